@@ -37,3 +37,68 @@ def test_samples_stay_in_kept_set_and_follow_distribution(top_k, top_p):
     tok3, _ = S.sample(z, temp, top_p, top_k, seed=11, step=4)
     assert not torch.equal(tok, tok3)
     assert tok.unique().numel() > 1                           # rows draw independently
+
+
+def _kept(z, temp, top_k, top_p):
+    """The filter in 64 bits: e = exp(z / temp - max) at least the largest multiple of 2^-26 that keeps top_k tokens, then the
+    largest that keeps a mass of top_p among them. Also where rounding in 32 bits may decide otherwise."""
+    e = torch.exp((z.double() / temp) - (z.double() / temp).max(-1, keepdim=True).values)
+    u = 2.0 ** -26
+    lo = torch.zeros(e.shape[0], 1, dtype=torch.float64, device=z.device)
+    if top_k:
+        lo = (e.topk(top_k, -1).values[:, -1:] / u).floor() * u
+    keep = e >= lo
+    if top_p:
+        s, _ = torch.where(keep, e, 0.0).sort(-1, descending=True)
+        need = (s.cumsum(-1) >= top_p * s.sum(-1, keepdim=True)).float().argmax(-1, keepdim=True)
+        lo = torch.maximum(lo, (s.gather(-1, need) / u).floor() * u)
+    return e >= lo * (1 - 1e-5) - 1e-7, e
+
+
+@pytest.mark.parametrize("shape", ["flat", "peaked", "ties", "forbidden"])
+@pytest.mark.parametrize("V", [3, 1023, 32771, 151936])
+@pytest.mark.parametrize("top_k,top_p", [(1, None), (50, 0.95), (None, 0.95), (None, 0.9999), (40000, 0.5)])
+def test_filtered_draws_for_any_split_of_the_row(shape, V, top_k, top_p):
+    """Rows are split over 8, 4, 2 or 1 thread blocks by the batch size; the draw of a row does not depend on it."""
+    from tunix_b200.ops import sampling_kernels as S
+    if top_k and top_k >= V:
+        top_k = 2
+    torch.manual_seed(V)
+    B, temp = 300, 0.9
+    z = torch.randn(B, V, device="cuda") * {"flat": 0.01, "peaked": 4.0}.get(shape, 1.5)
+    if shape == "ties":
+        z = (z * 2).round() / 2
+    forbidden = None
+    if shape == "forbidden":
+        forbidden = torch.arange(0, V - 1, 2, dtype=torch.int32, device="cuda")
+    ref = z.clone()
+    if forbidden is not None:
+        ref[:, forbidden.long()] = float("-inf")
+    kept, _ = _kept(ref, temp, top_k, top_p)
+    want = torch.log_softmax(ref.double() / temp, -1)
+    whole = None
+    for n in (300, 100, 60, 5, 1):
+        tok, lp = S.sample(z[:n].clone(), temp, top_p, top_k, seed=7, step=2, want_logprob=True, forbidden=forbidden)
+        whole = tok if whole is None else whole
+        assert torch.equal(tok, whole[:n])
+        assert kept[:n].gather(1, tok[:, None]).all()
+        # 32-bit exponentials (2 ulp) and sums of up to 151936 terms in blocks: a relative error of the sum below 1e-5
+        assert (lp - want[:n].gather(1, tok[:, None])[:, 0]).abs().max().item() < 1e-4
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_values_that_are_not_finite(value):
+    """An infinite logit is drawn, rows of nothing but -inf give token 0, and a NaN is never drawn."""
+    from tunix_b200.ops import sampling_kernels as S
+    z = torch.zeros(2, 9000, device="cuda")
+    z[0, 77] = value
+    if value == float("-inf"):
+        z[1] = value
+    for top_k, top_p in ((None, None), (30, 0.9), (None, 0.9)):
+        tok, _ = S.sample(z.clone(), 1.0, top_p, top_k, seed=1, step=1, want_logprob=True)
+        if value == float("inf"):
+            assert tok[0].item() == 77
+        else:
+            assert tok[0].item() != 77
+        if value == float("-inf"):
+            assert tok[1].item() == 0
