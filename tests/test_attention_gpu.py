@@ -137,3 +137,62 @@ def test_attention_backward(case):
     _close(dv, vf.grad, "dv")
     _close(dk, kf.grad, "dk")
     _close(dq, qf.grad, "dq")
+
+
+def _segments(layout, B, Tq, Tk):
+    g = torch.Generator().manual_seed(3)
+    if layout == "whole_blocks":                # boundaries on block edges: listed blocks hold one id
+        seg = (torch.arange(Tk) // 128).expand(B, Tk)
+    elif layout == "mixed":                     # ids in no order, negative ones among them: every block is compared
+        seg = torch.randint(-2, 3, (B, Tk), generator=g)
+    elif layout == "pads":                      # padding on both sides of a row, a row of padding alone
+        seg = torch.zeros(B, Tk, dtype=torch.long)
+        seg[0, 37:Tk - 70] = 1
+    else:                                       # "unseen": the ids of some queries occur in no key
+        seg = (torch.arange(Tk) // 100).expand(B, Tk)
+    seg_k = seg.to(torch.int32).contiguous().cuda()
+    seg_q = seg_k[:, Tk - Tq:].contiguous()
+    if layout == "unseen":
+        seg_q = torch.where(seg_q == 2, 1 << 20, seg_q).int().contiguous()
+    return seg_q, seg_k
+
+
+@pytest.mark.parametrize("H", [64, 128, 256])
+@pytest.mark.parametrize("window", [0, 150])
+@pytest.mark.parametrize("layout", ["whole_blocks", "mixed", "pads", "unseen"])
+def test_segment_blocks(layout, window, H):
+    """Key blocks that the segment ids leave out, let pass unseen, or have compared element by element."""
+    from tunix_b200 import _lib
+    from tunix_b200.ops import kernels as k_
+    B, Tq, Tk, N, KH = 2, 509, 573, 4, 2
+    q, k, v, _, _ = _make(B, Tq, Tk, N, KH, H, False)
+    seg_q, seg_k = _segments(layout, B, Tq, Tk)
+    do = torch.randn(B, Tq, N, H, device="cuda", dtype=torch.bfloat16)
+    qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
+    ref = ref_attention(qf, kf, vf, H ** -0.5, True, window, 0.0, seg_q, seg_k)
+    ref.backward(do.float())
+    kw = dict(scale=H ** -0.5, causal=True, window=window, seg_q=seg_q, seg_k=seg_k)
+    o, lse = k_.attn_fwd(q, k, v, **kw)
+    grads = k_.attn_bwd(do, q, k, v, o, lse, **kw)
+    _lib.raise_if_kernel_error()
+    # bf16 operands (2^-9 each) in sums of products: the bounds of the tests above
+    assert _rel(o, ref) < 2e-2
+    _close(o, ref, "o")
+    for name, got, want in zip(("dq", "dk", "dv"), grads, (qf.grad, kf.grad, vf.grad)):
+        assert _rel(got, want) < 3e-2, (name, _rel(got, want))
+        _close(got, want, name)
+
+
+def test_segments_past_the_block_list():
+    """More key blocks than the list of a tile holds."""
+    from tunix_b200 import _lib
+    from tunix_b200.ops import kernels as k_
+    Tq, Tk = 64, 64 * 2048 + 100
+    q, k, v, _, _ = _make(1, Tq, Tk, 1, 1, 64, False)
+    seg_k = (torch.arange(Tk, device="cuda") // 50000).int()[None].contiguous()
+    seg_q = torch.full((1, Tq), 1, dtype=torch.int32, device="cuda")
+    seg_q[0, 40:] = 2
+    o, _ = k_.attn_fwd(q, k, v, scale=0.125, causal=False, seg_q=seg_q, seg_k=seg_k)
+    _lib.raise_if_kernel_error()
+    ref = ref_attention(q, k, v, 0.125, False, 0, 0.0, seg_q, seg_k)
+    assert _rel(o, ref) < 2e-2

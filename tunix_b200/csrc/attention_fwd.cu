@@ -14,6 +14,13 @@
 // learned sinks and output gates per head, and queries and keys whose heads lie further apart than they are wide.
 // Every mbarrier wait is bounded; a timeout sets *status and the CTA unwinds.
 //
+// Bound by the softmax warps (64 exponentials a row and block share the special-function units with the other CTA of the SM).
+// Segment ids are compared per key block where they decide for the whole of it, and by warp votes elsewhere, not by one load a
+// score; K and V share a ring, so that no product waits for a load issued in its own block. B200, 32 / 8 heads of 128, causal,
+// before -> after: rollouts padded at both ends, 8 x 1024 519 -> 135 us, 16 x 1024 970 -> 245, 8 x 4096 6320 -> 939; packed rows
+// of 777, 14 / 2 heads of 64, 92 -> 31; without segments 2 x 2048 136 -> 116, 8 x 2048 452 -> 369, 1 x 16384 2228 -> 2206;
+// 4 x 1001 with heads of 256 and a soft-cap 265 -> 97.
+//
 // Replaces the eager [B,N,T,S] attention and the TPU-only splash attention of the reference
 // (tunix/models/llama3/model.py:379-396, tunix/models/qwen3/model.py:607-793,
 //  tunix/models/gemma/model.py:442-483).
@@ -58,6 +65,98 @@ struct AttnArgs {
   float out_scale;           // paged: factor of the output
 };
 
+// Segment ids (packed rows, padding) decide for most key blocks as a whole. A tile lists the blocks with any id between the
+// smallest and the largest of its rows, and marks those where all ids are the one that all its rows have; the others are never
+// loaded. Elements are compared in the rest only.
+constexpr int SEG_BLOCKS = 2048;            // blocks that the list can hold; longer ranges are walked without one
+constexpr uint16_t SEG_SAME = 0x8000, SEG_ID = 0x7fff;
+struct SegList {
+  uint16_t id[SEG_BLOCKS];
+  int lo[8], hi[8], n;
+};
+
+// All threads of the CTA: key blocks jb0 .. jb0 + nblk - 1 for the rows q0 .. q0 + nrows - 1 -> the number listed. Each half-warp
+// reads four consecutive ids a lane, four blocks in flight.
+__device__ __forceinline__ int build_seg_list(SegList& s, const AttnArgs& a, int b, int q0, int nrows, int jb0, int nblk) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  int lo = 0x7fffffff, hi = -0x7fffffff - 1;
+  for (int i = tid; i < min(nrows, BQ); i += blockDim.x) {
+    const int v = a.seg_q ? a.seg_q[(long long)b * a.Tq + q0 + i] : 0;
+    lo = min(lo, v);
+    hi = max(hi, v);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) {
+    s.lo[warp] = lo;
+    s.hi[warp] = hi;
+  }
+  __syncthreads();
+  for (int w = 0; w < nwarp; ++w) {
+    lo = min(lo, s.lo[w]);
+    hi = max(hi, s.hi[w]);
+  }
+  const int* seg = a.seg_k + (long long)b * a.Tk;
+  for (int j0 = warp * 8; j0 < nblk; j0 += nwarp * 8) {
+    int v[4][4];
+    bool in[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = j0 + 2 * u + (lane >> 4), k = (jb0 + j) * BKV + (lane & 15) * 4 + e;
+        in[u][e] = j < nblk && k < a.Tk;
+        v[u][e] = in[u][e] ? __ldg(seg + k) : 0;
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      bool any = false, same = lo == hi;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        any = any || (in[u][e] && v[u][e] >= lo && v[u][e] <= hi);
+        same = same && in[u][e] && v[u][e] == lo;
+      }
+      const uint32_t half = (lane & 16) ? 0xffff0000u : 0xffffu;
+      const uint32_t anys = __ballot_sync(0xffffffffu, any) & half, sames = __ballot_sync(0xffffffffu, same) & half;
+      const int j = j0 + 2 * u + (lane >> 4);
+      if ((lane & 15) == 0 && j < nblk) s.id[j] = anys ? (uint16_t)(j | (sames == half ? SEG_SAME : 0)) : (uint16_t)SEG_ID;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {                                  // in place: entry n is written after entries up to n have been read
+    int n = 0;
+    for (int j = lane; j - lane < nblk; j += 32) {
+      const uint16_t v = j < nblk ? s.id[j] : SEG_ID;
+      const uint32_t take = __ballot_sync(0xffffffffu, v != SEG_ID);
+      if (v != SEG_ID) s.id[n + __popc(take & ((1u << lane) - 1))] = v;
+      n += __popc(take);
+      __syncwarp();
+    }
+    if (lane == 0) s.n = n;
+  }
+  __syncthreads();
+  return s.n;
+}
+
+__device__ __forceinline__ uint32_t bits_below(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1; }
+
+// Clears the bits of the 64 keys from k0 whose id is not the row's: one vote per id among the rows of the warp.
+__device__ __forceinline__ void seg_bits(const int* seg, int k0, int Tk, int mine, uint32_t (&keep)[2]) {
+  const int lane = threadIdx.x & 31;
+  const int v0 = k0 + lane < Tk ? __ldg(seg + k0 + lane) : 0, v1 = k0 + 32 + lane < Tk ? __ldg(seg + k0 + 32 + lane) : 0;
+  uint32_t todo = ~0u;
+  while (todo) {
+    const int id = __shfl_sync(0xffffffffu, mine, __ffs(todo) - 1);
+    const uint32_t b0 = __ballot_sync(0xffffffffu, v0 == id), b1 = __ballot_sync(0xffffffffu, v1 == id);
+    const bool now = mine == id;
+    if (now) {
+      keep[0] &= b0;
+      keep[1] &= b1;
+    }
+    todo &= ~__ballot_sync(0xffffffffu, now);
+  }
+}
+
 // H: query / key head size, HV: value head size
 template <int H, int HV>
 struct FwdCfg {
@@ -67,13 +166,15 @@ struct FwdCfg {
   static constexpr int K_BYTES = HS * BKV * 128;    // slabs [64 x 128B]
   static constexpr int V_BYTES = HVS * BKV * 128;
   static constexpr int P_BYTES = BQ * 128;
-  // two V buffers, or one where that lets a second CTA share the SM
-  static constexpr int FIXED = Q_BYTES + K_BYTES + P_BYTES + 128 + 1024;
-  static constexpr int NV = FIXED + 2 * V_BYTES > 113 * 1024 && FIXED + V_BYTES <= 113 * 1024 ? 1 : 2;
+  // A ring of three tiles that K and V share, in the order in which they are read (K0 K1 V0 K2 V1 K3 ...): the load of a K runs
+  // a whole block ahead of its product. One buffer each where only that lets a second CTA share the SM.
+  static constexpr int SLOT = K_BYTES > V_BYTES ? K_BYTES : V_BYTES;
+  static constexpr int FIXED = Q_BYTES + P_BYTES + 128 + 1024;
+  static constexpr bool RING = FIXED + 3 * SLOT <= 113 * 1024 || FIXED + K_BYTES + V_BYTES > 113 * 1024;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_K = OFF_Q + Q_BYTES;
-  static constexpr int OFF_V = OFF_K + K_BYTES;
-  static constexpr int OFF_P = OFF_V + NV * V_BYTES;
+  static constexpr int OFF_V = OFF_K + K_BYTES;                       // not RING
+  static constexpr int OFF_P = OFF_K + (RING ? 3 * SLOT : K_BYTES + V_BYTES);
   static constexpr int OFF_BAR = OFF_P + P_BYTES;
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
   static constexpr int TMEM_S = 0;                  // two S buffers of 64 columns
@@ -87,14 +188,13 @@ __global__ void __launch_bounds__(160, FwdCfg<H, HV>::SMEM_BYTES <= 113 * 1024 ?
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmR, const AttnArgs a) {
   using C_ = FwdCfg<H, HV>;
-  constexpr int NV = C_::NV;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sptr = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t sQ = sbase + C_::OFF_Q, sK = sbase + C_::OFF_K, sV = sbase + C_::OFF_V,
                  sP = sbase + C_::OFF_P, bars = sbase + C_::OFF_BAR;
-  // barriers: 0 Q, 1 K, 2-3 V[2], 4-5 S[2], 6 P, 7 PV
-  const uint32_t barQ = bars, barK = bars + 8, barV0 = bars + 16, barS0 = bars + 32,
+  // barriers: 0 Q, 1-3 ring (or 1 K, 2 V), 4-5 S[2], 6 P, 7 PV
+  const uint32_t barQ = bars, barK = bars + 8, barV = bars + 16, barS0 = bars + 32,
                  barP = bars + 48, barPV = bars + 56;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sptr + C_::OFF_BAR + 64);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sptr + C_::OFF_BAR + 68);
@@ -128,8 +228,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (PAGED && a.chunk > 0) kv_start = max(kv_start, i0 - i0 % a.chunk);
   const int jb0 = kv_start / BKV;
   const int n_sink = PAGED ? min((min(a.keep, Tk) + BKV - 1) / BKV, jb0) : 0;
-  const int nblk = n_sink + (kv_end > jb0 * BKV ? (kv_end - jb0 * BKV + BKV - 1) / BKV : 0);
-  auto block_key = [&](int j) { return (j < n_sink ? j : jb0 + j - n_sink) * BKV; };      // first key of block j
+  int nblk = n_sink + (kv_end > jb0 * BKV ? (kv_end - jb0 * BKV + BKV - 1) / BKV : 0);
+  const SegList* list = nullptr;
+  if constexpr (!PAGED) {
+    __shared__ SegList s_list;
+    if (a.seg_k && nblk <= SEG_BLOCKS) {
+      list = &s_list;
+      nblk = build_seg_list(s_list, a, b, qt * BQ, nrows, jb0, nblk);
+    }
+  }
+  auto block_key = [&](int j) {                                                           // first key of block j
+    if (!PAGED && list) j = list->id[j] & SEG_ID;
+    return (j < n_sink ? j : jb0 + j - n_sink) * BKV;
+  };
   auto block_row = [&](int j) {                                                           // its row in the K / V maps
     const int k = block_key(j);
     return PAGED ? pages[k / a.page_size] * a.page_size + k % a.page_size : b * Tk + k;
@@ -137,9 +248,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   if (threadIdx.x == 0) {
     mbar_init(barQ, 1);
-    mbar_init(barK, 1);
-    mbar_init(barV0, 1);
-    mbar_init(barV0 + 8, 1);
+    for (int i = 0; i < 3; ++i) mbar_init(barK + 8 * i, 1);
     mbar_init(barS0, 1);
     mbar_init(barS0 + 8, 1);
     mbar_init(barP, 128);
@@ -161,41 +270,48 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (nblk > 0 && elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
       const uint32_t idesc_o = make_idesc_bf16(BQ, HV, 0, 1);
+      // RING: K_j is item 0 or 2j - 1 and V_j item 2j + 2 of the order above, item i in slot i % 3
+      auto slot_k = [](int j) { return C_::RING ? (j ? 2 * j - 1 : 0) : 3 * j; };
+      auto slot_v = [](int j) { return C_::RING ? 2 * j + 2 : 3 * j + 1; };
       auto load_k = [&](int j) {
-        mbar_expect_tx(barK, C_::K_BYTES);
+        const uint32_t bar = barK + 8 * (slot_k(j) % 3), dst = sK + slot_k(j) % 3 * C_::SLOT;
+        mbar_expect_tx(bar, C_::K_BYTES);
         const int row = block_row(j);
 #pragma unroll
         for (int c = 0; c < C_::HS; ++c) {
-          if (!PAGED) tma_load_2d(sK + c * (BKV * 128), &tmK, barK, kvh * H + 64 * c, row);
-          else if (c < a.k_own) tma_load_2d(sK + c * (BKV * 128), &tmK, barK, (kvh * a.k_own + c) * 64, row);
-          else tma_load_2d(sK + c * (BKV * 128), &tmR, barK, a.k_col + (c - a.k_own) * 64, row);
+          if (!PAGED) tma_load_2d(dst + c * (BKV * 128), &tmK, bar, kvh * H + 64 * c, row);
+          else if (c < a.k_own) tma_load_2d(dst + c * (BKV * 128), &tmK, bar, (kvh * a.k_own + c) * 64, row);
+          else tma_load_2d(dst + c * (BKV * 128), &tmR, bar, a.k_col + (c - a.k_own) * 64, row);
         }
       };
+      auto v_tile = [&](int j) { return C_::RING ? sK + slot_v(j) % 3 * C_::SLOT : sV; };
       auto load_v = [&](int j) {
-        const int buf = j % NV;
-        const uint32_t bar = barV0 + 8 * buf;
+        const uint32_t bar = barK + 8 * (slot_v(j) % 3);
         mbar_expect_tx(bar, C_::V_BYTES);
         const int row = block_row(j);
 #pragma unroll
         for (int c = 0; c < C_::HVS; ++c)
-          tma_load_2d(sV + buf * C_::V_BYTES + c * (BKV * 128), &tmV, bar, kvh * HV + 64 * c, row);
+          tma_load_2d(v_tile(j) + c * (BKV * 128), &tmV, bar, kvh * HV + 64 * c, row);
       };
       auto issue_s = [&](int j) {
-        const uint32_t d = tmem + C_::TMEM_S + (j & 1) * BKV;
+        const uint32_t d = tmem + C_::TMEM_S + (j & 1) * BKV, kt = sK + slot_k(j) % 3 * C_::SLOT;
 #pragma unroll
         for (int kk = 0; kk < H / 16; ++kk) {
           const uint64_t ad = make_smem_desc(sQ + (kk >> 2) * (BQ * 128) + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc(sK + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024);
+          const uint64_t bd = make_smem_desc(kt + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024);
           umma_f16_ss(d, ad, bd, idesc_s, kk != 0);
         }
         umma_commit(barS0 + 8 * (j & 1));
       };
+#define FWD_WAIT(bar, par, code) \
+  if (!mbar_wait_bounded((bar), (par), abort_flag, a.status, (code))) { ok = false; break; }
       bool ok = true;
       mbar_expect_tx(barQ, C_::Q_BYTES);
 #pragma unroll
       for (int c = 0; c < C_::HS; ++c)
         tma_load_2d(sQ + c * (BQ * 128), &tmQ, barQ, n * (PAGED ? a.q_heads : H) + 64 * c, row0);
       load_k(0);
+      if (C_::RING && nblk > 1) load_k(1);
       load_v(0);
       ok = ok && mbar_wait_bounded(barQ, 0, abort_flag, a.status, ST_TIMEOUT_PRODUCER);
       ok = ok && mbar_wait_bounded(barK, 0, abort_flag, a.status, ST_TIMEOUT_PRODUCER);
@@ -204,28 +320,39 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         issue_s(0);
       }
       for (int j = 0; j < nblk && ok; ++j) {
-        if (j + 1 < nblk) {
-          // S_j retired -> the K buffer is free again
-          if (!mbar_wait_bounded(barS0 + 8 * (j & 1), (j >> 1) & 1, abort_flag, a.status, ST_TIMEOUT_MMA)) { ok = false; break; }
-          load_k(j + 1);
-          if (!mbar_wait_bounded(barK, (j + 1) & 1, abort_flag, a.status, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
-          tc_fence_after();
-          issue_s(j + 1);
-          // V buffer (j+1)&1 was last read by PV_{j-1}
-          if (NV == 2) {
-            if (j >= 1 && !mbar_wait_bounded(barPV, (j - 1) & 1, abort_flag, a.status, ST_TIMEOUT_MMA)) { ok = false; break; }
+        if (C_::RING) {
+          if (j + 1 < nblk) {
+            FWD_WAIT(barK + 8 * (slot_k(j + 1) % 3), (slot_k(j + 1) / 3) & 1, ST_TIMEOUT_PRODUCER);
+            tc_fence_after();
+            issue_s(j + 1);
+          }
+          if (j + 2 < nblk) {                   // K_{j+2} takes the slot of V_{j-1}, or of K_0
+            if (j >= 1) { FWD_WAIT(barPV, (j - 1) & 1, ST_TIMEOUT_MMA); }
+            else { FWD_WAIT(barS0, 0, ST_TIMEOUT_MMA); }
+            load_k(j + 2);
+          }
+          if (j + 1 < nblk) {                   // V_{j+1} takes that of K_{j+1}
+            FWD_WAIT(barS0 + 8 * ((j + 1) & 1), ((j + 1) >> 1) & 1, ST_TIMEOUT_MMA);
             load_v(j + 1);
           }
+        } else {
+          if (j + 1 < nblk) {
+            // S_j retired -> the K buffer is free again
+            FWD_WAIT(barS0 + 8 * (j & 1), (j >> 1) & 1, ST_TIMEOUT_MMA);
+            load_k(j + 1);
+            FWD_WAIT(barK, (j + 1) & 1, ST_TIMEOUT_PRODUCER);
+            tc_fence_after();
+            issue_s(j + 1);
+          }
+          if (j >= 1) {                         // the only V buffer was last read by PV_{j-1}
+            FWD_WAIT(barPV, (j - 1) & 1, ST_TIMEOUT_MMA);
+            load_v(j);
+          }
         }
-        // the only V buffer was last read by PV_{j-1}
-        if (NV == 1 && j >= 1) {
-          if (!mbar_wait_bounded(barPV, (j - 1) & 1, abort_flag, a.status, ST_TIMEOUT_MMA)) { ok = false; break; }
-          load_v(j);
-        }
-        if (!mbar_wait_bounded(barP, j & 1, abort_flag, a.status, ST_TIMEOUT_MMA)) { ok = false; break; }
-        if (!mbar_wait_bounded(barV0 + 8 * (j % NV), (j / NV) & 1, abort_flag, a.status, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
+        FWD_WAIT(barP, j & 1, ST_TIMEOUT_MMA);
+        FWD_WAIT(C_::RING ? barK + 8 * (slot_v(j) % 3) : barV, (slot_v(j) / 3) & 1, ST_TIMEOUT_PRODUCER);
         tc_fence_after();
-        const uint32_t vb = sV + (j % NV) * C_::V_BYTES;
+        const uint32_t vb = v_tile(j);
 #pragma unroll
         for (int kk = 0; kk < BKV / 16; ++kk) {
           const uint64_t ad = make_smem_desc(sP + kk * 32, 16, 1024);
@@ -234,6 +361,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         umma_commit(barPV);
       }
+#undef FWD_WAIT
     }
   } else {
     // ---------------------------------------------------------- softmax warps
@@ -250,6 +378,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float m_used = 0.f, l = 0.f;
     bool ok = true;
     for (int j = 0; j < nblk && ok; ++j) {
+      const int k0 = block_key(j);
+      // most key blocks of a causal tile lie fully below the diagonal: skip the per-element mask there
+      bool by_seg = !PAGED && a.seg_k && !(list && (list->id[j] & SEG_SAME));
+      const bool need_mask = (k0 + BKV > Tk) || by_seg || (a.causal && (k0 + BKV - 1 > i0)) ||
+                             (a.window > 0 && (k0 <= i0 + BQ - 1 - a.window)) ||
+                             (PAGED && a.chunk > 0 && k0 < i0 + nrows - 1 - (i0 + nrows - 1) % a.chunk);
+      // the keys of the block that this row sees, one bit each
+      uint32_t keep[2] = {~0u, ~0u};
+      if (!PAGED && need_mask) {
+        int hi = Tk - k0;
+        if (a.causal) hi = min(hi, qpos + 1 - k0);
+        const int lo = a.window > 0 ? qpos - a.window + 1 - k0 : 0;
+        keep[0] = bits_below(hi) & ~bits_below(lo);
+        keep[1] = bits_below(hi - 32) & ~bits_below(lo - 32);
+        if (by_seg) seg_bits(a.seg_k + (long long)b * a.Tk, k0, a.Tk, my_seg, keep);
+      }
       if (!mbar_wait_bounded(barS0 + 8 * (j & 1), (j >> 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
       uint32_t sraw[64];
@@ -261,61 +405,46 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int i = 0; i < 32; ++i) { sraw[i] = t0[i]; sraw[32 + i] = t1[i]; }
       }
-      const int k0 = block_key(j);
       float z[64];
-      float mx = -INFINITY;
-      const int* segk = a.seg_k ? a.seg_k + (long long)b * a.Tk + k0 : nullptr;
-      // most key blocks of a causal tile lie fully below the diagonal: skip the per-element mask there
-      const bool need_mask = (k0 + BKV > Tk) || (segk != nullptr) || (a.causal && (k0 + BKV - 1 > i0)) ||
-                             (a.window > 0 && (k0 <= i0 + BQ - 1 - a.window)) ||
-                             (PAGED && a.chunk > 0 && k0 < i0 + nrows - 1 - (i0 + nrows - 1) % a.chunk);
-      if (PAGED) {
-        if (a.softcap > 0.f) {
+      // z holds scores in log2 units, or raw ones whose scale is left to the exponent's multiply-add (scale > 0: a maximum
+      // stays a maximum)
+      const bool raw = a.scale > 0.f && a.softcap <= 0.f && !(PAGED && bias);
+      if (a.softcap > 0.f) {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) z[i] = cap_score(__uint_as_float(sraw[i]) * a.scale, a.softcap, inv_cap) * LOG2E;
-          if (bias) {
+        for (int i = 0; i < 64; ++i) z[i] = cap_score(__uint_as_float(sraw[i]) * a.scale, a.softcap, inv_cap) * LOG2E;
+        if (PAGED && bias) {
 #pragma unroll
-            for (int i = 0; i < 64; ++i) z[i] += __ldg(bias + min(max(qpos - k0 - i, 0), a.far)) * LOG2E;
-          }
-        } else if (bias) {
-#pragma unroll
-          for (int i = 0; i < 64; ++i)
-            z[i] = fmaf(__uint_as_float(sraw[i]), sc2, __ldg(bias + min(max(qpos - k0 - i, 0), a.far)) * LOG2E);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 64; ++i) z[i] = __uint_as_float(sraw[i]) * sc2;
+          for (int i = 0; i < 64; ++i) z[i] += __ldg(bias + min(max(qpos - k0 - i, 0), a.far)) * LOG2E;
         }
-        if (need_mask) {
+      } else if (PAGED && bias) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          z[i] = fmaf(__uint_as_float(sraw[i]), sc2, __ldg(bias + min(max(qpos - k0 - i, 0), a.far)) * LOG2E);
+      } else {
+        const float f = raw ? 1.f : sc2;
+#pragma unroll
+        for (int i = 0; i < 64; ++i) z[i] = __uint_as_float(sraw[i]) * f;
+      }
+      if (need_mask) {
+        if (PAGED) {
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
             const int kp = k0 + i;
             if (kp > qpos || (((a.window > 0 && kp <= qpos - a.window) || kp < chunk0) && kp >= a.keep)) z[i] = -INFINITY;
           }
-        }
+        } else {
 #pragma unroll
-        for (int i = 0; i < 64; ++i) mx = fmaxf(mx, z[i]);
-      } else if (!need_mask && a.softcap <= 0.f) {
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          z[i] = __uint_as_float(sraw[i]) * sc2;
-          mx = fmaxf(mx, z[i]);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          const int kp = k0 + i;
-          float s = __uint_as_float(sraw[i]);
-          if (a.softcap > 0.f) s = cap_score(s * a.scale, a.softcap, inv_cap) * LOG2E;
-          else s *= sc2;
-          bool keep = kp < a.Tk;
-          if (a.causal) keep = keep && (kp <= qpos);
-          if (a.window > 0) keep = keep && (kp > qpos - a.window);
-          if (segk) keep = keep && (kp < a.Tk) && (__ldg(segk + (kp < a.Tk ? i : 0)) == my_seg);
-          s = keep ? s : -INFINITY;
-          z[i] = s;
-          mx = fmaxf(mx, s);
+          for (int i = 0; i < 64; ++i)
+            if (!(keep[i >> 5] >> (i & 31) & 1)) z[i] = -INFINITY;
         }
       }
+      float mq[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};        // four chains instead of one of 64
+#pragma unroll
+      for (int i = 0; i < 64; i += 8)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mq[c] = fmaxf(fmaxf(mq[c], z[i + c]), z[i + 4 + c]);
+      const float mul = raw ? sc2 : 1.f;
+      const float mx = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3])) * mul;
       float alpha = 1.f;
       bool need = false;
       if (mx != -INFINITY) {
@@ -328,16 +457,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
       const bool warp_need = __any_sync(0xffffffffu, need);
-      float psum = 0.f;
+      float ps[4] = {0.f, 0.f, 0.f, 0.f};
       uint32_t pk[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        const float p0 = exp2f(z[2 * i] - m_used);
-        const float p1 = exp2f(z[2 * i + 1] - m_used);
-        psum += p0 + p1;
+        const float p0 = exp2f(fmaf(z[2 * i], mul, -m_used));
+        const float p1 = exp2f(fmaf(z[2 * i + 1], mul, -m_used));
+        ps[i & 3] += p0 + p1;
         pk[i] = pack_bf16(p0, p1);
       }
-      l = l * alpha + psum;
+      l = l * alpha + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
       if (j > 0) {
         // PV_{j-1} retired: P buffer reusable and O consistent
         if (!mbar_wait_bounded(barPV, (j - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
