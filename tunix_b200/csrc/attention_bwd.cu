@@ -17,8 +17,7 @@
 //
 // Counterpart in the reference: autodiff of the attention in tunix/models/*/model.py
 // (e.g. tunix/models/llama3/model.py:379-396); no hand-written backward exists there.
-#include "common.cuh"
-#include <cstdlib>
+#include "segments.cuh"
 
 using namespace tb;
 
@@ -26,6 +25,7 @@ namespace {
 
 constexpr int BK_ = 128;  // keys per CTA
 constexpr int BQ_ = 64;   // queries per iteration
+constexpr int RG_ = 2;    // row-thread groups
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct BwdArgs {
@@ -45,12 +45,13 @@ struct BwdArgs {
 
 template <int H>
 struct BwdCfg {
-  static constexpr bool PIPE = (H <= 128);          // software-pipelined schedule (needs double buffers)
+  static constexpr bool PIPE = (H <= 128);          // software-pipelined schedule (needs room for more than one query tile)
   static constexpr int HS = H / 64;
   static constexpr int HO = H < 128 ? H : 128;
   static constexpr int NHALF = H / HO;
   static constexpr int NST = PIPE ? 3 : 1;          // Q / dO tile stages
-  static constexpr int NPB = PIPE ? 2 : 1;          // Pt / dSt staging buffers
+  static constexpr int NDS = PIPE ? 2 : 1;          // dSt staging buffers
+  static constexpr int SEG_BLOCKS = PIPE ? 2048 : 64;       // query tiles that the list can hold (what shared memory leaves)
   static constexpr int KV_BYTES = HS * BK_ * 128;
   static constexpr int Q_BYTES = HS * BQ_ * 128;
   static constexpr int P_BYTES = BK_ * 128;
@@ -59,27 +60,33 @@ struct BwdCfg {
   static constexpr int OFF_Q = OFF_V + KV_BYTES;
   static constexpr int OFF_DO = OFF_Q + NST * Q_BYTES;
   static constexpr int OFF_PT = OFF_DO + NST * Q_BYTES;
-  static constexpr int OFF_DST = OFF_PT + NPB * P_BYTES;
-  static constexpr int OFF_STAT = OFF_DST + NPB * P_BYTES;   // [2][3][64] 4-byte values
-  static constexpr int OFF_BAR = OFF_STAT + 2 * 3 * 64 * 4;
+  static constexpr int OFF_DST = OFF_PT + P_BYTES;
+  static constexpr int OFF_STAT = OFF_DST + NDS * P_BYTES;   // [3][2][64] lse and delta of three query tiles
+  static constexpr int OFF_BAR = OFF_STAT + 3 * 2 * 64 * 4;
   static constexpr int SMEM_BYTES = OFF_BAR + 192 + 1024;
-  // TMEM columns. PIPE: St/dQt buffers at 0 and 64, dPt buffers at 128 and 192, dV at 256, dK after it.
-  // Otherwise: St 0, dPt 64, dQt 128, dV 192, dK after it.
-  static constexpr int TM_DV = PIPE ? 256 : 192;
+  // TMEM columns: St (two buffers if PIPE), dPt, dQt, dV, dK
+  static constexpr int TM_DPT = PIPE ? 128 : 64;
+  static constexpr int TM_DQT = TM_DPT + 64;
+  static constexpr int TM_DV = TM_DQT + 64;
   static constexpr int TM_DK = TM_DV + HO;
   static constexpr int TMEM_COLS = 512;
-  __host__ __device__ static constexpr int tm_st(int buf) { return PIPE ? buf * 64 : 0; }
-  __host__ __device__ static constexpr int tm_dpt(int buf) { return PIPE ? 128 + buf * 64 : 64; }
-  __host__ __device__ static constexpr int tm_dqt(int buf) { return PIPE ? buf * 64 : 128; }
+  __host__ __device__ static constexpr int tm_st(int it) { return PIPE ? (it & 1) * 64 : 0; }
 };
 
-// Schedule (PIPE): while the row threads work on query tile `it` (P, then dS), the tensor core already
-// holds St/dPt of tile it+1 (issued at mid-iteration) and finishes dV/dK/dQt of tile it-1; the dQt of
-// tile it-1 is drained between the two phases of tile it. Handoffs never wait on a just-issued MMA.
-// RG_: row-thread groups. The BQ_ query columns of a key row are split over RG_ threads (one per warpgroup), so the
-// element-wise work between the MMAs runs on 128 * RG_ threads.
-template <int H, int RG_>
-__global__ void __launch_bounds__(128 * RG_ + 32, 1)   // 9 warps are allocated as 12: 168 registers per thread
+// Bound by the chain S -> P -> dS -> dK / dQ of one CTA an SM (512 TMEM columns, 208 KB), of which the products are 1280 cycles
+// a tile at the tensor cores' rate. B200, 32 / 8 heads of 128, causal, the whole backward (with delta and the fp32 dQ passes),
+// before -> after these roles, this schedule and the order of the grid: 2 x 2048 546 -> 297 us, 8 x 2048 1546 -> 1214,
+// 1 x 16384 8569 -> 6845; rollouts padded at both ends 8 x 1024 864 -> 406; packed rows 3 x 777 with 14 / 2 heads of 64 375 -> 112;
+// 4 x 1001, 16 / 8 heads of 256, soft-cap 610 -> 378.
+//
+// Roles: row threads (P and dS), four warps that add dQt to dQ and fetch lse / delta of later tiles, one issuer.
+// Schedule (PIPE): St runs two query tiles ahead and dPt of the next tile is the first product behind dSt, so the row threads go
+// from dS of one tile to P of the next without a wait; dK, dQt and the next St follow while they work. dQt leaves through its own
+// warps, off the row threads' path.
+// The BQ_ query columns of a key row are split over RG_ threads (one per warpgroup), so the element-wise work between the MMAs
+// runs on 128 * RG_ threads.
+template <int H>
+__global__ void __launch_bounds__(128 * RG_ + 160, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const BwdArgs a) {
@@ -95,20 +102,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t sK = sbase + C_::OFF_K, sV = sbase + C_::OFF_V, sQ = sbase + C_::OFF_Q,
                  sdO = sbase + C_::OFF_DO, sPt = sbase + C_::OFF_PT, sdSt = sbase + C_::OFF_DST,
                  bars = sbase + C_::OFF_BAR;
-  // barriers (8 bytes each): 0 KV | 1-3 Q[3] | 4-6 Qfree[3] | 7-8 St[2] | 9-10 dPt[2] | 11 Pt | 12 dSt |
-  //                          13 dQ | 14 dQ drained | 15 row-thread sync ; then tmem slot + abort flag
-  const uint32_t barKV = bars, barQ0 = bars + 8, barQF0 = bars + 32, barSt0 = bars + 56, bardPt0 = bars + 72,
-                 barPt = bars + 88, bardSt = bars + 96, bardQ = bars + 104, barDQfree = bars + 112,
-                 barSync = bars + 120;
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sptr + C_::OFF_BAR + 128);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(sptr + C_::OFF_BAR + 132);
+  // barriers (8 bytes each): 0 KV | 1-3 Q[3] | 4-6 Qfree[3] | 7-8 St[2] | 9 dPt | 10 Pt | 11 dSt | 12 dQ | 13 dQ drained |
+  //                          14 dV | 15-17 stats[3] ; tmem slot + abort flag ; 20 everything retired
+  const uint32_t barKV = bars, barQ0 = bars + 8, barQF0 = bars + 32, barSt0 = bars + 56, bardPt = bars + 72,
+                 barPt = bars + 80, bardSt = bars + 88, bardQ = bars + 96, barDQfree = bars + 104, bardV = bars + 112,
+                 barStat0 = bars + 120, barDone = bars + 160;
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sptr + C_::OFF_BAR + 144);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(sptr + C_::OFF_BAR + 148);
   float* s_stat = reinterpret_cast<float*>(sptr + C_::OFF_STAT);
 
   const int warp = threadIdx.x >> 5;
-  const int kt = blockIdx.x;
-  const int half = (C_::NHALF > 1) ? (blockIdx.y % C_::NHALF) : 0;
-  const int kvh = blockIdx.y / C_::NHALF;
-  const int b = blockIdx.z;
+  const int kt = blockIdx.z;               // heavy (early) causal tiles of all heads and rows first: a last wave of light ones
+  const int half = (C_::NHALF > 1) ? (blockIdx.x % C_::NHALF) : 0;
+  const int kvh = blockIdx.x / C_::NHALF;
+  const int b = blockIdx.y;
   const int G = a.N / a.KH;
   const int k0 = kt * BK_;
 
@@ -117,28 +124,56 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (a.causal) q_lo = max(0, k0 - a.q_off);
   if (a.window > 0) q_hi = min(a.Tq, k0 + BK_ + a.window - 1 - a.q_off);
   const int qt0 = q_lo / BQ_;
-  const int nq = q_hi > qt0 * BQ_ ? (q_hi - qt0 * BQ_ + BQ_ - 1) / BQ_ : 0;
+  int nq = q_hi > qt0 * BQ_ ? (q_hi - qt0 * BQ_ + BQ_ - 1) / BQ_ : 0;
+  __shared__ SegList<C_::SEG_BLOCKS> s_list;
+  const bool listed = a.seg_k && a.seg_q && nq <= C_::SEG_BLOCKS;
+  if (listed)
+    nq = build_seg_list(s_list, a.seg_k + (long long)b * a.Tk + k0, min(BK_, a.Tk - k0), a.seg_q + (long long)b * a.Tq, a.Tq, qt0, nq);
   const int nit = nq * G;
+  // walks the query tiles of a head, head after head
+  struct Walk {
+    int n, i, base;
+    bool same;                             // the ids of keys and queries are all one
+  };
+  auto tile_at = [&](Walk& w) {
+    const int e = listed ? s_list.id[w.i] : w.i;
+    w.base = (qt0 + (e & SEG_ID)) * BQ_;
+    w.same = listed && (e & SEG_SAME);
+  };
+  auto first_tile = [&] {
+    Walk w{kvh * G, 0, 0, false};
+    if (nit > 0) tile_at(w);
+    return w;
+  };
+  auto next_tile = [&](Walk& w) {
+    if (++w.i == nq) {
+      w.i = 0;
+      ++w.n;
+    }
+    tile_at(w);
+  };
 
   if (threadIdx.x == 0) {
     mbar_init(barKV, 1);
     for (int s = 0; s < 3; ++s) {
       mbar_init(barQ0 + 8 * s, 1);
       mbar_init(barQF0 + 8 * s, 1);
+      mbar_init(barStat0 + 8 * s, 64);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(barSt0 + 8 * s, 1);
-      mbar_init(bardPt0 + 8 * s, 1);
     }
+    mbar_init(bardPt, 1);
+    mbar_init(bardV, 1);
+    mbar_init(barDone, 1);
     mbar_init(barPt, NROW_);
     mbar_init(bardSt, NROW_);
     mbar_init(bardQ, 1);
-    mbar_init(barDQfree, NROW_);
-    mbar_init(barSync, NROW_);
+    mbar_init(barDQfree, 128);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 4 * RG_) {
+  if (warp == 4 * RG_ + 4) {
     tmem_alloc(smem_u32((const void*)tmem_slot), C_::TMEM_COLS);
     tmem_relinquish();
   }
@@ -146,11 +181,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  // TMEM buffer / barrier index and parity of the per-tile St and dPt results
-  auto sbuf = [&](int it) { return PIPE ? (it & 1) : 0; };
-  auto spar = [&](int it) { return PIPE ? ((it >> 1) & 1) : (it & 1); };
-
-  if (warp == 4 * RG_) {
+  if (warp == 4 * RG_ + 4) {
     // ------------------------------------------------------------ issuer warp
     if (nit > 0 && elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(128, BQ_, 0, 0);     // K-major x K-major, N = 64
@@ -158,50 +189,52 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t idesc_dq = make_idesc_bf16(128, BQ_, 1, 1);    // both MN-major, N = 64
       const uint32_t col_off = half * (HO / 64) * (BQ_ * 128);      // slab offset of this half in Q/dO tiles
       const uint32_t k_half = sK + half * (HO / 64) * (BK_ * 128);
+      Walk wl = first_tile();              // of the next load
       auto load_q = [&](int it) {
         const int st = it % NST;
-        const int g = it / nq, qt = qt0 + it % nq;
-        const int n = kvh * G + g;
         const uint32_t bar = barQ0 + 8 * st;
         mbar_expect_tx(bar, 2 * C_::Q_BYTES);
 #pragma unroll
         for (int c = 0; c < C_::HS; ++c) {
-          tma_load_2d(sQ + st * C_::Q_BYTES + c * (BQ_ * 128), &tmQ, bar, n * H + 64 * c, b * a.Tq + qt * BQ_);
-          tma_load_2d(sdO + st * C_::Q_BYTES + c * (BQ_ * 128), &tmdO, bar, n * H + 64 * c, b * a.Tq + qt * BQ_);
+          tma_load_2d(sQ + st * C_::Q_BYTES + c * (BQ_ * 128), &tmQ, bar, wl.n * H + 64 * c, b * a.Tq + wl.base);
+          tma_load_2d(sdO + st * C_::Q_BYTES + c * (BQ_ * 128), &tmdO, bar, wl.n * H + 64 * c, b * a.Tq + wl.base);
         }
+        if (it + 1 < nit) next_tile(wl);
       };
       // St = K Q^T ; dPt = V dO^T  (contraction over the full head dim)
-      auto issue_s_dp = [&](int it) {
-        const int st = it % NST;
-        const uint32_t q_s = sQ + st * C_::Q_BYTES, do_s = sdO + st * C_::Q_BYTES;
+      auto issue_s = [&](int it) {
+        const uint32_t q_s = sQ + (it % NST) * C_::Q_BYTES;
 #pragma unroll
         for (int kk = 0; kk < H / 16; ++kk) {
           const uint64_t ad = make_smem_desc(sK + (kk >> 2) * (BK_ * 128) + (kk & 3) * 32, 16, 1024);
           const uint64_t bd = make_smem_desc(q_s + (kk >> 2) * (BQ_ * 128) + (kk & 3) * 32, 16, 1024);
-          umma_f16_ss(tmem + C_::tm_st(sbuf(it)), ad, bd, idesc_s, kk != 0);
+          umma_f16_ss(tmem + C_::tm_st(it), ad, bd, idesc_s, kk != 0);
         }
-        umma_commit(barSt0 + 8 * sbuf(it));
+        umma_commit(barSt0 + (PIPE ? 8 * (it & 1) : 0));
+      };
+      auto issue_dp = [&](int it) {
+        const uint32_t do_s = sdO + (it % NST) * C_::Q_BYTES;
 #pragma unroll
         for (int kk = 0; kk < H / 16; ++kk) {
           const uint64_t ad = make_smem_desc(sV + (kk >> 2) * (BK_ * 128) + (kk & 3) * 32, 16, 1024);
           const uint64_t bd = make_smem_desc(do_s + (kk >> 2) * (BQ_ * 128) + (kk & 3) * 32, 16, 1024);
-          umma_f16_ss(tmem + C_::tm_dpt(sbuf(it)), ad, bd, idesc_s, kk != 0);
+          umma_f16_ss(tmem + C_::TM_DPT, ad, bd, idesc_s, kk != 0);
         }
-        umma_commit(bardPt0 + 8 * sbuf(it));
+        umma_commit(bardPt);
       };
       // dV += Pt dO   (A = Pt K-major over 64 queries, B = dO MN-major, this CTA's column half)
       auto issue_dv = [&](int it) {
         const uint32_t do_s = sdO + (it % NST) * C_::Q_BYTES;
-        const uint32_t pt = sPt + (PIPE ? (it & 1) : 0) * C_::P_BYTES;
 #pragma unroll
         for (int kk = 0; kk < BQ_ / 16; ++kk) {
-          const uint64_t ad = make_smem_desc(pt + kk * 32, 16, 1024);
+          const uint64_t ad = make_smem_desc(sPt + kk * 32, 16, 1024);
           const uint64_t bd = make_smem_desc(do_s + col_off + kk * 2048, BQ_ * 128, 1024);
           umma_f16_ss(tmem + C_::TM_DV, ad, bd, idesc_dv, (it | kk) != 0);
         }
+        umma_commit(bardV);
       };
-      // dK += dSt Q ; dQt = K^T dS^T
-      auto issue_dk_dq = [&](int it) {
+      // dK += dSt Q
+      auto issue_dk = [&](int it) {
         const uint32_t q_s = sQ + (it % NST) * C_::Q_BYTES;
         const uint32_t ds = sdSt + (PIPE ? (it & 1) : 0) * C_::P_BYTES;
 #pragma unroll
@@ -210,12 +243,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const uint64_t bd = make_smem_desc(q_s + col_off + kk * 2048, BQ_ * 128, 1024);
           umma_f16_ss(tmem + C_::TM_DK, ad, bd, idesc_dv, (it | kk) != 0);
         }
+      };
+      // dQt = K^T dS^T
+      auto issue_dq = [&](int it) {
+        const uint32_t ds = sdSt + (PIPE ? (it & 1) : 0) * C_::P_BYTES;
 #pragma unroll
         for (int kk = 0; kk < BK_ / 16; ++kk) {
           // A = K^T: M (head dim) contiguous, 64-wide M chunks BK_*128 bytes apart; 16 keys per step
           const uint64_t ad = make_smem_desc(k_half + kk * 2048, BK_ * 128, 1024);
           const uint64_t bd = make_smem_desc(ds + kk * 2048, BK_ * 128, 1024);
-          umma_f16_ss(tmem + C_::tm_dqt(sbuf(it)), ad, bd, idesc_dq, kk != 0);
+          umma_f16_ss(tmem + C_::TM_DQT, ad, bd, idesc_dq, kk != 0);
         }
         umma_commit(barQF0 + 8 * (it % NST));
         umma_commit(bardQ);
@@ -235,27 +272,38 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         ok = ok && mbar_wait_bounded(barQ0, 0, abort_flag, a.status, ST_TIMEOUT_PRODUCER);
         if (ok) {
           tc_fence_after();
-          issue_s_dp(0);
+          issue_s(0);
+          issue_dp(0);
+        }
+        if (nit > 1 && ok) {
+          ok = mbar_wait_bounded(barQ0 + 8, 0, abort_flag, a.status, ST_TIMEOUT_PRODUCER);
+          if (ok) {
+            tc_fence_after();
+            issue_s(1);
+          }
         }
         for (int it = 0; it < nit && ok; ++it) {
           BWD_WAIT(barPt, it & 1, ST_TIMEOUT_MMA);
           tc_fence_after();
           issue_dv(it);
-          if (it + 1 < nit) {
-            BWD_WAIT(barQ0 + 8 * ((it + 1) % NST), ((it + 1) / NST) & 1, ST_TIMEOUT_PRODUCER);
-            // St_{it+1} overwrites the TMEM buffer that held dQt_{it-1}: wait until it was drained
-            if (it >= 1) BWD_WAIT(barDQfree, (it - 1) & 1, ST_TIMEOUT_MMA);
-            tc_fence_after();
-            issue_s_dp(it + 1);
-          }
           if (it >= 1 && it + 2 < nit) {
             // the stage of tile it-1 is free once its dK / dQt retired
             BWD_WAIT(barQF0 + 8 * ((it - 1) % NST), ((it - 1) / NST) & 1, ST_TIMEOUT_MMA);
             load_q(it + 2);
           }
+          // dS of this tile is stored: its dPt has been read
           BWD_WAIT(bardSt, it & 1, ST_TIMEOUT_MMA);
           tc_fence_after();
-          issue_dk_dq(it);
+          if (it + 1 < nit) issue_dp(it + 1);
+          issue_dk(it);
+          if (it >= 1) BWD_WAIT(barDQfree, (it - 1) & 1, ST_TIMEOUT_MMA);
+          tc_fence_after();
+          issue_dq(it);
+          if (it + 2 < nit) {
+            BWD_WAIT(barQ0 + 8 * ((it + 2) % NST), ((it + 2) / NST) & 1, ST_TIMEOUT_PRODUCER);
+            tc_fence_after();
+            issue_s(it + 2);
+          }
         }
       } else {
         for (int it = 0; it < nit && ok; ++it) {
@@ -265,15 +313,75 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
           BWD_WAIT(barQ0, it & 1, ST_TIMEOUT_PRODUCER);
           tc_fence_after();
-          issue_s_dp(it);
+          issue_s(it);
+          issue_dp(it);
           BWD_WAIT(barPt, it & 1, ST_TIMEOUT_MMA);
           tc_fence_after();
           issue_dv(it);
           BWD_WAIT(bardSt, it & 1, ST_TIMEOUT_MMA);
           tc_fence_after();
-          issue_dk_dq(it);
+          issue_dk(it);
+          if (it >= 1) BWD_WAIT(barDQfree, (it - 1) & 1, ST_TIMEOUT_MMA);
+          tc_fence_after();
+          issue_dq(it);
         }
       }
+      if (ok) umma_commit(barDone);
+    }
+  } else if (warp >= 4 * RG_) {
+    // ------------------------------------------- dQ and the row statistics
+    const int r = threadIdx.x - NROW_;     // lane = head-dim index (within this CTA's half); column = query
+    const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+    const long long ld = (long long)a.N * H;
+    Walk w = first_tile(), ws = w;         // of the tile that is drained, and of the next statistics
+    auto fetch = [&](float& v_lse, float& v_delta) {
+      const int qi = ws.base + r;
+      const bool in = r < 64 && qi < a.Tq;
+      const long long o = ((long long)b * a.N + ws.n) * a.Tq + qi;
+      v_lse = in ? a.lse[o] * LOG2E : INFINITY;
+      v_delta = in ? a.delta[o] : 0.f;
+    };
+    auto put = [&](int it, float v_lse, float v_delta) {
+      if (r < 64) {
+        float* d = s_stat + (it % 3) * 128;
+        d[r] = v_lse;
+        d[64 + r] = v_delta;
+        mbar_arrive(barStat0 + 8 * (it % 3));
+      }
+    };
+    float v_lse, v_delta;
+    for (int it = 0; it < 3 && it < nit; ++it) {
+      fetch(v_lse, v_delta);
+      put(it, v_lse, v_delta);
+      if (it + 1 < nit) next_tile(ws);
+    }
+    bool ok = true;
+    for (int it = 0; it < nit && ok; ++it) {
+      if (it + 3 < nit) fetch(v_lse, v_delta);
+      BWD_WAIT(bardQ, it & 1, ST_TIMEOUT_EPILOGUE);
+      tc_fence_after();
+      if (it + 3 < nit) {                  // dQt of this tile is there: its dS is, and nobody reads its statistics any more
+        put(it + 3, v_lse, v_delta);
+        if (it + 4 < nit) next_tile(ws);
+      }
+      uint32_t t[2][32];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) tmem_ld_32x32(tmem + lane_addr + C_::TM_DQT + 32 * j, t[j]);
+      tmem_ld_wait();
+      tc_fence_before();
+      mbar_arrive(barDQfree);
+      if (r < HO) {
+        float* dq = a.dQ + ((long long)b * a.Tq + w.base) * ld + (long long)w.n * H + half * HO + r;
+        if (w.base + BQ_ <= a.Tq) {
+#pragma unroll
+          for (int i = 0; i < BQ_; ++i) atomicAdd(dq + i * ld, __uint_as_float(t[i >> 5][i & 31]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < BQ_; ++i)
+            if (w.base + i < a.Tq) atomicAdd(dq + i * ld, __uint_as_float(t[i >> 5][i & 31]));
+        }
+      }
+      if (it + 1 < nit) next_tile(w);
     }
   } else {
     // ------------------------------------------------------- per-key-row math
@@ -285,148 +393,87 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     const int my_seg = (a.seg_k && key_valid) ? a.seg_k[(long long)b * a.Tk + kp] : 0;
     bool ok = true;
-    auto stat_ptr = [&](int buf, int which) { return s_stat + (buf * 3 + which) * 64; };
-    auto tile_of = [&](int it, int& n, int& qbase) {
-      n = kvh * G + it / nq;
-      qbase = (qt0 + it % nq) * BQ_;
-    };
-    auto fetch_stats = [&](int it, float& v_lse, float& v_delta, int& v_seg) {
-      int n, qbase;
-      tile_of(it, n, qbase);
-      const int qi = qbase + (int)threadIdx.x;
-      if (threadIdx.x < 64 && qi < a.Tq) {
-        const long long o = ((long long)b * a.N + n) * a.Tq + qi;
-        v_lse = a.lse[o] * LOG2E;
-        v_delta = a.delta[o];
-        v_seg = a.seg_q ? a.seg_q[(long long)b * a.Tq + qi] : 0;
-      } else {
-        v_lse = INFINITY;
-        v_delta = 0.f;
-        v_seg = -1;
-      }
-    };
-    // dQt tile of `it`: lane = head-dim index (within this CTA's half), column = query
-    auto drain_dq = [&](int it) {
-      int n, qbase;
-      tile_of(it, n, qbase);
-      uint32_t t[CW_ / 32][32];
+    const float sc2 = a.scale * LOG2E, inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
+    Walk w = first_tile();
+    for (int it = 0; it < nit && ok; ++it) {
+      const float* st_lse = s_stat + (it % 3) * 128 + c0;      // this thread's columns
+      const float* st_delta = st_lse + 64;
+      const int q0 = w.base + c0;
+      // does any (key, query) pair of this tile need masking?
+      const int qpos_lo = w.base + a.q_off, qpos_hi = w.base + BQ_ - 1 + a.q_off;
+      const bool by_seg = a.seg_k != nullptr && !w.same;
+      const bool need_mask = (k0 + BK_ > a.Tk) || (w.base + BQ_ > a.Tq) || by_seg || (a.causal && (k0 + BK_ - 1 > qpos_lo)) ||
+                             (a.window > 0 && (k0 <= qpos_hi - a.window));
+      uint32_t keep[CW_ / 32];             // the queries that see this key, one bit each
+      if (need_mask) {
+        int lo = 0, hi = key_valid ? a.Tq - q0 : 0;
+        if (a.causal) lo = kp - a.q_off - q0;
+        if (a.window > 0) hi = min(hi, kp + a.window - a.q_off - q0);
 #pragma unroll
-      for (int j = 0; j < CW_ / 32; ++j) tmem_ld_32x32(tmem + lane_addr + C_::tm_dqt(sbuf(it)) + c0 + 32 * j, t[j]);
-      tmem_ld_wait();
-      if (r < HO) {
-        float* dq = a.dQ + ((long long)b * a.Tq + qbase + c0) * ((long long)a.N * H) + (long long)n * H + half * HO + r;
-        const long long ld = (long long)a.N * H;
-        if (qbase + 64 <= a.Tq) {
-#pragma unroll
-          for (int i = 0; i < CW_; ++i) atomicAdd(dq + i * ld, __uint_as_float(t[i >> 5][i & 31]));
-        } else {
-#pragma unroll
-          for (int i = 0; i < CW_; ++i)
-            if (qbase + c0 + i < a.Tq) atomicAdd(dq + i * ld, __uint_as_float(t[i >> 5][i & 31]));
+        for (int j = 0; j < CW_ / 32; ++j) {
+          keep[j] = bits_below(hi - 32 * j) & ~bits_below(lo - 32 * j);
+          if (by_seg && a.seg_q) seg_bits(a.seg_q + (long long)b * a.Tq, q0 + 32 * j, a.Tq, my_seg, keep[j]);
+          else if (by_seg && my_seg != 0) keep[j] = 0;
         }
       }
-    };
-    if (nit > 0) {
-      float f0, f1;
-      int i2;
-      fetch_stats(0, f0, f1, i2);
-      if (threadIdx.x < 64) {
-        stat_ptr(0, 0)[threadIdx.x] = f0;
-        stat_ptr(0, 1)[threadIdx.x] = f1;
-        reinterpret_cast<int*>(stat_ptr(0, 2))[threadIdx.x] = i2;
-      }
-    }
-    for (int it = 0; it < nit && ok; ++it) {
-      // stats of tile `it` visible to every row thread; previous tile's stats fully consumed
-      mbar_arrive(barSync);
-      BWD_WAIT(barSync, it & 1, ST_TIMEOUT_EPILOGUE);
-      float nx_lse = INFINITY, nx_delta = 0.f;
-      int nx_seg = -1;
-      if (it + 1 < nit) fetch_stats(it + 1, nx_lse, nx_delta, nx_seg);
-      int n, qbase;
-      tile_of(it, n, qbase);
-      const float* st_lse = stat_ptr(it & 1, 0) + c0;          // this thread's columns
-      const float* st_delta = stat_ptr(it & 1, 1) + c0;
-      const int* st_seg = reinterpret_cast<const int*>(stat_ptr(it & 1, 2)) + c0;
-      const int pb = PIPE ? (it & 1) : 0;
-      // does any (key, query) pair of this tile need masking?
-      const int qpos_lo = qbase + a.q_off, qpos_hi = qbase + BQ_ - 1 + a.q_off;
-      const bool need_mask = (k0 + BK_ > a.Tk) || (qbase + BQ_ > a.Tq) || (a.seg_k != nullptr) ||
-                             (a.causal && (k0 + BK_ - 1 > qpos_lo)) ||
-                             (a.window > 0 && (k0 <= qpos_hi - a.window));
 
-      BWD_WAIT(barSt0 + 8 * sbuf(it), spar(it), ST_TIMEOUT_EPILOGUE);
+      BWD_WAIT(barStat0 + 8 * (it % 3), (it / 3) & 1, ST_TIMEOUT_EPILOGUE);
+      BWD_WAIT(barSt0 + (PIPE ? 8 * (it & 1) : 0), (PIPE ? it >> 1 : it) & 1, ST_TIMEOUT_EPILOGUE);
       tc_fence_after();
       float p[CW_];
+      uint32_t pk[CW_ / 2];
       {
         uint32_t t[CW_ / 32][32];
 #pragma unroll
-        for (int j = 0; j < CW_ / 32; ++j) tmem_ld_32x32(tmem + lane_addr + C_::tm_st(sbuf(it)) + c0 + 32 * j, t[j]);
+        for (int j = 0; j < CW_ / 32; ++j) tmem_ld_32x32(tmem + lane_addr + C_::tm_st(it) + c0 + 32 * j, t[j]);
         tmem_ld_wait();
-        const float sc2 = a.scale * LOG2E;
-        if (!need_mask && a.softcap <= 0.f) {
-#pragma unroll
-          for (int i = 0; i < CW_; ++i)
-            p[i] = exp2f(__uint_as_float(t[i >> 5][i & 31]) * sc2 - st_lse[i]);
-        } else {
+        if (a.softcap > 0.f) {
 #pragma unroll
           for (int i = 0; i < CW_; ++i) {
-            const float s = __uint_as_float(t[i >> 5][i & 31]);
-            const int qpos = qbase + c0 + i + a.q_off;
-            float z;
-            if (a.softcap > 0.f) z = a.softcap * tanhf(s * a.scale / a.softcap) * LOG2E;
-            else z = s * sc2;
-            bool keep = key_valid && (qbase + c0 + i < a.Tq);
-            if (a.causal) keep = keep && (kp <= qpos);
-            if (a.window > 0) keep = keep && (kp > qpos - a.window);
-            if (a.seg_k) keep = keep && (st_seg[i] == my_seg);
-            p[i] = keep ? exp2f(z - st_lse[i]) : 0.f;
+            const float z = cap_score(__uint_as_float(t[i >> 5][i & 31]) * a.scale, a.softcap, inv_cap);
+            t[i >> 5][i & 31] = __float_as_uint(z * inv_cap);
+            p[i] = exp2f(fmaf(z, LOG2E, -st_lse[i]));
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < CW_; ++i) p[i] = exp2f(fmaf(__uint_as_float(t[i >> 5][i & 31]), sc2, -st_lse[i]));
+        }
+        if (need_mask) {
+#pragma unroll
+          for (int i = 0; i < CW_; ++i)
+            if (!(keep[i >> 5] >> (i & 31) & 1)) p[i] = 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < CW_ / 2; ++i) pk[i] = pack_bf16(p[2 * i], p[2 * i + 1]);
+        if (a.softcap > 0.f) {             // dS passes through the cap's derivative
+#pragma unroll
+          for (int i = 0; i < CW_; ++i) {
+            const float th = __uint_as_float(t[i >> 5][i & 31]);
+            p[i] *= 1.f - th * th;
           }
         }
       }
+      // dV of the tile before has read the buffer of Pt (without PIPE it retired before this tile's St)
+      if (PIPE && it >= 1) BWD_WAIT(bardV, (it - 1) & 1, ST_TIMEOUT_EPILOGUE);
       {
-        uint8_t* prow = sptr + C_::OFF_PT + pb * C_::P_BYTES + r * 128;
+        uint8_t* prow = sptr + C_::OFF_PT + r * 128;
 #pragma unroll
-        for (int c = 0; c < CW_ / 8; ++c) {
-          uint4 v;
-          v.x = pack_bf16(p[8 * c + 0], p[8 * c + 1]);
-          v.y = pack_bf16(p[8 * c + 2], p[8 * c + 3]);
-          v.z = pack_bf16(p[8 * c + 4], p[8 * c + 5]);
-          v.w = pack_bf16(p[8 * c + 6], p[8 * c + 7]);
-          *reinterpret_cast<uint4*>(prow + (((c + c0 / 8) ^ (r & 7)) << 4)) = v;
-        }
+        for (int c = 0; c < CW_ / 8; ++c)
+          *reinterpret_cast<uint4*>(prow + (((c + c0 / 8) ^ (r & 7)) << 4)) =
+              make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
         fence_proxy_async_smem();
         tc_fence_before();
         mbar_arrive(barPt);
       }
-      if (PIPE && it >= 1) {
-        // drain dQt of the previous tile while the tensor core works on dV of this one
-        BWD_WAIT(bardQ, (it - 1) & 1, ST_TIMEOUT_EPILOGUE);
-        tc_fence_after();
-        drain_dq(it - 1);
-        tc_fence_before();
-        mbar_arrive(barDQfree);
-      }
-      BWD_WAIT(bardPt0 + 8 * sbuf(it), spar(it), ST_TIMEOUT_EPILOGUE);
+      BWD_WAIT(bardPt, it & 1, ST_TIMEOUT_EPILOGUE);
       tc_fence_after();
       {
         uint32_t t[CW_ / 32][32];
 #pragma unroll
-        for (int j = 0; j < CW_ / 32; ++j) tmem_ld_32x32(tmem + lane_addr + C_::tm_dpt(sbuf(it)) + c0 + 32 * j, t[j]);
+        for (int j = 0; j < CW_ / 32; ++j) tmem_ld_32x32(tmem + lane_addr + C_::TM_DPT + c0 + 32 * j, t[j]);
         tmem_ld_wait();
-        if (a.softcap > 0.f) {
-          uint32_t sv[CW_ / 32][32];
-#pragma unroll
-          for (int j = 0; j < CW_ / 32; ++j) tmem_ld_32x32(tmem + lane_addr + C_::tm_st(sbuf(it)) + c0 + 32 * j, sv[j]);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < CW_; ++i) {
-            const float s = __uint_as_float(sv[i >> 5][i & 31]);
-            const float t = tanhf(s * a.scale / a.softcap);
-            p[i] *= (1.f - t * t);
-          }
-        }
-        uint8_t* drow = sptr + C_::OFF_DST + pb * C_::P_BYTES + r * 128;
+        // (dSt of the tile before last was read by products that retired before this dPt)
+        uint8_t* drow = sptr + C_::OFF_DST + (PIPE ? (it & 1) : 0) * C_::P_BYTES + r * 128;
 #pragma unroll
         for (int c = 0; c < CW_ / 8; ++c) {
           float d[8];
@@ -447,24 +494,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc_fence_before();
         mbar_arrive(bardSt);
       }
-      if (!PIPE) {
-        BWD_WAIT(bardQ, it & 1, ST_TIMEOUT_EPILOGUE);
-        tc_fence_after();
-        drain_dq(it);
-        tc_fence_before();
-      }
-      if (it + 1 < nit && threadIdx.x < 64) {
-        stat_ptr((it + 1) & 1, 0)[threadIdx.x] = nx_lse;
-        stat_ptr((it + 1) & 1, 1)[threadIdx.x] = nx_delta;
-        reinterpret_cast<int*>(stat_ptr((it + 1) & 1, 2))[threadIdx.x] = nx_seg;
-      }
+      if (it + 1 < nit) next_tile(w);
     }
-    if (PIPE && nit > 0 && ok) {
-      // last tile's dQt; its completion also means every dV / dK MMA has retired
-      ok = mbar_wait_bounded(bardQ, (nit - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
-      tc_fence_after();
-      if (ok) drain_dq(nit - 1);
-    }
+    if (nit > 0 && ok) ok = mbar_wait_bounded(barDone, 0, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
 #undef BWD_WAIT
     // ------------------------------------------------------------- dK / dV
     tc_fence_after();
@@ -503,7 +535,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (*abort_flag) {
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
   }
-  if (warp == 4 * RG_) {
+  if (warp == 4 * RG_ + 4) {
     tc_fence_after();
     tmem_dealloc(tmem, C_::TMEM_COLS);
   }
@@ -545,15 +577,10 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* dout, co
   if (tb_make_tmap_2d_bf16(&tv, v, (uint64_t)a.B * a.Tk, (uint64_t)a.KH * H, ldv, BK_, 64, 1)) return -3;
   static DeviceOnce once;
   if (once.first() &&
-      (cudaFuncSetAttribute(attn_bwd_kernel<H, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM_BYTES) != cudaSuccess ||
-       cudaFuncSetAttribute(attn_bwd_kernel<H, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM_BYTES) != cudaSuccess))
+      cudaFuncSetAttribute(attn_bwd_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM_BYTES) != cudaSuccess)
     return -5;
-  dim3 grid((a.Tk + BK_ - 1) / BK_, a.KH * C_::NHALF, a.B);
-  // two row-thread groups (288 threads; B = 8, T = 2048, 32 / 8 heads, H = 128: 1.55 ms against 1.77 ms with one group);
-  // TUNIX_B200_ATTN_BWD_GROUPS=1 selects the single-warpgroup form for comparison
-  static const bool one_group = [] { const char* e = getenv("TUNIX_B200_ATTN_BWD_GROUPS"); return e && atoi(e) == 1; }();
-  if (one_group) attn_bwd_kernel<H, 1><<<grid, 160, C_::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, a);
-  else attn_bwd_kernel<H, 2><<<grid, 288, C_::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, a);
+  dim3 grid(a.KH * C_::NHALF, a.B, (a.Tk + BK_ - 1) / BK_);
+  attn_bwd_kernel<H><<<grid, 128 * RG_ + 160, C_::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

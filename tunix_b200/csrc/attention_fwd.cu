@@ -18,13 +18,13 @@
 // Segment ids are compared per key block where they decide for the whole of it, and by warp votes elsewhere, not by one load a
 // score; K and V share a ring, so that no product waits for a load issued in its own block. B200, 32 / 8 heads of 128, causal,
 // before -> after: rollouts padded at both ends, 8 x 1024 519 -> 135 us, 16 x 1024 970 -> 245, 8 x 4096 6320 -> 939; packed rows
-// of 777, 14 / 2 heads of 64, 92 -> 31; without segments 2 x 2048 136 -> 116, 8 x 2048 452 -> 369, 1 x 16384 2228 -> 2206;
-// 4 x 1001 with heads of 256 and a soft-cap 265 -> 97.
+// of 777, 14 / 2 heads of 64, 92 -> 31; without segments 2 x 2048 136 -> 95, 8 x 2048 452 -> 397, 1 x 16384 2228 -> 2046;
+// 4 x 1001 with heads of 256 and a soft-cap 265 -> 89.
 //
 // Replaces the eager [B,N,T,S] attention and the TPU-only splash attention of the reference
 // (tunix/models/llama3/model.py:379-396, tunix/models/qwen3/model.py:607-793,
 //  tunix/models/gemma/model.py:442-483).
-#include "common.cuh"
+#include "segments.cuh"
 #include <cstdlib>
 
 using namespace tb;
@@ -34,6 +34,7 @@ namespace {
 constexpr int BQ = 128;   // query rows per CTA
 constexpr int BKV = 64;   // keys per iteration
 constexpr float LOG2E = 1.4426950408889634f;
+constexpr int SEG_BLOCKS = 2048;           // key blocks that the list of a tile can hold; longer ranges are walked without one
 constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units
 
 struct AttnArgs {
@@ -64,98 +65,6 @@ struct AttnArgs {
                              // of rows that all heads share
   float out_scale;           // paged: factor of the output
 };
-
-// Segment ids (packed rows, padding) decide for most key blocks as a whole. A tile lists the blocks with any id between the
-// smallest and the largest of its rows, and marks those where all ids are the one that all its rows have; the others are never
-// loaded. Elements are compared in the rest only.
-constexpr int SEG_BLOCKS = 2048;            // blocks that the list can hold; longer ranges are walked without one
-constexpr uint16_t SEG_SAME = 0x8000, SEG_ID = 0x7fff;
-struct SegList {
-  uint16_t id[SEG_BLOCKS];
-  int lo[8], hi[8], n;
-};
-
-// All threads of the CTA: key blocks jb0 .. jb0 + nblk - 1 for the rows q0 .. q0 + nrows - 1 -> the number listed. Each half-warp
-// reads four consecutive ids a lane, four blocks in flight.
-__device__ __forceinline__ int build_seg_list(SegList& s, const AttnArgs& a, int b, int q0, int nrows, int jb0, int nblk) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
-  int lo = 0x7fffffff, hi = -0x7fffffff - 1;
-  for (int i = tid; i < min(nrows, BQ); i += blockDim.x) {
-    const int v = a.seg_q ? a.seg_q[(long long)b * a.Tq + q0 + i] : 0;
-    lo = min(lo, v);
-    hi = max(hi, v);
-  }
-  lo = __reduce_min_sync(0xffffffffu, lo);
-  hi = __reduce_max_sync(0xffffffffu, hi);
-  if (lane == 0) {
-    s.lo[warp] = lo;
-    s.hi[warp] = hi;
-  }
-  __syncthreads();
-  for (int w = 0; w < nwarp; ++w) {
-    lo = min(lo, s.lo[w]);
-    hi = max(hi, s.hi[w]);
-  }
-  const int* seg = a.seg_k + (long long)b * a.Tk;
-  for (int j0 = warp * 8; j0 < nblk; j0 += nwarp * 8) {
-    int v[4][4];
-    bool in[4][4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int j = j0 + 2 * u + (lane >> 4), k = (jb0 + j) * BKV + (lane & 15) * 4 + e;
-        in[u][e] = j < nblk && k < a.Tk;
-        v[u][e] = in[u][e] ? __ldg(seg + k) : 0;
-      }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      bool any = false, same = lo == hi;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        any = any || (in[u][e] && v[u][e] >= lo && v[u][e] <= hi);
-        same = same && in[u][e] && v[u][e] == lo;
-      }
-      const uint32_t half = (lane & 16) ? 0xffff0000u : 0xffffu;
-      const uint32_t anys = __ballot_sync(0xffffffffu, any) & half, sames = __ballot_sync(0xffffffffu, same) & half;
-      const int j = j0 + 2 * u + (lane >> 4);
-      if ((lane & 15) == 0 && j < nblk) s.id[j] = anys ? (uint16_t)(j | (sames == half ? SEG_SAME : 0)) : (uint16_t)SEG_ID;
-    }
-  }
-  __syncthreads();
-  if (warp == 0) {                                  // in place: entry n is written after entries up to n have been read
-    int n = 0;
-    for (int j = lane; j - lane < nblk; j += 32) {
-      const uint16_t v = j < nblk ? s.id[j] : SEG_ID;
-      const uint32_t take = __ballot_sync(0xffffffffu, v != SEG_ID);
-      if (v != SEG_ID) s.id[n + __popc(take & ((1u << lane) - 1))] = v;
-      n += __popc(take);
-      __syncwarp();
-    }
-    if (lane == 0) s.n = n;
-  }
-  __syncthreads();
-  return s.n;
-}
-
-__device__ __forceinline__ uint32_t bits_below(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1; }
-
-// Clears the bits of the 64 keys from k0 whose id is not the row's: one vote per id among the rows of the warp.
-__device__ __forceinline__ void seg_bits(const int* seg, int k0, int Tk, int mine, uint32_t (&keep)[2]) {
-  const int lane = threadIdx.x & 31;
-  const int v0 = k0 + lane < Tk ? __ldg(seg + k0 + lane) : 0, v1 = k0 + 32 + lane < Tk ? __ldg(seg + k0 + 32 + lane) : 0;
-  uint32_t todo = ~0u;
-  while (todo) {
-    const int id = __shfl_sync(0xffffffffu, mine, __ffs(todo) - 1);
-    const uint32_t b0 = __ballot_sync(0xffffffffu, v0 == id), b1 = __ballot_sync(0xffffffffu, v1 == id);
-    const bool now = mine == id;
-    if (now) {
-      keep[0] &= b0;
-      keep[1] &= b1;
-    }
-    todo &= ~__ballot_sync(0xffffffffu, now);
-  }
-}
 
 // H: query / key head size, HV: value head size
 template <int H, int HV>
@@ -200,8 +109,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sptr + C_::OFF_BAR + 68);
 
   const int warp = threadIdx.x >> 5;
-  const int qt = gridDim.x - 1 - blockIdx.x;  // heavy (late) causal tiles first
-  const int n = blockIdx.y, b = blockIdx.z;
+  // heavy (late) causal tiles of all heads and rows first: a last wave of light ones
+  const int qt = PAGED ? gridDim.x - 1 - blockIdx.x : gridDim.z - 1 - blockIdx.z;
+  const int n = PAGED ? blockIdx.y : blockIdx.x, b = PAGED ? 0 : blockIdx.y;
   const int kvh = n / (a.N / a.KH);
   // the tile's first row in Q and O, its valid rows, the position of its first query, the keys of its sequence
   int row0, nrows, i0, Tk;
@@ -229,12 +139,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int jb0 = kv_start / BKV;
   const int n_sink = PAGED ? min((min(a.keep, Tk) + BKV - 1) / BKV, jb0) : 0;
   int nblk = n_sink + (kv_end > jb0 * BKV ? (kv_end - jb0 * BKV + BKV - 1) / BKV : 0);
-  const SegList* list = nullptr;
+  const SegList<SEG_BLOCKS>* list = nullptr;
   if constexpr (!PAGED) {
-    __shared__ SegList s_list;
+    __shared__ SegList<SEG_BLOCKS> s_list;
     if (a.seg_k && nblk <= SEG_BLOCKS) {
       list = &s_list;
-      nblk = build_seg_list(s_list, a, b, qt * BQ, nrows, jb0, nblk);
+      nblk = build_seg_list(s_list, a.seg_q ? a.seg_q + (long long)b * a.Tq + qt * BQ : nullptr, min(nrows, BQ),
+                            a.seg_k + (long long)b * a.Tk, a.Tk, jb0, nblk);
     }
   }
   auto block_key = [&](int j) {                                                           // first key of block j
@@ -392,7 +303,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int lo = a.window > 0 ? qpos - a.window + 1 - k0 : 0;
         keep[0] = bits_below(hi) & ~bits_below(lo);
         keep[1] = bits_below(hi - 32) & ~bits_below(lo - 32);
-        if (by_seg) seg_bits(a.seg_k + (long long)b * a.Tk, k0, a.Tk, my_seg, keep);
+        if (by_seg) {
+          const int* seg = a.seg_k + (long long)b * a.Tk;
+          seg_bits(seg, k0, a.Tk, my_seg, keep[0]);
+          seg_bits(seg, k0 + 32, a.Tk, my_seg, keep[1]);
+        }
       }
       if (!mbar_wait_bounded(barS0 + 8 * (j & 1), (j >> 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
@@ -556,7 +471,7 @@ int launch_fwd(const void* q, const void* k, const void* v, const AttnArgs& a, l
   if (once.first() &&
       cudaFuncSetAttribute(attn_fwd_kernel<H, H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM_BYTES) != cudaSuccess)
     return -5;
-  dim3 grid((a.Tq + BQ - 1) / BQ, a.N, a.B);
+  dim3 grid(a.N, a.B, (a.Tq + BQ - 1) / BQ);
   attn_fwd_kernel<H, H, false><<<grid, 160, C_::SMEM_BYTES, stream>>>(tq, tk, tv, tk, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
