@@ -382,3 +382,23 @@ def test_packed_gemm_with_gated_epilogue(M, F, D, kind):
     assert out.shape == (M, F)
     assert _rel_err(out, ref) < 1e-2
     assert torch.allclose(out.float(), ref, atol=0.02 * ref.abs().max().item() + 1e-3, rtol=3e-2)
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K_", [(1, 8), (5, 264), (1030, 1536), (2050, 520), (72, 4104)])
+def test_gemm_few_rows(M, N, K_):
+    """Products of up to four rows: remainders of the row groups and of the steps over K, every epilogue."""
+    k = _k()
+    g = torch.Generator(device="cuda").manual_seed(8)
+    draw = lambda r, c: torch.randn(r, c + 8, device="cuda", generator=g).to(torch.bfloat16)[:, :c]  # noqa: E731
+    a, b, res = draw(M, K_), draw(N, K_), draw(M, N)
+    bias = torch.randn(N, device="cuda", generator=g).to(torch.bfloat16)
+    want = a.double() @ b.double().t()
+    # sums of K_ products in 32 bits: 2^-24 a term, far below the norm of the sum
+    assert _rel_err(k.gemm(a, b, out_dtype=torch.float32), want) < 1e-5
+    full = 0.5 * want + bias.double() + res.double()
+    assert _rel_err(k.gemm(a, b, bias=bias, residual=res, alpha=0.5), full) < 4e-3
+    for dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 4e-3)):
+        out = torch.ones(M, N + 3, device="cuda", dtype=dtype)[:, :N]
+        assert _rel_err(k.gemm(a, b, out=out, accumulate=True), want + 1) < tol
+    _check_status()
