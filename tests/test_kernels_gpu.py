@@ -402,3 +402,25 @@ def test_gemm_few_rows(M, N, K_):
         out = torch.ones(M, N + 3, device="cuda", dtype=dtype)[:, :N]
         assert _rel_err(k.gemm(a, b, out=out, accumulate=True), want + 1) < tol
     _check_status()
+
+
+@pytest.mark.parametrize("rows", [1, 3, 1301])
+@pytest.mark.parametrize("D", [8, 64, 72, 128, 136, 256, 264, 4096, 4104, 8192, 8200, 16384, 16392])
+def test_rmsnorm_widths(rows, D):
+    """Widths on both sides of every kernel's limit, rows that lie apart, dx added to what is there."""
+    k = _k()
+    g = torch.Generator(device="cuda").manual_seed(7)
+    draw = lambda: torch.randn(rows, D + 8, device="cuda", generator=g).to(torch.bfloat16)[:, :D]  # noqa: E731
+    x, dy, base = draw(), draw(), draw()
+    w = torch.randn(D, device="cuda", generator=g).to(torch.bfloat16)
+    y, rstd = k.rmsnorm_fwd(x, w, 1e-6, True)
+    into = base.clone()
+    dx, dw = k.rmsnorm_bwd(dy, x, w, rstd, True, dx_accumulate_into=into)
+    xd, dd, wd = x.double(), dy.double(), w.double() + 1
+    rs = torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6)
+    gx = dd * wd
+    want = base.double() + rs * (gx - xd * rs * (gx * xd * rs).mean(-1, keepdim=True))
+    # one rounding to bf16: 2^-9 of a value
+    assert _rel_err(y, xd * rs * wd) < 4e-3 and _rel_err(dx, want) < 4e-3
+    assert _rel_err(dw, (dd * xd * rs).sum(0)) < 1e-5          # 32-bit sums over the rows
+    _check_status()

@@ -63,6 +63,49 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, long lon
   }
 }
 
+// Same for rows of at most 256 columns (the norms of single heads): T lanes a row, 8 columns a lane, a row read once.
+template <int T>
+__global__ void __launch_bounds__(256)
+rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
+                          __nv_bfloat16* __restrict__ y, long long ldy, float* __restrict__ rstd_out, int rows, int D, float eps,
+                          float add_one) {
+  const int sub = threadIdx.x % T, col = sub * 8;
+  const bool in = col < D;
+  float g[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) g[i] = 0.f;
+  if (in) load8(w + col, g);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) g[i] += add_one;
+  constexpr int U = 4;                                     // rows in flight per lane
+  const long long step = (long long)gridDim.x * (256 / T), first = (long long)blockIdx.x * (256 / T) + threadIdx.x / T;
+  for (long long r0 = first; r0 - threadIdx.x / T < rows; r0 += U * step) {
+    float v[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[u][i] = 0.f;
+      if (r0 + u * step < rows && in) load8(x + (r0 + u * step) * ldx + col, v[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long r = r0 + u * step;
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ss += v[u][i] * v[u][i];
+#pragma unroll
+      for (int o = T / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float rstd = rsqrtf(ss / (float)D + eps);
+      if (r < rows && in) {
+        if (sub == 0 && rstd_out) rstd_out[r] = rstd;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[u][i] = v[u][i] * rstd * g[i];
+        store8(y + r * ldy + col, v[u]);
+      }
+    }
+  }
+}
+
 // Same, one CTA per row: with few rows (decode) the warp-per-row kernel is a handful of warps each walking a
 // whole row twice, and latency, not bandwidth, sets its time. The row is held in registers between the passes.
 template <int VPT>   // 8-element vectors per thread
@@ -103,8 +146,215 @@ rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const
   }
 }
 
-// dx = rstd * (dy*w' - xhat * mean(dy*w'*xhat)), xhat = x*rstd, w' = w + add_one.
-// If accumulate != 0, dx += (used when the residual stream's gradient is folded in).
+// dx = rstd * (dy*w' - xhat * mean(dy*w'*xhat)), xhat = x*rstd, w' = w + add_one (dx += with accumulate != 0), and
+// dw[c] += sum_rows dy[r,c] * x[r,c] * rstd[r] (fp32 atomics into a zeroed buffer), in one pass over x and dy: a row is held in
+// registers between its reduction and its dx, and a thread keeps the sums of its columns over all its rows.
+//
+// Bound by HBM: x, dy and dx once each. B200, dx and dw together, before (two kernels, three passes over x and dy) -> after:
+// 524288 x 128 691 -> 125 us, 16384 x 4096 219 -> 105, 8192 x 4096 117 -> 59, 4096 x 4096 59 -> 33, 2331 x 896 34 -> 22. Narrow
+// rows forward (a lane of 16 idle before): 524288 x 128 98 -> 64.
+__device__ __forceinline__ void add4(float* p, float a, float b, float c, float d) {     // p: 16-byte aligned
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// Rows of at most 256 columns (the norms of single heads): T lanes a row, 8 columns a lane.
+template <int T>
+__global__ void __launch_bounds__(256)
+rmsnorm_bwd_narrow_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv_bfloat16* __restrict__ x, long long ldx,
+                          const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
+                          long long lddx, float* __restrict__ dw, int rows, int D, float add_one, int accumulate) {
+  __shared__ float s_dw[T * 8];
+  const int sub = threadIdx.x % T, col = sub * 8;
+  const bool in = col < D;
+  for (int i = threadIdx.x; i < T * 8; i += blockDim.x) s_dw[i] = 0.f;
+  __syncthreads();
+  float g[8], acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) g[i] = acc[i] = 0.f;
+  if (in) load8(w + col, g);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) g[i] += add_one;
+  const float inv_d = 1.f / (float)D;
+  constexpr int U = 2;                                     // rows in flight per lane
+  const long long step = (long long)gridDim.x * (256 / T), first = (long long)blockIdx.x * (256 / T) + threadIdx.x / T;
+  // every lane of a warp makes the same number of turns: the shuffles below need all of them
+  for (long long r0 = first; r0 - threadIdx.x / T < rows; r0 += U * step) {
+    float v[U][8], d[U][8], rs[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long r = r0 + u * step;
+      rs[u] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[u][i] = d[u][i] = 0.f;
+      if (r < rows && in) {
+        load8(x + r * ldx + col, v[u]);
+        load8(dy + r * lddy + col, d[u]);
+        rs[u] = rstd_in[r];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long r = r0 + u * step;
+      float dot = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[u][i] *= rs[u];
+        acc[i] += d[u][i] * v[u][i];
+        d[u][i] *= g[i];
+        dot += d[u][i] * v[u][i];
+      }
+#pragma unroll
+      for (int o = T / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      dot *= inv_d;
+      if (r < rows && in && dx) {
+        float o[8];
+        if (accumulate) load8(dx + r * lddx + col, o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float t = rs[u] * (d[u][i] - v[u][i] * dot);
+          o[i] = accumulate ? o[i] + t : t;
+        }
+        store8(dx + r * lddx + col, o);
+      }
+    }
+  }
+  if (!dw) return;
+  if (in)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) atomicAdd(s_dw + col + i, acc[i]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < D; i += blockDim.x) atomicAdd(dw + i, s_dw[i]);
+}
+
+// Wider rows: up to 512 threads a row, VPT vectors of 8 columns a thread; the next row is loaded before the sum of this one is
+// formed. The groups of threads of a block (threadIdx.y) walk over rows of their own, and their column sums meet in shared memory
+// before they leave as one atomic a block and column.
+constexpr int RMS_GROUPS = 8;
+template <int VPT>
+__global__ void __launch_bounds__(VPT == 1 ? 1024 : 512, 1)
+rmsnorm_bwd_row_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv_bfloat16* __restrict__ x, long long ldx,
+                       const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
+                       long long lddx, float* __restrict__ dw, int rows, int D, float add_one, int accumulate) {
+  __shared__ float red[RMS_GROUPS][2][16];
+  extern __shared__ float s_dw[];                          // [D]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, grp = threadIdx.y;
+  constexpr int AHEAD = VPT == 1 ? 2 : 1;                  // rows that are loaded before their turn
+  float acc[VPT][8], ns[AHEAD];
+  uint4 nx[AHEAD][VPT], nd[AHEAD][VPT], wq[VPT];
+  auto col = [&](int j) { return (int)(threadIdx.x + j * blockDim.x) * 8; };
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
+    wq[j] = col(j) < D ? *reinterpret_cast<const uint4*>(w + col(j)) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  auto fetch = [&](long long r, uint4 (&fx)[VPT], uint4 (&fd)[VPT], float& fs) {
+    fs = r < rows ? rstd_in[r] : 0.f;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      fx[j] = fd[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (r < rows && col(j) < D) {
+        fx[j] = *reinterpret_cast<const uint4*>(x + r * ldx + col(j));
+        fd[j] = *reinterpret_cast<const uint4*>(dy + r * lddy + col(j));
+      }
+    }
+  };
+  auto unpack = [](const uint4& q, float (&v)[8]) {
+    const uint32_t t[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = bf16_lo(t[i]);
+      v[2 * i + 1] = bf16_hi(t[i]);
+    }
+  };
+  const float inv_d = 1.f / (float)D;
+  int turn = 0;
+  const long long first = (long long)blockIdx.x * blockDim.y + grp, step = (long long)gridDim.x * blockDim.y;
+#pragma unroll
+  for (int q = 0; q < AHEAD; ++q) fetch(first + q * step, nx[q], nd[q], ns[q]);
+  for (long long r = first; r < rows; r += step, turn ^= 1) {
+    uint4 cx[VPT], cd[VPT];
+    const float rs = ns[0];
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      cx[j] = nx[0][j];
+      cd[j] = nd[0][j];
+    }
+#pragma unroll
+    for (int q = 0; q + 1 < AHEAD; ++q) {
+      ns[q] = ns[q + 1];
+#pragma unroll
+      for (int j = 0; j < VPT; ++j) {
+        nx[q][j] = nx[q + 1][j];
+        nd[q][j] = nd[q + 1][j];
+      }
+    }
+    fetch(r + AHEAD * step, nx[AHEAD - 1], nd[AHEAD - 1], ns[AHEAD - 1]);
+    float dot = 0.f;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      if (col(j) >= D) continue;
+      float v[8], d[8], g[8];
+      unpack(cx[j], v);
+      unpack(cd[j], d);
+      unpack(wq[j], g);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float p = d[i] * (v[i] * rs);
+        acc[j][i] += p;
+        dot += p * (g[i] + add_one);
+      }
+    }
+    dot = warp_sum(dot);
+    if (lane == 0) red[grp][turn][warp] = dot;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"((int)blockDim.x) : "memory");   // of the group; the other buffer is next
+    dot = 0.f;
+    for (int i = 0; i < nw; ++i) dot += red[grp][turn][i];
+    dot *= inv_d;
+    if (!dx) continue;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      if (col(j) >= D) continue;
+      float v[8], d[8], g[8], o[8];
+      unpack(cx[j], v);
+      unpack(cd[j], d);
+      unpack(wq[j], g);
+      if (accumulate) load8(dx + r * lddx + col(j), o);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float t = rs * (d[i] * (g[i] + add_one) - v[i] * rs * dot);
+        o[i] = accumulate ? o[i] + t : t;
+      }
+      store8(dx + r * lddx + col(j), o);
+    }
+  }
+  if (!dw) return;
+  for (int g = 0; g < (int)blockDim.y; ++g) {
+    if (grp == g) {
+#pragma unroll
+      for (int j = 0; j < VPT; ++j) {
+        if (col(j) >= D) continue;
+        float4* d = reinterpret_cast<float4*>(s_dw + col(j));
+        float4 lo = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+        float4 hi = make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
+        if (g > 0) {
+          lo.x += d[0].x; lo.y += d[0].y; lo.z += d[0].z; lo.w += d[0].w;
+          hi.x += d[1].x; hi.y += d[1].y; hi.z += d[1].z; hi.w += d[1].w;
+        }
+        if (g + 1 < (int)blockDim.y) {
+          d[0] = lo;
+          d[1] = hi;
+        } else {
+          add4(dw + col(j), lo.x, lo.y, lo.z, lo.w);
+          add4(dw + col(j) + 4, hi.x, hi.y, hi.z, hi.w);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The same in two kernels, for rows too wide for the registers of a block.
 __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy,
                                       const __nv_bfloat16* __restrict__ x, long long ldx,
                                       const __nv_bfloat16* __restrict__ w,
@@ -349,6 +599,18 @@ TB_API int tb_rmsnorm_fwd(const void* x, long long ldx, const void* w, void* y, 
     return e == cudaSuccess ? 0 : -5;
   }
   const int block = 256;
+  if (D <= 256) {
+    const int t = D <= 64 ? 8 : D <= 128 ? 16 : 32;
+    const int grid = grid_for((long long)rows * t, 256 * 2, 148 * 16);
+    auto run = [&](auto kernel) {
+      kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, ldy, rstd, rows, D, eps,
+                                       add_one);
+    };
+    if (t == 8) run(rmsnorm_fwd_narrow_kernel<8>);
+    else if (t == 16) run(rmsnorm_fwd_narrow_kernel<16>);
+    else run(rmsnorm_fwd_narrow_kernel<32>);
+    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  }
   rmsnorm_fwd_kernel<<<grid_for((long long)rows * 32, block), block, 0, stream>>>(
       (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, ldy, rstd, rows, D,
       eps, add_one);
@@ -360,16 +622,42 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
                           int rows, int D, float add_one, int accumulate_dx, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (D % 8) return -2;
-  const int block = 256;
-  if (dx)
-    rmsnorm_bwd_dx_kernel<<<grid_for((long long)rows * 32, block), block, 0, stream>>>(
-        (const __nv_bfloat16*)dy, lddy, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, rstd,
-        (__nv_bfloat16*)dx, lddx, rows, D, add_one, accumulate_dx);
-  if (dw) {
-    dim3 grid((D + 127) / 128, (unsigned)min(128, (rows + 3) / 4));
-    rmsnorm_bwd_dw_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, lddy,
-                                                    (const __nv_bfloat16*)x, ldx, rstd, dw, rows, D);
+  if (!dx && !dw) return 0;
+  // up to 256 columns by lanes of a warp, up to 16384 by threads of a block; the SMs are filled once, so that the sums over columns
+  // meet in few atomics
+#define RMS_BWD_ARGS                                                                                                          \
+  (const __nv_bfloat16*)dy, lddy, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, rstd, (__nv_bfloat16*)dx, lddx, dw, rows, D, \
+      add_one, accumulate_dx
+  const bool wide = D > 16384 || (D > 256 && (reinterpret_cast<uintptr_t>(dw) & 15));
+  if (wide) {
+    const int block = 256;
+    if (dx)
+      rmsnorm_bwd_dx_kernel<<<grid_for((long long)rows * 32, block), block, 0, stream>>>(
+          (const __nv_bfloat16*)dy, lddy, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, rstd,
+          (__nv_bfloat16*)dx, lddx, rows, D, add_one, accumulate_dx);
+    if (dw) {
+      dim3 grid((D + 127) / 128, (unsigned)min(128, (rows + 3) / 4));
+      rmsnorm_bwd_dw_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, lddy,
+                                                      (const __nv_bfloat16*)x, ldx, rstd, dw, rows, D);
+    }
+  } else if (D <= 256) {
+    const int t = D <= 64 ? 8 : D <= 128 ? 16 : 32;
+    const int grid = grid_for((long long)rows * t, 256 * 4, 148 * 6);
+    if (t == 8) rmsnorm_bwd_narrow_kernel<8><<<grid, 256, 0, stream>>>(RMS_BWD_ARGS);
+    else if (t == 16) rmsnorm_bwd_narrow_kernel<16><<<grid, 256, 0, stream>>>(RMS_BWD_ARGS);
+    else rmsnorm_bwd_narrow_kernel<32><<<grid, 256, 0, stream>>>(RMS_BWD_ARGS);
+  } else {
+    const int vecs = D / 8, vpt = vecs <= 512 ? 1 : vecs <= 1024 ? 2 : 4;
+    const int threads = ((vecs + vpt - 1) / vpt + 31) / 32 * 32, most = vpt == 1 ? 1024 : 512;
+    const int groups = min(RMS_GROUPS, most / threads);
+    const int grid = min((rows + groups - 1) / groups, 148 * (most / (threads * groups)));
+    const dim3 block(threads, groups);
+    const size_t smem = groups > 1 ? (size_t)D * 4 : 0;      // at most 16 KB: more than one group has at most 4096 columns
+    if (vpt == 1) rmsnorm_bwd_row_kernel<1><<<grid, block, smem, stream>>>(RMS_BWD_ARGS);
+    else if (vpt == 2) rmsnorm_bwd_row_kernel<2><<<grid, block, smem, stream>>>(RMS_BWD_ARGS);
+    else rmsnorm_bwd_row_kernel<4><<<grid, block, smem, stream>>>(RMS_BWD_ARGS);
   }
+#undef RMS_BWD_ARGS
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -150,7 +150,7 @@ def rmsnorm_bwd(dy, x, w, rstd, add_one: bool = False, want_dw: bool = True,
                                     rstd.data_ptr(), dx.data_ptr(), dx.stride(0), _lib.ptr(dw), rows, D,
                                     1.0 if add_one else 0.0, acc, _lib.stream_ptr())
     _lib.check(rc, "tb_rmsnorm_bwd")
-    _count(2 if want_dw else 1)
+    _count(2 if want_dw and D > 16384 else 1)
     return dx, dw
 
 
