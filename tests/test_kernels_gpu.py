@@ -424,3 +424,20 @@ def test_rmsnorm_widths(rows, D):
     assert _rel_err(y, xd * rs * wd) < 4e-3 and _rel_err(dx, want) < 4e-3
     assert _rel_err(dw, (dd * xd * rs).sum(0)) < 1e-5          # 32-bit sums over the rows
     _check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,D", [(1, 8), (37, 264), (300, 10)])
+def test_embedding_bwd_tables(tokens, D, dtype):
+    """Both tables, rows of whole 16-byte pieces and by pairs; ids outside the table are left out."""
+    k = _k()
+    g = torch.Generator(device="cuda").manual_seed(10)
+    ids = torch.randint(-1, 41, (tokens,), device="cuda", generator=g, dtype=torch.int32)
+    dout = torch.randn(tokens, D, device="cuda", generator=g).to(torch.bfloat16)
+    table = torch.zeros(40, D, device="cuda", dtype=dtype)
+    k.embedding_bwd(ids, dout, table, scale=0.5)
+    ok = (ids >= 0) & (ids < 40)
+    want = torch.zeros(40, D, device="cuda").index_add_(0, ids[ok].long(), 0.5 * dout.float()[ok])
+    # up to some 20 terms a row: a bf16 rounding each where the table is bf16
+    assert _rel_err(table, want) < (2e-2 if dtype == torch.bfloat16 else 1e-6)
+    _check_status()

@@ -36,6 +36,7 @@ _CUDA_SIGS = {
     "tb_glu_bwd": [P, LL, P, LL, P, LL, P, LL, P, LL, LL, I, I, P],
     "tb_embedding_fwd": [P, P, LL, P, LL, LL, I, I, F, P],
     "tb_embedding_bwd": [P, P, LL, P, LL, LL, I, I, F, P],
+    "tb_embedding_bwd_f32": [P, P, LL, P, LL, LL, I, I, F, P],
     "tb_add_bf16": [P, P, P, LL, P],
     "tb_logsoftmax_gather": [P, LL, P, P, P, P, I, I, F, F, P],
     "tb_dlogits": [P, LL, P, P, P, P, P, P, LL, I, I, F, F, P],

@@ -354,7 +354,7 @@ class _EmbeddingFn(torch.autograd.Function):
         table = ctx.table_ref
         d2 = _flat2d(dout)
         mg = getattr(table, "main_grad", None)
-        if mg is not None and mg.dtype == torch.bfloat16:
+        if mg is not None and mg.dtype in (torch.bfloat16, torch.float32) and mg.stride(-1) == 1:
             K.embedding_bwd(ids32, d2, mg, ctx.scale)
             table.grad_added_to_main_grad = True
             return None, None, None

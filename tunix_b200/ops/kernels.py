@@ -210,11 +210,13 @@ def embedding_fwd(ids: torch.Tensor, table: torch.Tensor, scale: float = 1.0) ->
 
 
 def embedding_bwd(ids: torch.Tensor, dout: torch.Tensor, dtable: torch.Tensor, scale: float = 1.0) -> None:
-    """dtable[ids] += dout * scale (dtable bf16, accumulated in place)."""
+    """dtable[ids] += dout * scale (dtable bf16 or fp32, accumulated in place)."""
+    assert dtable.dtype in (torch.bfloat16, torch.float32) and dtable.stride(1) == 1
     tokens = ids.numel()
     V, D = dtable.shape
-    rc = _lib.cuda().tb_embedding_bwd(ids.data_ptr(), dout.data_ptr(), dout.stride(0), dtable.data_ptr(),
-                                      dtable.stride(0), tokens, D, V, float(scale), _lib.stream_ptr())
+    fn = _lib.cuda().tb_embedding_bwd if dtable.dtype == torch.bfloat16 else _lib.cuda().tb_embedding_bwd_f32
+    rc = fn(ids.data_ptr(), dout.data_ptr(), dout.stride(0), dtable.data_ptr(), dtable.stride(0), tokens, D, V,
+            float(scale), _lib.stream_ptr())
     _lib.check(rc, "tb_embedding_bwd")
     _count()
 
