@@ -441,3 +441,20 @@ def test_embedding_bwd_tables(tokens, D, dtype):
     # up to some 20 terms a row: a bf16 rounding each where the table is bf16
     assert _rel_err(table, want) < (2e-2 if dtype == torch.bfloat16 else 1e-6)
     _check_status()
+
+
+@pytest.mark.parametrize("tokens,heads,H,gap", [(1, 1, 16, 0), (33, 3, 64, 64), (70, 5, 128, 0), (129, 4, 256, 8), (20, 6, 40, 0), (9, 4, 64, 4)])
+def test_rope_widths(tokens, heads, H, gap):
+    """Head groups that are not full, rows that lie apart, and sizes without whole 16-byte pieces (H = 40, a gap of 4)."""
+    k = _k()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x = torch.randn(tokens, heads * H + gap, device="cuda", generator=g).to(torch.bfloat16)
+    v = x[:, :heads * H].unflatten(1, (heads, H))
+    pos = torch.randint(0, 50, (tokens,), device="cuda", generator=g, dtype=torch.int32)
+    ang = torch.randn(50, H // 2, device="cuda", generator=g)
+    c, s = ang.cos()[pos.long()][:, None], ang.sin()[pos.long()][:, None]
+    a, b = v.float()[..., :H // 2], v.float()[..., H // 2:]
+    want, rest = torch.cat([a * c - b * s, b * c + a * s], -1), x[:, heads * H:].clone()
+    k.rope_(v, pos, ang.cos(), ang.sin())
+    assert _rel_err(v, want) < 4e-3 and torch.equal(x[:, heads * H:], rest)
+    _check_status()

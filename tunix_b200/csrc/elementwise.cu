@@ -440,7 +440,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const i
     const int rem = (int)(i - tok * pairs_per_token);
     const int h = rem / (half >> 1);
     const int j = (rem - h * (half >> 1)) * 2;
-    const int p = pos[tok];
+    const int p = max(pos[tok], 0);                        // idle rows carry position -1
     const float2 c = *reinterpret_cast<const float2*>(cos_t + (long long)p * half + j);
     float2 s = *reinterpret_cast<const float2*>(sin_t + (long long)p * half + j);
     s.x *= sign;
@@ -452,6 +452,49 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const i
     *reinterpret_cast<uint32_t*>(base + j) = pack_bf16(a0 * c.x - b0 * s.x, a1 * c.y - b1 * s.y);
     *reinterpret_cast<uint32_t*>(base + half + j) =
         pack_bf16(b0 * c.x + a0 * s.x, b1 * c.y + a1 * s.y);
+  }
+}
+
+// The same with 16-byte accesses: a thread rotates 8 pairs of ROPE_HEADS heads of a token by the same angles. Bound by HBM: x read
+// and written once. B200, before -> after: 16384 x 32 x 128 79 -> 46 us, 4096 x 32 x 128 22 -> 14, 4004 x 16 x 256 21 -> 14.
+constexpr int ROPE_HEADS = 4;
+__global__ void __launch_bounds__(256)
+rope_vec_kernel(__nv_bfloat16* __restrict__ x, long long ld, const int* __restrict__ pos, const float* __restrict__ cos_t,
+                const float* __restrict__ sin_t, unsigned total, int heads, int H, float sign) {
+  const int half = H >> 1;
+  const unsigned vecs = half >> 3, per_token = vecs * ((heads + ROPE_HEADS - 1) / ROPE_HEADS);
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned tok = i / per_token, rem = i - tok * per_token, grp = rem / vecs;
+    const int j = (int)(rem - grp * vecs) << 3, h0 = (int)grp * ROPE_HEADS;
+    __nv_bfloat16* base = x + (long long)tok * ld + (long long)h0 * H + j;
+    uint4 lo[ROPE_HEADS], hi[ROPE_HEADS];
+#pragma unroll
+    for (int h = 0; h < ROPE_HEADS; ++h)
+      if (h0 + h < heads) {
+        lo[h] = *reinterpret_cast<const uint4*>(base + h * H);
+        hi[h] = *reinterpret_cast<const uint4*>(base + h * H + half);
+      }
+    float c[8], s[8];
+    const long long at = (long long)max(pos[tok], 0) * half + j;    // idle rows carry position -1
+#pragma unroll
+    for (int k = 0; k < 8; k += 4) {
+      const float4 cv = *reinterpret_cast<const float4*>(cos_t + at + k), sv = *reinterpret_cast<const float4*>(sin_t + at + k);
+      c[k] = cv.x; c[k + 1] = cv.y; c[k + 2] = cv.z; c[k + 3] = cv.w;
+      s[k] = sv.x * sign; s[k + 1] = sv.y * sign; s[k + 2] = sv.z * sign; s[k + 3] = sv.w * sign;
+    }
+#pragma unroll
+    for (int h = 0; h < ROPE_HEADS; ++h) {
+      if (h0 + h >= heads) break;
+      uint32_t a[4] = {lo[h].x, lo[h].y, lo[h].z, lo[h].w}, b[4] = {hi[h].x, hi[h].y, hi[h].z, hi[h].w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float a0 = bf16_lo(a[k]), a1 = bf16_hi(a[k]), b0 = bf16_lo(b[k]), b1 = bf16_hi(b[k]);
+        a[k] = pack_bf16(a0 * c[2 * k] - b0 * s[2 * k], a1 * c[2 * k + 1] - b1 * s[2 * k + 1]);
+        b[k] = pack_bf16(b0 * c[2 * k] + a0 * s[2 * k], b1 * c[2 * k + 1] + a1 * s[2 * k + 1]);
+      }
+      *reinterpret_cast<uint4*>(base + h * H) = make_uint4(a[0], a[1], a[2], a[3]);
+      *reinterpret_cast<uint4*>(base + h * H + half) = make_uint4(b[0], b[1], b[2], b[3]);
+    }
   }
 }
 
@@ -696,6 +739,14 @@ TB_API int tb_rope(void* x, long long ld, const int* pos, const float* cos_t, co
                    long long tokens, int heads, int H, int backward, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (H % 4) return -2;
+  const long long units = tokens * (H / 16) * ((heads + ROPE_HEADS - 1) / ROPE_HEADS);
+  // whole 16-byte pieces of both halves; a unit's number, and a turn's step beyond the last, fit 32 bits
+  if (H % 16 == 0 && ld % 8 == 0 && units < (1LL << 31) &&
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15) == 0) {
+    rope_vec_kernel<<<grid_for(units, 256), 256, 0, stream>>>((__nv_bfloat16*)x, ld, pos, cos_t, sin_t, (unsigned)units, heads, H,
+                                                              backward ? -1.f : 1.f);
+    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  }
   const long long total = tokens * heads * (H / 4);
   rope_kernel<<<grid_for(total, 256), 256, 0, stream>>>((__nv_bfloat16*)x, ld, pos, cos_t, sin_t,
                                                        tokens, heads, H, backward ? -1.f : 1.f);
