@@ -458,3 +458,15 @@ def test_rope_widths(tokens, heads, H, gap):
     k.rope_(v, pos, ang.cos(), ang.sin())
     assert _rel_err(v, want) < 4e-3 and torch.equal(x[:, heads * H:], rest)
     _check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,off", [(1, 0), (7, 0), (4099, 1), (5_000_003, 0), (5_000_003, 3)])
+def test_sumsq_tails(n, off, dtype):
+    """Lengths that are not whole vectors, and a start that is not aligned to one."""
+    k = _k()
+    x = torch.randn(n + off, device="cuda", generator=torch.Generator(device="cuda").manual_seed(11)).to(dtype)[off:]
+    out = torch.full((1,), 2.0, device="cuda")
+    k.sumsq(x, out)
+    want = 2.0 + x.double().square().sum().item()
+    assert abs(out.item() - want) < 1e-5 * want                # 32-bit partial sums

@@ -5,6 +5,7 @@
 // Replaces the optax update + clip_by_global_norm chain of the reference trainer
 // (tunix/sft/peft_trainer.py:517-548, tunix/cli/config.py:286-378).
 #include "common.cuh"
+#include <algorithm>
 
 using namespace tb;
 
@@ -17,18 +18,38 @@ __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// out[0] += sum(g^2)
+// out[0] += sum(g^2). Bound by HBM: 16-byte loads, eight of a thread in flight, four sums.
+// B200: 654 M bf16 340 -> 189 us (6.9 TB/s), 500 M fp32 318 -> 283.
 template <typename T>
-__global__ void sumsq_kernel(const T* __restrict__ g, long long n, float* __restrict__ out) {
+__global__ void __launch_bounds__(512, 2)
+sumsq_kernel(const T* __restrict__ g, long long n, float* __restrict__ out) {
   __shared__ float red[33];
-  float acc = 0.f;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const float v = to_f<T>(g[i]);
-    acc += v * v;
+  constexpr int W = 16 / sizeof(T);
+  const bool vec = (reinterpret_cast<uintptr_t>(g) & 15) == 0;
+  const long long nv = vec ? n / W : 0, step = (long long)gridDim.x * blockDim.x;
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (long long i = first; i < nv; i += 8 * step) {
+    uint4 q[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      q[u] = i + u * step < nv ? __ldg(reinterpret_cast<const uint4*>(g) + i + u * step) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t w[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if constexpr (sizeof(T) == 4) acc[u & 3] += __uint_as_float(w[k]) * __uint_as_float(w[k]);
+        else acc[u & 3] += bf16_lo(w[k]) * bf16_lo(w[k]) + bf16_hi(w[k]) * bf16_hi(w[k]);
+      }
+    }
   }
-  acc = block_sum(acc, red);
-  if (threadIdx.x == 0) atomicAdd(out, acc);
+  for (long long i = nv * W + first; i < n; i += step) {
+    const float v = to_f<T>(g[i]);
+    acc[0] += v * v;
+  }
+  const float sum = block_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), red);
+  if (threadIdx.x == 0) atomicAdd(out, sum);
 }
 
 struct AdamArgs {
@@ -155,9 +176,9 @@ inline int grid_for(long long n, int block) {
 TB_API int tb_sumsq(const void* g, long long n, int is_bf16, float* out, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (is_bf16)
-    sumsq_kernel<__nv_bfloat16><<<grid_for(n, 512), 512, 0, stream>>>((const __nv_bfloat16*)g, n, out);
+    sumsq_kernel<__nv_bfloat16><<<(int)std::min<long long>(148 * 2, (n + 512 * 8 - 1) / (512 * 8)), 512, 0, stream>>>((const __nv_bfloat16*)g, n, out);
   else
-    sumsq_kernel<float><<<grid_for(n, 512), 512, 0, stream>>>((const float*)g, n, out);
+    sumsq_kernel<float><<<(int)std::min<long long>(148 * 2, (n + 512 * 4 - 1) / (512 * 4)), 512, 0, stream>>>((const float*)g, n, out);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
