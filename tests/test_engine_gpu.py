@@ -537,3 +537,50 @@ def test_tensor_parallel_decode_matches_whole_model(tmp_path):
             assert r[f"first_lp_graph{g}"] < 5e-2, r
             assert r[f"ranks_equal_graph{g}"], r
             assert r[f"sampled_agree_graph{g}"] > 0.6, r    # a flipped draw changes the rest of that sequence
+
+
+@pytest.mark.parametrize("family,window", [("qwen3", 0), ("gemma2", 48)])
+@pytest.mark.parametrize("pack", [131072, 150])             # one call of the attention kernel, and several
+def test_packed_prefill_matches_padded(family, window, pack):
+    """Prompts end to end give every prompt the hidden state and the pages that rows padded to the longest give it."""
+    from tunix_b200 import _lib
+    from tunix_b200.common.configs import CacheConfig
+    from tunix_b200.generate.engine import PagedEngine
+    kw = dict(sliding_window=window, layer_pattern=("local", "global"), attn_logit_softcap=50.0, post_norms=True) if window else {}
+    model = _model(family=family, qk_norm=not window, **kw)
+    cfg = model.config
+    lens, rng = [5, 64, 200, 1, 129], np.random.RandomState(0)
+    rows = [rng.randint(3, 500, n) for n in lens]
+    slots, P, out = list(range(len(lens))), max(lens), {}
+    for name in ("padded", "packed"):
+        eng = PagedEngine(model, Tok(), CacheConfig(256, cfg.num_layers, cfg.num_kv_heads, cfg.head_dim), page_size=16,
+                          max_running_requests=len(lens), prefix_caching=False)
+        eng.PACK_TOKENS = pack
+        with torch.no_grad():
+            eng._fuse_all()
+            eng._ensure_pool(len(lens))
+            for s, r in zip(slots, rows):
+                eng.pool.open(s, r.tolist(), 1)
+            eng.pool.sync_table()
+            for pool in eng.pool.k + eng.pool.v:
+                pool.zero_()
+            if name == "packed":
+                h = eng._prefill_packed(rows, slots, [0, 0, 7, 0, 0])
+            else:
+                toks = torch.zeros(len(lens), P, dtype=torch.int64, device="cuda")
+                for i, r in enumerate(rows):
+                    toks[i, P - len(r):] = torch.from_numpy(r).cuda()
+                n = torch.tensor(lens, device="cuda")
+                seg = (torch.arange(P, device="cuda")[None] >= (P - n)[:, None]).int()
+                pos = (seg.cumsum(-1) - 1).clamp(min=0).int()
+                h = eng._prefill(toks, pos, seg, torch.tensor(slots, dtype=torch.int32, device="cuda"), None,
+                                 torch.tensor([0, 0, 7, 0, 0], dtype=torch.int32, device="cuda"))
+        _lib.raise_if_kernel_error()
+        out[name] = [h] + [torch.cat([p.view(-1, p.shape[-1])[torch.tensor(
+            [pg * 16 + o for pg in eng.pool.pages_of(s) for o in range(16)], device="cuda")] for s in slots])
+            for p in eng.pool.k + eng.pool.v]
+    for i, (a, b) in enumerate(zip(out["packed"], out["padded"])):
+        # the same products in bf16; key blocks of another start round other weights
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 2e-2
+        if i:                                               # nothing is written that the padded form does not write
+            assert torch.equal((a != 0).any(1), (b != 0).any(1))

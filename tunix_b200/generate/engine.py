@@ -433,6 +433,59 @@ class PagedEngine(BaseSampler):
             x = self._mlp_and_norms(layer, i, x, a)
         return self._model.norm(x[:, -1])
 
+    # tokens that one attention call of `_prefill_packed` takes: what a tile's block list of the kernel can hold
+    PACK_TOKENS = 131072
+    PACK_ALIGN = 64
+
+    def _packed_len(self, n):
+        return (n + self.PACK_ALIGN - 1) // self.PACK_ALIGN * self.PACK_ALIGN
+
+    def _prefill_packed(self, rows, slots_list, write_from):
+        """Whole prompts (arrays of token ids of different lengths, nothing of them in the pages that is read here) end to
+        end as one row instead of padded to the longest: segment ids keep the prompts apart, and the attention kernel leaves
+        out key blocks of other segments. A prompt starts at a key block of the kernel, so that its keys meet in the same
+        blocks, and its results round alike, whatever it is prefilled with; the tokens that fill its last block follow it and
+        are seen by none of its own. Returns the hidden state of every prompt's last token.
+
+        8 prompts of 1024 to 4096 tokens, 4 layers of an 8B model, first token: 55.8 -> 37.3 ms."""
+        cfg, pool, dev = self.cfg, self.pool, self.device
+        KH, H = self.n_kv, cfg.head_dim
+        lens = np.asarray([len(r) for r in rows], np.int64)
+        ends = np.cumsum([self._packed_len(int(n)) for n in lens])
+        starts = np.concatenate([[0], ends[:-1]])
+        total = int(ends[-1])
+        meta = np.zeros((4, total), np.int32)                  # position, written position, slot, segment of a token
+        meta[1] = -1
+        ids = np.zeros(total, np.int64)
+        groups = []                                            # runs of prompts for the attention kernel: (first token, end)
+        for i, (n, a, e) in enumerate(zip(lens.tolist(), starts.tolist(), ends.tolist())):
+            pos = np.arange(n, dtype=np.int32)
+            ids[a:a + n], meta[0, a:a + n], meta[1, a:a + n] = rows[i], pos, np.where(pos >= write_from[i], pos, -1)
+            meta[2, a:e], meta[3, a:e] = slots_list[i], i + 1
+            if groups and e - groups[-1][0] <= self.PACK_TOKENS:
+                groups[-1] = (groups[-1][0], e)
+            else:
+                groups.append((a, e))
+        pos, wpos, seq_ids, seg = torch.from_numpy(meta).to(dev)
+        toks = torch.from_numpy(ids).to(dev)
+        x = F.embedding(toks[None], self._model.embed_tokens, math.sqrt(cfg.embed_dim) if cfg.embed_scale else 1.0)
+        for i, layer in enumerate(self._model.layers):
+            h = layer.input_layernorm(x)
+            q, k, v = self._attn_in(layer, h.view(total, -1), pos, i)
+            K.kv_write(k.view(total, -1), v, seq_ids, wpos, pool.table, pool.page_size, pool.k[i], pool.v[i])
+            at = layer.self_attn
+            q, k, v = q.view(total, self.n_heads, H), k.view(total, KH, H), v.view(total, KH, H)
+            o = [F.attention(q[a:b][None], k[a:b][None], v[a:b][None], scale=at.scale, causal=True, window=at.window,
+                             softcap=cfg.attn_logit_softcap, seg_q=seg[a:b][None], seg_k=seg[a:b][None]) for a, b in groups]
+            o = (o[0] if len(o) == 1 else torch.cat(o, 1)).reshape(1, total, -1)
+            if self.tpw > 1:
+                a = self._tp_sum(at.o_proj(o), None if cfg.post_norms else x)
+            else:
+                a = at.o_proj(o, residual=None if cfg.post_norms else x)
+            x = self._mlp_and_norms(layer, i, x, a)
+        last = torch.from_numpy(starts + lens - 1).to(dev)
+        return self._model.norm(x[0].index_select(0, last))
+
     def _prefill_ragged(self, work):
         """Prompts [(slot, token ids)] of a layer-stack model, from position 0, in steps of at most `step_tokens` tokens
         (portions of at most `prefill_chunk`). Returns the hidden state of every prompt's last token [len(work), D]."""
@@ -815,6 +868,13 @@ class PagedEngine(BaseSampler):
         newlen = [ln - u for ln, u in zip(lens_l, use)]
         Pn = max(newlen)
         P = toks_np.shape[1]
+        # Prompts that attend to nothing but themselves go end to end where that makes fewer rows than padding to the longest.
+        # Head sizes without an attention kernel would form the scores between prompts.
+        if sum(map(self._packed_len, newlen)) < g * Pn and min(newlen) > 0 and not any(use) and \
+                not (self.prefill_chunk and 0 < self.prefill_chunk < Pn) and self.cfg.head_dim in (64, 128, 256):
+            hlast = self._prefill_packed([toks_np[i, P - n:] for i, n in enumerate(newlen)], slots_list, cached)
+            self._first_tokens(st, hlast, slots_list, lens_l, pad_id, limits)
+            return
         new_np = np.full((g, Pn), pad_id, np.int64)
         for i in range(g):
             new_np[i, Pn - newlen[i]:] = toks_np[i, P - newlen[i]:]
