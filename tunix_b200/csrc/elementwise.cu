@@ -716,7 +716,8 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
     }
   } else if (D <= 256) {
     const int t = D <= 64 ? 8 : D <= 128 ? 16 : 32;
-    const int grid = grid_for((long long)rows * t, 256 * 4, 148 * 6);
+    // four rows a lane once that fills the SMs
+    const int grid = max(grid_for((long long)rows * t, 256 * 4, 148 * 6), grid_for((long long)rows * t, 256, 148));
     if (t == 8) rmsnorm_bwd_narrow_kernel<8><<<grid, 256, 0, stream>>>(RMS_BWD_ARGS);
     else if (t == 16) rmsnorm_bwd_narrow_kernel<16><<<grid, 256, 0, stream>>>(RMS_BWD_ARGS);
     else rmsnorm_bwd_narrow_kernel<32><<<grid, 256, 0, stream>>>(RMS_BWD_ARGS);
