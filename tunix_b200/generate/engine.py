@@ -195,6 +195,7 @@ class PagedEngine(BaseSampler):
         self.pool: Optional[PagePool] = None
         self._graph = None
         self._graph_key = None
+        self._capture: Optional[tuple] = None       # stream of the captures, and the last decode graph
 
     # ----------------------------------------------------------------- plumbing
     @property
@@ -815,7 +816,7 @@ class PagedEngine(BaseSampler):
             # ---- decode until the next check point; no slot can run past its token limit, which bounds the steps
             # to the next look at the done flags
             if graph is None and self.use_graph and max_steps > 2:
-                graph = self._capture(st)
+                graph = self._capture_step(st)
             running = [s for s in range(B) if slot_req[s] is not None]
             left = [slot_lim[s] - slot_cnt[s] for s in running]
             n_steps = max(1, min(self.check_every, min(left) if source.more_waiting() else max(left)))
@@ -917,7 +918,7 @@ class PagedEngine(BaseSampler):
         st["positions"][ix] = torch.where(done, st["neg1"][ix], lens.to(torch.int32))
         st["seq_lens"][ix] = torch.where(done, st["zero"][ix], (lens + 1).to(torch.int32))
 
-    def _capture(self, st):
+    def _capture_step(self, st):
         """Warm the decode path once outside capture (lazy kernel attribute setup, tensor-map cache), then capture
         one step; the state the warm-up and the capture touched is put back."""
         keys = ("tokens", "positions", "seq_lens", "done", "out_tokens", "out_lp", "out_pos", "step")
@@ -930,9 +931,20 @@ class PagedEngine(BaseSampler):
             st[k].copy_(v)
         torch.cuda.synchronize()
         graph = torch.cuda.CUDAGraph()
-        # thread-local capture: other threads of the process (a trainer, another engine) keep using CUDA meanwhile
-        with torch.cuda.graph(graph, capture_error_mode="thread_local"):
-            self._decode_step(st)
+        # Captured by hand: `torch.cuda.graph` first returns the allocator's cached blocks to the driver, and every call would
+        # pay for freeing and allocating them again. A graph takes the memory pool of the engine's last one, which lives until it
+        # has. Where little memory is left the pool may need the cached blocks.
+        if torch.cuda.mem_get_info(self.device)[0] < 4 << 30:
+            torch.cuda.empty_cache()
+        stream, last = self._capture or (torch.cuda.Stream(self.device), None)
+        with torch.cuda.stream(stream):
+            # thread-local capture: other threads of the process (a trainer, another engine) keep using CUDA meanwhile
+            graph.capture_begin(*(() if last is None else (last.pool(),)), capture_error_mode="thread_local")
+            try:
+                self._decode_step(st)
+            finally:
+                graph.capture_end()
+        self._capture = stream, graph
         for k, v in snap.items():
             st[k].copy_(v)
         return graph
