@@ -584,3 +584,33 @@ def test_packed_prefill_matches_padded(family, window, pack):
         assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 2e-2
         if i:                                               # nothing is written that the padded form does not write
             assert torch.equal((a != 0).any(1), (b != 0).any(1))
+
+
+def test_biased_projections_decode_fused_like_one_by_one(monkeypatch):
+    """q, k and v with biases as one product per layer, before and after the biases were changed from outside."""
+    from tunix_b200 import _lib
+    from tunix_b200.common.configs import CacheConfig
+    from tunix_b200.generate.engine import PagedEngine
+    model = _model(family="qwen2", qk_norm=False, qkv_bias=True, head_dim=64)
+    with torch.no_grad():
+        for layer in model.layers:
+            for proj in (layer.self_attn.q_proj, layer.self_attn.k_proj, layer.self_attn.v_proj):
+                proj.bias.normal_(0, 0.5)
+    cc = CacheConfig(cache_size=128, num_layers=2, num_kv_heads=2, head_dim=64)
+    rng = np.random.default_rng(3)
+    prompts = [[1] + rng.integers(3, 500, size=n).tolist() for n in (9, 30, 17)]
+    call = dict(prompt_token_ids=prompts, max_generation_steps=4, eos_tokens=[-1], return_logprobs=True)
+    fused = PagedEngine(model, Tok(), cc, page_size=16, max_running_requests=3, prefix_caching=False)
+    apart = PagedEngine(model, Tok(), cc, page_size=16, max_running_requests=3, prefix_caching=False)
+    plain = PagedEngine._fused_weight
+    monkeypatch.setattr(apart, "_fused_weight", lambda mods, bias=False: plain(mods))
+    for _ in range(2):
+        a, b = fused(**call), apart(**call)
+        assert all(w is not None for w in fused._wqkv) and all(w is None for w in apart._wqkv)
+        # first tokens come from the prefill, which both share; those behind it from decode steps that round alike up to the
+        # order of bf16 sums
+        for x, y in zip(a.logprobs, b.logprobs):
+            assert abs(x[0] - y[0]) < 1e-6 and abs(x[1] - y[1]) < 5e-2
+        with torch.no_grad():
+            model.layers[0].self_attn.k_proj.bias.add_(1.0)
+    _lib.raise_if_kernel_error()

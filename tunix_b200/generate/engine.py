@@ -195,6 +195,7 @@ class PagedEngine(BaseSampler):
         self.pool: Optional[PagePool] = None
         self._graph = None
         self._graph_key = None
+        self._bqkv: list = []       # per layer: the q, k and v biases end to end, or None
         self._capture: Optional[tuple] = None       # stream of the captures, and the last decode graph
 
     # ----------------------------------------------------------------- plumbing
@@ -215,6 +216,8 @@ class PagedEngine(BaseSampler):
         for name, w in updated_weights.items():
             if own[name].data_ptr() != w.data_ptr():
                 own[name].copy_(w.to(own[name].device, own[name].dtype))
+        if any(b is not None for b in self._bqkv):
+            self._fuse_all()
 
     def delete_cache(self) -> None:
         self.pool = None
@@ -231,13 +234,13 @@ class PagedEngine(BaseSampler):
 
     # ---------------------------------------------------------------- the model
     @staticmethod
-    def _fused_weight(mods):
+    def _fused_weight(mods, bias: bool = False):
         """One [sum(out_i), in] view over the weights of `mods`, so that projections sharing an input run as a
         single GEMM. Weights already back to back in one storage (the optimizer's flat buffer lays q/k/v and
         gate/up out that way) are viewed in place; weights that own their storage are moved, once, into a joint
-        tensor and stay views of it. Anything else (bias, LoRA, quantised base, foreign layout) returns None and
-        the caller runs the projections one by one."""
-        if any(m.quant is not None or m.bias is not None or (m.lora_a is not None and m.lora_enabled) for m in mods):
+        tensor and stay views of it. Anything else (LoRA, quantised base, foreign layout, biases unless the caller adds
+        them: `bias`) returns None and the caller runs the projections one by one."""
+        if any(m.quant is not None or (m.bias is not None and not bias) or (m.lora_a is not None and m.lora_enabled) for m in mods):
             return None
         ws = [m.weight for m in mods]
         cols = ws[0].shape[1]
@@ -270,11 +273,26 @@ class PagedEngine(BaseSampler):
             self.exec.pk = self._pk
             return
         self._wqkv, self._wgu = [], []
+        biases = self._bqkv if len(self._bqkv) == len(self._model.layers) else [None] * len(self._model.layers)
+        self._bqkv = []
         for layer in self._model.layers:
             at = layer.self_attn
-            self._wqkv.append(self._fused_weight([at.q_proj, at.k_proj, at.v_proj]))
+            projs = [at.q_proj, at.k_proj, at.v_proj]
+            biased = all(m.bias is not None for m in projs)
+            self._wqkv.append(self._fused_weight(projs, biased))
+            self._bqkv.append(self._joint_bias(projs, biases[len(self._bqkv)]) if biased and self._wqkv[-1] is not None else None)
             # a mixture-of-experts block keeps its stacked expert weights and runs through the grouped GEMM
             self._wgu.append(None if self.cfg.is_moe else self._fused_weight([layer.mlp.gate_proj, layer.mlp.up_proj]))
+
+    @staticmethod
+    def _joint_bias(mods, have):
+        """The biases of `mods` end to end: a copy, refreshed in place (a captured decode graph reads it) at the start of every
+        call, as the packed weights are."""
+        rows = sum(m.bias.shape[0] for m in mods)
+        if have is None or have.shape[0] != rows or have.dtype != mods[0].bias.dtype:
+            have = torch.empty(rows, dtype=mods[0].bias.dtype, device=mods[0].bias.device)
+        torch.cat([m.bias.detach() for m in mods], out=have)
+        return have
 
     @staticmethod
     def _plain(mod) -> bool:
@@ -530,7 +548,8 @@ class PagedEngine(BaseSampler):
             at = layer.self_attn
             if self._wqkv[i] is not None:
                 pq = self._pk(i, "qkv")
-                qkv = K.gemm_packed(h, pq) if pq is not None else F.linear(h, self._wqkv[i])
+                bq = self._bqkv[i]
+                qkv = K.gemm_packed(h, pq, bias=bq) if pq is not None else F.linear(h, self._wqkv[i], bq)
                 cos, sin = self._rope(i)
                 qn, kn = (at.q_norm, at.k_norm) if cfg.qk_norm else (None, None)
                 K.qkv_post(qkv, st["slots"], pos, qn.weight if qn is not None else None,
