@@ -5,7 +5,7 @@
 // One CTA handles 128 query rows of one head. Five warps:
 //   warps 0..3 : one thread per query row. S is read from TMEM (tcgen05.ld), masked and
 //                exponentiated in registers (row max / row sum are thread-local: no shuffles),
-//                P is written to shared memory in the 128-byte-swizzled K-major layout,
+//                P goes back to TMEM over its scores, as the left operand of P V,
 //                O stays in TMEM and is rescaled there only when a row max grows by > 2^8.
 //   warp 4     : one elected thread issues every TMA load (no multicast) and every
 //                tcgen05.mma: S_{j+1} = Q K_{j+1}^T is in flight while the softmax of block j runs.
@@ -17,9 +17,10 @@
 // Bound by the softmax warps (64 exponentials a row and block share the special-function units with the other CTA of the SM).
 // Segment ids are compared per key block where they decide for the whole of it, and by warp votes elsewhere, not by one load a
 // score; K and V share a ring, so that no product waits for a load issued in its own block. B200, 32 / 8 heads of 128, causal,
-// before -> after: rollouts padded at both ends, 8 x 1024 519 -> 135 us, 16 x 1024 970 -> 245, 8 x 4096 6320 -> 939; packed rows
-// of 777, 14 / 2 heads of 64, 92 -> 31; without segments 2 x 2048 136 -> 95, 8 x 2048 452 -> 397, 1 x 16384 2228 -> 2046;
-// 4 x 1001 with heads of 256 and a soft-cap 265 -> 89.
+// before -> after: rollouts padded at both ends, 8 x 1024 519 -> 140 us, 16 x 1024 970 -> 258, 8 x 4096 6320 -> 920; packed rows
+// of 777, 14 / 2 heads of 64, 92 -> 26; without segments 2 x 2048 136 -> 93, 8 x 2048 452 -> 389, 1 x 16384 2228 -> 1990;
+// 4 x 1001 with heads of 256 and a soft-cap 265 -> 87. P in TMEM instead of shared memory (whose 128 bytes a cycle the operands of
+// S fill otherwise) is 4 to 10 % of it.
 //
 // Replaces the eager [B,N,T,S] attention and the TPU-only splash attention of the reference
 // (tunix/models/llama3/model.py:379-396, tunix/models/qwen3/model.py:607-793,
@@ -74,19 +75,17 @@ struct FwdCfg {
   static constexpr int Q_BYTES = HS * BQ * 128;     // K-major slabs [128 x 128B]
   static constexpr int K_BYTES = HS * BKV * 128;    // slabs [64 x 128B]
   static constexpr int V_BYTES = HVS * BKV * 128;
-  static constexpr int P_BYTES = BQ * 128;
   // A ring of three tiles that K and V share, in the order in which they are read (K0 K1 V0 K2 V1 K3 ...): the load of a K runs
   // a whole block ahead of its product. One buffer each where only that lets a second CTA share the SM.
   static constexpr int SLOT = K_BYTES > V_BYTES ? K_BYTES : V_BYTES;
-  static constexpr int FIXED = Q_BYTES + P_BYTES + 128 + 1024;
+  static constexpr int FIXED = Q_BYTES + 128 + 1024;
   static constexpr bool RING = FIXED + 3 * SLOT <= 113 * 1024 || FIXED + K_BYTES + V_BYTES > 113 * 1024;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_K = OFF_Q + Q_BYTES;
   static constexpr int OFF_V = OFF_K + K_BYTES;                       // not RING
-  static constexpr int OFF_P = OFF_K + (RING ? 3 * SLOT : K_BYTES + V_BYTES);
-  static constexpr int OFF_BAR = OFF_P + P_BYTES;
+  static constexpr int OFF_BAR = OFF_K + (RING ? 3 * SLOT : K_BYTES + V_BYTES);
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
-  static constexpr int TMEM_S = 0;                  // two S buffers of 64 columns
+  static constexpr int TMEM_S = 0;                  // two S buffers of 64 columns; P takes the first 32 of its S
   static constexpr int TMEM_O = 128;
   static constexpr int TMEM_COLS = (128 + HV) <= 256 ? 256 : 512;
 };
@@ -101,7 +100,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sptr = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t sQ = sbase + C_::OFF_Q, sK = sbase + C_::OFF_K, sV = sbase + C_::OFF_V,
-                 sP = sbase + C_::OFF_P, bars = sbase + C_::OFF_BAR;
+                 bars = sbase + C_::OFF_BAR;
   // barriers: 0 Q, 1-3 ring (or 1 K, 2 V), 4-5 S[2], 6 P, 7 PV
   const uint32_t barQ = bars, barK = bars + 8, barV = bars + 16, barS0 = bars + 32,
                  barP = bars + 48, barPV = bars + 56;
@@ -266,9 +265,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint32_t vb = v_tile(j);
 #pragma unroll
         for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint64_t ad = make_smem_desc(sP + kk * 32, 16, 1024);
           const uint64_t bd = make_smem_desc(vb + kk * 2048, BKV * 128, 1024);
-          umma_f16_ss(tmem + C_::TMEM_O, ad, bd, idesc_o, (j | kk) != 0);
+          umma_f16_ts(tmem + C_::TMEM_O, tmem + C_::TMEM_S + (j & 1) * BKV + kk * 8, bd, idesc_o, (j | kk) != 0);
         }
         umma_commit(barPV);
       }
@@ -383,7 +381,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       l = l * alpha + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
       if (j > 0) {
-        // PV_{j-1} retired: P buffer reusable and O consistent
+        // PV_{j-1} retired: O consistent
         if (!mbar_wait_bounded(barPV, (j - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
         tc_fence_after();
         if (warp_need) {
@@ -399,14 +397,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_st_wait();
         }
       }
-      // P row -> smem, K-major 128-byte swizzle: 16-byte chunk c of row r lands at c ^ (r & 7)
-      uint8_t* prow = sptr + C_::OFF_P + r * 128;
+      // P row -> TMEM, two weights a column, over the scores that it comes from
+      {
+        uint32_t lo[16], hi[16];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint4 v = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-        *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = v;
+        for (int i = 0; i < 16; ++i) { lo[i] = pk[i]; hi[i] = pk[16 + i]; }
+        tmem_st_32x16(tmem + lane_addr + C_::TMEM_S + (j & 1) * BKV, lo);
+        tmem_st_32x16(tmem + lane_addr + C_::TMEM_S + (j & 1) * BKV + 16, hi);
+        tmem_st_wait();
       }
-      fence_proxy_async_smem();
       tc_fence_before();
       mbar_arrive(barP);
     }
