@@ -51,7 +51,7 @@ struct BwdCfg {
   static constexpr int NHALF = H / HO;
   static constexpr int NST = PIPE ? 3 : 1;          // Q / dO tile stages
   static constexpr int NDS = PIPE ? 2 : 1;          // dSt staging buffers
-  static constexpr int SEG_BLOCKS = 2048;           // query tiles that the list can hold; longer ranges are walked without one
+  static constexpr int SEG_BLOCKS = PIPE ? 2048 : 64;       // query tiles that the list can hold (what shared memory leaves)
   static constexpr int KV_BYTES = HS * BK_ * 128;
   static constexpr int Q_BYTES = HS * BQ_ * 128;
   static constexpr int P_BYTES = BK_ * 128;
@@ -59,12 +59,12 @@ struct BwdCfg {
   static constexpr int OFF_V = OFF_K + KV_BYTES;
   static constexpr int OFF_Q = OFF_V + KV_BYTES;
   static constexpr int OFF_DO = OFF_Q + NST * Q_BYTES;
-  static constexpr int OFF_DST = OFF_DO + NST * Q_BYTES;
+  static constexpr int OFF_PT = OFF_DO + NST * Q_BYTES;
+  static constexpr int OFF_DST = OFF_PT + P_BYTES;
   static constexpr int OFF_STAT = OFF_DST + NDS * P_BYTES;   // [3][2][64] lse and delta of three query tiles
   static constexpr int OFF_BAR = OFF_STAT + 3 * 2 * 64 * 4;
   static constexpr int SMEM_BYTES = OFF_BAR + 192 + 1024;
-  // TMEM columns: St (two buffers if PIPE), dPt, dQt, dV, dK. Each half of St's columns, which one thread of a row reads, holds that
-  // thread's bf16 Pt in its first quarter-buffer and dSt in the next: the left operands of dV and dK.
+  // TMEM columns: St (two buffers if PIPE), dPt, dQt, dV, dK
   static constexpr int TM_DPT = PIPE ? 128 : 64;
   static constexpr int TM_DQT = TM_DPT + 64;
   static constexpr int TM_DV = TM_DQT + 64;
@@ -73,11 +73,13 @@ struct BwdCfg {
   __host__ __device__ static constexpr int tm_st(int it) { return PIPE ? (it & 1) * 64 : 0; }
 };
 
-// Bound by the chain S -> P -> dS -> dK / dQ of one CTA an SM (512 TMEM columns, 192 KB), of which the products are 1280 cycles
+// Bound by the chain S -> P -> dS -> dK / dQ of one CTA an SM (512 TMEM columns, 208 KB), of which the products are 1280 cycles
 // a tile at the tensor cores' rate. B200, 32 / 8 heads of 128, causal, the whole backward (with delta and the fp32 dQ passes),
-// before -> after these roles, this schedule and the order of the grid: 2 x 2048 546 -> 266 us, 8 x 2048 1546 -> 1135,
-// 1 x 16384 8569 -> 6350; rollouts padded at both ends 8 x 1024 864 -> 361; packed rows 3 x 777 with 14 / 2 heads of 64 375 -> 112;
-// 4 x 1001, 16 / 8 heads of 256, soft-cap 610 -> 356. Pt and dSt as operands in TMEM instead of shared memory are 3 to 18 % of it.
+// before -> after these roles, this schedule and the order of the grid: 2 x 2048 546 -> 297 us, 8 x 2048 1546 -> 1214,
+// 1 x 16384 8569 -> 6750; rollouts padded at both ends 8 x 1024 864 -> 406; packed rows 3 x 777 with 14 / 2 heads of 64 375 -> 112;
+// 4 x 1001, 16 / 8 heads of 256, soft-cap 610 -> 385. Pt and dSt as operands in TMEM were tried: 1 x 16384 6759 -> 6585 us, heads of 64
+// 239 -> 260 and packed rows 112 -> 128 (a vote before each store to TMEM, and a barrier of the issuer's: row warps wait for dV of the
+// tile before ahead of Pt, or one that is ahead arrives twice for a tile).
 //
 // Roles: row threads (P and dS), four warps that add dQt to dQ and fetch lse / delta of later tiles, one issuer.
 // Schedule (PIPE): St runs two query tiles ahead and dPt of the next tile is the first product behind dSt, so the row threads go
@@ -92,7 +94,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const BwdArgs a) {
   using C_ = BwdCfg<H>;
   constexpr int CW_ = BQ_ / RG_;           // query columns per row thread
-  static_assert(CW_ == 32, "a thread's Pt and dSt take the 32 columns of its scores");
   constexpr int NROW_ = 128 * RG_;         // row threads per CTA (plus the issuer warp)
   constexpr int HO = C_::HO;
   constexpr int NST = C_::NST;
@@ -101,12 +102,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sptr = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t sK = sbase + C_::OFF_K, sV = sbase + C_::OFF_V, sQ = sbase + C_::OFF_Q,
-                 sdO = sbase + C_::OFF_DO, sdSt = sbase + C_::OFF_DST,
+                 sdO = sbase + C_::OFF_DO, sPt = sbase + C_::OFF_PT, sdSt = sbase + C_::OFF_DST,
                  bars = sbase + C_::OFF_BAR;
   // barriers (8 bytes each): 0 KV | 1-3 Q[3] | 4-6 Qfree[3] | 7-8 St[2] | 9 dPt | 10 Pt | 11 dSt | 12 dQ | 13 dQ drained |
-  //                          15-17 stats[3] ; tmem slot + abort flag ; 20 everything retired
+  //                          14 dV | 15-17 stats[3] ; tmem slot + abort flag ; 20 everything retired
   const uint32_t barKV = bars, barQ0 = bars + 8, barQF0 = bars + 32, barSt0 = bars + 56, bardPt = bars + 72,
-                 barPt = bars + 80, bardSt = bars + 88, bardQ = bars + 96, barDQfree = bars + 104,
+                 barPt = bars + 80, bardSt = bars + 88, bardQ = bars + 96, barDQfree = bars + 104, bardV = bars + 112,
                  barStat0 = bars + 120, barDone = bars + 160;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sptr + C_::OFF_BAR + 144);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sptr + C_::OFF_BAR + 148);
@@ -165,6 +166,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(barSt0 + 8 * s, 1);
     }
     mbar_init(bardPt, 1);
+    mbar_init(bardV, 1);
     mbar_init(barDone, 1);
     mbar_init(barPt, NROW_);
     mbar_init(bardSt, NROW_);
@@ -227,17 +229,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint32_t do_s = sdO + (it % NST) * C_::Q_BYTES;
 #pragma unroll
         for (int kk = 0; kk < BQ_ / 16; ++kk) {
+          const uint64_t ad = make_smem_desc(sPt + kk * 32, 16, 1024);
           const uint64_t bd = make_smem_desc(do_s + col_off + kk * 2048, BQ_ * 128, 1024);
-          umma_f16_ts(tmem + C_::TM_DV, tmem + C_::tm_st(it) + (kk >> 1) * 32 + (kk & 1) * 8, bd, idesc_dv, (it | kk) != 0);
+          umma_f16_ss(tmem + C_::TM_DV, ad, bd, idesc_dv, (it | kk) != 0);
         }
+        umma_commit(bardV);
       };
       // dK += dSt Q
       auto issue_dk = [&](int it) {
         const uint32_t q_s = sQ + (it % NST) * C_::Q_BYTES;
+        const uint32_t ds = sdSt + (PIPE ? (it & 1) : 0) * C_::P_BYTES;
 #pragma unroll
         for (int kk = 0; kk < BQ_ / 16; ++kk) {
+          const uint64_t ad = make_smem_desc(ds + kk * 32, 16, 1024);
           const uint64_t bd = make_smem_desc(q_s + col_off + kk * 2048, BQ_ * 128, 1024);
-          umma_f16_ts(tmem + C_::TM_DK, tmem + C_::tm_st(it) + 16 + (kk >> 1) * 32 + (kk & 1) * 8, bd, idesc_dv, (it | kk) != 0);
+          umma_f16_ss(tmem + C_::TM_DK, ad, bd, idesc_dv, (it | kk) != 0);
         }
       };
       // dQt = K^T dS^T
@@ -449,10 +455,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
         }
       }
-      tmem_st_32x16(tmem + lane_addr + C_::tm_st(it) + c0, pk);
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(barPt);
+      // dV of the tile before has read the buffer of Pt (without PIPE it retired before this tile's St)
+      if (PIPE && it >= 1) BWD_WAIT(bardV, (it - 1) & 1, ST_TIMEOUT_EPILOGUE);
+      {
+        uint8_t* prow = sptr + C_::OFF_PT + r * 128;
+#pragma unroll
+        for (int c = 0; c < CW_ / 8; ++c)
+          *reinterpret_cast<uint4*>(prow + (((c + c0 / 8) ^ (r & 7)) << 4)) =
+              make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+        fence_proxy_async_smem();
+        tc_fence_before();
+        mbar_arrive(barPt);
+      }
       BWD_WAIT(bardPt, it & 1, ST_TIMEOUT_EPILOGUE);
       tc_fence_after();
       {
@@ -463,22 +477,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // (dSt of the tile before last was read by products that retired before this dPt)
         uint8_t* drow = sptr + C_::OFF_DST + (PIPE ? (it & 1) : 0) * C_::P_BYTES + r * 128;
 #pragma unroll
-        for (int i = 0; i < CW_ / 2; ++i) {
-          float d[2];
+        for (int c = 0; c < CW_ / 8; ++c) {
+          float d[8];
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float dp = __uint_as_float(t[i >> 4][(2 * i + e) & 31]);
-            d[e] = p[2 * i + e] * (dp - st_delta[2 * i + e]) * a.scale;
+          for (int e = 0; e < 8; ++e) {
+            const int i = 8 * c + e;
+            const float dp = __uint_as_float(t[i >> 5][i & 31]);
+            d[e] = p[i] * (dp - st_delta[i]) * a.scale;
           }
-          pk[i] = pack_bf16(d[0], d[1]);
+          uint4 v;
+          v.x = pack_bf16(d[0], d[1]);
+          v.y = pack_bf16(d[2], d[3]);
+          v.z = pack_bf16(d[4], d[5]);
+          v.w = pack_bf16(d[6], d[7]);
+          *reinterpret_cast<uint4*>(drow + (((c + c0 / 8) ^ (r & 7)) << 4)) = v;
         }
-        tmem_st_32x16(tmem + lane_addr + C_::tm_st(it) + c0 + 16, pk);
-        // the right operand of dQt
-#pragma unroll
-        for (int c = 0; c < CW_ / 8; ++c)
-          *reinterpret_cast<uint4*>(drow + (((c + c0 / 8) ^ (r & 7)) << 4)) =
-              make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-        tmem_st_wait();
         fence_proxy_async_smem();
         tc_fence_before();
         mbar_arrive(bardSt);

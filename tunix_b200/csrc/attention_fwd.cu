@@ -17,10 +17,10 @@
 // Bound by the softmax warps (64 exponentials a row and block share the special-function units with the other CTA of the SM).
 // Segment ids are compared per key block where they decide for the whole of it, and by warp votes elsewhere, not by one load a
 // score; K and V share a ring, so that no product waits for a load issued in its own block. B200, 32 / 8 heads of 128, causal,
-// before -> after: rollouts padded at both ends, 8 x 1024 519 -> 140 us, 16 x 1024 970 -> 258, 8 x 4096 6320 -> 920; packed rows
-// of 777, 14 / 2 heads of 64, 92 -> 26; without segments 2 x 2048 136 -> 93, 8 x 2048 452 -> 389, 1 x 16384 2228 -> 1990;
-// 4 x 1001 with heads of 256 and a soft-cap 265 -> 87. P in TMEM instead of shared memory (whose 128 bytes a cycle the operands of
-// S fill otherwise) is 4 to 10 % of it.
+// before -> after: rollouts padded at both ends, 8 x 1024 519 -> 143 us, 16 x 1024 970 -> 264, 8 x 4096 6320 -> 984; packed rows
+// of 777, 14 / 2 heads of 64, 92 -> 26; without segments 2 x 2048 136 -> 96, 8 x 2048 452 -> 391, 1 x 16384 2228 -> 2011;
+// 4 x 1001 with heads of 256 and a soft-cap 265 -> 94. P in TMEM instead of shared memory (whose 128 bytes a cycle the operands of
+// S fill otherwise) is 2 to 5 % of it.
 //
 // Replaces the eager [B,N,T,S] attention and the TPU-only splash attention of the reference
 // (tunix/models/llama3/model.py:379-396, tunix/models/qwen3/model.py:607-793,
@@ -307,7 +307,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           seg_bits(seg, k0 + 32, a.Tk, my_seg, keep[1]);
         }
       }
-      if (!mbar_wait_bounded(barS0 + 8 * (j & 1), (j >> 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
+      // a failed wait is acted upon at the next vote of the warp
+      const bool here = mbar_wait_bounded(barS0 + 8 * (j & 1), (j >> 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
       tc_fence_after();
       uint32_t sraw[64];
       {
@@ -380,9 +381,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         pk[i] = pack_bf16(p0, p1);
       }
       l = l * alpha + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
+      // PV_{j-1} retired: O consistent (and the issuer has seen all of P_{j-1})
+      ok = __all_sync(0xffffffffu, here && (j == 0 || mbar_wait_bounded(barPV, (j - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)));
+      if (!ok) break;
       if (j > 0) {
-        // PV_{j-1} retired: O consistent
-        if (!mbar_wait_bounded(barPV, (j - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
         tc_fence_after();
         if (warp_need) {
 #pragma unroll 1
@@ -411,7 +413,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     // ------------------------------------------------------------- epilogue
     if (ok && nblk > 0)
-      ok = mbar_wait_bounded(barPV, (nblk - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
+      ok = mbar_wait_warp(barPV, (nblk - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
     tc_fence_after();
     const int vd = PAGED ? a.vd : HV;
     float inv_l = (l > 0.f) ? 1.f / l : 0.f;

@@ -108,6 +108,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
+// The same for all lanes of a warp, with one answer. Lanes may leave the polls apart, and where a failed wait leaves the caller's loop
+// the compiler has no earlier place to bring them together again; what follows may be a `.sync.aligned` instruction.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code));
+}
+
 // --------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* tm, uint32_t bar,
                                             int x, int y) {
