@@ -196,3 +196,24 @@ def test_segments_past_the_block_list():
     _lib.raise_if_kernel_error()
     ref = ref_attention(q, k, v, 0.125, False, 0, 0.0, seg_q, seg_k)
     assert _rel(o, ref) < 2e-2
+
+
+@pytest.mark.parametrize("H", [64, 128])
+def test_gradients_of_rollouts_repeat(H):
+    """Rows padded at both ends make the warps of a block run apart (they fetch segment ids on their own): what the kernels sum in a
+    fixed order is the same bit for bit in every run."""
+    from tunix_b200 import _lib
+    from tunix_b200.ops import kernels as k_
+    B, T, N, KH = 8, 1024, 16, 4
+    q, k, v, _, _ = _make(B, T, T, N, KH, H, False)
+    do = torch.randn(B, T, N, H, device="cuda", dtype=torch.bfloat16)
+    at = torch.arange(T, device="cuda")[None]
+    seg = ((at >= 23 * torch.arange(B, device="cuda")[:, None]) & (at < T - 61 * torch.arange(B, device="cuda")[:, None])).int().contiguous()
+    first = None
+    for _ in range(40):
+        o, lse = k_.attn_fwd(q, k, v, scale=H ** -0.5, seg_q=seg, seg_k=seg)
+        _, dk, dv = k_.attn_bwd(do, q, k, v, o, lse, scale=H ** -0.5, seg_q=seg, seg_k=seg)
+        got = (o, lse, dk, dv)
+        first = first or [t.clone() for t in got]
+        assert all(torch.equal(a, b) for a, b in zip(got, first))
+    _lib.raise_if_kernel_error()
