@@ -77,9 +77,10 @@ struct BwdCfg {
 // a tile at the tensor cores' rate. B200, 32 / 8 heads of 128, causal, the whole backward (with delta and the fp32 dQ passes),
 // before -> after these roles, this schedule and the order of the grid: 2 x 2048 546 -> 297 us, 8 x 2048 1546 -> 1214,
 // 1 x 16384 8569 -> 6750; rollouts padded at both ends 8 x 1024 864 -> 406; packed rows 3 x 777 with 14 / 2 heads of 64 375 -> 112;
-// 4 x 1001, 16 / 8 heads of 256, soft-cap 610 -> 385. Pt and dSt as operands in TMEM were tried: 1 x 16384 6759 -> 6585 us, heads of 64
-// 239 -> 260 and packed rows 112 -> 128 (a vote before each store to TMEM, and a barrier of the issuer's: row warps wait for dV of the
-// tile before ahead of Pt, or one that is ahead arrives twice for a tile).
+// 4 x 1001, 16 / 8 heads of 256, soft-cap 610 -> 385. Pt and dSt as operands in TMEM were tried: 1 x 16384 6759 -> 6585 us and
+// 2 x 2048 290 -> 276, but no gain beyond what runs differ by at 8 x 2048, in packed rows or with heads of 64, once a vote before each
+// store to TMEM and a barrier of the issuer's were added (the row warps' wait for dV of the tile before is also what keeps one that is
+// ahead from arriving twice for a tile).
 //
 // Roles: row threads (P and dS), four warps that add dQt to dQ and fetch lse / delta of later tiles, one issuer.
 // Schedule (PIPE): St runs two query tiles ahead and dPt of the next tile is the first product behind dSt, so the row threads go
@@ -114,10 +115,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   float* s_stat = reinterpret_cast<float*>(sptr + C_::OFF_STAT);
 
   const int warp = threadIdx.x >> 5;
-  const int kt = blockIdx.z;               // heavy (early) causal tiles of all heads and rows first: a last wave of light ones
-  const int half = (C_::NHALF > 1) ? (blockIdx.x % C_::NHALF) : 0;
-  const int kvh = blockIdx.x / C_::NHALF;
-  const int b = blockIdx.y;
+  // heavy (early) causal tiles of all heads and rows first: a last wave of light ones
+  const unsigned heads = (unsigned)a.KH * C_::NHALF, head = blockIdx.x % heads;
+  const int kt = blockIdx.x / (heads * a.B);
+  const int half = (C_::NHALF > 1) ? (head % C_::NHALF) : 0;
+  const int kvh = head / C_::NHALF;
+  const int b = blockIdx.x / heads % a.B;
   const int G = a.N / a.KH;
   const int k0 = kt * BK_;
 
@@ -614,7 +617,9 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* dout, co
   if (once.first() &&
       cudaFuncSetAttribute(attn_bwd_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM_BYTES) != cudaSuccess)
     return -5;
-  dim3 grid(a.KH * C_::NHALF, a.B, (a.Tk + BK_ - 1) / BK_);
+  const long long ctas = (long long)a.KH * C_::NHALF * a.B * ((a.Tk + BK_ - 1) / BK_);
+  if (ctas > 0x7fffffffLL) return -2;
+  const dim3 grid((unsigned)ctas);
   attn_bwd_kernel<H><<<grid, 128 * RG_ + 160, C_::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -109,8 +109,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int warp = threadIdx.x >> 5;
   // heavy (late) causal tiles of all heads and rows first: a last wave of light ones
-  const int qt = PAGED ? gridDim.x - 1 - blockIdx.x : gridDim.z - 1 - blockIdx.z;
-  const int n = PAGED ? blockIdx.y : blockIdx.x, b = PAGED ? 0 : blockIdx.y;
+  const int qt = PAGED ? gridDim.x - 1 - blockIdx.x : (a.Tq + BQ - 1) / BQ - 1 - blockIdx.x / ((unsigned)a.N * a.B);
+  const int n = PAGED ? blockIdx.y : blockIdx.x % a.N, b = PAGED ? 0 : blockIdx.x / a.N % a.B;
   const int kvh = n / (a.N / a.KH);
   // the tile's first row in Q and O, its valid rows, the position of its first query, the keys of its sequence
   int row0, nrows, i0, Tk;
@@ -472,7 +472,9 @@ int launch_fwd(const void* q, const void* k, const void* v, const AttnArgs& a, l
   if (once.first() &&
       cudaFuncSetAttribute(attn_fwd_kernel<H, H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM_BYTES) != cudaSuccess)
     return -5;
-  dim3 grid(a.N, a.B, (a.Tq + BQ - 1) / BQ);
+  const long long ctas = (long long)a.N * a.B * ((a.Tq + BQ - 1) / BQ);
+  if (ctas > 0x7fffffffLL) return -2;
+  const dim3 grid((unsigned)ctas);
   attn_fwd_kernel<H, H, false><<<grid, 160, C_::SMEM_BYTES, stream>>>(tq, tk, tv, tk, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
