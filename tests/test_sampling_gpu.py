@@ -102,3 +102,22 @@ def test_values_that_are_not_finite(value):
             assert tok[0].item() != 77
         if value == float("-inf"):
             assert tok[1].item() == 0
+
+
+@pytest.mark.parametrize("temp", [1e-4, 1e-5, 1e-6, 1e-7])
+@pytest.mark.parametrize("top_k,top_p", [(1, None), (50, 0.95), (None, 0.95), (None, 0.9999), (3000, 0.5)])
+def test_filtered_draws_at_low_temperatures(temp, top_k, top_p):
+    """z / temperature up to 4e8, where the rounding of a product is many nats: no weight lies above the best token's, which leads by
+    more than the draw's noise and is always the one, and log-probs are those of 64 bits. Rows on 1, 2, 4 and 8 thread blocks."""
+    from tunix_b200.ops import sampling_kernels as S
+    for V, B in ((5000, 40), (9000, 40), (151936, 300), (151936, 60), (151936, 5)):
+        g = torch.Generator(device="cuda").manual_seed(B)
+        z = torch.rand(B, V, device="cuda", generator=g) * 30 + 9.9
+        best = torch.randint(0, V, (B,), device="cuda", generator=g)
+        # the others end at 39.9: at least 0.1 / 1e-4 nats of lead against 23 of noise
+        z.scatter_(1, best[:, None], 40 + torch.rand(B, 1, device="cuda", generator=g))
+        tok, lp = S.sample(z, temp, top_p, top_k, seed=3, step=1, want_logprob=True)
+        assert torch.equal(tok, best), (V, B)
+        want = torch.log_softmax(z.double() / torch.tensor(temp, dtype=torch.float32).item(), -1).gather(1, best[:, None])[:, 0]
+        # a weight's exponent is off by 2^-23 of itself, which nothing within 20 nats of the best token sees; sums as above
+        assert (lp - want).abs().max().item() < 1e-4, (V, B)

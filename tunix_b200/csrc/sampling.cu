@@ -202,7 +202,7 @@ sample_kernel(float* __restrict__ logits, long long ld, int V, float inv_temp, i
   };
   float all[8][2];
   // Best candidate of the whole cluster -> the row's result, then the barrier before any CTA may leave.
-  auto finish = [&](ArgMax best, float m, float log_s) {
+  auto finish = [&](ArgMax best, auto&& log_prob) {
     best = block_amax(best, sh.s_v, sh.s_i);
     if (tid == 0) {
       sh.pv = best.v;
@@ -216,7 +216,7 @@ sample_kernel(float* __restrict__ logits, long long ld, int V, float inv_temp, i
       }
       const int tok = best.i < V ? best.i : 0;
       tokens[row] = tok;
-      if (logprobs) logprobs[row] = z[tok] * inv_temp - m - log_s;
+      if (logprobs) logprobs[row] = log_prob(z[tok]);
     }
     csync();
   };
@@ -258,21 +258,25 @@ sample_kernel(float* __restrict__ logits, long long ld, int V, float inv_temp, i
     float m = -INFINITY, s = 0.f;
     for (int r = 0; r < C; ++r) m = fmaxf(m, all[r][0]);
     for (int r = 0; r < C; ++r) s += all[r][0] == -INFINITY ? 0.f : all[r][1] * __expf(all[r][0] - m);
-    finish(best, m, logf(s));
+    const float log_s = logf(s);
+    finish(best, [&](float v) { return v * inv_temp - m - log_s; });
     return;
   }
 
   float lm = -INFINITY;
-  walk([&](int, float v) { lm = fmaxf(lm, v * inv_temp); });
+  walk([&](int, float v) { lm = fmaxf(lm, v); });
   for (int b = tid; b < BINS; b += nt) sh.hist[b] = 0;
   if (tid == 0) sh.ncand = 0;
   lm = block_max(lm, sh.red);
   exchange(lm, 0.f, all);                               // and rank 0's histogram is clear
-  float m = -INFINITY;
-  for (int r = 0; r < C; ++r) m = fmaxf(m, all[r][0]);
+  float top = -INFINITY;
+  for (int r = 0; r < C; ++r) top = fmaxf(top, all[r][0]);
+  const float m = __fmul_rn(top, inv_temp);
   const bool finite = fabsf(m) < INFINITY;
   constexpr float PER = BINS / BIN_SPAN;
-  auto below = [&](float v) { return fmaf(v, inv_temp, -m); };      // log of a token's weight, one rounding
+  // Log of a token's weight: the difference to the largest logit, then the scale. It is never positive, so that a bin is never
+  // negative and no weight above 1; the product first would leave its rounding, half an ulp of m: 110 bins at a temperature of 1e-6.
+  auto below = [&](float v) { return __fmul_rn(__fadd_rn(v, -top), inv_temp); };
   float ls = 0.f;
   walk([&](int, float v) {
     const float x = below(v);
@@ -398,7 +402,7 @@ sample_kernel(float* __restrict__ logits, long long ld, int V, float inv_temp, i
         if (tid == 0) {
           const int tok = best.i < V ? best.i : 0;
           tokens[row] = tok;
-          if (logprobs) logprobs[row] = z[tok] * inv_temp - m - log_s;
+          if (logprobs) logprobs[row] = below(z[tok]) - log_s;
         }
       } else if (tid == 0) {
         sh.cut = by_p ? -1 : -2;                        // the list is too short; or the threshold is 0 and all are drawn from
@@ -486,7 +490,7 @@ sample_kernel(float* __restrict__ logits, long long ld, int V, float inv_temp, i
       best = amax(best, ArgMax{zi - __logf(-__logf(u01(rr[j]))), i4 + j});
     }
   }
-  finish(best, m, log_s);
+  finish(best, [&](float v) { return below(v) - log_s; });
 }
 
 // CTAs per row: up to 8, as long as the grid is one wave of two CTAs an SM. More CTAs shorten every pass over the row; past
