@@ -121,3 +121,37 @@ def test_filtered_draws_at_low_temperatures(temp, top_k, top_p):
         want = torch.log_softmax(z.double() / torch.tensor(temp, dtype=torch.float32).item(), -1).gather(1, best[:, None])[:, 0]
         # a weight's exponent is off by 2^-23 of itself, which nothing within 20 nats of the best token sees; sums as above
         assert (lp - want).abs().max().item() < 1e-4, (V, B)
+
+
+@pytest.mark.parametrize("temp", [0.6, 0.9, 1.0, 1.3])
+@pytest.mark.parametrize("weights,top_k,top_p,n_kept,crowd", [
+    ((1.0, 0.97), 2, None, 2, None), ((0.9, 0.4, 0.3, 0.25, 0.2, 0.1), 5, None, 5, None),
+    ((0.9, 0.1), None, 0.95, 2, None), ((0.55, 0.3, 0.15), None, 0.8, 2, None), ((0.55, 0.3, 0.15), None, 0.9, 3, None),
+    ((0.5, 0.3, 0.2), 3, 0.75, 2, None),
+    # more candidates than the list holds, so that the halvings run over the row: behind the k-th token in its own bin, or of no weight
+    ((1.0, 0.8, 0.6), 3, None, 3, (0.594, 0.599)), ((0.5, 0.3, 0.2), 2500, 0.75, 2, (1e-6, 2e-6))])
+def test_every_kept_token_is_drawn(weights, top_k, top_p, n_kept, crowd, temp):
+    """The k-th token, or the one that completes the mass, comes as often as its weight says, at any rounding of z / temperature."""
+    from tunix_b200.ops import sampling_kernels as S
+    rows, draws, V = 256, 128, 16384
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w = torch.tensor(weights, dtype=torch.float64, device="cuda")
+    base = torch.rand(rows, 1, device="cuda", generator=g, dtype=torch.float64) * 20 + 10
+    z = torch.full((rows, V), -60.0, dtype=torch.float64, device="cuda")
+    at = torch.rand(rows, V, device="cuda", generator=g).argsort(-1)
+    z.scatter_(1, at[:, :len(weights)], base + temp * w.log())
+    if crowd:
+        c = torch.linspace(*crowd, 3000, dtype=torch.float64, device="cuda")
+        z.scatter_(1, at[:, len(weights):len(weights) + 3000], base + temp * c.log())
+    z = z.float()
+    kept = at[:, :n_kept]
+    p = (z.double().gather(1, kept) / temp).softmax(-1)
+    n = torch.zeros(rows, V, device="cuda")
+    for step in range(draws):
+        tok, _ = S.sample(z, temp, top_p, top_k, seed=17, step=step)
+        n[torch.arange(rows, device="cuda"), tok] += 1
+    n = n.gather(1, kept)
+    assert (n.sum(1) == draws).all()                          # nothing else is drawn
+    # counts of independent draws: 6 standard deviations over at most 1280 of them
+    assert ((n - draws * p).abs() <= 6 * (draws * p * (1 - p)).sqrt()).all()
+    assert ((n.sum(0) - draws * p.sum(0)).abs() <= 5 * (draws * (p * (1 - p)).sum(0)).sqrt()).all()
