@@ -332,6 +332,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
       if (ok) umma_commit(barDone);
+#undef BWD_WAIT
     }
   } else if (warp >= 4 * RG_) {
     // ------------------------------------------- dQ and the row statistics
@@ -363,7 +364,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     bool ok = true;
     for (int it = 0; it < nit && ok; ++it) {
       if (it + 3 < nit) fetch(v_lse, v_delta);
-      BWD_WAIT(bardQ, it & 1, ST_TIMEOUT_EPILOGUE);
+      if (!mbar_wait_warp(bardQ, it & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
       if (it + 3 < nit) {                  // dQt of this tile is there: its dS is, and nobody reads its statistics any more
         put(it + 3, v_lse, v_delta);
@@ -422,8 +423,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
 
-      BWD_WAIT(barStat0 + 8 * (it % 3), (it / 3) & 1, ST_TIMEOUT_EPILOGUE);
-      BWD_WAIT(barSt0 + (PIPE ? 8 * (it & 1) : 0), (PIPE ? it >> 1 : it) & 1, ST_TIMEOUT_EPILOGUE);
+      // One answer for a warp ahead of the aligned loads from TMEM, and before anybody leaves the loop: the votes over segment ids
+      // above need every lane.
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(barStat0 + 8 * (it % 3), (it / 3) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE) &&
+                                       mbar_wait_bounded(barSt0 + (PIPE ? 8 * (it & 1) : 0), (PIPE ? it >> 1 : it) & 1, abort_flag,
+                                                         a.status, ST_TIMEOUT_EPILOGUE));
+      if (!ok) break;
       tc_fence_after();
       float p[CW_];
       uint32_t pk[CW_ / 2];
@@ -459,7 +464,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
       // dV of the tile before has read the buffer of Pt (without PIPE it retired before this tile's St)
-      if (PIPE && it >= 1) BWD_WAIT(bardV, (it - 1) & 1, ST_TIMEOUT_EPILOGUE);
+      bool free = true;                    // a failed wait is acted upon at the next vote
+      if (PIPE && it >= 1) free = mbar_wait_bounded(bardV, (it - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
       {
         uint8_t* prow = sptr + C_::OFF_PT + r * 128;
 #pragma unroll
@@ -470,7 +476,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc_fence_before();
         mbar_arrive(barPt);
       }
-      BWD_WAIT(bardPt, it & 1, ST_TIMEOUT_EPILOGUE);
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(bardPt, it & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE) && free);
+      if (!ok) break;
       tc_fence_after();
       {
         uint32_t t[CW_ / 32][32];
@@ -501,8 +508,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       if (it + 1 < nit) next_tile(w);
     }
-    if (nit > 0 && ok) ok = mbar_wait_bounded(barDone, 0, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
-#undef BWD_WAIT
+    if (nit > 0 && ok) ok = mbar_wait_warp(barDone, 0, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
     // ------------------------------------------------------------- dK / dV
     tc_fence_after();
     __nv_bfloat16* dkrow = a.dK + ((long long)b * a.Tk + kp) * a.lddk + (long long)kvh * H + half * HO;

@@ -701,7 +701,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     bool ok = true;
     for (int i = 0; i < nx && ok; ++i) {
       const int j = lo_x + i;
-      if (!mbar_wait_bounded(barS + 8 * (i & 1), (i >> 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
+      // one answer for a warp: votes and aligned accesses to TMEM follow every wait
+      if (!mbar_wait_warp(barS + 8 * (i & 1), (i >> 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
       uint32_t sraw[32];
       tmem_ld_32x32(tmem + lane_addr + C_::tm_s(x, i & 1) + half * 32, sraw);
@@ -746,7 +747,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       float* slot = s_mx + (((i & 1) * 2 + x) * 2) * 128;
       slot[half * 128 + r] = mx;
       mbar_arrive(barX);
-      if (!mbar_wait_bounded(barX, i & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
+      if (!mbar_wait_warp(barX, i & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
       mx = fmaxf(mx, slot[(half ^ 1) * 128 + r]);
       float alpha = 1.f;
       bool need = false;
@@ -778,7 +779,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       l = l * alpha + ((p0s + p1s) + (p2s + p3s));
       if (i > 0) {
         // PV(i-1) retired: P buffer reusable and O consistent
-        if (!mbar_wait_bounded(barPV, (i - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
+        if (!mbar_wait_warp(barPV, (i - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
         tc_fence_after();
         if (warp_need) {
 #pragma unroll 1
@@ -805,13 +806,13 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_arrive(barP);
     }
     // ------------------------------------------------------------- epilogue
-    if (ok && nx > 0) ok = mbar_wait_bounded(barPV, (nx - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
+    if (ok && nx > 0) ok = mbar_wait_warp(barPV, (nx - 1) & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
     tc_fence_after();
     // the row sum is the two halves' shares together
     float* lslot = s_mx + ((nx & 1) * 2 + x) * 2 * 128;
     lslot[half * 128 + r] = l;
     mbar_arrive(barX);
-    if (ok) ok = mbar_wait_bounded(barX, nx & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
+    if (ok) ok = mbar_wait_warp(barX, nx & 1, abort_flag, a.status, ST_TIMEOUT_EPILOGUE);
     if (ok) l += lslot[(half ^ 1) * 128 + r];
     const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
     __nv_bfloat16* orow = a.O + ((long long)b * a.Tq + qi) * a.ldo + (long long)n * H + half * HH;

@@ -108,8 +108,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
-// The same for all lanes of a warp, with one answer. Lanes may leave the polls apart, and where a failed wait leaves the caller's loop
-// the compiler has no earlier place to bring them together again; what follows may be a `.sync.aligned` instruction.
+// The same for all lanes of a warp, with one answer. Lanes give up one by one (each reads its own clock and the abort flag on its own),
+// and a lane that left the caller's loop never comes to the votes, shuffles and barriers of a warp that follow: the others would wait
+// for it without a limit. Lanes may also leave the polls apart, and where a failed wait leaves the loop the compiler has no earlier place
+// to bring them together again; what follows may be a `.sync.aligned` instruction.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code));
 }

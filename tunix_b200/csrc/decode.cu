@@ -242,7 +242,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     if (TMA) {
       // the buffer of tile + STAGES - 1 was read in the previous iteration, which ended with a barrier
       if (tid == 0 && tile + STAGES - 1 < n_tiles) issue_tma(tile + STAGES - 1, (tile + STAGES - 1) % STAGES);
-      if (!mbar_wait_bounded(smem_u32(&full_bars[buf]), (tile / STAGES) & 1, &abort_flag, status, ST_TIMEOUT_PRODUCER)) break;
+      if (!mbar_wait_warp(smem_u32(&full_bars[buf]), (tile / STAGES) & 1, &abort_flag, status, ST_TIMEOUT_PRODUCER)) break;
     } else {
       if (tile + 1 < n_tiles) {
         issue(tile + 1, buf ^ 1);

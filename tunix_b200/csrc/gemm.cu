@@ -306,7 +306,7 @@ __device__ void reducer_role(const ReduceArgs& ra, int rank, int world, int N, i
       const int c = c_first + q / world, s = q % world;
       if (tid == 0) issue_upto(q + NBUF);
       const int b = (int)(consumed % NBUF);
-      if (!mbar_wait_bounded(full(b), (ph_full >> b) & 1u, abort_flag, status, ST_TIMEOUT_EPILOGUE)) return;
+      if (!mbar_wait_warp(full(b), (ph_full >> b) & 1u, abort_flag, status, ST_TIMEOUT_EPILOGUE)) return;
       ph_full ^= 1u << b;
       ++consumed;
       const uint8_t* buf = smem_al + b * PIECE;
@@ -610,8 +610,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int M = td.m_end;                       // shadows the problem's M: rows of this tile that exist
       const long long c_off = td.c_off;
       const bool empty_k = td.kb1 <= td.kb0;        // nothing was accumulated: the tile's value is zero
-      if (!empty_k && !mbar_wait_bounded(tfull_bar(acc), acc_phase, abort_flag, args.status,
-                                         ST_TIMEOUT_EPILOGUE)) {
+      if (!empty_k && !mbar_wait_warp(tfull_bar(acc), acc_phase, abort_flag, args.status,
+                                      ST_TIMEOUT_EPILOGUE)) {
         ok = false;
         break;
       }

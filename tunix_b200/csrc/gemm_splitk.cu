@@ -152,7 +152,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const int r = q * 32 + lane;
     const bool have = kb_end > kb_begin;
     bool ok = true;
-    if (have) ok = mbar_wait_bounded(tfull_bar, 0, abort_flag, args.status, ST_TIMEOUT_EPILOGUE);
+    if (have) ok = mbar_wait_warp(tfull_bar, 0, abort_flag, args.status, ST_TIMEOUT_EPILOGUE);
     tc_fence_after();
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
