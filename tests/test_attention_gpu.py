@@ -217,3 +217,23 @@ def test_gradients_of_rollouts_repeat(H):
         first = first or [t.clone() for t in got]
         assert all(torch.equal(a, b) for a, b in zip(got, first))
     _lib.raise_if_kernel_error()
+
+
+def test_backward_past_32768_query_tiles():
+    """More query tiles than the block numbers of a segment list count: every query meets the keys once."""
+    from tunix_b200 import _lib
+    from tunix_b200.ops import kernels as k_
+    Tq, Tk, H = 64 * 32768 + 130, 40, 64
+    q, k, v, _, _ = _make(1, Tq, Tk, 1, 1, H, False)
+    do = torch.randn(1, Tq, 1, H, device="cuda", dtype=torch.bfloat16)
+    kw = dict(scale=H ** -0.5, causal=False)
+    o, lse = k_.attn_fwd(q, k, v, **kw)
+    dq, dk, dv = k_.attn_bwd(do, q, k, v, o, lse, **kw)
+    _lib.raise_if_kernel_error()
+    qf, kf, vf, df = (t[0, :, 0].float() for t in (q, k, v, do))
+    p = (qf @ kf.T * H ** -0.5).softmax(-1)
+    ds = p * (df @ vf.T - (df * (p @ vf)).sum(-1, keepdim=True)) * H ** -0.5
+    # the bounds of the tests above
+    for name, got, want in (("dq", dq, ds @ kf), ("dk", dk, ds.T @ qf), ("dv", dv, p.T @ df)):
+        assert _rel(got[0, :, 0], want) < 3e-2, (name, _rel(got[0, :, 0], want))
+    assert _rel(dq[0, -130:, 0], (ds @ kf)[-130:]) < 3e-2

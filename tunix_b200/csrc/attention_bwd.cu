@@ -141,8 +141,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     bool same;                             // the ids of keys and queries are all one
   };
   auto tile_at = [&](Walk& w) {
-    const int e = listed ? s_list.id[w.i] : w.i;
-    w.base = (qt0 + (e & SEG_ID)) * BQ_;
+    const int e = listed ? s_list.id[w.i] : 0;             // without a list a tile's number has no mark, and may take more than 15 bits
+    w.base = (qt0 + (listed ? e & SEG_ID : w.i)) * BQ_;
     w.same = listed && (e & SEG_SAME);
   };
   auto first_tile = [&] {
