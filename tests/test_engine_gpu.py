@@ -614,3 +614,28 @@ def test_biased_projections_decode_fused_like_one_by_one(monkeypatch):
         with torch.no_grad():
             model.layers[0].self_attn.k_proj.bias.add_(1.0)
     _lib.raise_if_kernel_error()
+
+
+def test_deleted_cache_gives_the_decode_graph_back():
+    """No private memory pool of the engine outlives `delete_cache`; captures before and after it give the same tokens."""
+    import gc
+    from tunix_b200.common.configs import CacheConfig
+    from tunix_b200.generate.engine import PagedEngine
+
+    def pools():
+        gc.collect()
+        torch.cuda.empty_cache()
+        return {s["segment_pool_id"] for s in torch.cuda.memory_snapshot()}
+
+    model = _model()
+    before = pools()
+    eng = PagedEngine(model, Tok(), CacheConfig(128, 2, 2, model.config.head_dim), page_size=16, max_running_requests=2)
+    call = dict(prompt_token_ids=[[1, 5, 9, 4], [1, 7]], max_generation_steps=12, eos_tokens=[-1])
+    outs = []
+    for _ in range(3):
+        outs += [eng(**call).tokens, eng(**call).tokens]
+        assert pools() - before
+        eng.delete_cache()
+        assert not pools() - before
+        eng.reinitialize_cache()
+    assert all(all(np.array_equal(a, b) for a, b in zip(o, outs[0])) for o in outs)

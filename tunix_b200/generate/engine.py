@@ -193,10 +193,8 @@ class PagedEngine(BaseSampler):
         self.preemptions = 0
         self.forbidden: Optional[torch.Tensor] = None
         self.pool: Optional[PagePool] = None
-        self._graph = None
-        self._graph_key = None
         self._bqkv: list = []       # per layer: the q, k and v biases end to end, or None
-        self._capture: Optional[tuple] = None       # stream of the captures, and the last decode graph
+        self._capture: Optional[tuple] = None       # stream of the captures, and the last decode graph (until `delete_cache`)
 
     # ----------------------------------------------------------------- plumbing
     @property
@@ -220,8 +218,10 @@ class PagedEngine(BaseSampler):
             self._fuse_all()
 
     def delete_cache(self) -> None:
+        """Gives back the device memory that the engine keeps from call to call: the pages, and the last decode graph with its
+        memory pool."""
         self.pool = None
-        self._graph = None
+        self._capture = None
 
     def reinitialize_cache(self) -> None:
         self._ensure_pool(self.max_running)
@@ -329,7 +329,6 @@ class PagedEngine(BaseSampler):
             # gated activation (no [rows, 2F] intermediate, no separate activation kernel)
             self._packed = [{name: (K.PackedWeight(w, glu=(name == "gu" and w.shape[0] % 32 == 0)) if w is not None else None)
                              for name, w in src.items()} for src in srcs]
-            self._graph = None          # a captured graph points at the old buffers
             return
         for have, src in zip(self._packed, srcs):
             for name, w in src.items():
