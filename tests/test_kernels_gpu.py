@@ -470,3 +470,19 @@ def test_sumsq_tails(n, off, dtype):
     k.sumsq(x, out)
     want = 2.0 + x.double().square().sum().item()
     assert abs(out.item() - want) < 1e-5 * want                # 32-bit partial sums
+
+
+@pytest.mark.parametrize("D", [8, 128, 264, 4096, 16392])
+def test_rmsnorm_weight_gradient_alone(D):
+    """Without dx the entry point asks for no weight and no 16-byte alignment of x and dy."""
+    from tunix_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(12)
+    rows, ld = 37, D + 6
+    x, dy = (torch.randn(rows * ld + 2, device="cuda", generator=g).to(torch.bfloat16)[2:].view(rows, ld)[:, :D] for _ in range(2))
+    assert x.data_ptr() % 16 == 4
+    rstd = torch.rand(rows, device="cuda", generator=g) + 0.5
+    dw = torch.zeros(D, device="cuda")
+    rc = _lib.cuda().tb_rmsnorm_bwd(dy.data_ptr(), ld, x.data_ptr(), ld, 0, rstd.data_ptr(), 0, 0, dw.data_ptr(), rows, D, 0.0, 0,
+                                    _lib.stream_ptr())
+    assert rc == 0
+    assert _rel_err(dw, (dy.double() * x.double() * rstd.double()[:, None]).sum(0)) < 1e-5      # 32-bit sums over the rows

@@ -206,7 +206,7 @@ rmsnorm_bwd_narrow_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, 
 #pragma unroll
       for (int o = T / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
       dot *= inv_d;
-      if (r < rows && in && dx) {
+      if (r < rows && in) {
         float o[8];
         if (accumulate) load8(dx + r * lddx + col, o);
 #pragma unroll
@@ -311,7 +311,6 @@ rmsnorm_bwd_row_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, con
     dot = 0.f;
     for (int i = 0; i < nw; ++i) dot += red[grp][turn][i];
     dot *= inv_d;
-    if (!dx) continue;
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       if (col(j) >= D) continue;
@@ -354,7 +353,7 @@ rmsnorm_bwd_row_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, con
   }
 }
 
-// The same in two kernels, for rows too wide for the registers of a block.
+// The same in two kernels, for rows too wide for the registers of a block and for dw alone (x and dy 4-byte aligned, no w).
 __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy,
                                       const __nv_bfloat16* __restrict__ x, long long ldx,
                                       const __nv_bfloat16* __restrict__ w,
@@ -698,11 +697,11 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
   if (D % 8) return -2;
   if (!dx && !dw) return 0;
   // up to 256 columns by lanes of a warp, up to 16384 by threads of a block; the SMs are filled once, so that the sums over columns
-  // meet in few atomics
+  // meet in few atomics. dw alone needs no weight and no rows of 16-byte pieces: that call keeps the kernel for wide rows.
 #define RMS_BWD_ARGS                                                                                                          \
   (const __nv_bfloat16*)dy, lddy, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, rstd, (__nv_bfloat16*)dx, lddx, dw, rows, D, \
       add_one, accumulate_dx
-  const bool wide = D > 16384 || (D > 256 && (reinterpret_cast<uintptr_t>(dw) & 15));
+  const bool wide = !dx || D > 16384 || (D > 256 && (reinterpret_cast<uintptr_t>(dw) & 15));
   if (wide) {
     const int block = 256;
     if (dx)
