@@ -237,3 +237,18 @@ def test_backward_past_32768_query_tiles():
     for name, got, want in (("dq", dq, ds @ kf), ("dk", dk, ds.T @ qf), ("dv", dv, p.T @ df)):
         assert _rel(got[0, :, 0], want) < 3e-2, (name, _rel(got[0, :, 0], want))
     assert _rel(dq[0, -130:, 0], (ds @ kf)[-130:]) < 3e-2
+
+
+@pytest.mark.parametrize("H,off,gap", [(128, 0, 0), (128, 2, 0), (64, 0, 2), (96, 0, 0), (30, 2, 6)])
+def test_delta_rows(H, off, gap):
+    """Row sums of dO * O of rows without whole 16-byte pieces, and of head sizes that the attention kernels do not take."""
+    from tunix_b200 import _lib
+    B, T, N = 2, 37, 3
+    g = torch.Generator(device="cuda").manual_seed(13)
+    ld = N * H + gap
+    o, do = (torch.randn(B * T * ld + off, device="cuda", generator=g).to(torch.bfloat16)[off:].view(B, T, ld)[..., :N * H] for _ in range(2))
+    delta = torch.empty(B, N, T, device="cuda")
+    rc = _lib.cuda().tb_attn_delta(o.data_ptr(), ld, do.data_ptr(), ld, delta.data_ptr(), B, T, N, H, _lib.stream_ptr())
+    assert rc == 0
+    want = (o.double() * do.double()).unflatten(-1, (N, H)).sum(-1).transpose(1, 2)
+    assert ((delta.double() - want).norm() / want.norm()).item() < 1e-6          # 32-bit sums of up to 128 terms

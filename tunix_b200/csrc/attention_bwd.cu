@@ -592,11 +592,35 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long ldo, const __nv
   }
 }
 
+// The same by pairs, a warp a row, for rows that are not whole 16-byte pieces and other head sizes.
+__global__ void attn_delta_pairs_kernel(const __nv_bfloat16* __restrict__ o, long long ldo, const __nv_bfloat16* __restrict__ dout,
+                                        long long lddo, float* __restrict__ delta, int B, int T, int N, int H) {
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const long long total = (long long)B * T * N;
+  for (long long w = (long long)blockIdx.x * warps + (threadIdx.x >> 5); w < total; w += (long long)gridDim.x * warps) {
+    const long long bt = w / N, n = w - bt * N, b = bt / T;
+    const __nv_bfloat16 *po = o + bt * ldo + n * H, *pd = dout + bt * lddo + n * H;
+    float acc = 0.f;
+    for (int c = lane * 2; c < H; c += 64) {
+      const uint32_t x = *reinterpret_cast<const uint32_t*>(po + c), y = *reinterpret_cast<const uint32_t*>(pd + c);
+      acc += bf16_lo(x) * bf16_lo(y) + bf16_hi(x) * bf16_hi(y);
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) delta[(b * N + n) * T + (bt - b * T)] = acc;
+  }
+}
+
 int launch_delta(const void* o, long long ldo, const void* dout, long long lddo, float* delta, int B, int T, int N, int H,
                  cudaStream_t stream) {
   const long long total = (long long)B * T * N;
   if (total <= 0) return 0;
-  if (ldo % 8 || lddo % 8 || ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15)) return -2;
+  const bool vec = ldo % 8 == 0 && lddo % 8 == 0 && ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15) == 0;
+  if (!vec || (H != 64 && H != 128 && H != 256)) {
+    const long long blocks = (total + 7) / 8;
+    attn_delta_pairs_kernel<<<(int)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, stream>>>(
+        (const __nv_bfloat16*)o, ldo, (const __nv_bfloat16*)dout, lddo, delta, B, T, N, H);
+    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  }
   auto run = [&](auto kernel, int per) {
     const long long blocks = (total + 2 * per - 1) / (2 * per);
     kernel<<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream>>>((const __nv_bfloat16*)o, ldo, (const __nv_bfloat16*)dout, lddo,
@@ -605,8 +629,7 @@ int launch_delta(const void* o, long long ldo, const void* dout, long long lddo,
   const bool small = total < (1LL << 30);             // row numbers, and what a turn adds to them, in 32 bits
   if (H == 64) small ? run(attn_delta_kernel<64, uint32_t>, 32) : run(attn_delta_kernel<64, long long>, 32);
   else if (H == 128) small ? run(attn_delta_kernel<128, uint32_t>, 16) : run(attn_delta_kernel<128, long long>, 16);
-  else if (H == 256) small ? run(attn_delta_kernel<256, uint32_t>, 8) : run(attn_delta_kernel<256, long long>, 8);
-  else return -2;
+  else small ? run(attn_delta_kernel<256, uint32_t>, 8) : run(attn_delta_kernel<256, long long>, 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -742,7 +765,7 @@ TB_API int tb_attn_bwd_noalloc(const void* q, const void* k, const void* v, cons
   const long long ldq = (long long)N * H, ldkv = (long long)KH * H;
   // The scratch keeps the previous call's contents: the dQ accumulator must start at zero.
   noalloc_zero_kernel<<<592, 256, 0, stream>>>(dq32, dq_elems);
-  if (int rc = launch_delta(o, ldq, dout, ldq, delta, B, Tq, N, H, stream)) return noalloc_fail(rc, "row sums: bad alignment or launch");
+  if (int rc = launch_delta(o, ldq, dout, ldq, delta, B, Tq, N, H, stream)) return noalloc_fail(rc, "row sums: launch failed");
   BwdArgs a;
   a.B = B; a.Tq = Tq; a.Tk = Tk; a.N = N; a.KH = KH;
   a.scale = scale; a.softcap = softcap; a.causal = causal; a.window = window; a.q_off = Tk - Tq;
