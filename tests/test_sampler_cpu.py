@@ -333,3 +333,18 @@ def test_openai_front_end_routes_conversations_over_several_engines():
     finally:
         for e in engines.values():
             e.close()
+
+
+def test_joint_bias_follows_its_model():
+    """The engine's copy of the q, k and v biases is refreshed in place, and made anew where the model has moved or changed its type."""
+    from types import SimpleNamespace
+    from tunix_b200.generate.engine import PagedEngine
+    mods = [SimpleNamespace(bias=torch.nn.Parameter(torch.randn(n))) for n in (8, 4, 4)]
+    have = PagedEngine._joint_bias(mods, None)
+    with torch.no_grad():
+        mods[1].bias.add_(1.0)
+    again = PagedEngine._joint_bias(mods, have)
+    assert again is have and torch.equal(have, torch.cat([m.bias for m in mods]))
+    for other in (have.to("meta"), have.double(), have[:8].clone()):
+        moved = PagedEngine._joint_bias(mods, other)
+        assert moved.device.type == "cpu" and torch.equal(moved, have)

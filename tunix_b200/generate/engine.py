@@ -288,9 +288,9 @@ class PagedEngine(BaseSampler):
     def _joint_bias(mods, have):
         """The biases of `mods` end to end: a copy, refreshed in place (a captured decode graph reads it) at the start of every
         call, as the packed weights are."""
-        rows = sum(m.bias.shape[0] for m in mods)
-        if have is None or have.shape[0] != rows or have.dtype != mods[0].bias.dtype:
-            have = torch.empty(rows, dtype=mods[0].bias.dtype, device=mods[0].bias.device)
+        rows, like = sum(m.bias.shape[0] for m in mods), mods[0].bias
+        if have is None or (have.shape[0], have.dtype, have.device) != (rows, like.dtype, like.device):
+            have = torch.empty(rows, dtype=like.dtype, device=like.device)
         torch.cat([m.bias.detach() for m in mods], out=have)
         return have
 
