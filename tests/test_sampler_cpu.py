@@ -348,3 +348,35 @@ def test_joint_bias_follows_its_model():
     for other in (have.to("meta"), have.double(), have[:8].clone()):
         moved = PagedEngine._joint_bias(mods, other)
         assert moved.device.type == "cpu" and torch.equal(moved, have)
+
+
+def test_packed_prompts_share_short_attention_calls():
+    """An attention call reads segment ids with the square of its tokens: no run of several prompts is longer than 16384 of them, every
+    prompt starts at a key block and lies in one run."""
+    from tunix_b200.generate.engine import PagedEngine
+    eng = PagedEngine.__new__(PagedEngine)
+    rng = np.random.default_rng(0)
+    for lens in ([1], [5, 64, 65, 1], rng.integers(1, 300, 900).tolist(), [20000, 3, 16384, 16000, 500, 40000, 7]):
+        n, starts, ends, groups = eng._pack_layout(lens)
+        assert n.tolist() == list(lens) and (starts % 64 == 0).all() and starts[0] == 0 and (starts[1:] == ends[:-1]).all()
+        assert ((ends - starts >= n) & (ends - starts < n + 64)).all()
+        assert groups[0][0] == 0 and groups[-1][1] == ends[-1] and all(a[1] == b[0] for a, b in zip(groups, groups[1:]))
+        for a, b in groups:
+            inside = [i for i in range(len(lens)) if a <= starts[i] < b]
+            assert starts[inside[0]] == a and ends[inside[-1]] == b and (b - a <= 16384 or len(inside) == 1)
+
+
+def test_prompts_of_like_lengths_stay_padded():
+    """End to end only where that leaves out more than a tenth of the rows: the segment ids cost more than a few rows."""
+    from types import SimpleNamespace
+    from tunix_b200.generate.engine import PagedEngine
+    eng, routes = PagedEngine.__new__(PagedEngine), []
+    eng.cfg = SimpleNamespace(head_dim=64)
+    eng.exec, eng.prefill_chunk, eng.pool, eng.device = None, 0, SimpleNamespace(page_size=16), torch.device("cpu")
+    eng._prefill_packed = lambda *a: routes.append("packed")
+    eng._prefill = lambda *a: routes.append("padded")
+    eng._first_tokens = lambda *a: None
+    for lens in ([256] * 7 + [192], [256, 250, 240, 256], [256, 64, 100, 200], [1000, 10]):
+        toks = np.ones((len(lens), max(lens)), np.int64)
+        eng._admit({}, list(range(len(lens))), toks, np.asarray(lens), 0, [1] * len(lens))
+    assert routes == ["padded", "padded", "packed", "packed"]

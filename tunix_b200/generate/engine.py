@@ -451,12 +451,33 @@ class PagedEngine(BaseSampler):
             x = self._mlp_and_norms(layer, i, x, a)
         return self._model.norm(x[:, -1])
 
-    # tokens that one attention call of `_prefill_packed` takes: what a tile's block list of the kernel can hold
-    PACK_TOKENS = 131072
+    # Tokens that one attention call of `_prefill_packed` takes, unless a single prompt has more: every tile of the kernel reads the
+    # segment ids of all tokens in front of it, which short prompts do not pay back. 512 prompts of 128 to 256 tokens, us a layer,
+    # 14 heads of 64 / 32 of 128, in calls of 131072, 32768, 16384, 8192, 4096 tokens: 1992, 822, 649, 614, 1063 / 4612, 1900, 1507,
+    # 1375, 1411 (padded 368 / 1134).
+    PACK_TOKENS = 16384
+    # Rows end to end that pay for those reads, as a share of the padded ones. Padded -> packed, ms, for 14 heads of 64 and 896 columns
+    # (4 layers), where a row costs least: 768 to 1024 tokens, share 0.90, 21.3 -> 21.2; 128 to 256, 0.89, 20.0 -> 19.6; 64 to 256, 0.74,
+    # 20.5 -> 17.1; 192 to 256, 0.99, 19.8 -> 22.3. 32 heads of 128 and 4096 columns (2 layers): 0.99 110 -> 111, 0.89 111 -> 96.
+    PACK_SHARE = 0.9
     PACK_ALIGN = 64
 
     def _packed_len(self, n):
         return (n + self.PACK_ALIGN - 1) // self.PACK_ALIGN * self.PACK_ALIGN
+
+    def _pack_layout(self, lens):
+        """Prompts of these lengths end to end: their lengths, first tokens and ends, and the runs of prompts that one attention
+        call takes, (first token, end)."""
+        lens = np.asarray(lens, np.int64)
+        ends = np.cumsum(self._packed_len(lens))
+        starts = np.concatenate([[0], ends[:-1]])
+        groups = []
+        for a, e in zip(starts.tolist(), ends.tolist()):
+            if groups and e - groups[-1][0] <= self.PACK_TOKENS:
+                groups[-1] = (groups[-1][0], e)
+            else:
+                groups.append((a, e))
+        return lens, starts, ends, groups
 
     def _prefill_packed(self, rows, slots_list, write_from):
         """Whole prompts (arrays of token ids of different lengths, nothing of them in the pages that is read here) end to
@@ -465,36 +486,31 @@ class PagedEngine(BaseSampler):
         blocks, and its results round alike, whatever it is prefilled with; the tokens that fill its last block follow it and
         are seen by none of its own. Returns the hidden state of every prompt's last token.
 
-        8 prompts of 1024 to 4096 tokens, 4 layers of an 8B model, first token: 55.8 -> 37.3 ms."""
+        8 prompts of 1024 to 4096 tokens, 2 layers of an 8B model, padded -> packed: 54 -> 34 ms."""
         cfg, pool, dev = self.cfg, self.pool, self.device
         KH, H = self.n_kv, cfg.head_dim
-        lens = np.asarray([len(r) for r in rows], np.int64)
-        ends = np.cumsum([self._packed_len(int(n)) for n in lens])
-        starts = np.concatenate([[0], ends[:-1]])
-        total = int(ends[-1])
-        meta = np.zeros((4, total), np.int32)                  # position, written position, slot, segment of a token
-        meta[1] = -1
-        ids = np.zeros(total, np.int64)
-        groups = []                                            # runs of prompts for the attention kernel: (first token, end)
-        for i, (n, a, e) in enumerate(zip(lens.tolist(), starts.tolist(), ends.tolist())):
-            pos = np.arange(n, dtype=np.int32)
-            ids[a:a + n], meta[0, a:a + n], meta[1, a:a + n] = rows[i], pos, np.where(pos >= write_from[i], pos, -1)
-            meta[2, a:e], meta[3, a:e] = slots_list[i], i + 1
-            if groups and e - groups[-1][0] <= self.PACK_TOKENS:
-                groups[-1] = (groups[-1][0], e)
-            else:
-                groups.append((a, e))
-        pos, wpos, seq_ids, seg = torch.from_numpy(meta).to(dev)
-        toks = torch.from_numpy(ids).to(dev)
+        lens, starts, ends, groups = self._pack_layout([len(r) for r in rows])
+        total, fill = int(ends[-1]), np.zeros(self.PACK_ALIGN, np.int64)
+        toks = torch.from_numpy(np.concatenate([t for r, n in zip(rows, ends - starts - lens) for t in (r, fill[:n])])).to(dev)
+        # per prompt -> per token: position, written position, slot, segment
+        per = torch.from_numpy(np.stack([starts, lens, np.asarray(write_from, np.int64), np.asarray(slots_list, np.int64), ends - starts])).to(dev)
+        row = torch.repeat_interleave(torch.arange(len(rows), device=dev), per[4], output_size=total)
+        at, n, w, seq_ids = per[:4].index_select(1, row).to(torch.int32)
+        pos = torch.arange(total, dtype=torch.int32, device=dev) - at
+        real = pos < n
+        wpos = pos.masked_fill(~real | (pos < w), -1)
+        pos, seg = pos.masked_fill(~real, 0), (row + 1).to(torch.int32)
+        seg = [seg[None, a:b] for a, b in groups]
         x = F.embedding(toks[None], self._model.embed_tokens, math.sqrt(cfg.embed_dim) if cfg.embed_scale else 1.0)
         for i, layer in enumerate(self._model.layers):
             h = layer.input_layernorm(x)
             q, k, v = self._attn_in(layer, h.view(total, -1), pos, i)
             K.kv_write(k.view(total, -1), v, seq_ids, wpos, pool.table, pool.page_size, pool.k[i], pool.v[i])
             at = layer.self_attn
-            q, k, v = q.view(total, self.n_heads, H), k.view(total, KH, H), v.view(total, KH, H)
-            o = [F.attention(q[a:b][None], k[a:b][None], v[a:b][None], scale=at.scale, causal=True, window=at.window,
-                             softcap=cfg.attn_logit_softcap, seg_q=seg[a:b][None], seg_k=seg[a:b][None]) for a, b in groups]
+            q, k, v = q.view(1, total, self.n_heads, H), k.view(1, total, KH, H), v.view(1, total, KH, H)
+            qkv = [(q, k, v)] if len(groups) == 1 else [tuple(t[0, a:b][None] for t in (q, k, v)) for a, b in groups]
+            o = [F.attention(*t, scale=at.scale, causal=True, window=at.window, softcap=cfg.attn_logit_softcap, seg_q=s, seg_k=s)
+                 for t, s in zip(qkv, seg)]
             o = (o[0] if len(o) == 1 else torch.cat(o, 1)).reshape(1, total, -1)
             if self.tpw > 1:
                 a = self._tp_sum(at.o_proj(o), None if cfg.post_norms else x)
@@ -887,9 +903,9 @@ class PagedEngine(BaseSampler):
         newlen = [ln - u for ln, u in zip(lens_l, use)]
         Pn = max(newlen)
         P = toks_np.shape[1]
-        # Prompts that attend to nothing but themselves go end to end where that makes fewer rows than padding to the longest.
+        # Prompts that attend to nothing but themselves go end to end where that makes clearly fewer rows than padding to the longest.
         # Head sizes without an attention kernel would form the scores between prompts.
-        if sum(map(self._packed_len, newlen)) < g * Pn and min(newlen) > 0 and not any(use) and \
+        if sum(map(self._packed_len, newlen)) <= self.PACK_SHARE * g * Pn and min(newlen) > 0 and not any(use) and \
                 not (self.prefill_chunk and 0 < self.prefill_chunk < Pn) and self.cfg.head_dim in (64, 128, 256):
             hlast = self._prefill_packed([toks_np[i, P - n:] for i, n in enumerate(newlen)], slots_list, cached)
             self._first_tokens(st, hlast, slots_list, lens_l, pad_id, limits)
