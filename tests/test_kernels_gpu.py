@@ -486,3 +486,26 @@ def test_rmsnorm_weight_gradient_alone(D):
                                     _lib.stream_ptr())
     assert rc == 0
     assert _rel_err(dw, (dy.double() * x.double() * rstd.double()[:, None]).sum(0)) < 1e-5      # 32-bit sums over the rows
+
+
+@pytest.mark.parametrize("gap,off", [(0, 0), (4, 0), (3, 0), (4, 1)])
+@pytest.mark.parametrize("M,N", [(2048, 1536), (1999, 1560), (2311, 1533)])
+def test_scaled_sums_into_fp32(M, N, gap, off):
+    """Large products added to fp32 with a factor: whole 32-column blocks as reductions, remainders of rows and columns, and results
+    without 16-byte rows (a gap of 3, an offset of 1), as the epilogue before."""
+    k = _k()
+    g = torch.Generator(device="cuda").manual_seed(14)
+    K_ = 256
+    a = torch.randn(K_, (M + 7) // 8 * 8, device="cuda", generator=g).to(torch.bfloat16)[:, :M]
+    b = torch.randn(K_, (N + 7) // 8 * 8, device="cuda", generator=g).to(torch.bfloat16)[:, :N]
+    buf = torch.randn(M * (N + gap) + off, device="cuda", generator=g)
+    before, out = buf.clone(), buf[off:].view(M, N + gap)[:, :N]
+    want = out.double() - 0.375 * (a.double().t() @ b.double())
+    k.gemm(a, b, a_mn=True, b_mn=True, out=out, accumulate=True, alpha=-0.375)
+    _check_status()
+    # sums of K_ products in 32 bits
+    assert _rel_err(out, want) < 1e-6
+    rest = torch.ones(M, N + gap, dtype=torch.bool, device="cuda")
+    rest[:, :N] = False
+    assert torch.equal(buf[off:].view(M, N + gap)[rest], before[off:].view(M, N + gap)[rest])
+    assert torch.equal(buf[:off], before[:off])
