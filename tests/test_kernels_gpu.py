@@ -509,3 +509,15 @@ def test_scaled_sums_into_fp32(M, N, gap, off):
     rest[:, :N] = False
     assert torch.equal(buf[off:].view(M, N + gap)[rest], before[off:].view(M, N + gap)[rest])
     assert torch.equal(buf[:off], before[:off])
+
+
+@pytest.mark.parametrize("M,N,K_", [(1, 32768, 4096), (1, 32776, 4096), (2, 16384, 4096), (2, 16392, 4096), (3, 4096, 4096), (4, 4104, 4096),
+                                    (3, 12288, 1024), (4, 12296, 1024)])
+def test_gemm_few_rows_at_the_limits(M, N, K_):
+    """The largest weights of the few-row kernel, and the next size, which the tensor cores take."""
+    k = _k()
+    g = torch.Generator(device="cuda").manual_seed(15)
+    a, b = (torch.randn(r, K_, device="cuda", generator=g).to(torch.bfloat16) for r in (M, N))
+    want = torch.cat([a.double() @ p.double().t() for p in b.split(4096)], 1)
+    assert _rel_err(k.gemm(a, b, out_dtype=torch.float32), want) < 1e-5      # sums of K_ products in 32 bits
+    _check_status()

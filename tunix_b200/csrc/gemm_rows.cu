@@ -120,11 +120,14 @@ gemm_rows_kernel(const RowsArgs a) {
 // error. Same conventions as tb_gemm_bf16.
 int tb_gemm_rows_try(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                      int flags, const void* bias, const void* resid, long long ldr, float alpha, cudaStream_t stream) {
-  // Rows of 16-byte pieces; no other flag than the epilogue's. Three and four rows go to the tensor cores from 16 M weights on
-  // (4096 x 4096, 4 rows: 12.7 us here, 12.5 there), two rows from 64 M on (24576 x 4096: 37.5 against 37.8), where the stream of
-  // the weight bounds both and the multiply-adds of further rows only add to it.
+  // Rows of 16-byte pieces; no other flag than the epilogue's. Above these numbers of weights the stream of the weight bounds both
+  // kernels and the multiply-adds of further rows only add to it. us, here / on the tensor cores: one row, 32768 x 4096 43.5 / 48.0,
+  // 49152 x 4096 69.6 / 66.3, 151936 x 896 47.6 / 46.0; two, 16384 x 4096 24.8 / 27.1, 24576 x 4096 37.5 / 37.8; three, 4096 x 4096
+  // 9.9 / 12.3, 6144 x 4096 14.7 / 14.8; four, 12.6 / 12.3 and 14.7 / 14.7. Three and four rows of many short columns already meet
+  // there below: four, 9728 x 896 8.4 / 8.8, 16384 x 1024 14.4 / 10.9, 65536 x 256 14.1 / 11.7 (1024 x 16384 12.3 / 18.6).
   if (M > 4 || K % 8 || (flags & ~(GF_OUT_F32 | GF_ACCUM | GF_BIAS | GF_RESIDUAL))) return 0;
-  if (M > 1 && (long long)N * K > (M == 2 ? 64LL : 16LL) << 20) return 0;
+  const long long most = (M == 1 ? 128LL : M == 2 ? 64LL : N <= 4096 ? 16LL : 12LL) << 20;
+  if ((long long)N * K > most) return 0;
   RowsArgs a;
   a.A = reinterpret_cast<const __nv_bfloat16*>(A); a.B = reinterpret_cast<const __nv_bfloat16*>(B);
   a.lda = lda; a.ldb = ldb; a.ldc = ldc; a.ldr = ldr; a.N = N; a.K = K; a.flags = flags; a.C = C;
