@@ -521,3 +521,29 @@ def test_gemm_few_rows_at_the_limits(M, N, K_):
     want = torch.cat([a.double() @ p.double().t() for p in b.split(4096)], 1)
     assert _rel_err(k.gemm(a, b, out_dtype=torch.float32), want) < 1e-5      # sums of K_ products in 32 bits
     _check_status()
+
+
+@pytest.mark.parametrize("rows,D", [(4095, 64), (4099, 8), (4099, 128), (4099, 136), (8191, 72), (8195, 8), (8195, 64), (8195, 72), (8195, 128),
+                                    (8195, 136), (16383, 264), (16389, 512), (513, 2304), (512, 2304), (3000, 4104), (9, 16384), (2049, 16384),
+                                    (8195, 3584), (8191, 3584)])
+def test_rmsnorm_rows_and_frozen_weights(rows, D):
+    """Numbers of rows on both sides of every kernel's limit, with and without a gradient of the weight."""
+    k = _k()
+    g = torch.Generator(device="cuda").manual_seed(16)
+    draw = lambda: torch.randn(rows, D + 8, device="cuda", generator=g).to(torch.bfloat16)[:, :D]  # noqa: E731
+    x, dy, base = draw(), draw(), draw()
+    w = torch.randn(D, device="cuda", generator=g).to(torch.bfloat16)
+    y, rstd = k.rmsnorm_fwd(x, w, 1e-6)
+    xd, dd, wd = x.double(), dy.double(), w.double()
+    rs = torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6)
+    gx = dd * wd
+    want = rs * (gx - xd * rs * (gx * xd * rs).mean(-1, keepdim=True))
+    dx, dw = k.rmsnorm_bwd(dy, x, w, rstd)
+    frozen, none = k.rmsnorm_bwd(dy, x, w, rstd, want_dw=False)
+    into = base.clone()
+    k.rmsnorm_bwd(dy, x, w, rstd, want_dw=False, dx_accumulate_into=into)
+    assert none is None
+    # one rounding to bf16: 2^-9 of a value; 32-bit sums over the rows
+    assert _rel_err(y, xd * rs * wd) < 4e-3 and _rel_err(dx, want) < 4e-3 and _rel_err(frozen, want) < 4e-3
+    assert _rel_err(into, base.double() + want) < 4e-3 and _rel_err(dw, (dd * xd * rs).sum(0)) < 1e-5
+    _check_status()

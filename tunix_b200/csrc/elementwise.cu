@@ -63,7 +63,9 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, long lon
   }
 }
 
-// Same for rows of at most 256 columns (the norms of single heads): T lanes a row, 8 columns a lane, a row read once.
+// Same for many rows of at most 128 columns (the norms of single heads), which leave half of a warp idle or more: T lanes a row,
+// 8 columns a lane, a row read once. B200, a warp a row -> here: 524288 x 128 95 -> 62 us, 131072 x 64 21 -> 12, 8192 x 128 3.4 -> 3.0;
+// fewer rows fit one round of warps (4096 x 128 2.4, here 2.7), and rows of more columns fill them (131072 x 256 29, here 35).
 template <int T>
 __global__ void __launch_bounds__(256)
 rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
@@ -151,8 +153,8 @@ rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const
 // registers between its reduction and its dx, and a thread keeps the sums of its columns over all its rows.
 //
 // Bound by HBM: x, dy and dx once each. B200, dx and dw together, before (two kernels, three passes over x and dy) -> after:
-// 524288 x 128 691 -> 125 us, 16384 x 4096 219 -> 105, 8192 x 4096 117 -> 59, 4096 x 4096 59 -> 33, 2331 x 896 34 -> 22. Narrow
-// rows forward (a lane of 16 idle before): 524288 x 128 98 -> 64.
+// 524288 x 128 686 -> 120 us, 16384 x 4096 214 -> 99, 8192 x 4096 109 -> 54, 4096 x 4096 51 -> 30, 2048 x 896 10.5 -> 9.1,
+// 4096 x 512 10.3 -> 8.8, 4096 x 64 7.5 -> 4.4 (8.4 without the sums over the lanes of a warp in front of the atomics).
 __device__ __forceinline__ void add4(float* p, float a, float b, float c, float d) {     // p: 16-byte aligned
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
@@ -219,7 +221,11 @@ rmsnorm_bwd_narrow_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, 
     }
   }
   if (!dw) return;
-  if (in)
+#pragma unroll
+  for (int o = 16; o >= T; o >>= 1)                        // the lanes of a warp that have the same columns
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+  if (in && (threadIdx.x & 31) < T)
 #pragma unroll
     for (int i = 0; i < 8; ++i) atomicAdd(s_dw + col + i, acc[i]);
   __syncthreads();
@@ -353,7 +359,8 @@ rmsnorm_bwd_row_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, con
   }
 }
 
-// The same in two kernels, for rows too wide for the registers of a block and for dw alone (x and dy 4-byte aligned, no w).
+// The same in two kernels: for rows too wide for the registers of a block, for most calls without dw, and for dw alone (x and dy
+// 4-byte aligned, no w).
 __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy,
                                       const __nv_bfloat16* __restrict__ x, long long ldx,
                                       const __nv_bfloat16* __restrict__ w,
@@ -672,16 +679,15 @@ TB_API int tb_rmsnorm_fwd(const void* x, long long ldx, const void* w, void* y, 
     return e == cudaSuccess ? 0 : -5;
   }
   const int block = 256;
-  if (D <= 256) {
-    const int t = D <= 64 ? 8 : D <= 128 ? 16 : 32;
+  if (D <= 128 && rows >= 8192) {
+    const int t = D <= 64 ? 8 : 16;
     const int grid = grid_for((long long)rows * t, 256 * 2, 148 * 16);
     auto run = [&](auto kernel) {
       kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, ldy, rstd, rows, D, eps,
                                        add_one);
     };
     if (t == 8) run(rmsnorm_fwd_narrow_kernel<8>);
-    else if (t == 16) run(rmsnorm_fwd_narrow_kernel<16>);
-    else run(rmsnorm_fwd_narrow_kernel<32>);
+    else run(rmsnorm_fwd_narrow_kernel<16>);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
   rmsnorm_fwd_kernel<<<grid_for((long long)rows * 32, block), block, 0, stream>>>(
@@ -696,13 +702,21 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
   if (rows <= 0) return 0;
   if (D % 8) return -2;
   if (!dx && !dw) return 0;
-  // up to 256 columns by lanes of a warp, up to 16384 by threads of a block; the SMs are filled once, so that the sums over columns
-  // meet in few atomics. dw alone needs no weight and no rows of 16-byte pieces: that call keeps the kernel for wide rows.
+  // dx and dw: up to 256 columns by lanes of a warp, up to 16384 by threads of a block; the SMs are filled once, so that the sums over
+  // columns meet in few atomics (a second block an SM pays from 16384 rows on: 4096 x 512 11.6 us with two, 8.8 with one, 16384 x 512
+  // 17.6 and 18.2).
+  // dx alone gains nothing from sums that stay in registers; a warp a row / here, us: 16384 x 1536 34 / 38, 4096 x 2304 12.2 / 16.6,
+  // 524288 x 256 151 / 226, 4096 x 16384 123 / 156. It comes here where a warp a row is too few warps or too wide a
+  // row for their registers (128 x 4096 8.1 / 4.1, 4096 x 8192 64 / 39, 16384 x 4096 109 / 97), or leaves half of it idle (524288 x 128 142 / 116).
+  // dw alone needs no weight and no rows of 16-byte pieces: that call keeps the kernel for wide rows.
 #define RMS_BWD_ARGS                                                                                                          \
   (const __nv_bfloat16*)dy, lddy, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, rstd, (__nv_bfloat16*)dx, lddx, dw, rows, D, \
       add_one, accumulate_dx
-  const bool wide = !dx || D > 16384 || (D > 256 && (reinterpret_cast<uintptr_t>(dw) & 15));
-  if (wide) {
+  const bool narrow = dx && (dw ? D <= 256 : D <= 128 && rows >= 4096);
+  const bool fits = dx && D > 256 && D <= 16384;
+  const bool by_row = dw ? fits && !(reinterpret_cast<uintptr_t>(dw) & 15)
+                         : fits && D > 2048 && (rows <= 512 || (D > 4096 ? D <= 8192 || rows <= 2048 : D > 3072 && rows >= 8192));
+  if (!narrow && !by_row) {
     const int block = 256;
     if (dx)
       rmsnorm_bwd_dx_kernel<<<grid_for((long long)rows * 32, block), block, 0, stream>>>(
@@ -713,7 +727,7 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
       rmsnorm_bwd_dw_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, lddy,
                                                       (const __nv_bfloat16*)x, ldx, rstd, dw, rows, D);
     }
-  } else if (D <= 256) {
+  } else if (narrow) {
     const int t = D <= 64 ? 8 : D <= 128 ? 16 : 32;
     // four rows a lane once that fills the SMs
     const int grid = max(grid_for((long long)rows * t, 256 * 4, 148 * 6), grid_for((long long)rows * t, 256, 148));
@@ -724,7 +738,7 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
     const int vecs = D / 8, vpt = vecs <= 512 ? 1 : vecs <= 1024 ? 2 : 4;
     const int threads = ((vecs + vpt - 1) / vpt + 31) / 32 * 32, most = vpt == 1 ? 1024 : 512;
     const int groups = min(RMS_GROUPS, most / threads);
-    const int grid = min((rows + groups - 1) / groups, 148 * (most / (threads * groups)));
+    const int grid = min((rows + groups - 1) / groups, 148 * (rows >= 16384 ? most / (threads * groups) : 1));
     const dim3 block(threads, groups);
     const size_t smem = groups > 1 ? (size_t)D * 4 : 0;      // at most 16 KB: more than one group has at most 4096 columns
     if (vpt == 1) rmsnorm_bwd_row_kernel<1><<<grid, block, smem, stream>>>(RMS_BWD_ARGS);
