@@ -547,3 +547,10 @@ def test_rmsnorm_rows_and_frozen_weights(rows, D):
     assert _rel_err(y, xd * rs * wd) < 4e-3 and _rel_err(dx, want) < 4e-3 and _rel_err(frozen, want) < 4e-3
     assert _rel_err(into, base.double() + want) < 4e-3 and _rel_err(dw, (dd * xd * rs).sum(0)) < 1e-5
     _check_status()
+
+
+@pytest.mark.parametrize("tokens,heads,H,gap", [(5461, 3, 48, 16), (5462, 3, 48, 16), (2050, 5, 64, 8), (1030, 32, 64, 0), (300, 30, 128, 0),
+                                                (129, 41, 256, 8), (9000, 4, 64, 4)])
+def test_rope_of_many_heads(tokens, heads, H, gap):
+    """Sizes of the vector kernel, from the smallest on: head groups that are not full, rows that lie apart or without 16-byte pieces."""
+    test_rope_widths(tokens, heads, H, gap)

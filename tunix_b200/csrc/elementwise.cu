@@ -754,8 +754,10 @@ TB_API int tb_rope(void* x, long long ld, const int* pos, const float* cos_t, co
   if (tokens <= 0) return 0;
   if (H % 4) return -2;
   const long long units = tokens * (H / 16) * ((heads + ROPE_HEADS - 1) / ROPE_HEADS);
-  // whole 16-byte pieces of both halves; a unit's number, and a turn's step beyond the last, fit 32 bits
-  if (H % 16 == 0 && ld % 8 == 0 && units < (1LL << 31) &&
+  // whole 16-byte pieces of both halves; a unit's number, and a turn's step beyond the last, fit 32 bits. Fewer units than these are
+  // one short round of either kernel, of which the one by pairs has more threads (64 x 32 heads of 128, 4096 units: 2.2 us, 2.5 by
+  // vectors; 256 x 32, 16384 units: 3.4, 2.7).
+  if (units >= 16384 && H % 16 == 0 && ld % 8 == 0 && units < (1LL << 31) &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15) == 0) {
     rope_vec_kernel<<<grid_for(units, 256), 256, 0, stream>>>((__nv_bfloat16*)x, ld, pos, cos_t, sin_t, (unsigned)units, heads, H,
                                                               backward ? -1.f : 1.f);
