@@ -351,8 +351,8 @@ def test_joint_bias_follows_its_model():
 
 
 def test_packed_prompts_share_short_attention_calls():
-    """An attention call reads segment ids with the square of its tokens: no run of several prompts is longer than 16384 of them, every
-    prompt starts at a key block and lies in one run."""
+    """An attention call reads segment ids with the square of its tokens: no run of several prompts is longer than 16384 of them
+    or eight times the longest prompt, every prompt starts at a key block and lies in one run."""
     from tunix_b200.generate.engine import PagedEngine
     eng = PagedEngine.__new__(PagedEngine)
     rng = np.random.default_rng(0)
@@ -363,7 +363,7 @@ def test_packed_prompts_share_short_attention_calls():
         assert groups[0][0] == 0 and groups[-1][1] == ends[-1] and all(a[1] == b[0] for a, b in zip(groups, groups[1:]))
         for a, b in groups:
             inside = [i for i in range(len(lens)) if a <= starts[i] < b]
-            assert starts[inside[0]] == a and ends[inside[-1]] == b and (b - a <= 16384 or len(inside) == 1)
+            assert starts[inside[0]] == a and ends[inside[-1]] == b and b - a <= max(16384, 8 * max(lens))
 
 
 def test_prompts_of_like_lengths_stay_padded():
