@@ -75,12 +75,12 @@ struct BwdCfg {
 
 // Bound by the chain S -> P -> dS -> dK / dQ of one CTA an SM (512 TMEM columns, 208 KB), of which the products are 1280 cycles
 // a tile at the tensor cores' rate. B200, 32 / 8 heads of 128, causal, the whole backward (with delta and the fp32 dQ passes),
-// before -> after these roles, this schedule and the order of the grid: 2 x 2048 546 -> 297 us, 8 x 2048 1546 -> 1214,
-// 1 x 16384 8569 -> 6750; rollouts padded at both ends 8 x 1024 864 -> 406; packed rows 3 x 777 with 14 / 2 heads of 64 375 -> 112;
-// 4 x 1001, 16 / 8 heads of 256, soft-cap 610 -> 385. Pt and dSt as operands in TMEM were tried: 1 x 16384 6759 -> 6585 us and
-// 2 x 2048 290 -> 276, but no gain beyond what runs differ by at 8 x 2048, in packed rows or with heads of 64, once a vote before each
-// store to TMEM and a barrier of the issuer's were added (the row warps' wait for dV of the tile before is also what keeps one that is
-// ahead from arriving twice for a tile).
+// before -> after these roles, this schedule and the order of the grid: 2 x 2048 546 -> 279 us, 8 x 2048 1546 -> 1147,
+// 1 x 16384 8569 -> 6620 (runs differ by 4 %); rollouts padded at both ends 8 x 1024 864 -> 375; packed rows 3 x 777 with 14 / 2 heads
+// of 64 375 -> 110; 4 x 1001, 16 / 8 heads of 256, soft-cap 610 -> 376. Pt and dSt as operands in TMEM were tried: 3 to 5 % less at
+// 1 x 16384 and 2 x 2048, nothing beyond what runs differ by at 8 x 2048 and in packed rows, and with heads of 64 between nothing and a
+// loss of 14 %, once a vote before each store to TMEM and a barrier of the issuer's were added (the row warps' wait for dV of the tile
+// before is also what keeps one that is ahead from arriving twice for a tile).
 //
 // Roles: row threads (P and dS), four warps that add dQt to dQ and fetch lse / delta of later tiles, one issuer.
 // Schedule (PIPE): St runs two query tiles ahead and dPt of the next tile is the first product behind dSt, so the row threads go
@@ -440,6 +440,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (a.softcap > 0.f) {
 #pragma unroll
           for (int i = 0; i < CW_; ++i) {
+            // as in the forward, whose row sums it then matches. Also the closer form in this file's fast-math build: against 64 bits,
+            // cap 50, scores up to 150, the capped score is off by 3.2e-6 rms (1.4e-5 at most), with tanhf by 1.3e-4 (3.9e-4); the
+            // cap's derivative by 1.1e-7 and 4.2e-6.
             const float z = cap_score(__uint_as_float(t[i >> 5][i & 31]) * a.scale, a.softcap, inv_cap);
             t[i >> 5][i & 31] = __float_as_uint(z * inv_cap);
             p[i] = exp2f(fmaf(z, LOG2E, -st_lse[i]));

@@ -17,9 +17,9 @@
 // Bound by the softmax warps (64 exponentials a row and block share the special-function units with the other CTA of the SM).
 // Segment ids are compared per key block where they decide for the whole of it, and by warp votes elsewhere, not by one load a
 // score; K and V share a ring, so that no product waits for a load issued in its own block. B200, 32 / 8 heads of 128, causal,
-// before -> after: rollouts padded at both ends, 8 x 1024 519 -> 143 us, 16 x 1024 970 -> 264, 8 x 4096 6320 -> 984; packed rows
-// of 777, 14 / 2 heads of 64, 92 -> 26; without segments 2 x 2048 136 -> 96, 8 x 2048 452 -> 391, 1 x 16384 2228 -> 2011;
-// 4 x 1001 with heads of 256 and a soft-cap 265 -> 94. P in TMEM instead of shared memory (whose 128 bytes a cycle the operands of
+// before -> after: rollouts padded at both ends, 8 x 1024 519 -> 136 us, 8 x 4096 6320 -> 906; packed rows
+// of 777, 14 / 2 heads of 64, 92 -> 26; without segments 2 x 2048 136 -> 91, 8 x 2048 452 -> 375, 1 x 16384 2228 -> 2012;
+// 4 x 1001 with heads of 256 and a soft-cap 265 -> 88. P in TMEM instead of shared memory (whose 128 bytes a cycle the operands of
 // S fill otherwise) is 2 to 5 % of it.
 //
 // Replaces the eager [B,N,T,S] attention and the TPU-only splash attention of the reference

@@ -2,7 +2,9 @@
 //
 // Ids decide for most blocks of 64 tokens as a whole. A tile of rows lists the blocks with any id between the smallest and the
 // largest of its rows, and marks those where all ids are the one that all its rows have; the others are never loaded. Elements
-// are compared in the rest only, by warp votes.
+// are compared in the rest only, by warp votes. Every tile of every head reads the ids of all blocks that it may see: with the square
+// of a row's tokens, so rows of very many short segments are better cut into several calls (512 segments of 128 to 256 tokens, 32
+// heads of 128: 4612 us in one call, 1507 in calls of 16384 tokens).
 #pragma once
 #include "common.cuh"
 

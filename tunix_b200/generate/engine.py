@@ -487,7 +487,7 @@ class PagedEngine(BaseSampler):
         blocks, and its results round alike, whatever it is prefilled with; the tokens that fill its last block follow it and
         are seen by none of its own. Returns the hidden state of every prompt's last token.
 
-        8 prompts of 1024 to 4096 tokens, 2 layers of an 8B model, padded -> packed: 54 -> 34 ms."""
+        8 prompts of 1024 to 4096 tokens, 2 layers of an 8B model, padded -> packed: 24 -> 16 ms."""
         cfg, pool, dev = self.cfg, self.pool, self.device
         KH, H = self.n_kv, cfg.head_dim
         lens, starts, ends, groups = self._pack_layout([len(r) for r in rows])
