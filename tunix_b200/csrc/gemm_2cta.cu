@@ -34,12 +34,12 @@ constexpr int STAGES = 6;
 constexpr int A_BYTES = HM * BK * 2, B_BYTES = HN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int STAGING_BYTES = 4 * 32 * 128;        // a 32 x 32 block of fp32 results per epilogue warp
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + STAGING_BYTES + 1024;
-constexpr int GROUP_M = 8;
 
 enum { GF_A_MN = 1, GF_B_MN = 2, GF_OUT_F32 = 4, GF_ACCUM = 8, GF_BIAS = 16, GF_RESIDUAL = 32 };
 
 struct Args2 {
   int M, N, K, flags;
+  int group;             // tiles are walked in groups of this many rows of tiles (negative: columns), see tile_group
   // second contraction segment accumulated into the same TMEM tile: C += A2[M, K2] * B2[N, K2]^T with the layouts of
   // A and B (a low-rank adapter update x A^T B^T carried by the base projection's GEMM); K2 = 0 when absent
   int K2;
@@ -167,13 +167,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   const uint32_t tmem_base = *tmem_ptr_smem;
 
   auto tile_coords = [&](int t, int& mt, int& nt) {
-    const int per_group = GROUP_M * num_n;
-    const int g = t / per_group;
-    const int first_m = g * GROUP_M;
-    const int gsz = min(GROUP_M, num_m - first_m);
-    const int r = t - g * per_group;
-    mt = first_m + (r % gsz);
-    nt = r / gsz;
+    const bool by_n = args.group < 0;
+    const int size = by_n ? -args.group : args.group, along = by_n ? num_n : num_m, across = by_n ? num_m : num_n;
+    const int g = t / (size * across), first = g * size, r = t - first * across, here = min(size, along - first);
+    const int a = first + r % here, b = r / here;
+    mt = by_n ? b : a;
+    nt = by_n ? a : b;
   };
 
   if (warp == 0) {
@@ -475,6 +474,16 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 }
 
 int g_sms2 = 0;
+// The order of the tiles: groups of at most 16 rows (or columns) of tiles, a group's tiles column by column, in the direction that
+// reads the fewest 256-wide panels of A and B: a group's own once, all of the other operand once a group. 16 panels and the 4 or 5
+// columns that 74 pairs work on at a time stay in L2; a side of up to 16 tiles is one group, and each panel of the other side is read in
+// one go. Under the power cap a loop of products takes, against groups of 8 rows whatever the shape (us, bf16 out): 16384 x 4096 x 4096
+// 432 -> 410, 8192 x 4096 x 4096 216 -> 210, 4096 x 14336 x 4096 388 -> 375, 4096 x 4096 x 14336 (dgrad) 390 -> 375, 4096^3 115 -> 112.
+// Groups of 32 lose again (8192 x 4096 x 4096 228, 16384 x 12288 x 4096 1284 -> 1357).
+int tile_group(int num_m, int num_n) {
+  const int gm = (num_m + 15) / 16, gn = (num_n + 15) / 16;
+  return num_m + (long long)gm * num_n <= num_n + (long long)gn * num_m ? (num_m + gm - 1) / gm : -((num_n + gn - 1) / gn);
+}
 struct LseArgs {           // log-softmax epilogue request; partial == nullptr for a plain GEMM
   const int* targets = nullptr;
   float* partial = nullptr;
@@ -570,6 +579,7 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
   }
   Args2 a;
   a.K2 = seg.K2;
+  a.group = tile_group(num_m, num_n);
   a.M = M; a.N = N; a.K = K; a.flags = flags; a.C = C; a.ldc = ldc;
   a.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   a.resid = reinterpret_cast<const __nv_bfloat16*>(resid);
