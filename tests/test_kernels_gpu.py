@@ -554,3 +554,74 @@ def test_rmsnorm_rows_and_frozen_weights(rows, D):
 def test_rope_of_many_heads(tokens, heads, H, gap):
     """Sizes of the vector kernel, from the smallest on: head groups that are not full, rows that lie apart or without 16-byte pieces."""
     test_rope_widths(tokens, heads, H, gap)
+
+
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("tokens,N,KH,H,gap", [(1, 1, 1, 64, 0), (37, 14, 2, 64, 0), (130, 4, 5, 128, 24), (1000, 32, 8, 128, 0), (67, 16, 8, 256, 8)])
+def test_qk_rope(tokens, N, KH, H, gap, norm):
+    """Head groups that are not full, rows that lie apart, one token, more units than one round of blocks takes; forward and backward."""
+    k = _k()
+    g = torch.Generator(device="cuda").manual_seed(13)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)  # noqa: E731
+    xs = [rnd(tokens, n * H + gap)[:, :n * H] for n in (N, KH)]
+    ws = [1 + 0.2 * rnd(H), 1 + 0.2 * rnd(H)] if norm else [None, None]
+    ds = [rnd(tokens, n * H) for n in (N, KH)]
+    pos = torch.randint(0, 50, (tokens,), device="cuda", generator=g, dtype=torch.int32)
+    ang = torch.randn(50, H // 2, device="cuda", generator=g)
+    cos, sin = ang.cos(), ang.sin()
+    want, leaves = [], []
+    for x, w in zip(xs, ws):
+        x = x.double().unflatten(1, (-1, H)).requires_grad_()
+        w = None if w is None else w.double().requires_grad_()
+        leaves.append((x, w))
+        y = x if w is None else x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * (w + 1)
+        c, s = cos.double()[pos.long()][:, None], sin.double()[pos.long()][:, None]
+        a, b = y[..., :H // 2], y[..., H // 2:]
+        want.append(torch.cat([a * c - b * s, b * c + a * s], -1).flatten(1))
+    yq, yk, rq, rk = k.qk_rope(*xs, H, pos, cos, sin, wq=ws[0], wk=ws[1], eps=1e-6, add_one=True, want_rstd=norm)
+    # one rounding to bf16: at most 2^-9 of a value, about 2^-9 / sqrt(3) in the norm
+    assert _rel_err(yq, want[0]) < 2e-3 and _rel_err(yk, want[1]) < 2e-3
+    torch.autograd.backward(want, [d.double() for d in ds])
+    if norm:
+        dxq, dxk, dwq, dwk = k.qk_rope_bwd(*ds, *xs, H, pos, cos, sin, *ws, rq, rk, True)
+        assert _rel_err(dwq, leaves[0][1].grad) < 1e-4 and _rel_err(dwk, leaves[1][1].grad) < 1e-4      # 32-bit sums
+        assert k.qk_rope_bwd(*ds, *xs, H, pos, cos, sin, *ws, rq, rk, True, want_dw=False)[2] is None
+    else:
+        dxq, dxk, _, _ = k.qk_rope(*ds, H, pos, cos, sin, backward=True)
+    assert _rel_err(dxq, leaves[0][0].grad.flatten(1)) < 2e-3 and _rel_err(dxk, leaves[1][0].grad.flatten(1)) < 2e-3
+    again = [x.clone() for x in xs]
+    k.qk_rope(*again, H, pos, cos, sin, wq=ws[0], wk=ws[1], eps=1e-6, add_one=True, out=again)          # over its inputs
+    assert torch.equal(again[0], yq) and torch.equal(again[1], yk)
+    assert k.qk_rope(xs[0], rnd(tokens, KH * H + 4)[:, :KH * H], H, pos, cos, sin) is None              # rows without 16-byte pieces
+    _check_status()
+
+
+@pytest.mark.parametrize("qk_norm", [False, True])
+def test_model_joint_rotation_matches_separate(qk_norm):
+    """The attention layer with the joint kernel and, made to by a hook or by a refusing kernel, with norm and rotation one by one."""
+    from tunix_b200.models.config import ModelConfig
+    from tunix_b200.models.transformer import Attention
+    from tunix_b200.ops import functional as F
+    cfg = ModelConfig(family="qwen3", num_layers=1, vocab_size=64, embed_dim=128, hidden_dim=128, num_heads=4, head_dim=64, num_kv_heads=2,
+                      qk_norm=qk_norm, dtype=torch.bfloat16, max_position=64)
+    att = Attention(cfg, 0, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    with torch.no_grad():
+        for p in att.parameters():
+            p.copy_(torch.randn(p.shape, device="cuda", generator=g) * 0.1 + (1.0 if p.dim() == 1 else 0.0))
+    x = torch.randn(2, 33, 128, device="cuda", generator=g).to(torch.bfloat16)
+    pos = torch.arange(33, device="cuda", dtype=torch.int32)[None].expand(2, 33).contiguous()
+    ang = torch.randn(64, 32, device="cuda", generator=g)
+    def run():
+        leaf = x.clone().requires_grad_()
+        y, _ = att(leaf, pos, (ang.cos(), ang.sin()))
+        return [y.detach(), *torch.autograd.grad(y.float().pow(2).sum(), [leaf, *att.parameters()])]
+    joint, sep = run(), None
+    real, F.qk_rope = F.qk_rope, lambda *a, **k: None
+    try:
+        sep = run()
+    finally:
+        F.qk_rope = real
+    for a, b in zip(joint, sep):
+        assert _rel_err(a, b) < 2e-2, (a.shape, _rel_err(a, b))        # a few roundings to bf16 apart
+    _check_status()

@@ -30,6 +30,7 @@ import numpy as np
 import torch
 
 from ..common.configs import CacheConfig
+from ..models.transformer import RMSNorm, _bare
 from ..ops import functional as F
 from ..ops import kernels as K
 from ..ops import sampling_kernels as S
@@ -345,24 +346,31 @@ class PagedEngine(BaseSampler):
         """Projections + QK-norm + RoPE on flat rows h2 [n, D] -> q [n,N,H], k [n,K,H], v [n,K*H]."""
         cfg, at = self.cfg, layer.self_attn
         N, KH, H = self.n_heads, self.n_kv, cfg.head_dim
-        q = F.linear(h2, at.q_proj.base_weight(), at.q_proj.bias).view(-1, N, H)
-        k = F.linear(h2, at.k_proj.base_weight(), at.k_proj.bias).view(-1, KH, H)
-        v = F.linear(h2, at.v_proj.base_weight(), at.v_proj.bias)
+        q, k, v = (F.linear(h2, p.base_weight(), p.bias) for p in (at.q_proj, at.k_proj, at.v_proj))
         for proj, name in ((at.q_proj, "q"), (at.k_proj, "k"), (at.v_proj, "v")):
             if proj.lora_a is not None and proj.lora_enabled:
                 delta = F.linear(F.linear(h2, proj.lora_a), proj.lora_b) * proj.lora_scale
                 if name == "q":
-                    q = q + delta.view_as(q)
+                    q = q + delta
                 elif name == "k":
-                    k = k + delta.view_as(k)
+                    k = k + delta
                 else:
                     v = v + delta
-        if cfg.qk_norm:
-            q = at.q_norm(q)
-            k = at.k_norm(k)
         cos, sin = self._rope(i)
-        K.rope_(q, positions_flat, cos, sin)
-        K.rope_(k, positions_flat, cos, sin)
+        norms = (at.q_norm, at.k_norm) if cfg.qk_norm else ()
+        if not norms:
+            done = K.qk_rope(q, k, H, positions_flat, cos, sin, out=(q, k))
+        elif all(_bare(n, RMSNorm) for n in norms) and norms[0].eps == norms[1].eps and norms[0].add_one == norms[1].add_one:
+            done = K.qk_rope(q, k, H, positions_flat, cos, sin, wq=norms[0].weight, wk=norms[1].weight, eps=norms[0].eps,
+                             add_one=norms[0].add_one, out=(q, k))
+        else:
+            done = None
+        q, k = q.view(-1, N, H), k.view(-1, KH, H)
+        if done is None:
+            if norms:
+                q, k = at.q_norm(q), at.k_norm(k)
+            K.rope_(q, positions_flat, cos, sin)
+            K.rope_(k, positions_flat, cos, sin)
         return q, k, v
 
     def _lin(self, mod, x, residual=None):

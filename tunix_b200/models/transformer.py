@@ -19,6 +19,7 @@ from typing import Optional
 
 import torch
 import torch.nn as nn
+from torch.nn.modules.module import _has_any_global_hook
 from torch.utils.checkpoint import checkpoint as _torch_checkpoint
 
 from ..ops import functional as F
@@ -126,6 +127,12 @@ class RMSNorm(nn.Module):
         return F.rmsnorm(x, self.weight, self.eps, self.add_one)
 
 
+def _bare(mod: nn.Module, kind: type) -> bool:
+    """Whether calling `mod` is no more than `kind.forward`: a joint kernel may then read its parameters and leave the call out."""
+    return type(mod) is kind and "forward" not in mod.__dict__ and not (
+        mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks or _has_any_global_hook())
+
+
 class Attention(nn.Module):
     def __init__(self, cfg: ModelConfig, layer_idx: int, device=None):
         super().__init__()
@@ -143,6 +150,22 @@ class Attention(nn.Module):
         self.window = cfg.sliding_window if self.is_local else 0
         qpas = cfg.query_pre_attn_scalar if cfg.query_pre_attn_scalar else float(H)
         self.scale = 1.0 / math.sqrt(qpas)
+
+    def _norm_and_rotate(self, q, k, positions, rope):
+        """Per-head norms (where the family has them) and rotary embedding of q, k [B, T, heads * H] -> [B, T, heads, H]."""
+        cfg, H, (cos, sin) = self.cfg, self.cfg.head_dim, rope
+        norms = (self.q_norm, self.k_norm) if cfg.qk_norm else ()
+        out = None
+        if not norms:
+            out = F.qk_rope(q, k, positions, cos, sin, H)
+        elif all(_bare(n, RMSNorm) for n in norms) and norms[0].eps == norms[1].eps and norms[0].add_one == norms[1].add_one:
+            out = F.qk_rope(q, k, positions, cos, sin, H, norms[0].weight, norms[1].weight, norms[0].eps, norms[0].add_one)
+        if out is not None:
+            return tuple(t.view(*t.shape[:2], -1, H) for t in out)
+        q, k = (t.view(*t.shape[:2], -1, H) for t in (q, k))
+        if norms:
+            q, k = self.q_norm(q), self.k_norm(k)
+        return F.rope(q, positions, cos, sin), F.rope(k, positions, cos, sin)
 
     def forward(self, x, positions, rope, cache=None, segment_ids=None, attention_mask=None, residual=None):
         cfg = self.cfg
@@ -162,24 +185,18 @@ class Attention(nn.Module):
                 qkv = tp_lib.column_parallel_linear(x, w, b, tp)
                 B, N, K = qkv.shape[0], N // tp.world, K // tp.world
                 q, k, v = qkv.split([N * H, K * H, K * H], dim=-1)
-                q, k, v = (t.contiguous().view(B, T, -1, H) for t in (q, k, v))
+                q, k, v = (t.contiguous() for t in (q, k, v))
             else:
                 # adapters or a quantised base: gather the tokens once, then this rank's slices run as local projections
                 xg = tp_lib.gather_tokens(x, tp)
                 B, N, K = xg.shape[0], N // tp.world, K // tp.world
-                q = self.q_proj(xg).view(B, T, N, H)
-                k = self.k_proj(xg).view(B, T, K, H)
-                v = self.v_proj(xg).view(B, T, K, H)
+                q = self.q_proj(xg)
+                k = self.k_proj(xg)
+                v = self.v_proj(xg)
         else:
-            q = self.q_proj(x).view(B, T, N, H)
-            k = self.k_proj(x).view(B, T, K, H)
-            v = self.v_proj(x).view(B, T, K, H)
-        if cfg.qk_norm:
-            q = self.q_norm(q)
-            k = self.k_norm(k)
-        cos, sin = rope
-        q = F.rope(q, positions, cos, sin)
-        k = F.rope(k, positions, cos, sin)
+            q, k, v = self.q_proj(x), self.k_proj(x), self.v_proj(x)
+        q, k = self._norm_and_rotate(q, k, positions, rope)
+        v = v.view(B, T, K, H)
         seg_q = seg_k = segment_ids
         q_off = None
         new_cache = None

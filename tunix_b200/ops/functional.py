@@ -273,6 +273,69 @@ def rope(x, positions, cos, sin):
     return R.rope_ref(x, positions, cos, sin)
 
 
+def _aligned16(*ts) -> bool:
+    return all(t.data_ptr() % 16 == 0 for t in ts)
+
+
+class _QKRopeFn(torch.autograd.Function):
+    """q, k [B, T, heads * H] -> normed per head (where weights are given) and rotated, one launch for both. Without norms they are
+    rotated in place: the projections' outputs as a whole, since autograd copies the gradient of a view that is written to."""
+
+    @staticmethod
+    def forward(ctx, q, k, wq, wk, positions, cos, sin, H, eps, add_one):
+        pos = positions.reshape(-1)
+        q2, k2 = q.view(-1, q.shape[-1]), k.view(-1, k.shape[-1])
+        ctx.cfg = (H, add_one)
+        if wq is None:
+            fresh = not (q._is_view() or k._is_view() or q.is_leaf and q.requires_grad or k.is_leaf and k.requires_grad)
+            yq, yk = (q, k) if fresh else (torch.empty_like(q), torch.empty_like(k))
+            K.qk_rope(q2, k2, H, pos, cos, sin, out=(yq.view(q2.shape), yk.view(k2.shape)))
+            ctx.save_for_backward(positions, cos, sin)
+            if fresh:
+                ctx.mark_dirty(q, k)
+            return yq, yk
+        yq, yk = torch.empty_like(q), torch.empty_like(k)
+        _, _, rq, rk = K.qk_rope(q2, k2, H, pos, cos, sin, wq=wq, wk=wk, eps=eps, add_one=add_one, want_rstd=True,
+                                 out=(yq.view(q2.shape), yk.view(k2.shape)))
+        ctx.save_for_backward(positions, cos, sin, q, k, wq, wk, rq, rk)
+        ctx.refs = (wq, wk)
+        return yq, yk
+
+    @staticmethod
+    def backward(ctx, dq, dk):
+        positions, cos, sin, *normed = ctx.saved_tensors
+        H, add_one = ctx.cfg
+        pos = positions.reshape(-1)
+        dq, dk = dq.contiguous(), dk.contiguous()
+        if not _aligned16(dq, dk):
+            dq, dk = dq.clone(), dk.clone()
+        d2 = dq.view(-1, dq.shape[-1]), dk.view(-1, dk.shape[-1])
+        if not normed:
+            yq, yk, _, _ = K.qk_rope(*d2, H, pos, cos, sin, backward=True)
+            return yq.view(dq.shape), yk.view(dk.shape), *(None,) * 8
+        q, k, wq, wk, rq, rk = normed
+        want_dw = ctx.needs_input_grad[2] or ctx.needs_input_grad[3]
+        dxq, dxk, dwq, dwk = K.qk_rope_bwd(*d2, q.view(d2[0].shape), k.view(d2[1].shape), H, pos, cos, sin, wq, wk, rq, rk, add_one,
+                                           want_dw=want_dw)
+        dws = [_deliver_grad(p, dw if getattr(p, "main_grad", None) is not None else dw.to(p.dtype)) if need else None
+               for p, dw, need in zip(ctx.refs, (dwq, dwk), ctx.needs_input_grad[2:4])]
+        return dxq.view(dq.shape), dxk.view(dk.shape), *dws, *(None,) * 6
+
+
+def qk_rope(q, k, positions, cos, sin, H: int, wq=None, wk=None, eps: float = 1e-6, add_one: bool = False):
+    """Rotary embedding of q [B, T, N * H] and k [B, T, K * H], behind a norm over each head where wq and wk are given. q and k are fresh
+    projection outputs, which may be overwritten. None where the joint kernel does not take the call."""
+    if not (_native(q) and _native(k) and H in (64, 128, 256) and q.dim() == k.dim() == 3 and q.shape[:2] == k.shape[:2] and q.is_contiguous()
+            and k.is_contiguous() and q.shape[0] * q.shape[1] * (q.shape[2] // H + k.shape[2] // H + 8) < 1 << 30
+            and q.numel() and k.numel() and cos.shape[-1] == H // 2 and _aligned16(q, k, cos, sin)):
+        return None
+    if wq is not None and not (wq.dtype == wk.dtype == torch.bfloat16 and wq.numel() == wk.numel() == H and wq.is_contiguous()
+                               and wk.is_contiguous() and _aligned16(wq, wk)):
+        return None
+    pos = positions if positions.dtype == torch.int32 else positions.to(torch.int32)
+    return _QKRopeFn.apply(q, k, wq, wk, pos.contiguous(), cos, sin, int(H), float(eps), bool(add_one))
+
+
 # -------------------------------------------------------------------------------- glu
 class _GluFn(torch.autograd.Function):
     @staticmethod

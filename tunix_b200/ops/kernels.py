@@ -171,6 +171,52 @@ def rope_(x: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: torc
     return x
 
 
+def qk_rope(q: torch.Tensor, k: torch.Tensor, H: int, positions: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, *, wq=None, wk=None,
+            eps: float = 0.0, add_one: bool = False, want_rstd: bool = False, out=None, backward: bool = False):
+    """Rotary embedding of q [tokens, N * H] and k [tokens, K * H] in one launch, behind a norm over each head where its weights are
+    given. `out` = (yq, yk), the inputs themselves among them. Returns (yq, yk, rstd_q, rstd_k), or None where the kernel does not
+    take the call (other head sizes, rows that are not whole 16-byte pieces, weights that are not bf16)."""
+    tokens, N, KH = q.shape[0], q.shape[1] // H, k.shape[1] // H
+    assert _is2d_rowmajor(q) and _is2d_rowmajor(k) and q.dtype == k.dtype == torch.bfloat16 and k.shape[0] == tokens
+    assert positions.dtype == torch.int32 and positions.numel() == tokens and positions.is_contiguous()
+    assert cos.dtype == torch.float32 and cos.shape[1] == H // 2 and cos.is_contiguous() and sin.is_contiguous()
+    if wq is not None and not all(w.dtype == torch.bfloat16 and w.numel() == H and w.is_contiguous() for w in (wq, wk)):
+        return None
+    yq, yk = out if out is not None else (torch.empty((tokens, N * H), dtype=q.dtype, device=q.device),
+                                          torch.empty((tokens, KH * H), dtype=q.dtype, device=q.device))
+    rq = rk = None
+    if want_rstd:
+        rq, rk = torch.empty(tokens * (N + KH), dtype=torch.float32, device=q.device).split((tokens * N, tokens * KH))
+    rc = _lib.cuda().tb_qk_rope(q.data_ptr(), q.stride(0), yq.data_ptr(), yq.stride(0), _lib.ptr(wq), _lib.ptr(rq), N, k.data_ptr(),
+                                k.stride(0), yk.data_ptr(), yk.stride(0), _lib.ptr(wk), _lib.ptr(rk), KH, positions.data_ptr(),
+                                cos.data_ptr(), sin.data_ptr(), tokens, H, float(eps), 1.0 if add_one else 0.0, 1 if backward else 0,
+                                _lib.stream_ptr())
+    if rc == -2:
+        return None
+    _lib.check(rc, "tb_qk_rope")
+    _count()
+    return yq, yk, rq, rk
+
+
+def qk_rope_bwd(dq, dk, xq, xk, H: int, positions, cos, sin, wq, wk, rstd_q, rstd_k, add_one: bool = False, want_dw: bool = True):
+    """Gradients of `qk_rope` with norms: (dxq, dxk, dwq, dwk), the last two fp32 [H] or None; None for rows that are not whole 16-byte
+    pieces."""
+    tokens, N, KH = xq.shape[0], xq.shape[1] // H, xk.shape[1] // H
+    assert all(_is2d_rowmajor(t) and t.dtype == torch.bfloat16 for t in (dq, dk, xq, xk)) and dq.shape == xq.shape and dk.shape == xk.shape
+    dxq = torch.empty((tokens, N * H), dtype=torch.bfloat16, device=xq.device)
+    dxk = torch.empty((tokens, KH * H), dtype=torch.bfloat16, device=xq.device)
+    dwq, dwk = torch.zeros(2, H, dtype=torch.float32, device=xq.device).unbind(0) if want_dw else (None, None)
+    rc = _lib.cuda().tb_qk_rope_bwd(dq.data_ptr(), dq.stride(0), xq.data_ptr(), xq.stride(0), wq.data_ptr(), rstd_q.data_ptr(),
+                                    dxq.data_ptr(), N * H, _lib.ptr(dwq), N, dk.data_ptr(), dk.stride(0), xk.data_ptr(), xk.stride(0),
+                                    wk.data_ptr(), rstd_k.data_ptr(), dxk.data_ptr(), KH * H, _lib.ptr(dwk), KH, positions.data_ptr(),
+                                    cos.data_ptr(), sin.data_ptr(), tokens, H, 1.0 if add_one else 0.0, _lib.stream_ptr())
+    if rc == -2:
+        return None
+    _lib.check(rc, "tb_qk_rope_bwd")
+    _count()
+    return dxq, dxk, dwq, dwk
+
+
 GLU_SILU, GLU_GELU = 0, 1
 
 
