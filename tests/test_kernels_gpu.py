@@ -625,3 +625,48 @@ def test_model_joint_rotation_matches_separate(qk_norm):
     for a, b in zip(joint, sep):
         assert _rel_err(a, b) < 2e-2, (a.shape, _rel_err(a, b))        # a few roundings to bf16 apart
     _check_status()
+
+
+def _normal(*shape, seed):
+    return torch.randn(*shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
+
+
+@pytest.mark.parametrize("M,N,Ks", [(2065, 1304, (320, 136, 64)), (2065, 1304, (64, 8, 320)), (300, 72, (128, 64, 72))])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_gemm_sum_of_three_products(M, N, Ks, b_mn):
+    """Contractions that end inside a k-block, in any of the products; the last size is left to one GEMM a product."""
+    k = _k()
+    xs = [_normal(M, K_, seed=i).bfloat16() for i, K_ in enumerate(Ks)]
+    ws = [_normal(*((K_, N) if b_mn else (N, K_)), seed=9 + i).bfloat16() for i, K_ in enumerate(Ks)]
+    want = sum(x.double() @ (w.double() if b_mn else w.double().t()) for x, w in zip(xs, ws))
+    out = k.gemm_ext(*(t for p in zip(xs, ws) for t in p), b_mn=b_mn)
+    assert _rel_err(out, want) < (2e-3 if M > 300 else 5e-3)                 # one rounding, or one a product
+    _check_status()
+
+
+@pytest.mark.parametrize("M", [2065, 70])
+def test_joint_projections(M):
+    """Three projections of one input, with and without biases, into gradients of their own and into `main_grad`."""
+    from tunix_b200.ops import functional as F
+    D, outs = 328, (1024, 264, 264)
+    x = _normal(M, D, seed=1).bfloat16()
+    ws = [(0.1 * _normal(o, D, seed=2 + i)).bfloat16() for i, o in enumerate(outs)]
+    bs = [_normal(outs[0], seed=7).bfloat16(), None, _normal(outs[2], seed=8).bfloat16()]
+    dys = [_normal(M, o, seed=20 + i).bfloat16() for i, o in enumerate(outs)]
+    leaf = x.clone().requires_grad_()
+    wl = [w.clone().requires_grad_() for w in ws]
+    bl = [None if b is None else b.clone().requires_grad_() for b in bs]
+    wl[1].main_grad = torch.ones_like(wl[1], dtype=torch.float32)
+    ys = F.joint_linear(leaf, list(zip(wl, bl)))
+    torch.autograd.backward(ys, dys)
+    for y, w, b in zip(ys, ws, bs):
+        assert _rel_err(y, x.double() @ w.double().t() + (0 if b is None else b.double())) < 2e-3
+    assert _rel_err(leaf.grad, sum(d.double() @ w.double() for d, w in zip(dys, ws))) < (2e-3 if M > 100 else 5e-3)
+    for i, (w, d) in enumerate(zip(wl, dys)):
+        want = d.double().t() @ x.double()
+        if i == 1:
+            assert w.grad is None and w.grad_added_to_main_grad and _rel_err(w.main_grad, want + 1) < 1e-5
+        else:
+            assert _rel_err(w.grad, want) < 2e-3
+    assert _rel_err(bl[0].grad, dys[0].double().sum(0)) < 2e-3 and bl[1] is None
+    _check_status()

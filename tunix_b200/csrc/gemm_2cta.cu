@@ -40,9 +40,9 @@ enum { GF_A_MN = 1, GF_B_MN = 2, GF_OUT_F32 = 4, GF_ACCUM = 8, GF_BIAS = 16, GF_
 struct Args2 {
   int M, N, K, flags;
   int group;             // tiles are walked in groups of this many rows of tiles (negative: columns), see tile_group
-  // second contraction segment accumulated into the same TMEM tile: C += A2[M, K2] * B2[N, K2]^T with the layouts of
-  // A and B (a low-rank adapter update x A^T B^T carried by the base projection's GEMM); K2 = 0 when absent
-  int K2;
+  // further products accumulated into the same TMEM tile, C += A_i[M, K_i] * B_i[N, K_i]^T with the layouts of A and B (a low-rank adapter
+  // update carried by the base projection's GEMM, the input gradients of projections that share their input); 0 when absent
+  int K2, K3;
   void* C;
   long long ldc;
   const __nv_bfloat16* bias;
@@ -64,6 +64,11 @@ struct Args2 {
   const float* dz_dlogp;
   const float* dz_dent;
   const float* dz_ent;
+};
+
+constexpr int SEGS = 3;
+struct Maps2 {
+  CUtensorMap a[SEGS], b[SEGS];
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -114,8 +119,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
 }
 
 __global__ void __launch_bounds__(192, 1)
-gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-             const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2, const Args2 args) {
+gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -134,7 +138,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   const int M = args.M, N = args.N, K = args.K;
   const int num_m = (M + BM - 1) / BM, num_n = (N + BN - 1) / BN;
   const int num_kb1 = (K + BK - 1) / BK;                         // k-blocks of the main operands ...
-  const int num_kb = num_kb1 + (args.K2 + BK - 1) / BK;          // ... followed by those of the second segment
+  const int num_kb2 = num_kb1 + (args.K2 + BK - 1) / BK;         // ... followed by those of the second ...
+  const int num_kb = num_kb2 + (args.K3 + BK - 1) / BK;          // ... and the third product
   const int num_tiles = num_m * num_n;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const bool a_mn = args.flags & GF_A_MN, b_mn = args.flags & GF_B_MN;
@@ -150,12 +155,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     }
     *abort_flag = 0;
     mbar_fence_init();
-    if (args.K2 > 0) {
-      prefetch_tensormap(&tmA2);
-      prefetch_tensormap(&tmB2);
-    }
-    prefetch_tensormap(&tmA);
-    prefetch_tensormap(&tmB);
+    for (int i = 0; i < SEGS; ++i)
+      if (i == 0 || (i == 1 ? args.K2 : args.K3) > 0) {
+        prefetch_tensormap(&maps.a[i]);
+        prefetch_tensormap(&maps.b[i]);
+      }
   }
   if (warp == 1) {
     tmem_alloc2(smem_u32((const void*)tmem_ptr_smem), 2 * BN);
@@ -194,11 +198,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           const uint32_t sb = sa + A_BYTES;
           const uint32_t fb = mapa_u32(full_bar(stage), 0);           // the leader's barrier for this stage
           if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
-          // the second segment's maps zero-fill past K2, so a rank below 64 costs one padded k-block
-          const bool seg2 = kb >= num_kb1;
-          const CUtensorMap* ta = seg2 ? &tmA2 : &tmA;
-          const CUtensorMap* tb_ = seg2 ? &tmB2 : &tmB;
-          const int k0 = (seg2 ? kb - num_kb1 : kb) * BK;
+          // the maps zero-fill past the end of their contraction, so a rank below 64 costs one padded k-block
+          const int seg = kb < num_kb1 ? 0 : kb < num_kb2 ? 1 : 2;
+          const CUtensorMap *ta = &maps.a[seg], *tb_ = &maps.b[seg];
+          const int k0 = (kb - (seg == 0 ? 0 : seg == 1 ? num_kb1 : num_kb2)) * BK;
           if (!a_mn) {
             tma2_load_2d(sa, ta, fb, k0, m0);
           } else {
@@ -493,11 +496,10 @@ struct LseArgs {           // log-softmax epilogue request; partial == nullptr f
   const float* dz_dent = nullptr;
   const float* dz_ent = nullptr;
 };
-struct Seg2 {              // second contraction segment; K2 == 0 when absent
-  const void* A2 = nullptr;
-  const void* B2 = nullptr;
-  int K2 = 0;
-  long long lda2 = 0, ldb2 = 0;
+struct Product {           // a further product of the sum; K == 0 when absent
+  const void *A = nullptr, *B = nullptr;
+  int K = 0;
+  long long lda = 0, ldb = 0;
 };
 
 // partial [M, num_n, 4] -> logp[row] = z[target] - lse (0 for targets outside [0, V)), lse, entropy = lse - E[z]
@@ -541,7 +543,7 @@ __global__ void lse_combine_kernel(const float* __restrict__ partial, const int*
 namespace {
 int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                 int flags, const void* bias, const void* resid, long long ldr, float alpha, int* status,
-                cudaStream_t stream, const LseArgs& lse, const Seg2& seg = Seg2{}) {
+                cudaStream_t stream, const LseArgs& lse, const Product& p2 = Product{}, const Product& p3 = Product{}) {
   static const bool off = getenv("TUNIX_B200_NO_2CTA") != nullptr;
   if (off) return 0;
   static DeviceOnce once;
@@ -557,28 +559,27 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
   // worth it when the pairs have at least a wave of 256 x 256 tiles and the K loop amortises the prologue
   if (N < 256 || M < 256 || K < 256 || (long long)num_m * num_n < (pairs * 3) / 5) return 0;
   const bool a_mn = flags & GF_A_MN, b_mn = flags & GF_B_MN;
-  CUtensorMap tmA, tmB;
-  int r;
-  if (!a_mn) r = tb_make_tmap_2d_bf16(&tmA, A, M, K, lda, HM, BK, 1);
-  else       r = tb_make_tmap_2d_bf16(&tmA, A, K, M, lda, BK, 64, 1);
-  if (r) return -3;
-  if (!b_mn) r = tb_make_tmap_2d_bf16(&tmB, B, N, K, ldb, HN, BK, 1);
-  else       r = tb_make_tmap_2d_bf16(&tmB, B, K, N, ldb, BK, 64, 1);
-  if (r) return -4;
-  CUtensorMap tmA2 = tmA, tmB2 = tmB;
-  if (seg.K2 > 0) {
-    if ((seg.lda2 % 8) || (seg.ldb2 % 8) || (reinterpret_cast<uintptr_t>(seg.A2) & 15) ||
-        (reinterpret_cast<uintptr_t>(seg.B2) & 15))
-      return -2;
-    if (!a_mn) r = tb_make_tmap_2d_bf16(&tmA2, seg.A2, M, seg.K2, seg.lda2, HM, BK, 1);
-    else       r = tb_make_tmap_2d_bf16(&tmA2, seg.A2, seg.K2, M, seg.lda2, BK, 64, 1);
+  const Product sum[SEGS] = {{A, B, K, lda, ldb}, p2, p3};
+  Maps2 maps;
+  for (int i = 0; i < SEGS; ++i) {
+    const Product& q = sum[i];
+    if (q.K <= 0) {                                       // never loaded from
+      maps.a[i] = maps.a[0];
+      maps.b[i] = maps.b[0];
+      continue;
+    }
+    if ((q.lda % 8) || (q.ldb % 8) || ((reinterpret_cast<uintptr_t>(q.A) | reinterpret_cast<uintptr_t>(q.B)) & 15)) return -2;
+    int r;
+    if (!a_mn) r = tb_make_tmap_2d_bf16(&maps.a[i], q.A, M, q.K, q.lda, HM, BK, 1);
+    else       r = tb_make_tmap_2d_bf16(&maps.a[i], q.A, q.K, M, q.lda, BK, 64, 1);
     if (r) return -3;
-    if (!b_mn) r = tb_make_tmap_2d_bf16(&tmB2, seg.B2, N, seg.K2, seg.ldb2, HN, BK, 1);
-    else       r = tb_make_tmap_2d_bf16(&tmB2, seg.B2, seg.K2, N, seg.ldb2, BK, 64, 1);
+    if (!b_mn) r = tb_make_tmap_2d_bf16(&maps.b[i], q.B, N, q.K, q.ldb, HN, BK, 1);
+    else       r = tb_make_tmap_2d_bf16(&maps.b[i], q.B, q.K, N, q.ldb, BK, 64, 1);
     if (r) return -4;
   }
   Args2 a;
-  a.K2 = seg.K2;
+  a.K2 = p2.K;
+  a.K3 = p3.K;
   a.group = tile_group(num_m, num_n);
   a.M = M; a.N = N; a.K = K; a.flags = flags; a.C = C; a.ldc = ldc;
   a.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
@@ -600,7 +601,7 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, gemm2_kernel, tmA, tmB, tmA2, tmB2, a) != cudaSuccess) return -5;
+  if (cudaLaunchKernelEx(&cfg, gemm2_kernel, maps, a) != cudaSuccess) return -5;
   return 1;
 }
 }  // namespace
@@ -612,21 +613,21 @@ int tb_gemm_2cta_try(const void* A, const void* B, void* C, int M, int N, int K,
   return launch_2cta(A, B, C, M, N, K, lda, ldb, ldc, flags, bias, resid, ldr, alpha, status, stream, LseArgs{});
 }
 
-// C = epilogue(A * B^T + A2 * B2^T): the base projection with a low-rank update accumulated into the same TMEM tile
-// (A2 [M, K2] or [K2, M], B2 [N, K2] or [K2, N], laid out like A and B; K2 is the adapter rank, any multiple of 8).
-// Returns 1 when launched, 0 when the problem is too small for the two-SM kernel (the caller then runs the two
-// products separately), negative on error.
+// C = epilogue(A * B^T + A2 * B2^T (+ A3 * B3^T)): products accumulated into the same TMEM tile (a base projection with a low-rank update, the
+// input gradient of projections that share their input). A2 [M, K2] or [K2, M], B2 [N, K2] or [K2, N] and so on, laid out like A and B; K3 may
+// be 0. The output's rounding and its passes over memory happen once.
+// Returns 1 when launched, 0 when the problem is too small for the two-SM kernel (the caller then runs the products one by one), negative on
+// error.
 TB_API int tb_gemm_bf16_ext(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                             long long ldc, int flags, const void* bias, const void* resid, long long ldr, float alpha,
-                            const void* A2, const void* B2, int K2, long long lda2, long long ldb2, int* status,
-                            cudaStream_t stream) {
+                            const void* A2, const void* B2, int K2, long long lda2, long long ldb2, const void* A3, const void* B3, int K3,
+                            long long lda3, long long ldb3, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || K2 <= 0 || (K2 % 8) || (lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
+  if (K <= 0 || K2 <= 0 || (K2 % 8) || K3 < 0 || (K3 % 8) || (lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
       (reinterpret_cast<uintptr_t>(B) & 15))
     return -2;
-  Seg2 seg;
-  seg.A2 = A2; seg.B2 = B2; seg.K2 = K2; seg.lda2 = lda2; seg.ldb2 = ldb2;
-  return launch_2cta(A, B, C, M, N, K, lda, ldb, ldc, flags, bias, resid, ldr, alpha, status, stream, LseArgs{}, seg);
+  return launch_2cta(A, B, C, M, N, K, lda, ldb, ldc, flags, bias, resid, ldr, alpha, status, stream, LseArgs{}, {A2, B2, K2, lda2, ldb2},
+                     {A3, B3, K3, lda3, ldb3});
 }
 
 // log p(target) (and optionally lse / entropy) of z = softcap(h W^T) / temperature without materialising z:

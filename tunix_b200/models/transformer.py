@@ -76,6 +76,12 @@ def _joint_rows(parts):
     return joint
 
 
+def _bare(mod: nn.Module, kind: type) -> bool:
+    """Whether calling `mod` is no more than `kind.forward`: a joint kernel may then read its parameters and leave the call out."""
+    return type(mod) is kind and "forward" not in mod.__dict__ and not (
+        mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks or _has_any_global_hook())
+
+
 class Linear(nn.Module):
     """Linear layer with optional bias, LoRA adapters and NF4-quantised frozen base (QLoRA)."""
 
@@ -116,6 +122,13 @@ class Linear(nn.Module):
         return F.linear(x, self.weight, self.bias, residual)
 
 
+def _project(projs, x):
+    """The outputs of projections of one input, as one function where they are plain."""
+    if all(_bare(p, Linear) and p.lora_a is None and p.quant is None and getattr(p, "dp_shard", None) is None for p in projs):
+        return F.joint_linear(x, [(p.weight, p.bias) for p in projs])
+    return tuple(p(x) for p in projs)
+
+
 class RMSNorm(nn.Module):
     def __init__(self, dim: int, eps: float, add_one: bool, dtype=torch.float32, device=None):
         super().__init__()
@@ -125,12 +138,6 @@ class RMSNorm(nn.Module):
 
     def forward(self, x):
         return F.rmsnorm(x, self.weight, self.eps, self.add_one)
-
-
-def _bare(mod: nn.Module, kind: type) -> bool:
-    """Whether calling `mod` is no more than `kind.forward`: a joint kernel may then read its parameters and leave the call out."""
-    return type(mod) is kind and "forward" not in mod.__dict__ and not (
-        mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks or _has_any_global_hook())
 
 
 class Attention(nn.Module):
@@ -194,7 +201,7 @@ class Attention(nn.Module):
                 k = self.k_proj(xg)
                 v = self.v_proj(xg)
         else:
-            q, k, v = self.q_proj(x), self.k_proj(x), self.v_proj(x)
+            q, k, v = _project((self.q_proj, self.k_proj, self.v_proj), x)
         q, k = self._norm_and_rotate(q, k, positions, rope)
         v = v.view(B, T, K, H)
         seg_q = seg_k = segment_ids
@@ -258,7 +265,7 @@ class MLP(nn.Module):
             g, u = gu.split(gu.shape[-1] // 2, dim=-1)
             h = F.glu(g.contiguous(), u.contiguous(), self.kind)
             return tp_lib.row_parallel_linear(h, self.down_proj.weight, residual, tp)
-        h = F.glu(self.gate_proj(x), self.up_proj(x), self.kind)
+        h = F.glu(*_project((self.gate_proj, self.up_proj), x), self.kind)
         return self.down_proj(h, residual=residual)
 
 

@@ -109,6 +109,55 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
     return y if residual is None else y + residual
 
 
+def _weight_grad(w, dy2, x2):
+    """dy^T x, added into the weight's `main_grad` (None then) or returned."""
+    mg = getattr(w, "main_grad", None)
+    if mg is None:
+        return K.gemm(dy2, x2, a_mn=True, b_mn=True)
+    K.gemm(dy2, x2, a_mn=True, b_mn=True, out=mg, accumulate=True)
+    w.grad_added_to_main_grad = True
+    return None
+
+
+class _JointLinearFn(torch.autograd.Function):
+    """Two or three projections of one input. The gradient of the input is one sum of products (one launch, one rounding), where
+    projections on their own write one each for autograd to add."""
+
+    @staticmethod
+    def forward(ctx, x, *wb):
+        x2 = _flat2d(x)
+        ws, bs = wb[0::2], wb[1::2]
+        ys = []
+        for w, b in zip(ws, bs):
+            y = torch.empty((*x.shape[:-1], w.shape[0]), dtype=torch.bfloat16, device=x.device)
+            K.gemm(x2, w, bias=b, out=y.view(-1, w.shape[0]))
+            ys.append(y)
+        ctx.save_for_backward(x2, *ws)
+        ctx.refs, ctx.x_shape = wb, x.shape
+        return tuple(ys)
+
+    @staticmethod
+    def backward(ctx, *dys):
+        x2, *ws = ctx.saved_tensors
+        dy2 = [_flat2d(d) for d in dys]
+        dx = None
+        if ctx.needs_input_grad[0]:
+            dx = K.gemm_ext(*(t for d, w in zip(dy2, ws) for t in (d, w)), b_mn=True).view(ctx.x_shape)
+        out = []
+        for i, (d, (w, b)) in enumerate(zip(dy2, zip(ctx.refs[0::2], ctx.refs[1::2]))):
+            out.append(_weight_grad(w, d, x2) if ctx.needs_input_grad[1 + 2 * i] else None)
+            out.append(_deliver_grad(b, d.float().sum(0).to(d.dtype)) if b is not None and ctx.needs_input_grad[2 + 2 * i] else None)
+        return dx, *out
+
+
+def joint_linear(x, projs):
+    """[x @ w^T (+ bias)] for two or three (w, bias) of one input."""
+    if _native(x) and x.shape[-1] % 8 == 0 and len(projs) in (2, 3) and all(
+            w.dtype == torch.bfloat16 and w.shape[0] % 8 == 0 for w, _ in projs):
+        return _JointLinearFn.apply(x, *(t for p in projs for t in p))
+    return tuple(linear(x, w, b) for w, b in projs)
+
+
 class _LoraDeltaFn(torch.autograd.Function):
     """y = base + scale * (x A^T) B^T with A [r, in], B [out, r]."""
 

@@ -75,20 +75,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     return out
 
 
-def gemm_ext(a: torch.Tensor, b: torch.Tensor, a2: torch.Tensor, b2: torch.Tensor, *, b_mn: bool = False,
-             out: torch.Tensor | None = None, bias: torch.Tensor | None = None,
+def gemm_ext(a: torch.Tensor, b: torch.Tensor, a2: torch.Tensor, b2: torch.Tensor, a3: torch.Tensor | None = None,
+             b3: torch.Tensor | None = None, *, b_mn: bool = False, out: torch.Tensor | None = None, bias: torch.Tensor | None = None,
              residual: torch.Tensor | None = None) -> torch.Tensor:
-    """C = A @ op(B)^T + A2 @ op(B2)^T (+ bias) (+ residual) in ONE launch: the second product (a low-rank adapter
-    update) is a few extra k-blocks accumulated into the same TMEM tile.
+    """C = A @ op(B)^T + A2 @ op(B2)^T (+ A3 @ op(B3)^T) (+ bias) (+ residual) in ONE launch: the further products (a low-rank adapter
+    update, the input gradients of projections of the same input) are more k-blocks accumulated into the same TMEM tile.
 
-    a [M, K], a2 [M, r]; b [N, K] and b2 [N, r] (b_mn=False) or b [K, N] and b2 [r, N] (b_mn=True). Problems too small
-    for the two-SM kernel run as two GEMMs (the second adds the first as its residual)."""
-    assert a.dtype == b.dtype == a2.dtype == b2.dtype == torch.bfloat16
-    assert all(_is2d_rowmajor(t) for t in (a, b, a2, b2))
+    a [M, K], a2 [M, K2]; b [N, K] and b2 [N, K2] (b_mn=False) or b [K, N] and b2 [K2, N] (b_mn=True). Problems too small
+    for the two-SM kernel run as a GEMM a product (each adds the ones before as its residual)."""
+    prods = [(a, b), (a2, b2)] + ([(a3, b3)] if a3 is not None else [])
+    assert all(t.dtype == torch.bfloat16 and _is2d_rowmajor(t) for p in prods for t in p)
     M, K = a.shape
     N = b.shape[1] if b_mn else b.shape[0]
-    r = a2.shape[1]
-    assert a2.shape[0] == M and (b2.shape == (r, N) if b_mn else b2.shape == (N, r))
+    for x, w in prods[1:]:
+        assert x.shape[0] == M and (w.shape == (x.shape[1], N) if b_mn else w.shape == (N, x.shape[1]))
     if out is None:
         out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
     assert out.dtype == torch.bfloat16 and out.shape == (M, N) and out.stride(1) == 1
@@ -104,11 +104,12 @@ def gemm_ext(a: torch.Tensor, b: torch.Tensor, a2: torch.Tensor, b2: torch.Tenso
     if M == 0 or N == 0:
         return out
     rc = 0
-    if r % 8 == 0 and a2.stride(0) % 8 == 0 and b2.stride(0) % 8 == 0:
+    if all(x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 for x, w in prods[1:]):
         status = _lib.status_buffer(a.device)
+        more = [v for x, w in prods[1:] for v in (x.data_ptr(), w.data_ptr(), x.shape[1], x.stride(0), w.stride(0))]
         rc = _lib.cuda().tb_gemm_bf16_ext(
             a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), flags,
-            _lib.ptr(bias), _lib.ptr(residual), ldr, 1.0, a2.data_ptr(), b2.data_ptr(), r, a2.stride(0), b2.stride(0),
+            _lib.ptr(bias), _lib.ptr(residual), ldr, 1.0, *more, *((None, None, 0, 0, 0) if a3 is None else ()),
             status.data_ptr(), _lib.stream_ptr())
         if rc < 0:
             _lib.check(rc, "tb_gemm_bf16_ext")
@@ -116,7 +117,9 @@ def gemm_ext(a: torch.Tensor, b: torch.Tensor, a2: torch.Tensor, b2: torch.Tenso
         _count()
         return out
     gemm(a, b, b_mn=b_mn, out=out, bias=bias, residual=residual)
-    return gemm(a2, b2, b_mn=b_mn, out=out, residual=out)
+    for x, w in prods[1:]:
+        gemm(x, w, b_mn=b_mn, out=out, residual=out)
+    return out
 
 
 def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float, add_one: bool = False,
