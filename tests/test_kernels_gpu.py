@@ -644,6 +644,24 @@ def test_gemm_sum_of_three_products(M, N, Ks, b_mn):
     _check_status()
 
 
+@pytest.mark.parametrize("rows,D", [(1, 64), (77, 896), (300, 4096), (40, 6144), (9, 12288)])
+@pytest.mark.parametrize("frozen", [False, True])
+def test_rmsnorm_with_the_streams_gradient(rows, D, frozen):
+    """The norm's gradient and the one that passes it by, in one kernel, against their sum; in the kernels for narrow, wide and widest rows."""
+    from tunix_b200.ops import functional as F
+    x, w = _normal(rows, D, seed=1).bfloat16(), (1 + 0.1 * _normal(D, seed=2)).bfloat16()
+    dy, dres = _normal(rows, D, seed=3).bfloat16(), _normal(rows, D, seed=4).bfloat16()
+    leaf, wl = x.clone().requires_grad_(), w.clone().requires_grad_(not frozen)
+    y, kept = F.rmsnorm_keep(leaf, wl, 1e-6)
+    torch.autograd.backward([y, kept], [dy, dres])
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    yd = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * wd
+    torch.autograd.backward([yd, xd * 1.0], [dy.double(), dres.double()])
+    assert _rel_err(y, yd) < 2e-3 and torch.equal(kept, x) and _rel_err(leaf.grad, xd.grad) < 2e-3       # one rounding
+    assert frozen or _rel_err(wl.grad, wd.grad) < 4e-3
+    _check_status()
+
+
 @pytest.mark.parametrize("M", [2065, 70])
 def test_joint_projections(M):
     """Three projections of one input, with and without biases, into gradients of their own and into `main_grad`."""

@@ -31,6 +31,7 @@ _CUDA_SIGS = {
     "tb_tmap_cache_clear": [],
     "tb_rmsnorm_fwd": [P, LL, P, P, LL, P, I, I, F, F, P],
     "tb_rmsnorm_bwd": [P, LL, P, LL, P, P, P, LL, P, I, I, F, I, P],
+    "tb_rmsnorm_bwd_add": [P, LL, P, LL, P, P, P, LL, P, I, I, F, P, LL, P],
     "tb_rope": [P, LL, P, P, P, LL, I, I, I, P],
     "tb_qk_rope": [P, LL, P, LL, P, P, I, P, LL, P, LL, P, P, I, P, P, P, LL, I, F, F, I, P],
     "tb_qk_rope_bwd": [P, LL, P, LL, P, P, P, LL, P, I, P, LL, P, LL, P, P, P, LL, P, I, P, P, P, LL, I, F, P],

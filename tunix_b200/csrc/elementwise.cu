@@ -148,7 +148,7 @@ rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const
   }
 }
 
-// dx = rstd * (dy*w' - xhat * mean(dy*w'*xhat)), xhat = x*rstd, w' = w + add_one (dx += with accumulate != 0), and
+// dx = rstd * (dy*w' - xhat * mean(dy*w'*xhat)) (+ add: the residual stream's gradient, or dx itself), xhat = x*rstd, w' = w + add_one, and
 // dw[c] += sum_rows dy[r,c] * x[r,c] * rstd[r] (fp32 atomics into a zeroed buffer), in one pass over x and dy: a row is held in
 // registers between its reduction and its dx, and a thread keeps the sums of its columns over all its rows.
 //
@@ -164,7 +164,7 @@ template <int T>
 __global__ void __launch_bounds__(256)
 rmsnorm_bwd_narrow_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv_bfloat16* __restrict__ x, long long ldx,
                           const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                          long long lddx, float* __restrict__ dw, int rows, int D, float add_one, int accumulate) {
+                          long long lddx, float* __restrict__ dw, int rows, int D, float add_one, const __nv_bfloat16* add, long long ldadd) {
   __shared__ float s_dw[T * 8];
   const int sub = threadIdx.x % T, col = sub * 8;
   const bool in = col < D;
@@ -210,11 +210,11 @@ rmsnorm_bwd_narrow_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, 
       dot *= inv_d;
       if (r < rows && in) {
         float o[8];
-        if (accumulate) load8(dx + r * lddx + col, o);
+        if (add) load8(add + r * ldadd + col, o);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float t = rs[u] * (d[u][i] - v[u][i] * dot);
-          o[i] = accumulate ? o[i] + t : t;
+          o[i] = add ? o[i] + t : t;
         }
         store8(dx + r * lddx + col, o);
       }
@@ -240,7 +240,7 @@ template <int VPT>
 __global__ void __launch_bounds__(VPT == 1 ? 1024 : 512, 1)
 rmsnorm_bwd_row_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, const __nv_bfloat16* __restrict__ x, long long ldx,
                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                       long long lddx, float* __restrict__ dw, int rows, int D, float add_one, int accumulate) {
+                       long long lddx, float* __restrict__ dw, int rows, int D, float add_one, const __nv_bfloat16* add, long long ldadd) {
   __shared__ float red[RMS_GROUPS][2][16];
   extern __shared__ float s_dw[];                          // [D]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, grp = threadIdx.y;
@@ -279,12 +279,14 @@ rmsnorm_bwd_row_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, con
 #pragma unroll
   for (int q = 0; q < AHEAD; ++q) fetch(first + q * step, nx[q], nd[q], ns[q]);
   for (long long r = first; r < rows; r += step, turn ^= 1) {
-    uint4 cx[VPT], cd[VPT];
+    constexpr int EARLY = VPT <= 2 ? VPT : 1;              // of `add`: wider rows have no registers left for it
+    uint4 cx[VPT], cd[VPT], ca[EARLY];
     const float rs = ns[0];
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       cx[j] = nx[0][j];
       cd[j] = nd[0][j];
+      if (j < EARLY) ca[j] = add && col(j) < D ? *reinterpret_cast<const uint4*>(add + r * ldadd + col(j)) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int q = 0; q + 1 < AHEAD; ++q) {
@@ -324,12 +326,15 @@ rmsnorm_bwd_row_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy, con
       unpack(cx[j], v);
       unpack(cd[j], d);
       unpack(wq[j], g);
-      if (accumulate) load8(dx + r * lddx + col(j), o);
+      if (j < EARLY) {
+        unpack(ca[j], o);
+      } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float t = rs * (d[i] * (g[i] + add_one) - v[i] * rs * dot);
-        o[i] = accumulate ? o[i] + t : t;
+        for (int i = 0; i < 8; ++i) o[i] = 0.f;
+        if (add) load8(add + r * ldadd + col(j), o);
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] += rs * (d[i] * (g[i] + add_one) - v[i] * rs * dot);
       store8(dx + r * lddx + col(j), o);
     }
   }
@@ -366,7 +371,7 @@ __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, long
                                       const __nv_bfloat16* __restrict__ w,
                                       const float* __restrict__ rstd_in,
                                       __nv_bfloat16* __restrict__ dx, long long lddx, int rows,
-                                      int D, float add_one, int accumulate) {
+                                      int D, float add_one, const __nv_bfloat16* add, long long ldadd) {
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   for (long long row = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5); row < rows;
@@ -390,11 +395,11 @@ __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, long
       load8(xr + c, v);
       load8(w + c, g);
       load8(dyr + c, d);
-      if (accumulate) load8(dxr + c, o);
+      if (add) load8(add + row * ldadd + c, o);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         float r = rstd * (d[i] * (g[i] + add_one) - v[i] * rstd * dot);
-        o[i] = accumulate ? o[i] + r : r;
+        o[i] = add ? o[i] + r : r;
       }
       store8(dxr + c, o);
     }
@@ -696,9 +701,10 @@ TB_API int tb_rmsnorm_fwd(const void* x, long long ldx, const void* w, void* y, 
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long long ldx,
+// add: null, or [rows, D] bf16 (row stride ldadd, 16-byte pieces) that dx takes on top, dx itself among them
+TB_API int tb_rmsnorm_bwd_add(const void* dy, long long lddy, const void* x, long long ldx,
                           const void* w, const float* rstd, void* dx, long long lddx, float* dw,
-                          int rows, int D, float add_one, int accumulate_dx, cudaStream_t stream) {
+                          int rows, int D, float add_one, const void* add, long long ldadd, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (D % 8) return -2;
   if (!dx && !dw) return 0;
@@ -711,7 +717,7 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
   // dw alone needs no weight and no rows of 16-byte pieces: that call keeps the kernel for wide rows.
 #define RMS_BWD_ARGS                                                                                                          \
   (const __nv_bfloat16*)dy, lddy, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, rstd, (__nv_bfloat16*)dx, lddx, dw, rows, D, \
-      add_one, accumulate_dx
+      add_one, (const __nv_bfloat16*)add, ldadd
   const bool narrow = dx && (dw ? D <= 256 : D <= 128 && rows >= 4096);
   const bool fits = dx && D > 256 && D <= 16384;
   const bool by_row = dw ? fits && !(reinterpret_cast<uintptr_t>(dw) & 15)
@@ -721,7 +727,7 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
     if (dx)
       rmsnorm_bwd_dx_kernel<<<grid_for((long long)rows * 32, block), block, 0, stream>>>(
           (const __nv_bfloat16*)dy, lddy, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, rstd,
-          (__nv_bfloat16*)dx, lddx, rows, D, add_one, accumulate_dx);
+          (__nv_bfloat16*)dx, lddx, rows, D, add_one, (const __nv_bfloat16*)add, ldadd);
     if (dw) {
       dim3 grid((D + 127) / 128, (unsigned)min(128, (rows + 3) / 4));
       rmsnorm_bwd_dw_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, lddy,
@@ -747,6 +753,11 @@ TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long lo
   }
 #undef RMS_BWD_ARGS
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+TB_API int tb_rmsnorm_bwd(const void* dy, long long lddy, const void* x, long long ldx, const void* w, const float* rstd, void* dx,
+                          long long lddx, float* dw, int rows, int D, float add_one, int accumulate_dx, cudaStream_t stream) {
+  return tb_rmsnorm_bwd_add(dy, lddy, x, ldx, w, rstd, dx, lddx, dw, rows, D, add_one, accumulate_dx ? dx : nullptr, lddx, stream);
 }
 
 TB_API int tb_rope(void* x, long long ld, const int* pos, const float* cos_t, const float* sin_t,

@@ -315,6 +315,11 @@ class MoELayer(nn.Module):
         return y if residual is None else y + residual
 
 
+def _norm_keep(norm, x):
+    """(norm(x), x), for the residual stream to go on from the second: one function where the norm is plain."""
+    return F.rmsnorm_keep(x, norm.weight, norm.eps, norm.add_one) if _bare(norm, RMSNorm) else (norm(x), x)
+
+
 class DecoderLayer(nn.Module):
     def __init__(self, cfg: ModelConfig, layer_idx: int, device=None):
         super().__init__()
@@ -331,16 +336,17 @@ class DecoderLayer(nn.Module):
 
     def forward(self, x, positions, rope, cache=None, segment_ids=None, attention_mask=None, forced_experts=None):
         cfg = self.cfg
-        h = self.input_layernorm(x)
+        h, x = _norm_keep(self.input_layernorm, x)
         kw = {"forced_experts": forced_experts} if (forced_experts is not None and cfg.is_moe) else {}
         if cfg.post_norms:
             a, new_cache = self.self_attn(h, positions, rope, cache, segment_ids, attention_mask)
-            x = x + self.post_attn_norm(a)
-            m = self.mlp(self.post_attention_layernorm(x), **kw)
+            h, x = _norm_keep(self.post_attention_layernorm, x + self.post_attn_norm(a))
+            m = self.mlp(h, **kw)
             x = x + self.post_ffw_norm(m)
         else:
             x, new_cache = self.self_attn(h, positions, rope, cache, segment_ids, attention_mask, residual=x)
-            x = self.mlp(self.post_attention_layernorm(x), residual=x, **kw)
+            h, x = _norm_keep(self.post_attention_layernorm, x)
+            x = self.mlp(h, residual=x, **kw)
         return x, new_cache
 
 

@@ -271,10 +271,13 @@ class _RMSNormFn(torch.autograd.Function):
         return y
 
     @staticmethod
-    def backward(ctx, dy):
+    def backward(ctx, dy, add=None):
         x2, w, rstd = ctx.saved_tensors
         want_dw = ctx.needs_input_grad[1]
-        dx, dw = K.rmsnorm_bwd(_flat2d(dy), x2, w, rstd, ctx.add_one, want_dw=want_dw)
+        add = None if add is None else _flat2d(add)
+        if add is not None and (add.dtype != torch.bfloat16 or add.stride(0) % 8 or not _aligned16(add)):
+            add = add.to(torch.bfloat16).clone(memory_format=torch.contiguous_format)
+        dx, dw = K.rmsnorm_bwd(_flat2d(dy), x2, w, rstd, ctx.add_one, want_dw=want_dw, add=add)
         if dw is not None:
             mg = getattr(ctx.w_ref, "main_grad", None)
             if mg is not None:
@@ -284,6 +287,25 @@ class _RMSNormFn(torch.autograd.Function):
             else:
                 dw = dw.to(w.dtype)
         return dx.view(dy.shape), dw, None, None
+
+
+class _RMSNormKeepFn(torch.autograd.Function):
+    """(norm of x, x): what reaches x past the norm, the residual stream's gradient, joins the norm's own in one kernel."""
+
+    @staticmethod
+    def forward(ctx, x, w, eps, add_one):
+        return _RMSNormFn.forward(ctx, x, w, eps, add_one), x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, dres):
+        return _RMSNormFn.backward(ctx, dy, dres)
+
+
+def rmsnorm_keep(x, w, eps: float = 1e-6, add_one: bool = False):
+    """(rmsnorm(x), x) for a residual stream that goes on from x."""
+    if _native(x) and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and x.requires_grad and torch.is_grad_enabled():
+        return _RMSNormKeepFn.apply(x, w, eps, add_one)
+    return rmsnorm(x, w, eps, add_one), x
 
 
 def rmsnorm(x, w, eps: float = 1e-6, add_one: bool = False):

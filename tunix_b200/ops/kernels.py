@@ -138,20 +138,22 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float, add_one: bool = Fa
 
 
 def rmsnorm_bwd(dy, x, w, rstd, add_one: bool = False, want_dw: bool = True,
-                dx_accumulate_into: torch.Tensor | None = None):
-    """Returns (dx bf16 [rows,D], dw fp32 [D] or None)."""
+                dx_accumulate_into: torch.Tensor | None = None, add: torch.Tensor | None = None):
+    """Returns (dx bf16 [rows,D], dw fp32 [D] or None). `add` [rows, D] is added to dx (the gradient that reaches x past the norm);
+    `dx_accumulate_into` takes dx on top of what it holds."""
     rows, D = x.shape
     assert dy.stride(1) == 1 and x.stride(1) == 1
-    if dx_accumulate_into is not None:
-        dx = dx_accumulate_into
-        acc = 1
+    dx = dx_accumulate_into
+    if dx is not None:
+        assert add is None
+        add = dx
     else:
         dx = torch.empty((rows, D), dtype=torch.bfloat16, device=x.device)
-        acc = 0
+    assert add is None or (add.dtype == torch.bfloat16 and add.shape == (rows, D) and add.stride(1) == 1)
     dw = torch.zeros((D,), dtype=torch.float32, device=x.device) if want_dw else None
-    rc = _lib.cuda().tb_rmsnorm_bwd(dy.data_ptr(), dy.stride(0), x.data_ptr(), x.stride(0), w.data_ptr(),
-                                    rstd.data_ptr(), dx.data_ptr(), dx.stride(0), _lib.ptr(dw), rows, D,
-                                    1.0 if add_one else 0.0, acc, _lib.stream_ptr())
+    rc = _lib.cuda().tb_rmsnorm_bwd_add(dy.data_ptr(), dy.stride(0), x.data_ptr(), x.stride(0), w.data_ptr(),
+                                        rstd.data_ptr(), dx.data_ptr(), dx.stride(0), _lib.ptr(dw), rows, D, 1.0 if add_one else 0.0,
+                                        _lib.ptr(add), add.stride(0) if add is not None else 0, _lib.stream_ptr())
     _lib.check(rc, "tb_rmsnorm_bwd")
     _count(2 if want_dw and D > 16384 else 1)
     return dx, dw
