@@ -631,6 +631,32 @@ def _normal(*shape, seed):
     return torch.randn(*shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
 
 
+@pytest.mark.parametrize("M,N,K_,gap", [(2065, 1300, 320, 4), (2065, 1300, 320, 8), (2048, 1536, 256, 0), (5000, 776, 264, 24)])
+def test_gemm_result_blocks(M, N, K_, gap):
+    """Results of the two-SM kernel in blocks of 32 rows and 128 bytes: edges inside a block, rows that lie apart (1308 bf16 columns
+    are no whole 16-byte pieces and leave by a lane a row), every way the results leave, and nothing written beside them."""
+    k = _k()
+    a, b = _normal(M, K_, seed=1).bfloat16(), _normal(N, K_, seed=2).bfloat16()
+    bias, res = _normal(N, seed=3).bfloat16(), _normal(M, N, seed=4).bfloat16()
+    want = a.double() @ b.double().t()
+    for dtype, tol in ((torch.bfloat16, 2e-3), (torch.float32, 1e-5)):       # one rounding; sums of K_ products in 32 bits
+        for what in ("plain", "epilogue", "sum"):
+            wide = torch.full((M, N + gap), 3.0, device="cuda", dtype=dtype)
+            out = wide[:, :N]
+            if what == "plain":
+                k.gemm(a, b, out=out)
+                ref = want
+            elif what == "epilogue":
+                k.gemm(a, b, out=out, bias=bias, residual=res, alpha=0.5)
+                ref = 0.5 * want + bias.double() + res.double()
+            else:
+                k.gemm(a, b, out=out, accumulate=True, alpha=-0.25)
+                ref = 3.0 - 0.25 * want
+            assert _rel_err(out, ref) < tol, (dtype, what)
+            assert bool((wide[:, N:] == 3.0).all())
+    _check_status()
+
+
 @pytest.mark.parametrize("M,N,Ks", [(2065, 1304, (320, 136, 64)), (2065, 1304, (64, 8, 320)), (300, 72, (128, 64, 72))])
 @pytest.mark.parametrize("b_mn", [False, True])
 def test_gemm_sum_of_three_products(M, N, Ks, b_mn):

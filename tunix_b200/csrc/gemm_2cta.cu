@@ -32,8 +32,9 @@ constexpr int BM = 256, BN = 256, BK = 64, UMMA_K = 16;
 constexpr int HM = 128, HN = 128;                  // rows of A and of B staged by one CTA
 constexpr int STAGES = 6;
 constexpr int A_BYTES = HM * BK * 2, B_BYTES = HN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int STAGING_BYTES = 4 * 32 * 128;        // a 32 x 32 block of fp32 results per epilogue warp
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + STAGING_BYTES + 1024;
+constexpr int BLOCK_BYTES = 32 * 128;              // 32 rows of 64 bf16 or 32 fp32 results
+constexpr int STAGING_BYTES = 4 * 2 * BLOCK_BYTES; // two blocks per epilogue warp
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 256 + 1024;
 
 enum { GF_A_MN = 1, GF_B_MN = 2, GF_OUT_F32 = 4, GF_ACCUM = 8, GF_BIAS = 16, GF_RESIDUAL = 32 };
 
@@ -50,6 +51,7 @@ struct Args2 {
   long long ldr;
   float alpha;
   int* status;
+  int tma_c;               // the result leaves in blocks through maps.c
   // log-softmax epilogue (lm_head): instead of writing C, every tile leaves per row the online-softmax state of its
   // 256 columns and the target column's value, so logits never reach memory. partial: fp32 [M, num_n, 4] =
   // (max, sum exp(z - max), sum exp(z - max) z, z[target] or -inf when the target is in another tile).
@@ -69,6 +71,7 @@ struct Args2 {
 constexpr int SEGS = 3;
 struct Maps2 {
   CUtensorMap a[SEGS], b[SEGS];
+  CUtensorMap c;           // of the result, in blocks of 32 rows and 128 bytes
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -123,13 +126,13 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES + STAGING_BYTES;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };                       // used in the leader only
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };           // one per CTA
   auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };       // one per CTA
   auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + 2 + s); };  // used in the leader only
   volatile uint32_t* tmem_ptr_smem =
-      reinterpret_cast<volatile uint32_t*>(smem_al + STAGES * STAGE_BYTES + 8 * (2 * STAGES + 4));
+      reinterpret_cast<volatile uint32_t*>(smem_al + STAGES * STAGE_BYTES + STAGING_BYTES + 8 * (2 * STAGES + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -268,9 +271,9 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
     const bool c_al16 = (reinterpret_cast<uintptr_t>(args.C) & 15) == 0;
     const bool r_al16 = (reinterpret_cast<uintptr_t>(args.resid) & 15) == 0;
     const uint32_t tempty_leader0 = mapa_u32(tempty_bar(0), 0), tempty_leader1 = mapa_u32(tempty_bar(1), 0);
-    // sums into fp32 leave as reductions by rows of lanes (below)
-    const bool reduce = out_f32 && accum && !has_bias && !has_res && c_al16 && args.ldc % 4 == 0;
-    uint8_t* const staging = smem_al + STAGES * STAGE_BYTES + 256 + q * (32 * 128);
+    const bool b_al16 = (reinterpret_cast<uintptr_t>(args.bias) & 15) == 0;
+    uint8_t* const staging = smem_al + STAGES * STAGE_BYTES + q * 2 * BLOCK_BYTES;
+    int block = 0;                         // the staging block that is written next
     const bool lse_mode = args.partial != nullptr;
     const bool dz_mode = args.dz_lse != nullptr;
     for (int t = pair; t < num_tiles; t += num_pairs) {
@@ -338,120 +341,166 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         continue;
       }
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        const int col0 = n0 + c * 32;
-        if (col0 >= N) break;
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + c * 32, r);
-        tmem_ld_wait();
-        if (reduce && col0 + 32 <= N) {
-          // The block turns in shared memory, so that eight lanes add to a row's 128 bytes together, and nobody waits for C. With a
-          // lane a row every 16 bytes were loaded, added to and stored, 32 rows at a time: 4096 x 4096 x 4096 131 -> 106 us,
-          // 14336 x 4096 x 4096 406 -> 351 (358 by a lane a row). Results that are only stored leave faster by a lane a row.
+      // 32 columns of the row, up to what is stored
+      auto finish = [&](const uint32_t (&r)[32], int col0, float (&v)[32]) {
 #pragma unroll
-          for (int g = 0; g < 8; ++g)
-            *reinterpret_cast<float4*>(staging + lane * 128 + ((g ^ (lane & 7)) << 4)) =
-                make_float4(__uint_as_float(r[4 * g]) * alpha, __uint_as_float(r[4 * g + 1]) * alpha, __uint_as_float(r[4 * g + 2]) * alpha,
-                            __uint_as_float(r[4 * g + 3]) * alpha);
-          __syncwarp();
-          const int first = mt * BM + (int)rank * HM + q * 32 + (lane >> 3);
-          float* cp = reinterpret_cast<float*>(args.C) + col0 + (lane & 7) * 4;
+        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * alpha;
+        const bool full = (col0 + 32 <= N);
+        if (dz_mode) {
 #pragma unroll
-          for (int it = 0; it < 8; ++it) {
-            const int rr = it * 4 + (lane >> 3);
-            const float4 o = *reinterpret_cast<const float4*>(staging + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
-            if (first + it * 4 < M)
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(cp + (long long)(first + it * 4) * args.ldc), "f"(o.x),
-                           "f"(o.y), "f"(o.z), "f"(o.w) : "memory");
+          for (int i = 0; i < 32; ++i) {
+            float capped = v[i], chain = args.inv_temp;
+            if (args.softcap > 0.f) {
+              const float th = tanhf(v[i] / args.softcap);
+              capped = args.softcap * th;
+              chain *= (1.f - th * th);
+            }
+            const float z = capped * args.inv_temp;
+            const float p = __expf(z - dz_l);
+            float d = dz_gl * ((col0 + i == dz_t ? 1.f : 0.f) - p);
+            if (dz_ge != 0.f) d -= dz_ge * p * (z - dz_l + dz_en);
+            v[i] = d * chain;
           }
-          __syncwarp();
-          continue;
         }
-        if (row < M) {
-          float v[32];
+        if (has_bias) {
+          if (full && b_al16) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * alpha;
-          const bool full = (col0 + 32 <= N);
-          if (dz_mode) {
+            for (int g = 0; g < 4; ++g) {
+              const uint4 u = reinterpret_cast<const uint4*>(args.bias + col0)[g];
+              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              float capped = v[i], chain = args.inv_temp;
-              if (args.softcap > 0.f) {
-                const float th = tanhf(v[i] / args.softcap);
-                capped = args.softcap * th;
-                chain *= (1.f - th * th);
+              for (int j = 0; j < 4; ++j) {
+                v[g * 8 + 2 * j] += bf16_lo(w[j]);
+                v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
               }
-              const float z = capped * args.inv_temp;
-              const float p = __expf(z - dz_l);
-              float d = dz_gl * ((col0 + i == dz_t ? 1.f : 0.f) - p);
-              if (dz_ge != 0.f) d -= dz_ge * p * (z - dz_l + dz_en);
-              v[i] = d * chain;
-            }
-          }
-          if (has_bias) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (full || col0 + i < N) v[i] += __bfloat162float(args.bias[col0 + i]);
-          }
-          if (has_res) {
-            const __nv_bfloat16* rp = args.resid + (long long)row * args.ldr + col0;
-            if (full && (args.ldr % 8 == 0) && r_al16) {
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                const uint4 u = reinterpret_cast<const uint4*>(rp)[g];
-                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  v[g * 8 + 2 * j] += bf16_lo(w[j]);
-                  v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
-                }
-              }
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (col0 + i < N) v[i] += __bfloat162float(rp[i]);
-            }
-          }
-          if (out_f32) {
-            float* cp = reinterpret_cast<float*>(args.C) + (long long)row * args.ldc + col0;
-            if (full && (args.ldc % 4 == 0) && c_al16) {
-#pragma unroll
-              for (int g = 0; g < 8; ++g) {
-                float4 o = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-                if (accum) {
-                  const float4 p = reinterpret_cast<float4*>(cp)[g];
-                  o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w;
-                }
-                reinterpret_cast<float4*>(cp)[g] = o;
-              }
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (col0 + i < N) cp[i] = accum ? cp[i] + v[i] : v[i];
             }
           } else {
-            __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(args.C) + (long long)row * args.ldc + col0;
-            if (full && (args.ldc % 8 == 0) && c_al16) {
 #pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                if (accum) {
-                  const uint4 u = reinterpret_cast<uint4*>(cp)[g];
-                  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+            for (int i = 0; i < 32; ++i)
+              if (col0 + i < N) v[i] += __bfloat162float(args.bias[col0 + i]);
+          }
+        }
+        if (has_res) {
+          const __nv_bfloat16* rp = args.resid + (long long)row * args.ldr + col0;
+          if (full && (args.ldr % 8 == 0) && r_al16) {
 #pragma unroll
-                  for (int j = 0; j < 4; ++j) {
-                    v[g * 8 + 2 * j] += bf16_lo(w[j]);
-                    v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
+            for (int g = 0; g < 4; ++g) {
+              const uint4 u = reinterpret_cast<const uint4*>(rp)[g];
+              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                v[g * 8 + 2 * j] += bf16_lo(w[j]);
+                v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
+              }
+            }
+          } else {
+            for (int i = 0; i < 32; ++i)
+              if (col0 + i < N) v[i] += __bfloat162float(rp[i]);
+          }
+        }
+      };
+      if (args.tma_c) {
+        // Blocks of 32 rows and 128 bytes leave through shared memory and TMA, two in flight a warp: whole lines, and no thread waits for C
+        // or its address. Before, bf16 by a lane a row and fp32 sums by rows of lanes -> here (us, a loop under the power cap, the order of the
+        // tiles included): 4096^3 110 -> 107, 8192 x 1024 x 4096 (dgrad) 65 -> 58, added to bf16 4096^3 118 -> 113 and 4096 x 14336 x 4096
+        // 385 -> 364, added to fp32 404 -> 389.
+        const int row0 = mt * BM + (int)rank * HM + q * 32;
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; c += out_f32 ? 1 : 2) {
+          const int col0 = n0 + c * 32;
+          if (col0 >= N) break;
+          if (lane == 0) tma_store_wait_read<1>();         // the block's last store has read it
+          __syncwarp();
+          uint8_t* const to = staging + block * BLOCK_BYTES + lane * 128;
+          if (out_f32) {
+            uint32_t r[32];
+            tmem_ld_32x32(taddr + c * 32, r);
+            tmem_ld_wait();
+            float v[32];
+            if (row < M) finish(r, col0, v);
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              *reinterpret_cast<float4*>(to + ((g ^ (lane & 7)) << 4)) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+          } else {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              uint32_t r[32];
+              tmem_ld_32x32(taddr + (c + half) * 32, r);
+              tmem_ld_wait();
+              float v[32];
+              if (row < M) finish(r, col0 + half * 32, v);
+#pragma unroll
+              for (int g = 0; g < 4; ++g)
+                *reinterpret_cast<uint4*>(to + (((half * 4 + g) ^ (lane & 7)) << 4)) =
+                    make_uint4(pack_bf16(v[8 * g], v[8 * g + 1]), pack_bf16(v[8 * g + 2], v[8 * g + 3]),
+                               pack_bf16(v[8 * g + 4], v[8 * g + 5]), pack_bf16(v[8 * g + 6], v[8 * g + 7]));
+            }
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (row0 < M) {                                  // what lies past M or N in a block is left out by TMA
+            if (lane == 0) {
+              const uint32_t from = smem_u32(staging + block * BLOCK_BYTES);
+              if (out_f32 && accum) tma_reduce_add_2d(&maps.c, from, col0, row0);
+              else tma_store_2d(&maps.c, from, col0, row0);
+              tma_store_commit();
+            }
+            block ^= 1;
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          const int col0 = n0 + c * 32;
+          if (col0 >= N) break;
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + c * 32, r);
+          tmem_ld_wait();
+          if (row < M) {
+            float v[32];
+            finish(r, col0, v);
+            const bool full = (col0 + 32 <= N);
+            if (out_f32) {
+              float* cp = reinterpret_cast<float*>(args.C) + (long long)row * args.ldc + col0;
+              if (full && (args.ldc % 4 == 0) && c_al16) {
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                  float4 o = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+                  if (accum) {
+                    const float4 p = reinterpret_cast<float4*>(cp)[g];
+                    o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w;
                   }
+                  reinterpret_cast<float4*>(cp)[g] = o;
                 }
-                uint4 o;
-                o.x = pack_bf16(v[g * 8 + 0], v[g * 8 + 1]);
-                o.y = pack_bf16(v[g * 8 + 2], v[g * 8 + 3]);
-                o.z = pack_bf16(v[g * 8 + 4], v[g * 8 + 5]);
-                o.w = pack_bf16(v[g * 8 + 6], v[g * 8 + 7]);
-                reinterpret_cast<uint4*>(cp)[g] = o;
+              } else {
+                for (int i = 0; i < 32; ++i)
+                  if (col0 + i < N) cp[i] = accum ? cp[i] + v[i] : v[i];
               }
             } else {
-              for (int i = 0; i < 32; ++i)
-                if (col0 + i < N) cp[i] = __float2bfloat16(v[i] + (accum ? __bfloat162float(cp[i]) : 0.f));
+              __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(args.C) + (long long)row * args.ldc + col0;
+              if (full && (args.ldc % 8 == 0) && c_al16) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                  if (accum) {
+                    const uint4 u = reinterpret_cast<uint4*>(cp)[g];
+                    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                      v[g * 8 + 2 * j] += bf16_lo(w[j]);
+                      v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
+                    }
+                  }
+                  uint4 o;
+                  o.x = pack_bf16(v[g * 8 + 0], v[g * 8 + 1]);
+                  o.y = pack_bf16(v[g * 8 + 2], v[g * 8 + 3]);
+                  o.z = pack_bf16(v[g * 8 + 4], v[g * 8 + 5]);
+                  o.w = pack_bf16(v[g * 8 + 6], v[g * 8 + 7]);
+                  reinterpret_cast<uint4*>(cp)[g] = o;
+                }
+              } else {
+                for (int i = 0; i < 32; ++i)
+                  if (col0 + i < N) cp[i] = __float2bfloat16(v[i] + (accum ? __bfloat162float(cp[i]) : 0.f));
+              }
             }
           }
         }
@@ -461,6 +510,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       if (lane == 0) mbar_arrive_cluster(acc == 0 ? tempty_leader0 : tempty_leader1);
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
+    if (lane == 0) tma_store_wait_read<0>();
   }
 
   // ------------------------------------------------------------------ teardown
@@ -578,6 +628,19 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
     if (r) return -4;
   }
   Args2 a;
+  // Results in whole 16-byte pieces leave through TMA, columns included: what TMA leaves out past N it leaves out by such pieces. A sum into bf16 takes what is there as its residual, once and before the rounding
+  const bool f32 = flags & GF_OUT_F32;
+  a.tma_c = C != nullptr && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc % (f32 ? 4 : 8) == 0 && N % (f32 ? 4 : 8) == 0 &&
+            (f32 || (flags & (GF_ACCUM | GF_RESIDUAL)) != (GF_ACCUM | GF_RESIDUAL));
+  maps.c = maps.a[0];
+  if (a.tma_c) {
+    if (f32 ? tb_make_tmap_2d_f32(&maps.c, C, M, N, ldc, 32, 32) : tb_make_tmap_2d_bf16(&maps.c, C, M, N, ldc, 32, 64, 1)) return -4;
+    if (!f32 && (flags & GF_ACCUM)) {
+      flags = (flags & ~GF_ACCUM) | GF_RESIDUAL;
+      resid = C;
+      ldr = ldc;
+    }
+  }
   a.K2 = p2.K;
   a.K3 = p3.K;
   a.group = tile_group(num_m, num_n);
