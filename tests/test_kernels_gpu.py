@@ -579,7 +579,7 @@ def test_qk_rope(tokens, N, KH, H, gap, norm):
         a, b = y[..., :H // 2], y[..., H // 2:]
         want.append(torch.cat([a * c - b * s, b * c + a * s], -1).flatten(1))
     yq, yk, rq, rk = k.qk_rope(*xs, H, pos, cos, sin, wq=ws[0], wk=ws[1], eps=1e-6, add_one=True, want_rstd=norm)
-    # one rounding to bf16: at most 2^-9 of a value, about 2^-9 / sqrt(3) in the norm
+    # one rounding to bf16: at most 2^-8 of a value, about 1.7e-3 in the norm of many
     assert _rel_err(yq, want[0]) < 2e-3 and _rel_err(yk, want[1]) < 2e-3
     torch.autograd.backward(want, [d.double() for d in ds])
     if norm:
@@ -670,6 +670,37 @@ def test_gemm_sum_of_three_products(M, N, Ks, b_mn):
     _check_status()
 
 
+@pytest.mark.parametrize("kind", ["silu", "gelu"])
+@pytest.mark.parametrize("M,F_,D", [(2065, 1288, 1544), (4096, 768, 1536), (2065, 1288, 320)])
+def test_gated_products(M, F_, D, kind):
+    """The activation in the epilogue of the products in front of it; the last size is left to separate kernels."""
+    from tunix_b200.ops import functional as F
+    k = _k()
+    x, wg, wu = _normal(M, D, seed=1).bfloat16(), 0.05 * _normal(F_, D, seed=2), 0.05 * _normal(F_, D, seed=3)
+    wg, wu, wd = wg.bfloat16(), wu.bfloat16(), (0.1 * _normal(D, F_, seed=4)).bfloat16()
+    res, dy = _normal(M, D, seed=5).bfloat16(), _normal(M, D, seed=6).bfloat16()
+    kd = k.GLU_SILU if kind == "silu" else k.GLU_GELU
+    act = torch.nn.functional.silu if kind == "silu" else lambda t: torch.nn.functional.gelu(t, approximate="tanh")
+    g, u = x.double() @ wg.double().t(), x.double() @ wu.double().t()
+    kept, bare = k.gemm_glu(x, wg, wu, kd, keep=True), k.gemm_glu(x, wg, wu, kd)
+    assert (kept is None) == (D < 1536) and (bare is None) == (D < 1536)
+    # one rounding to bf16; the hardware tanh of the GELU adds an error of up to 5e-4 of a gate
+    tol = 2e-3 if kind == "silu" else 4e-3
+    if kept is not None:
+        assert _rel_err(kept[0], act(g) * u) < tol and _rel_err(kept[1], g) < 2e-3 and _rel_err(kept[2], u) < 2e-3
+        assert torch.equal(bare[0], kept[0]) and bare[1] is None
+    leaves = [t.clone().requires_grad_() for t in (x, wg, wu, wd, res)]
+    out = F.gated_mlp(*leaves[:4], kind, leaves[4])
+    ref = [t.double().requires_grad_() for t in (x, wg, wu, wd, res)]
+    want = (act(ref[0] @ ref[1].t()) * (ref[0] @ ref[2].t())) @ ref[3].t() + ref[4]
+    assert _rel_err(out, want) < 6e-3
+    out.backward(dy)
+    want.backward(dy.double())
+    for a, b in zip(leaves, ref):
+        assert _rel_err(a.grad, b.grad) < 1e-2, a.shape                      # gate, up and hidden rows rounded to bf16 on the way
+    _check_status()
+
+
 @pytest.mark.parametrize("rows,D", [(1, 64), (77, 896), (300, 4096), (40, 6144), (9, 12288)])
 @pytest.mark.parametrize("frozen", [False, True])
 def test_rmsnorm_with_the_streams_gradient(rows, D, frozen):
@@ -705,7 +736,8 @@ def test_joint_projections(M):
     torch.autograd.backward(ys, dys)
     for y, w, b in zip(ys, ws, bs):
         assert _rel_err(y, x.double() @ w.double().t() + (0 if b is None else b.double())) < 2e-3
-    assert _rel_err(leaf.grad, sum(d.double() @ w.double() for d, w in zip(dys, ws))) < (2e-3 if M > 100 else 5e-3)
+    # a rounding a product (1.7e-3 each in the norm), or one in all
+    assert _rel_err(leaf.grad, sum(d.double() @ w.double() for d, w in zip(dys, ws))) < 5e-3
     for i, (w, d) in enumerate(zip(wl, dys)):
         want = d.double().t() @ x.double()
         if i == 1:

@@ -5,6 +5,7 @@
 // Replaces the XLA elementwise fusions of the reference models
 // (RMSNorm: tunix/models/llama3/model.py:290-297, gemma (1+w): tunix/models/gemma/model.py:730-740,
 //  RoPE: tunix/models/llama3/model.py:249-270, SwiGLU/GeGLU: llama3/model.py:489-496, gemma/model.py:592-601).
+#include "activation.cuh"
 #include "common.cuh"
 
 using namespace tb;
@@ -509,22 +510,7 @@ rope_vec_kernel(__nv_bfloat16* __restrict__ x, long long ld, const int* __restri
   }
 }
 
-// ------------------------------------------------------------- gated activation
-__device__ __forceinline__ float act_fwd(float g, int kind) {
-  if (kind == 0) return g / (1.f + __expf(-g));  // SiLU
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;  // tanh-approximate GELU
-  return 0.5f * g * (1.f + tanhf(k0 * (g + k1 * g * g * g)));
-}
-__device__ __forceinline__ float act_bwd(float g, int kind) {
-  if (kind == 0) {
-    const float s = 1.f / (1.f + __expf(-g));
-    return s * (1.f + g * (1.f - s));
-  }
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float t = tanhf(k0 * (g + k1 * g * g * g));
-  return 0.5f * (1.f + t) + 0.5f * g * (1.f - t * t) * k0 * (1.f + 3.f * k1 * g * g);
-}
-
+// ------------------------------------------------------------- gated activation (act_fwd, act_bwd: activation.cuh)
 // h = act(g) * u ; all [rows, F] with row strides. F % 8 == 0.
 __global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ g, long long ldg,
                                const __nv_bfloat16* __restrict__ u, long long ldu,

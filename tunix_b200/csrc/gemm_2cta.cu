@@ -21,6 +21,7 @@
 //   * 6 stages x 32 KiB, TMEM 2 x 256 columns per CTA, every wait bounded, cluster barrier before teardown
 //
 // Operand layouts (K-major / MN-major) and epilogue flags are those of gemm.cu.
+#include "activation.cuh"
 #include "common.cuh"
 #include <cstdlib>
 
@@ -52,6 +53,9 @@ struct Args2 {
   float alpha;
   int* status;
   int tma_c;               // the result leaves in blocks through maps.c
+  // Gated feed-forward layers: B is the gate projection in maps.b[0] and the up projection in maps.b[1], a tile's columns 128 of
+  // each (N = their rows), and act(gate) * up leaves through maps.c[0], with gate and up through maps.c[1] and [2] if glu_keep.
+  int glu, glu_kind, glu_keep;
   // log-softmax epilogue (lm_head): instead of writing C, every tile leaves per row the online-softmax state of its
   // 256 columns and the target column's value, so logits never reach memory. partial: fp32 [M, num_n, 4] =
   // (max, sum exp(z - max), sum exp(z - max) z, z[target] or -inf when the target is in another tile).
@@ -71,7 +75,7 @@ struct Args2 {
 constexpr int SEGS = 3;
 struct Maps2 {
   CUtensorMap a[SEGS], b[SEGS];
-  CUtensorMap c;           // of the result, in blocks of 32 rows and 128 bytes
+  CUtensorMap c[3];        // of the results, in blocks of 32 rows and 128 bytes
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -139,7 +143,9 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int M = args.M, N = args.N, K = args.K;
-  const int num_m = (M + BM - 1) / BM, num_n = (N + BN - 1) / BN;
+  const bool glu = args.glu;
+  const int tile_n = glu ? BN / 2 : BN;
+  const int num_m = (M + BM - 1) / BM, num_n = (N + tile_n - 1) / tile_n;
   const int num_kb1 = (K + BK - 1) / BK;                         // k-blocks of the main operands ...
   const int num_kb2 = num_kb1 + (args.K2 + BK - 1) / BK;         // ... followed by those of the second ...
   const int num_kb = num_kb2 + (args.K3 + BK - 1) / BK;          // ... and the third product
@@ -191,7 +197,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
         int mt, nt;
         tile_coords(t, mt, nt);
-        const int m0 = mt * BM + (int)rank * HM, n0 = nt * BN + (int)rank * HN;
+        const int m0 = mt * BM + (int)rank * HM, n0 = nt * tile_n + (glu ? 0 : (int)rank * HN);
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1, abort_flag, args.status, ST_TIMEOUT_PRODUCER)) {
             ok = false;
@@ -203,7 +209,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
           if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
           // the maps zero-fill past the end of their contraction, so a rank below 64 costs one padded k-block
           const int seg = kb < num_kb1 ? 0 : kb < num_kb2 ? 1 : 2;
-          const CUtensorMap *ta = &maps.a[seg], *tb_ = &maps.b[seg];
+          const CUtensorMap *ta = &maps.a[seg], *tb_ = &maps.b[glu ? (int)rank : seg];
           const int k0 = (kb - (seg == 0 ? 0 : seg == 1 ? num_kb1 : num_kb2)) * BK;
           if (!a_mn) {
             tma2_load_2d(sa, ta, fb, k0, m0);
@@ -280,7 +286,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       int mt, nt;
       tile_coords(t, mt, nt);
       const int row = mt * BM + (int)rank * HM + q * 32 + lane;
-      const int n0 = nt * BN;
+      const int n0 = nt * tile_n;
       float dz_l = 0.f, dz_gl = 0.f, dz_ge = 0.f, dz_en = 0.f;
       int dz_t = -1;
       if (dz_mode && row < M) {
@@ -341,165 +347,195 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         continue;
       }
-      // 32 columns of the row, up to what is stored
-      auto finish = [&](const uint32_t (&r)[32], int col0, float (&v)[32]) {
+      const int row0 = mt * BM + (int)rank * HM + q * 32;
+      // a block of the staging memory, once its last store has read it; and its store (what lies past M or N is left out by TMA)
+      auto acquire = [&] {
+        if (lane == 0) tma_store_wait_read<1>();
+        __syncwarp();
+        return staging + block * BLOCK_BYTES + lane * 128;
+      };
+      auto release = [&](const CUtensorMap* to, int col0, bool sum) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (row0 >= M) return;
+        if (lane == 0) {
+          const uint32_t from = smem_u32(staging + block * BLOCK_BYTES);
+          if (sum) tma_reduce_add_2d(to, from, col0, row0);
+          else tma_store_2d(to, from, col0, row0);
+          tma_store_commit();
+        }
+        block ^= 1;
+      };
+      auto put = [&](uint8_t* to, int half, const float (&v)[32]) {       // 32 bf16 results of the lane's row
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          *reinterpret_cast<uint4*>(to + (((half * 4 + g) ^ (lane & 7)) << 4)) =
+              make_uint4(pack_bf16(v[8 * g], v[8 * g + 1]), pack_bf16(v[8 * g + 2], v[8 * g + 3]),
+                         pack_bf16(v[8 * g + 4], v[8 * g + 5]), pack_bf16(v[8 * g + 6], v[8 * g + 7]));
+      };
+      auto get = [&](int col, float (&v)[32]) {                           // 32 columns of the accumulator
+        uint32_t r[32];
+        __syncwarp();
+        tmem_ld_32x32(taddr + col, r);
+        tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * alpha;
-        const bool full = (col0 + 32 <= N);
-        if (dz_mode) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float capped = v[i], chain = args.inv_temp;
-            if (args.softcap > 0.f) {
-              const float th = tanhf(v[i] / args.softcap);
-              capped = args.softcap * th;
-              chain *= (1.f - th * th);
-            }
-            const float z = capped * args.inv_temp;
-            const float p = __expf(z - dz_l);
-            float d = dz_gl * ((col0 + i == dz_t ? 1.f : 0.f) - p);
-            if (dz_ge != 0.f) d -= dz_ge * p * (z - dz_l + dz_en);
-            v[i] = d * chain;
-          }
-        }
-        if (has_bias) {
-          if (full && b_al16) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const uint4 u = reinterpret_cast<const uint4*>(args.bias + col0)[g];
-              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                v[g * 8 + 2 * j] += bf16_lo(w[j]);
-                v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (col0 + i < N) v[i] += __bfloat162float(args.bias[col0 + i]);
-          }
-        }
-        if (has_res) {
-          const __nv_bfloat16* rp = args.resid + (long long)row * args.ldr + col0;
-          if (full && (args.ldr % 8 == 0) && r_al16) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const uint4 u = reinterpret_cast<const uint4*>(rp)[g];
-              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                v[g * 8 + 2 * j] += bf16_lo(w[j]);
-                v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
-              }
-            }
-          } else {
-            for (int i = 0; i < 32; ++i)
-              if (col0 + i < N) v[i] += __bfloat162float(rp[i]);
-          }
-        }
       };
-      if (args.tma_c) {
-        // Blocks of 32 rows and 128 bytes leave through shared memory and TMA, two in flight a warp: whole lines, and no thread waits for C
-        // or its address. Before, bf16 by a lane a row and fp32 sums by rows of lanes -> here (us, a loop under the power cap, the order of the
-        // tiles included): 4096^3 110 -> 107, 8192 x 1024 x 4096 (dgrad) 65 -> 58, added to bf16 4096^3 118 -> 113 and 4096 x 14336 x 4096
-        // 385 -> 364, added to fp32 404 -> 389.
-        const int row0 = mt * BM + (int)rank * HM + q * 32;
+      if (glu) {
 #pragma unroll 1
-        for (int c = 0; c < BN / 32; c += out_f32 ? 1 : 2) {
-          const int col0 = n0 + c * 32;
-          if (col0 >= N) break;
-          if (lane == 0) tma_store_wait_read<1>();         // the block's last store has read it
-          __syncwarp();
-          uint8_t* const to = staging + block * BLOCK_BYTES + lane * 128;
-          if (out_f32) {
-            uint32_t r[32];
-            tmem_ld_32x32(taddr + c * 32, r);
-            tmem_ld_wait();
-            float v[32];
-            if (row < M) finish(r, col0, v);
-#pragma unroll
-            for (int g = 0; g < 8; ++g)
-              *reinterpret_cast<float4*>(to + ((g ^ (lane & 7)) << 4)) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-          } else {
+        for (int c = 0; c < BN / 2; c += 64) {
+          if (n0 + c >= N) break;
+#pragma unroll 1
+          for (int o = args.glu_keep ? 2 : 0; o >= 0; --o) {
+            uint8_t* const to = acquire();
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-              uint32_t r[32];
-              tmem_ld_32x32(taddr + (c + half) * 32, r);
-              tmem_ld_wait();
               float v[32];
-              if (row < M) finish(r, col0 + half * 32, v);
+              get(c + half * 32 + (o == 2 ? BN / 2 : 0), v);
+              if (o == 0) {
+                float u[32];
+                get(BN / 2 + c + half * 32, u);
 #pragma unroll
-              for (int g = 0; g < 4; ++g)
-                *reinterpret_cast<uint4*>(to + (((half * 4 + g) ^ (lane & 7)) << 4)) =
-                    make_uint4(pack_bf16(v[8 * g], v[8 * g + 1]), pack_bf16(v[8 * g + 2], v[8 * g + 3]),
-                               pack_bf16(v[8 * g + 4], v[8 * g + 5]), pack_bf16(v[8 * g + 6], v[8 * g + 7]));
+                for (int i = 0; i < 32; ++i) v[i] = act_fwd(v[i], args.glu_kind) * u[i];
+              }
+              put(to, half, v);
             }
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (row0 < M) {                                  // what lies past M or N in a block is left out by TMA
-            if (lane == 0) {
-              const uint32_t from = smem_u32(staging + block * BLOCK_BYTES);
-              if (out_f32 && accum) tma_reduce_add_2d(&maps.c, from, col0, row0);
-              else tma_store_2d(&maps.c, from, col0, row0);
-              tma_store_commit();
-            }
-            block ^= 1;
+            release(&maps.c[o], n0 + c, false);
           }
         }
       } else {
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          const int col0 = n0 + c * 32;
-          if (col0 >= N) break;
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c * 32, r);
-          tmem_ld_wait();
-          if (row < M) {
-            float v[32];
-            finish(r, col0, v);
-            const bool full = (col0 + 32 <= N);
-            if (out_f32) {
-              float* cp = reinterpret_cast<float*>(args.C) + (long long)row * args.ldc + col0;
-              if (full && (args.ldc % 4 == 0) && c_al16) {
+        // 32 columns of the row, up to what is stored
+        auto finish = [&](float (&v)[32], int col0) {
+          const bool full = (col0 + 32 <= N);
+          if (dz_mode) {
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                  float4 o = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-                  if (accum) {
-                    const float4 p = reinterpret_cast<float4*>(cp)[g];
-                    o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w;
-                  }
-                  reinterpret_cast<float4*>(cp)[g] = o;
+            for (int i = 0; i < 32; ++i) {
+              float capped = v[i], chain = args.inv_temp;
+              if (args.softcap > 0.f) {
+                const float th = tanhf(v[i] / args.softcap);
+                capped = args.softcap * th;
+                chain *= (1.f - th * th);
+              }
+              const float z = capped * args.inv_temp;
+              const float p = __expf(z - dz_l);
+              float d = dz_gl * ((col0 + i == dz_t ? 1.f : 0.f) - p);
+              if (dz_ge != 0.f) d -= dz_ge * p * (z - dz_l + dz_en);
+              v[i] = d * chain;
+            }
+          }
+          if (has_bias) {
+            if (full && b_al16) {
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const uint4 u = reinterpret_cast<const uint4*>(args.bias + col0)[g];
+                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  v[g * 8 + 2 * j] += bf16_lo(w[j]);
+                  v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
                 }
-              } else {
-                for (int i = 0; i < 32; ++i)
-                  if (col0 + i < N) cp[i] = accum ? cp[i] + v[i] : v[i];
               }
             } else {
-              __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(args.C) + (long long)row * args.ldc + col0;
-              if (full && (args.ldc % 8 == 0) && c_al16) {
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                  if (accum) {
-                    const uint4 u = reinterpret_cast<uint4*>(cp)[g];
-                    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+              for (int i = 0; i < 32; ++i)
+                if (col0 + i < N) v[i] += __bfloat162float(args.bias[col0 + i]);
+            }
+          }
+          if (has_res) {
+            const __nv_bfloat16* rp = args.resid + (long long)row * args.ldr + col0;
+            if (full && (args.ldr % 8 == 0) && r_al16) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                      v[g * 8 + 2 * j] += bf16_lo(w[j]);
-                      v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
+              for (int g = 0; g < 4; ++g) {
+                const uint4 u = reinterpret_cast<const uint4*>(rp)[g];
+                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  v[g * 8 + 2 * j] += bf16_lo(w[j]);
+                  v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
+                }
+              }
+            } else {
+              for (int i = 0; i < 32; ++i)
+                if (col0 + i < N) v[i] += __bfloat162float(rp[i]);
+            }
+          }
+        };
+        if (args.tma_c) {
+          // Blocks of 32 rows and 128 bytes leave through shared memory and TMA, two in flight a warp: whole lines, and no thread waits for C
+          // or its address. bf16 results by a lane a row and fp32 sums by rows of lanes before (us): see launch_2cta.
+#pragma unroll 1
+          for (int c = 0; c < BN; c += out_f32 ? 32 : 64) {
+            const int col0 = n0 + c;
+            if (col0 >= N) break;
+            uint8_t* const to = acquire();
+            float v[32];
+            if (out_f32) {
+              get(c, v);
+              if (row < M) finish(v, col0);
+#pragma unroll
+              for (int g = 0; g < 8; ++g)
+                *reinterpret_cast<float4*>(to + ((g ^ (lane & 7)) << 4)) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+            } else {
+#pragma unroll
+              for (int half = 0; half < 2; ++half) {
+                get(c + half * 32, v);
+                if (row < M) finish(v, col0 + half * 32);
+                put(to, half, v);
+              }
+            }
+            release(&maps.c[0], col0, out_f32 && accum);
+          }
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < BN / 32; ++c) {
+            const int col0 = n0 + c * 32;
+            if (col0 >= N) break;
+            float v[32];
+            get(c * 32, v);
+            if (row < M) {
+              finish(v, col0);
+              const bool full = (col0 + 32 <= N);
+              if (out_f32) {
+                float* cp = reinterpret_cast<float*>(args.C) + (long long)row * args.ldc + col0;
+                if (full && (args.ldc % 4 == 0) && c_al16) {
+#pragma unroll
+                  for (int g = 0; g < 8; ++g) {
+                    float4 o = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+                    if (accum) {
+                      const float4 p = reinterpret_cast<float4*>(cp)[g];
+                      o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w;
                     }
+                    reinterpret_cast<float4*>(cp)[g] = o;
                   }
-                  uint4 o;
-                  o.x = pack_bf16(v[g * 8 + 0], v[g * 8 + 1]);
-                  o.y = pack_bf16(v[g * 8 + 2], v[g * 8 + 3]);
-                  o.z = pack_bf16(v[g * 8 + 4], v[g * 8 + 5]);
-                  o.w = pack_bf16(v[g * 8 + 6], v[g * 8 + 7]);
-                  reinterpret_cast<uint4*>(cp)[g] = o;
+                } else {
+                  for (int i = 0; i < 32; ++i)
+                    if (col0 + i < N) cp[i] = accum ? cp[i] + v[i] : v[i];
                 }
               } else {
-                for (int i = 0; i < 32; ++i)
-                  if (col0 + i < N) cp[i] = __float2bfloat16(v[i] + (accum ? __bfloat162float(cp[i]) : 0.f));
+                __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(args.C) + (long long)row * args.ldc + col0;
+                if (full && (args.ldc % 8 == 0) && c_al16) {
+#pragma unroll
+                  for (int g = 0; g < 4; ++g) {
+                    if (accum) {
+                      const uint4 u = reinterpret_cast<uint4*>(cp)[g];
+                      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                      for (int j = 0; j < 4; ++j) {
+                        v[g * 8 + 2 * j] += bf16_lo(w[j]);
+                        v[g * 8 + 2 * j + 1] += bf16_hi(w[j]);
+                      }
+                    }
+                    uint4 o;
+                    o.x = pack_bf16(v[g * 8 + 0], v[g * 8 + 1]);
+                    o.y = pack_bf16(v[g * 8 + 2], v[g * 8 + 3]);
+                    o.z = pack_bf16(v[g * 8 + 4], v[g * 8 + 5]);
+                    o.w = pack_bf16(v[g * 8 + 6], v[g * 8 + 7]);
+                    reinterpret_cast<uint4*>(cp)[g] = o;
+                  }
+                } else {
+                  for (int i = 0; i < 32; ++i)
+                    if (col0 + i < N) cp[i] = __float2bfloat16(v[i] + (accum ? __bfloat162float(cp[i]) : 0.f));
+                }
               }
             }
           }
@@ -545,6 +581,13 @@ struct LseArgs {           // log-softmax epilogue request; partial == nullptr f
   const float* dz_dlogp = nullptr;
   const float* dz_dent = nullptr;
   const float* dz_ent = nullptr;
+};
+struct GluArgs {           // gated form where `up` is given: B is the gate projection, up the other; g and u take the two unless null
+  int kind = 0;
+  const void* up = nullptr;
+  long long ldup = 0;
+  void *g = nullptr, *u = nullptr;
+  long long ldg = 0, ldu = 0;
 };
 struct Product {           // a further product of the sum; K == 0 when absent
   const void *A = nullptr, *B = nullptr;
@@ -593,7 +636,8 @@ __global__ void lse_combine_kernel(const float* __restrict__ partial, const int*
 namespace {
 int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                 int flags, const void* bias, const void* resid, long long ldr, float alpha, int* status,
-                cudaStream_t stream, const LseArgs& lse, const Product& p2 = Product{}, const Product& p3 = Product{}) {
+                cudaStream_t stream, const LseArgs& lse, const Product& p2 = Product{}, const Product& p3 = Product{},
+                const GluArgs& glu = GluArgs{}) {
   static const bool off = getenv("TUNIX_B200_NO_2CTA") != nullptr;
   if (off) return 0;
   static DeviceOnce once;
@@ -604,12 +648,14 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
     if (cudaFuncSetAttribute(gemm2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
       return -5;
   }
-  const int num_m = (M + BM - 1) / BM, num_n = (N + BN - 1) / BN;
+  const int tile_n = glu.up ? BN / 2 : BN;
+  const int num_m = (M + BM - 1) / BM, num_n = (N + tile_n - 1) / tile_n;
   const int pairs = g_sms2 / 2;
   // worth it when the pairs have at least a wave of 256 x 256 tiles and the K loop amortises the prologue
-  if (N < 256 || M < 256 || K < 256 || (long long)num_m * num_n < (pairs * 3) / 5) return 0;
+  if (N < tile_n || M < 256 || K < 256 || (long long)num_m * num_n < (pairs * 3) / 5) return 0;
   const bool a_mn = flags & GF_A_MN, b_mn = flags & GF_B_MN;
-  const Product sum[SEGS] = {{A, B, K, lda, ldb}, p2, p3};
+  // (the up projection takes the place of a second product: both read all of A)
+  const Product sum[SEGS] = {{A, B, K, lda, ldb}, glu.up ? Product{A, glu.up, K, lda, glu.ldup} : p2, p3};
   Maps2 maps;
   for (int i = 0; i < SEGS; ++i) {
     const Product& q = sum[i];
@@ -632,13 +678,25 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
   const bool f32 = flags & GF_OUT_F32;
   a.tma_c = C != nullptr && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc % (f32 ? 4 : 8) == 0 && N % (f32 ? 4 : 8) == 0 &&
             (f32 || (flags & (GF_ACCUM | GF_RESIDUAL)) != (GF_ACCUM | GF_RESIDUAL));
-  maps.c = maps.a[0];
+  for (CUtensorMap& c : maps.c) c = maps.a[0];
   if (a.tma_c) {
-    if (f32 ? tb_make_tmap_2d_f32(&maps.c, C, M, N, ldc, 32, 32) : tb_make_tmap_2d_bf16(&maps.c, C, M, N, ldc, 32, 64, 1)) return -4;
+    if (f32 ? tb_make_tmap_2d_f32(&maps.c[0], C, M, N, ldc, 32, 32) : tb_make_tmap_2d_bf16(&maps.c[0], C, M, N, ldc, 32, 64, 1)) return -4;
     if (!f32 && (flags & GF_ACCUM)) {
       flags = (flags & ~GF_ACCUM) | GF_RESIDUAL;
       resid = C;
       ldr = ldc;
+    }
+  }
+  a.glu = glu.up != nullptr;
+  a.glu_kind = glu.kind;
+  a.glu_keep = glu.g != nullptr;
+  if (glu.up) {
+    if (!a.tma_c) return 0;
+    auto rows_of_16 = [](const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 8 == 0; };
+    if (glu.g) {
+      if (!rows_of_16(glu.g, glu.ldg) || !rows_of_16(glu.u, glu.ldu)) return 0;
+      if (tb_make_tmap_2d_bf16(&maps.c[1], glu.g, M, N, glu.ldg, 32, 64, 1) || tb_make_tmap_2d_bf16(&maps.c[2], glu.u, M, N, glu.ldu, 32, 64, 1))
+        return -4;
     }
   }
   a.K2 = p2.K;
@@ -691,6 +749,22 @@ TB_API int tb_gemm_bf16_ext(const void* A, const void* B, void* C, int M, int N,
     return -2;
   return launch_2cta(A, B, C, M, N, K, lda, ldb, ldc, flags, bias, resid, ldr, alpha, status, stream, LseArgs{}, {A2, B2, K2, lda2, ldb2},
                      {A3, B3, K3, lda3, ldb3});
+}
+
+// h [M, F] = act(x Wg^T) * (x Wu^T), both products and the activation in one launch; gate and up projections [M, F] are written too where
+// g and u are given. x [M, K], Wg and Wu [F, K], bf16; F % 8 == 0. Returns 1 when launched, 0 when the call is left to separate kernels
+// (too small, or rows that are not whole 16-byte pieces), negative on error.
+// A loop under the power cap, us, two products and the activation by itself -> here, gate and up kept / not kept: 4096 x 14336 x 4096 742 -> 691 / 668,
+// 16384 x 12288 x 4096 2503 -> 2326 / 2230, 2048 x 8960 x 1536 115 -> 106 / 94, 512 x 8192 x 3072 61 -> 52 / 50. Below K = 1536 three results of a
+// tile take longer than its products: 2331 x 4864 x 896 59 -> 63 / 53. The activation's gradient in the epilogue of dy Wd was slower
+// everywhere (4096 x 14336 x 4096 442 -> 519): its rows of gate and up arrive by a lane a row.
+TB_API int tb_gemm_glu(const void* x, const void* wg, const void* wu, void* h, int M, int F, int K, long long ldx, long long ldwg,
+                       long long ldwu, long long ldh, void* g, void* u, long long ldg, long long ldu, int kind, int* status,
+                       cudaStream_t stream) {
+  if (M <= 0 || F <= 0 || K < 1536 || F % 8) return 0;
+  GluArgs a;
+  a.kind = kind; a.up = wu; a.ldup = ldwu; a.g = g; a.u = u; a.ldg = ldg; a.ldu = ldu;
+  return launch_2cta(x, wg, h, M, F, K, ldx, ldwg, ldh, 0, nullptr, nullptr, 0, 1.f, status, stream, LseArgs{}, Product{}, Product{}, a);
 }
 
 // log p(target) (and optionally lse / entropy) of z = softcap(h W^T) / temperature without materialising z:

@@ -389,7 +389,10 @@ class PagedEngine(BaseSampler):
         h2 = h.reshape(-1, h.shape[-1])
         pgu = self._pk(i, "gu") if decode else None
         kind = K.GLU_SILU if layer.mlp.kind == "silu" else K.GLU_GELU
-        if pgu is not None and pgu.glu:
+        joint = K.gemm_glu(h2, wgu[:Fd], wgu[Fd:], kind) if pgu is None else None
+        if joint is not None:
+            a = joint[0]
+        elif pgu is not None and pgu.glu:
             a = K.gemm_packed(h2, pgu, glu=kind)
         else:
             gu = K.gemm_packed(h2, pgu) if pgu is not None else F.linear(h2, wgu)

@@ -122,9 +122,14 @@ class Linear(nn.Module):
         return F.linear(x, self.weight, self.bias, residual)
 
 
+def _plain(projs) -> bool:
+    """Projections that are their weight and bias and nothing else, which a joint function may then read."""
+    return all(_bare(p, Linear) and p.lora_a is None and p.quant is None and getattr(p, "dp_shard", None) is None for p in projs)
+
+
 def _project(projs, x):
     """The outputs of projections of one input, as one function where they are plain."""
-    if all(_bare(p, Linear) and p.lora_a is None and p.quant is None and getattr(p, "dp_shard", None) is None for p in projs):
+    if _plain(projs):
         return F.joint_linear(x, [(p.weight, p.bias) for p in projs])
     return tuple(p(x) for p in projs)
 
@@ -265,7 +270,10 @@ class MLP(nn.Module):
             g, u = gu.split(gu.shape[-1] // 2, dim=-1)
             h = F.glu(g.contiguous(), u.contiguous(), self.kind)
             return tp_lib.row_parallel_linear(h, self.down_proj.weight, residual, tp)
-        h = F.glu(*_project((self.gate_proj, self.up_proj), x), self.kind)
+        projs = (self.gate_proj, self.up_proj, self.down_proj)
+        if _plain(projs) and all(p.bias is None for p in projs):
+            return F.gated_mlp(x, *(p.weight for p in projs), self.kind, residual)
+        h = F.glu(*_project(projs[:2], x), self.kind)
         return self.down_proj(h, residual=residual)
 
 

@@ -431,6 +431,53 @@ def glu(g, u, kind: str = "silu"):
     return R.glu_ref(g, u, kind)
 
 
+class _GatedMLPFn(torch.autograd.Function):
+    """act(x wg^T) * (x wu^T) wd^T (+ residual). Large calls apply the activation in the epilogue of the two products in front of it; the
+    gradient of x is one sum of products."""
+
+    @staticmethod
+    def forward(ctx, x, wg, wu, wd, residual, kind, keep):
+        x2 = _flat2d(x)
+        out = K.gemm_glu(x2, wg, wu, kind, keep)
+        if out is None:
+            g, u = K.gemm(x2, wg), K.gemm(x2, wu)
+            out = K.glu_fwd(g, u, kind), g, u
+        h, g, u = out
+        y = torch.empty((*x.shape[:-1], wd.shape[0]), dtype=torch.bfloat16, device=x.device)
+        K.gemm(h, wd, residual=_flat2d(residual) if residual is not None else None, out=y.view(-1, wd.shape[0]))
+        if keep:
+            ctx.save_for_backward(x2, wg, wu, wd, g, u, h)
+        ctx.refs, ctx.kind, ctx.x_shape = (wg, wu, wd), kind, x.shape
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x2, wg, wu, wd, g, u, h = ctx.saved_tensors
+        need_x, need_g, need_u, need_d, need_r = ctx.needs_input_grad[:5]
+        dy2 = _flat2d(dy)
+        dx = dwg = dwu = dwd = None
+        if need_x or need_g or need_u:
+            dg, du = K.glu_bwd(K.gemm(dy2, wd, b_mn=True), g, u, ctx.kind)
+        if need_d:
+            dwd = _weight_grad(ctx.refs[2], dy2, h)
+        if need_x:
+            dx = K.gemm_ext(dg, wg, du, wu, b_mn=True).view(ctx.x_shape)
+        if need_g:
+            dwg = _weight_grad(ctx.refs[0], dg, x2)
+        if need_u:
+            dwu = _weight_grad(ctx.refs[1], du, x2)
+        return dx, dwg, dwu, dwd, dy if need_r else None, None, None
+
+
+def gated_mlp(x, wg, wu, wd, kind: str = "silu", residual=None):
+    """act(x @ wg^T) * (x @ wu^T) @ wd^T (+ residual)."""
+    ws = (wg, wu, wd)
+    if _native(x) and all(w.dtype == torch.bfloat16 and w.shape[0] % 8 == 0 and w.shape[1] % 8 == 0 for w in ws):
+        keep = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, *ws, residual))
+        return _GatedMLPFn.apply(x, wg, wu, wd, residual, K.GLU_SILU if kind == "silu" else K.GLU_GELU, keep)
+    return linear(glu(linear(x, wg), linear(x, wu), kind), wd, residual=residual)
+
+
 # -------------------------------------------------------------------------- attention
 class _AttnFn(torch.autograd.Function):
     @staticmethod

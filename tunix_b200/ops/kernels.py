@@ -248,6 +248,25 @@ def glu_bwd(dh, g, u, kind: int, inplace: bool = False):
     return dg, du
 
 
+def gemm_glu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, kind: int, keep: bool = False):
+    """(act(x @ wg^T) * (x @ wu^T), gate, up), the last two only with `keep`, in one launch; None for calls that are left to separate
+    kernels (few rows, short rows, rows that are not whole 16-byte pieces)."""
+    assert all(t.dtype == torch.bfloat16 and _is2d_rowmajor(t) for t in (x, wg, wu)) and wg.shape == wu.shape and wg.shape[1] == x.shape[1]
+    (M, D), Fdim = x.shape, wg.shape[0]
+    if M < 256 or D < 1536 or Fdim % 8:
+        return None
+    h, g, u = (torch.empty((M, Fdim), dtype=torch.bfloat16, device=x.device) if want else None for want in (True, keep, keep))
+    rc = _lib.cuda().tb_gemm_glu(x.data_ptr(), wg.data_ptr(), wu.data_ptr(), h.data_ptr(), M, Fdim, D, x.stride(0), wg.stride(0),
+                                 wu.stride(0), Fdim, _lib.ptr(g), _lib.ptr(u), Fdim, Fdim, kind,
+                                 _lib.status_buffer(x.device).data_ptr(), _lib.stream_ptr())
+    if rc == 0:
+        return None
+    if rc < 0:
+        _lib.check(rc, "tb_gemm_glu")
+    _count()
+    return h, g, u
+
+
 def embedding_fwd(ids: torch.Tensor, table: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     assert ids.dtype == torch.int32 and ids.is_contiguous() and table.dtype == torch.bfloat16
     tokens = ids.numel()
