@@ -71,3 +71,55 @@ def test_moe_model_trains_and_matches_fallback():
     loss = logits.float().logsumexp(-1).mean()
     loss.backward()
     assert all(p.grad is not None and torch.isfinite(p.grad.float()).all() for p in layer.parameters())
+
+
+@pytest.mark.parametrize("T,E,k,D,Fd,acc", [(2100, 4, 2, 320, 384, None), (1100, 4, 1, 256, 320, torch.bfloat16), (1500, 3, 2, 512, 256, torch.float32)])
+def test_experts_on_sm_pairs(T, E, k, D, Fd, acc):
+    """Enough rows an expert for the products on SM pairs: segments of an odd number of 128 rows, an expert without rows, columns that end
+    inside a tile, gradients of their own and added to what is there."""
+    from tunix_b200 import _lib
+    from tunix_b200.ops import kernels as K
+    from tunix_b200.ops import moe
+    g = torch.Generator(device="cuda").manual_seed(0)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    x = (rnd(T, D) * 0.5).to(torch.bfloat16).requires_grad_()
+    ws = [(rnd(E, *s) * 0.08).to(torch.bfloat16).requires_grad_() for s in ((Fd, D), (Fd, D), (D, Fd))]
+    assert K.moe_on_pairs(T * k, E, Fd, D, *ws)
+    logits = rnd(T, E)
+    logits[:, 1] = -1e9 if k < E - 1 else -2.0            # an expert nobody picks
+    wts, idx = torch.topk(torch.softmax(logits, -1), k, -1)
+    wts = wts.detach().requires_grad_()
+    if acc is not None:
+        for w in ws:
+            w.main_grad = torch.full(w.shape, 0.5, device="cuda", dtype=acc)
+    out = moe.experts(x, wts, idx, *ws)
+    dout = rnd(T, D).to(torch.bfloat16)
+    out.backward(dout)
+    _lib.raise_if_kernel_error()
+    xr, wr, *rs = (t.detach().double().requires_grad_() for t in (x, wts, *ws))
+    sel = torch.nn.functional.one_hot(idx, E).double() * wr[..., None]
+    ref = sum(sel[:, :, e].sum(1, keepdim=True) * ((torch.nn.functional.silu(xr @ rs[0][e].t()) * (xr @ rs[1][e].t())) @ rs[2][e].t())
+              for e in range(E))
+    ref.backward(dout.double())
+
+    def rel(a, b):
+        return ((a.double() - b).norm() / (b.norm() + 1e-6)).item()
+    assert rel(out, ref) < 1e-2 and rel(x.grad, xr.grad) < 1e-2 and rel(wts.grad, wr.grad) < 1e-2
+    for w, r in zip(ws, rs):
+        assert rel(w.grad, r.grad) < 1e-2 if acc is None else rel(w.main_grad, r.grad + 0.5) < 1e-2
+
+
+def test_row_tiles_cover_every_segment_once():
+    """The planned tiles of 128 and 256 rows against the segments, empty ones and an odd number of 128 rows among them."""
+    import numpy as np
+    from tunix_b200.ops import kernels as K
+    sizes = [0, 128, 384, 0, 256, 1280, 128] + [128 * (i % 4) for i in range(120)]
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    seg = torch.tensor(off, dtype=torch.int32, device="cuda")
+    for kw, bm, bn in (({}, 128, 256), ({"pairs": True}, 256, 256), ({"pairs": True, "glu": True}, 256, 128)):
+        tl = K.moe_tiles_rows(seg, int(off[-1]), 640, 192, 640, **kw)
+        n = int(tl.count)
+        d = tl.desc[:n * 32].cpu().numpy().view(np.int32).reshape(n, 8)
+        want = [(off[e] + m, c, min(off[e] + m + bm, off[e + 1]), 0, 3, e * 640) for e in range(len(sizes)) for m in range(0, sizes[e], bm)
+                for c in range(0, 640, bn)]
+        assert n <= tl.max_tiles and [tuple(r[:6]) for r in d.tolist()] == [tuple(int(v) for v in w) for w in want]

@@ -39,7 +39,15 @@ constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 256 + 1024;
 
 enum { GF_A_MN = 1, GF_B_MN = 2, GF_OUT_F32 = 4, GF_ACCUM = 8, GF_BIAS = 16, GF_RESIDUAL = 32 };
 
+// Grouped products (mixtures of experts): the tiles come from a list in device memory, as in gemm.cu, planned for 256 rows a tile.
+struct TileDesc {          // must match gemm.cu
+  int m0, n0, m_end, kb0, kb1, b_row0;
+  long long c_off;
+};
+
 struct Args2 {
+  const TileDesc* tiles;   // null: a dense problem
+  const int* num_tiles_dev;
   int M, N, K, flags;
   int group;             // tiles are walked in groups of this many rows of tiles (negative: columns), see tile_group
   // further products accumulated into the same TMEM tile, C += A_i[M, K_i] * B_i[N, K_i]^T with the layouts of A and B (a low-rank adapter
@@ -149,7 +157,8 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
   const int num_kb1 = (K + BK - 1) / BK;                         // k-blocks of the main operands ...
   const int num_kb2 = num_kb1 + (args.K2 + BK - 1) / BK;         // ... followed by those of the second ...
   const int num_kb = num_kb2 + (args.K3 + BK - 1) / BK;          // ... and the third product
-  const int num_tiles = num_m * num_n;
+  const bool grouped = args.tiles != nullptr;
+  const int num_tiles = grouped ? *args.num_tiles_dev : num_m * num_n;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const bool a_mn = args.flags & GF_A_MN, b_mn = args.flags & GF_B_MN;
 
@@ -179,13 +188,20 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  auto tile_coords = [&](int t, int& mt, int& nt) {
+  // first row and column, end of the rows, k-blocks, what is added to B's row, and the row of C that row 0 of the output is
+  struct Tile {
+    int m0, n0, m_end, kb0, kb1, b_row0, c_row0;
+  };
+  auto tile_at = [&](int t) -> Tile {
+    if (grouped) {
+      const TileDesc d = args.tiles[t];
+      return {d.m0, d.n0, d.m_end, d.kb0, d.kb1, d.b_row0, d.c_off ? (int)(d.c_off / args.ldc) : 0};
+    }
     const bool by_n = args.group < 0;
     const int size = by_n ? -args.group : args.group, along = by_n ? num_n : num_m, across = by_n ? num_m : num_n;
     const int g = t / (size * across), first = g * size, r = t - first * across, here = min(size, along - first);
     const int a = first + r % here, b = r / here;
-    mt = by_n ? b : a;
-    nt = by_n ? a : b;
+    return {(by_n ? b : a) * BM, (by_n ? a : b) * tile_n, M, 0, num_kb, 0, 0};
   };
 
   if (warp == 0) {
@@ -195,10 +211,9 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       uint32_t phase = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-        int mt, nt;
-        tile_coords(t, mt, nt);
-        const int m0 = mt * BM + (int)rank * HM, n0 = nt * tile_n + (glu ? 0 : (int)rank * HN);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const Tile tile = tile_at(t);
+        const int m0 = tile.m0 + (int)rank * HM, n0 = tile.n0 + (glu ? 0 : (int)rank * HN);
+        for (int kb = tile.kb0; kb < tile.kb1; ++kb) {
           if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1, abort_flag, args.status, ST_TIMEOUT_PRODUCER)) {
             ok = false;
             break;
@@ -208,7 +223,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
           const uint32_t fb = mapa_u32(full_bar(stage), 0);           // the leader's barrier for this stage
           if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
           // the maps zero-fill past the end of their contraction, so a rank below 64 costs one padded k-block
-          const int seg = kb < num_kb1 ? 0 : kb < num_kb2 ? 1 : 2;
+          const int seg = kb < num_kb1 || grouped && args.K2 == 0 ? 0 : kb < num_kb2 ? 1 : 2;
           const CUtensorMap *ta = &maps.a[seg], *tb_ = &maps.b[glu ? (int)rank : seg];
           const int k0 = (kb - (seg == 0 ? 0 : seg == 1 ? num_kb1 : num_kb2)) * BK;
           if (!a_mn) {
@@ -218,10 +233,10 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
             for (int j = 0; j < HM / 64; ++j) tma2_load_2d(sa + j * 8192, ta, fb, m0 + 64 * j, k0);
           }
           if (!b_mn) {
-            tma2_load_2d(sb, tb_, fb, k0, n0);
+            tma2_load_2d(sb, tb_, fb, k0, n0 + tile.b_row0);
           } else {
 #pragma unroll
-            for (int j = 0; j < HN / 64; ++j) tma2_load_2d(sb + j * 8192, tb_, fb, n0 + 64 * j, k0);
+            for (int j = 0; j < HN / 64; ++j) tma2_load_2d(sb + j * 8192, tb_, fb, n0 + 64 * j, k0 + tile.b_row0);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -239,10 +254,15 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
+        int kb0 = 0, kb1 = num_kb;
+        if (grouped) {
+          kb0 = args.tiles[t].kb0;
+          kb1 = args.tiles[t].kb1;
+        }
         if (!mbar_wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag, args.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_bounded(full_bar(stage), phase, abort_flag, args.status, ST_TIMEOUT_MMA)) {
             ok = false;
             break;
@@ -254,7 +274,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t ad = make_smem_desc(sa + k * a_kstep, a_lbo, 1024);
             const uint64_t bd = make_smem_desc(sb + k * b_kstep, b_lbo, 1024);
-            umma2_f16_ss(tmem_d, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma2_f16_ss(tmem_d, ad, bd, idesc, kb > kb0 || k > 0 ? 1u : 0u);
           }
           umma2_commit(empty_bar(stage));                              // frees the stage here ...
           umma2_commit(mapa_u32(empty_bar(stage), 1));                 // ... and in the peer
@@ -283,13 +303,13 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
     const bool lse_mode = args.partial != nullptr;
     const bool dz_mode = args.dz_lse != nullptr;
     for (int t = pair; t < num_tiles; t += num_pairs) {
-      int mt, nt;
-      tile_coords(t, mt, nt);
-      const int row = mt * BM + (int)rank * HM + q * 32 + lane;
-      const int n0 = nt * tile_n;
+      const Tile tile = tile_at(t);
+      const int row = tile.m0 + (int)rank * HM + q * 32 + lane, row_end = tile.m_end, c_row = tile.c_row0 + row;
+      const int n0 = tile.n0;
+      const bool none = tile.kb1 <= tile.kb0;              // an expert without rows: its part of a sum over rows is zero
       float dz_l = 0.f, dz_gl = 0.f, dz_ge = 0.f, dz_en = 0.f;
       int dz_t = -1;
-      if (dz_mode && row < M) {
+      if (dz_mode && row < row_end) {
         dz_l = args.dz_lse[row];
         dz_ge = args.dz_dent ? args.dz_dent[row] : 0.f;
         dz_en = (args.dz_dent && args.dz_ent) ? args.dz_ent[row] : 0.f;
@@ -303,7 +323,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       if (lse_mode) {
         // one thread owns one row of the tile: the softmax statistics of its 256 columns need no communication
         float mx = -INFINITY, sm = 0.f, sz = 0.f, zt = -INFINITY;
-        const int tgt = row < M ? args.targets[row] : -1;
+        const int tgt = row < row_end ? args.targets[row] : -1;
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
           const int col0 = n0 + c * 32;
@@ -339,15 +359,15 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
           sz = sz * corr + z2;
           mx = nm;
         }
-        if (row < M)
-          *reinterpret_cast<float4*>(args.partial + ((long long)row * num_n + nt) * 4) = make_float4(mx, sm, sz, zt);
+        if (row < row_end)
+          *reinterpret_cast<float4*>(args.partial + ((long long)row * num_n + n0 / BN) * 4) = make_float4(mx, sm, sz, zt);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(acc == 0 ? tempty_leader0 : tempty_leader1);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         continue;
       }
-      const int row0 = mt * BM + (int)rank * HM + q * 32;
+      const int row0 = row - lane;
       // a block of the staging memory, once its last store has read it; and its store (what lies past M or N is left out by TMA)
       auto acquire = [&] {
         if (lane == 0) tma_store_wait_read<1>();
@@ -357,11 +377,11 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       auto release = [&](const CUtensorMap* to, int col0, bool sum) {
         fence_proxy_async_smem();
         __syncwarp();
-        if (row0 >= M) return;
+        if (row0 >= row_end) return;
         if (lane == 0) {
           const uint32_t from = smem_u32(staging + block * BLOCK_BYTES);
-          if (sum) tma_reduce_add_2d(to, from, col0, row0);
-          else tma_store_2d(to, from, col0, row0);
+          if (sum) tma_reduce_add_2d(to, from, col0, tile.c_row0 + row0);
+          else tma_store_2d(to, from, col0, tile.c_row0 + row0);
           tma_store_commit();
         }
         block ^= 1;
@@ -379,7 +399,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
         tmem_ld_32x32(taddr + col, r);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * alpha;
+        for (int i = 0; i < 32; ++i) v[i] = none ? 0.f : __uint_as_float(r[i]) * alpha;
       };
       if (glu) {
 #pragma unroll 1
@@ -442,7 +462,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
             }
           }
           if (has_res) {
-            const __nv_bfloat16* rp = args.resid + (long long)row * args.ldr + col0;
+            const __nv_bfloat16* rp = args.resid + (long long)c_row * args.ldr + col0;
             if (full && (args.ldr % 8 == 0) && r_al16) {
 #pragma unroll
               for (int g = 0; g < 4; ++g) {
@@ -471,7 +491,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
             float v[32];
             if (out_f32) {
               get(c, v);
-              if (row < M) finish(v, col0);
+              if (row < row_end) finish(v, col0);
 #pragma unroll
               for (int g = 0; g < 8; ++g)
                 *reinterpret_cast<float4*>(to + ((g ^ (lane & 7)) << 4)) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
@@ -479,7 +499,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
 #pragma unroll
               for (int half = 0; half < 2; ++half) {
                 get(c + half * 32, v);
-                if (row < M) finish(v, col0 + half * 32);
+                if (row < row_end) finish(v, col0 + half * 32);
                 put(to, half, v);
               }
             }
@@ -492,11 +512,11 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
             if (col0 >= N) break;
             float v[32];
             get(c * 32, v);
-            if (row < M) {
+            if (row < row_end) {
               finish(v, col0);
               const bool full = (col0 + 32 <= N);
               if (out_f32) {
-                float* cp = reinterpret_cast<float*>(args.C) + (long long)row * args.ldc + col0;
+                float* cp = reinterpret_cast<float*>(args.C) + (long long)c_row * args.ldc + col0;
                 if (full && (args.ldc % 4 == 0) && c_al16) {
 #pragma unroll
                   for (int g = 0; g < 8; ++g) {
@@ -512,7 +532,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
                     if (col0 + i < N) cp[i] = accum ? cp[i] + v[i] : v[i];
                 }
               } else {
-                __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(args.C) + (long long)row * args.ldc + col0;
+                __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(args.C) + (long long)c_row * args.ldc + col0;
                 if (full && (args.ldc % 8 == 0) && c_al16) {
 #pragma unroll
                   for (int g = 0; g < 4; ++g) {
@@ -634,20 +654,41 @@ __global__ void lse_combine_kernel(const float* __restrict__ partial, const int*
 }  // namespace
 
 namespace {
+bool setup_2cta() {
+  static DeviceOnce once;
+  if (once.first()) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_sms2, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaFuncSetAttribute(gemm2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return false;
+  }
+  return true;
+}
+
+int start_2cta(const Maps2& maps, const Args2& a, int tiles, cudaStream_t stream) {
+  const int pairs = g_sms2 / 2, use_pairs = tiles < pairs ? tiles : pairs;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * use_pairs, 1, 1);
+  cfg.blockDim = dim3(192, 1, 1);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, gemm2_kernel, maps, a) == cudaSuccess ? 1 : -5;
+}
+
 int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                 int flags, const void* bias, const void* resid, long long ldr, float alpha, int* status,
                 cudaStream_t stream, const LseArgs& lse, const Product& p2 = Product{}, const Product& p3 = Product{},
                 const GluArgs& glu = GluArgs{}) {
   static const bool off = getenv("TUNIX_B200_NO_2CTA") != nullptr;
   if (off) return 0;
-  static DeviceOnce once;
-  if (once.first()) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_sms2, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaFuncSetAttribute(gemm2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-      return -5;
-  }
+  if (!setup_2cta()) return -5;
   const int tile_n = glu.up ? BN / 2 : BN;
   const int num_m = (M + BM - 1) / BM, num_n = (N + tile_n - 1) / tile_n;
   const int pairs = g_sms2 / 2;
@@ -673,7 +714,7 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
     else       r = tb_make_tmap_2d_bf16(&maps.b[i], q.B, q.K, N, q.ldb, BK, 64, 1);
     if (r) return -4;
   }
-  Args2 a;
+  Args2 a = {};
   // Results in whole 16-byte pieces leave through TMA, columns included: what TMA leaves out past N it leaves out by such pieces. A sum into bf16 takes what is there as its residual, once and before the rounding
   const bool f32 = flags & GF_OUT_F32;
   a.tma_c = C != nullptr && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc % (f32 ? 4 : 8) == 0 && N % (f32 ? 4 : 8) == 0 &&
@@ -708,22 +749,7 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
   a.ldr = ldr; a.alpha = alpha; a.status = status;
   a.targets = lse.targets; a.partial = lse.partial; a.inv_temp = lse.inv_temp; a.softcap = lse.softcap;
   a.dz_lse = lse.dz_lse; a.dz_dlogp = lse.dz_dlogp; a.dz_dent = lse.dz_dent; a.dz_ent = lse.dz_ent;
-  const int tiles = num_m * num_n;
-  const int use_pairs = tiles < pairs ? tiles : pairs;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * use_pairs, 1, 1);
-  cfg.blockDim = dim3(192, 1, 1);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, gemm2_kernel, maps, a) != cudaSuccess) return -5;
-  return 1;
+  return start_2cta(maps, a, num_m * num_n, stream);
 }
 }  // namespace
 
@@ -749,6 +775,49 @@ TB_API int tb_gemm_bf16_ext(const void* A, const void* B, void* C, int M, int N,
     return -2;
   return launch_2cta(A, B, C, M, N, K, lda, ldb, ldc, flags, bias, resid, ldr, alpha, status, stream, LseArgs{}, {A2, B2, K2, lda2, ldb2},
                      {A3, B3, K3, lda3, ldb3});
+}
+
+// Grouped products on SM pairs over a tile list planned for 256 rows a tile (see tb_gemm_grouped_bf16, whose arguments these are). C is
+// [c_rows, ldc]-strided with whole 16-byte pieces, all experts' outputs one below the other. A2 / B2 (K2 > 0): a second product of the same
+// layouts and tiles, contracted over K2 behind the K of the first; the list's k-blocks count both.
+// up (not null): B and up are the stacked gate and up projections, tiles 128 columns wide, C takes act(gate) * up, g and u (null: not kept)
+// the two. All [c_rows, N] with stride ldc.
+// The weights of 512 rows an expert are read once a tile of 256 rows instead of 128, and the pair's halves of B fit the L2 -> SM port.
+TB_API int tb_gemm_grouped_pair(const void* A, long long a_rows, long long a_cols, long long lda, const void* B, long long b_rows,
+                                long long b_cols, long long ldb, void* C, long long c_rows, long long ldc, int N, int flags, const void* tiles,
+                                const int* num_tiles_dev, int max_tiles, int K, const void* A2, const void* B2, int K2, int glu_kind,
+                                const void* up, void* g, void* u, int* status, cudaStream_t stream) {
+  if (max_tiles <= 0) return 0;
+  const bool f32 = flags & GF_OUT_F32, a_mn = flags & GF_A_MN, b_mn = flags & GF_B_MN;
+  uintptr_t ptrs = 0;
+  for (const void* p : {A, B, (const void*)C, A2, B2, up, (const void*)g, (const void*)u}) ptrs |= reinterpret_cast<uintptr_t>(p);
+  if (lda % 8 || ldb % 8 || ldc % (f32 ? 4 : 8) || N % (f32 ? 4 : 8) || (ptrs & 15) || (K2 > 0 && K % BK) || (up && f32)) return -2;
+  if (!setup_2cta()) return -5;
+  Maps2 maps;
+  const void *as[SEGS] = {A, K2 > 0 ? A2 : A, A}, *bs[SEGS] = {B, up ? up : K2 > 0 ? B2 : B, B};
+  for (int i = 0; i < SEGS; ++i) {
+    if (a_mn ? tb_make_tmap_2d_bf16(&maps.a[i], as[i], a_rows, a_cols, lda, BK, 64, 1)
+             : tb_make_tmap_2d_bf16(&maps.a[i], as[i], a_rows, a_cols, lda, HM, BK, 1)) return -3;
+    if (b_mn ? tb_make_tmap_2d_bf16(&maps.b[i], bs[i], b_rows, b_cols, ldb, BK, 64, 1)
+             : tb_make_tmap_2d_bf16(&maps.b[i], bs[i], b_rows, b_cols, ldb, HN, BK, 1)) return -4;
+  }
+  const void* outs[3] = {C, up && g ? g : C, up && g ? u : C};
+  for (int i = 0; i < 3; ++i)
+    if (f32 ? tb_make_tmap_2d_f32(&maps.c[i], outs[i], c_rows, N, ldc, 32, 32) : tb_make_tmap_2d_bf16(&maps.c[i], outs[i], c_rows, N, ldc, 32, 64, 1))
+      return -4;
+  Args2 a = {};
+  a.tiles = reinterpret_cast<const TileDesc*>(tiles);
+  a.num_tiles_dev = num_tiles_dev;
+  a.N = N; a.K = K; a.K2 = K2; a.flags = flags; a.C = C; a.ldc = ldc; a.alpha = 1.f; a.status = status; a.tma_c = 1; a.group = 1;
+  a.inv_temp = 1.f;
+  if (!f32 && (flags & GF_ACCUM)) {
+    a.flags = (flags & ~GF_ACCUM) | GF_RESIDUAL;
+    a.resid = reinterpret_cast<const __nv_bfloat16*>(C);
+    a.ldr = ldc;
+  }
+  a.glu = up != nullptr; a.glu_kind = glu_kind; a.glu_keep = g != nullptr;
+  const int rc = start_2cta(maps, a, max_tiles, stream);
+  return rc == 1 ? 0 : rc;
 }
 
 // h [M, F] = act(x Wg^T) * (x Wu^T), both products and the activation in one launch; gate and up projections [M, F] are written too where

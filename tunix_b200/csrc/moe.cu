@@ -213,46 +213,66 @@ __global__ void moe_row_dot_kernel(const __nv_bfloat16* __restrict__ a, long lon
   if (lane == 0) out[w] = s;
 }
 
-// single CTA: tiles [expert][m tile of its segment][n tile]
-__global__ void moe_tiles_rows_kernel(const int* __restrict__ seg_off, int E, int num_n, int bn, int kblocks,
-                                      int b_rows_per_expert, TileDesc* __restrict__ tiles, int* __restrict__ num_tiles) {
-  __shared__ int base[1025];
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < E; ++e) {
-      base[e] = acc;
-      acc += ((seg_off[e + 1] - seg_off[e]) >> 7) * num_n;
+// single CTA: tiles [expert][m tile of its segment][n tile]. One thread an expert counts its tiles, a scan places them, and every thread
+// then finds the expert of its tiles by bisection (128 experts of 512 rows: 31 us with one thread counting and an expert at a time -> below 5).
+__global__ void __launch_bounds__(1024)
+moe_tiles_rows_kernel(const int* __restrict__ seg_off, int E, int num_n, int bm, int bn, int kblocks, int b_rows_per_expert,
+                      TileDesc* __restrict__ tiles, int* __restrict__ num_tiles) {
+  __shared__ int s_end[1024], s_off[1025], s_warp[32];     // tiles up to the end of an expert; where its rows begin
+  const int e0 = threadIdx.x, lane = e0 & 31, warp = e0 >> 5;
+  if (e0 <= E && e0 < 1024) s_off[e0] = seg_off[e0];
+  if (e0 == 0) s_off[E] = seg_off[E];
+  int n = e0 < E ? (seg_off[e0 + 1] - seg_off[e0] + bm - 1) / bm * num_n : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, n, o);
+    if (lane >= o) n += v;
+  }
+  if (lane == 31) s_warp[warp] = n;
+  __syncthreads();
+  if (warp == 0) {
+    int v = s_warp[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int w = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += w;
     }
-    base[E] = acc;
-    *num_tiles = acc;
+    s_warp[lane] = v;
   }
   __syncthreads();
-  for (int e = 0; e < E; ++e) {
-    const int n = base[e + 1] - base[e];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const int mt = i / num_n, nt = i - mt * num_n;
-      TileDesc d;
-      d.m0 = seg_off[e] + mt * 128;
-      d.n0 = nt * bn;
-      d.m_end = d.m0 + 128;
-      d.kb0 = 0;
-      d.kb1 = kblocks;
-      d.b_row0 = e * b_rows_per_expert;
-      d.c_off = 0;
-      tiles[base[e] + i] = d;
+  s_end[e0] = n + (warp ? s_warp[warp - 1] : 0);
+  __syncthreads();
+  const int total = s_end[E - 1];
+  if (e0 == 0) *num_tiles = total;
+  for (int i = e0; i < total; i += 1024) {
+    int lo = 0, hi = E - 1;
+    while (lo < hi) {                                      // the first expert whose tiles end past i
+      const int mid = (lo + hi) >> 1;
+      if (s_end[mid] > i) hi = mid;
+      else lo = mid + 1;
     }
+    const int r = i - (lo ? s_end[lo - 1] : 0), mt = r / num_n;
+    TileDesc d;
+    d.m0 = s_off[lo] + mt * bm;
+    d.n0 = (r - mt * num_n) * bn;
+    d.m_end = min(d.m0 + bm, s_off[lo + 1]);
+    d.kb0 = 0;
+    d.kb1 = kblocks;
+    d.b_row0 = lo * b_rows_per_expert;
+    d.c_off = 0;
+    tiles[i] = d;
   }
 }
 
 // tiles [expert][m tile][n tile] of a per-expert [M, N] output, contraction over the expert's row segment
-__global__ void moe_tiles_expert_kernel(const int* __restrict__ seg_off, int E, int M, int num_m, int num_n, int bn,
+__global__ void moe_tiles_expert_kernel(const int* __restrict__ seg_off, int E, int M, int num_m, int num_n, int bm, int bn,
                                         long long c_stride, TileDesc* __restrict__ tiles, int* __restrict__ num_tiles) {
   const int per = num_m * num_n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < E * per; i += gridDim.x * blockDim.x) {
     const int e = i / per, r = i - e * per;
     const int mt = r / num_n, nt = r - mt * num_n;
     TileDesc d;
-    d.m0 = mt * 128;
+    d.m0 = mt * bm;
     d.n0 = nt * bn;
     d.m_end = M;
     d.kb0 = seg_off[e] >> 6;
@@ -350,21 +370,22 @@ TB_API int tb_moe_row_dot(const void* a, long long lda, const void* b, long long
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-// seg_off int32 [E + 1], multiples of 128. tiles: room for (seg_off[E] / 128) * num_n descriptors of 32 bytes.
+// seg_off int32 [E + 1], multiples of 128. tiles: room for (seg_off[E] / 128) * num_n descriptors of 32 bytes; bm rows a tile: 128, or 256
+// for the products on SM pairs.
 TB_API int tb_moe_tiles_rows(const int* seg_off, int E, int num_n, int bn, int kblocks, int b_rows_per_expert,
-                             void* tiles, int* num_tiles, cudaStream_t stream) {
-  if (E <= 0 || E > 1024) return -2;
-  moe_tiles_rows_kernel<<<1, 1024, 0, stream>>>(seg_off, E, num_n, bn, kblocks, b_rows_per_expert,
+                             void* tiles, int* num_tiles, int bm, cudaStream_t stream) {
+  if (E <= 0 || E > 1024 || (bm != 128 && bm != 256)) return -2;
+  moe_tiles_rows_kernel<<<1, 1024, 0, stream>>>(seg_off, E, num_n, bm, bn, kblocks, b_rows_per_expert,
                                                 reinterpret_cast<TileDesc*>(tiles), num_tiles);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 TB_API int tb_moe_tiles_expert(const int* seg_off, int E, int M, int N, int bn, long long c_stride, void* tiles,
-                               int* num_tiles, cudaStream_t stream) {
-  if (E <= 0) return -2;
-  const int num_m = (M + 127) / 128, num_n = (N + bn - 1) / bn;
+                               int* num_tiles, int bm, cudaStream_t stream) {
+  if (E <= 0 || (bm != 128 && bm != 256)) return -2;
+  const int num_m = (M + bm - 1) / bm, num_n = (N + bn - 1) / bn;
   const int total = E * num_m * num_n;
-  moe_tiles_expert_kernel<<<(total + 255) / 256, 256, 0, stream>>>(seg_off, E, M, num_m, num_n, bn, c_stride,
+  moe_tiles_expert_kernel<<<(total + 255) / 256, 256, 0, stream>>>(seg_off, E, M, num_m, num_n, bm, bn, c_stride,
                                                                    reinterpret_cast<TileDesc*>(tiles), num_tiles);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

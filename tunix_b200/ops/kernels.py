@@ -588,48 +588,63 @@ _lib.register_cuda_sigs({
     "tb_moe_scatter_rows": [_lib.P, _lib.LL, _lib.P, _lib.P, _lib.P, _lib.LL, _lib.LL, _lib.I, _lib.I, _lib.P],
     "tb_moe_gather_sum": [_lib.P, _lib.LL, _lib.P, _lib.P, _lib.P, _lib.LL, _lib.P, _lib.LL, _lib.LL, _lib.I, _lib.I, _lib.P],
     "tb_moe_dot_rows": [_lib.P, _lib.LL, _lib.P, _lib.LL, _lib.P, _lib.P, _lib.LL, _lib.I, _lib.I, _lib.P],
-    "tb_moe_tiles_rows": [_lib.P, _lib.I, _lib.I, _lib.I, _lib.I, _lib.I, _lib.P, _lib.P, _lib.P],
-    "tb_moe_tiles_expert": [_lib.P, _lib.I, _lib.I, _lib.I, _lib.I, _lib.LL, _lib.P, _lib.P, _lib.P],
+    "tb_moe_tiles_rows": [_lib.P, _lib.I, _lib.I, _lib.I, _lib.I, _lib.I, _lib.P, _lib.P, _lib.I, _lib.P],
+    "tb_moe_tiles_expert": [_lib.P, _lib.I, _lib.I, _lib.I, _lib.I, _lib.LL, _lib.P, _lib.P, _lib.I, _lib.P],
+    "tb_gemm_grouped_pair": [_lib.P, _lib.LL, _lib.LL, _lib.LL, _lib.P, _lib.LL, _lib.LL, _lib.LL, _lib.P, _lib.LL, _lib.LL, _lib.I, _lib.I,
+                             _lib.P, _lib.P, _lib.I, _lib.I, _lib.P, _lib.P, _lib.I, _lib.I, _lib.P, _lib.P, _lib.P, _lib.P, _lib.P],
 })
 
 TILE_DESC_BYTES = 32
 
 
 class TileList:
-    """Device-resident tile list of a grouped GEMM: descriptors, their count (device int32) and a host bound."""
+    """Device-resident tile list of a grouped GEMM: descriptors, their count (device int32) and a host bound. Tiles of 256 rows (`bm`) are
+    for the kernel on SM pairs, `k` is then what one product contracts over (0: segments of rows) and `n` its columns."""
 
-    def __init__(self, max_tiles: int, bn: int, device):
+    def __init__(self, max_tiles: int, bn: int, device, bm: int = 128, k: int = 0, n: int = 0):
         self.desc = torch.empty(max(max_tiles, 1) * TILE_DESC_BYTES, dtype=torch.uint8, device=device)
         self.count = torch.zeros(1, dtype=torch.int32, device=device)
-        self.max_tiles, self.bn = max_tiles, bn
+        self.max_tiles, self.bn, self.bm, self.k, self.n = max_tiles, bn, bm, k, n
 
 
 def _grouped_bn(n: int) -> int:
     return 256 if n >= 256 else (128 if n >= 128 else 64)
 
 
-def moe_tiles_rows(seg_off: torch.Tensor, max_rows: int, n_out: int, k_contract: int, b_rows_per_expert: int) -> TileList:
+# Rows an expert from which grouped products run on SM pairs: a tile of 256 rows that is half empty costs what two of 128 do.
+PAIR_ROWS = 256
+
+
+def moe_on_pairs(rows: int, experts: int, Fdim: int, D: int, *tensors) -> bool:
+    """Whether the grouped products of `rows` rows over `experts` experts [Fdim, D] run on SM pairs: enough rows an expert, tiles
+    that are not mostly past a matrix's columns, and whole 16-byte pieces."""
+    return rows >= PAIR_ROWS * experts and Fdim >= 256 and D >= 256 and Fdim % 64 == 0 and D % 64 == 0 and \
+        all(t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def moe_tiles_rows(seg_off: torch.Tensor, max_rows: int, n_out: int, k_contract: int, b_rows_per_expert: int, *, pairs: bool = False,
+                   glu: bool = False, products: int = 1) -> TileList:
     """Tiles of a GEMM whose output rows are the permuted token rows: [max_rows, n_out] with the contraction
     k_contract over the feature dimension (the operands' inner one where it is no multiple of 64: reads past it are zeros) and
-    B = the stacked expert weights."""
+    B = the stacked expert weights. `pairs`: for the kernel on SM pairs; `glu` then is its gated form, `products` how many it sums."""
     E = seg_off.numel() - 1
-    bn = _grouped_bn(n_out)
+    bn = (128 if glu else 256) if pairs else _grouped_bn(n_out)
     num_n = (n_out + bn - 1) // bn
-    tl = TileList((max_rows // 128) * num_n, bn, seg_off.device)
-    rc = _lib.cuda().tb_moe_tiles_rows(seg_off.data_ptr(), E, num_n, bn, -(-k_contract // 64), b_rows_per_expert,
-                                       tl.desc.data_ptr(), tl.count.data_ptr(), _lib.stream_ptr())
+    tl = TileList((max_rows // 128) * num_n, bn, seg_off.device, 256 if pairs else 128, k_contract, n_out)
+    rc = _lib.cuda().tb_moe_tiles_rows(seg_off.data_ptr(), E, num_n, bn, -(-k_contract // 64) * products, b_rows_per_expert,
+                                       tl.desc.data_ptr(), tl.count.data_ptr(), tl.bm, _lib.stream_ptr())
     _lib.check(rc, "tb_moe_tiles_rows")
     _count()
     return tl
 
 
-def moe_tiles_expert(seg_off: torch.Tensor, m_out: int, n_out: int) -> TileList:
+def moe_tiles_expert(seg_off: torch.Tensor, m_out: int, n_out: int, *, pairs: bool = False) -> TileList:
     """Tiles of a GEMM with one [m_out, n_out] output per expert, contracted over the expert's row segment."""
     E = seg_off.numel() - 1
-    bn = _grouped_bn(n_out)
-    tl = TileList(E * ((m_out + 127) // 128) * ((n_out + bn - 1) // bn), bn, seg_off.device)
+    bn, bm = (256, 256) if pairs else (_grouped_bn(n_out), 128)
+    tl = TileList(E * ((m_out + bm - 1) // bm) * ((n_out + bn - 1) // bn), bn, seg_off.device, bm)
     rc = _lib.cuda().tb_moe_tiles_expert(seg_off.data_ptr(), E, m_out, n_out, bn, m_out * n_out, tl.desc.data_ptr(),
-                                         tl.count.data_ptr(), _lib.stream_ptr())
+                                         tl.count.data_ptr(), bm, _lib.stream_ptr())
     _lib.check(rc, "tb_moe_tiles_expert")
     _count()
     return tl
@@ -641,6 +656,8 @@ def gemm_grouped(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, n_limit: i
     dimension is contracted follows a_mn / b_mn as in `gemm`. out: bf16 or fp32, 2-D (per-expert outputs are
     addressed through the tile's element offset). n_limit: number of valid output columns per group."""
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and _is2d_rowmajor(a) and _is2d_rowmajor(b)
+    if tiles.bm == 256:
+        return _grouped_pair(a, b, out, n_limit, tiles, a_mn=a_mn, b_mn=b_mn, accumulate=accumulate)
     flags = (GF_A_MN if a_mn else 0) | (GF_B_MN if b_mn else 0) | (GF_OUT_F32 if out.dtype == torch.float32 else 0) | \
         (GF_ACCUM if accumulate else 0)
     rc = _lib.cuda().tb_gemm_grouped_bf16(a.data_ptr(), a.shape[0], a.shape[1], a.stride(0), b.data_ptr(), b.shape[0],
@@ -650,6 +667,35 @@ def gemm_grouped(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, n_limit: i
     _lib.check(rc, "tb_gemm_grouped_bf16")
     _count()
     return out
+
+
+def _grouped_pair(a, b, out, n_limit, tiles, *, a_mn=False, b_mn=False, accumulate=False, a2=None, b2=None, kind=0, up=None, g=None, u=None):
+    assert tiles.bm == 256 and (out.is_contiguous() or out.dim() == 2 and out.stride(1) == 1)
+    flags = (GF_A_MN if a_mn else 0) | (GF_B_MN if b_mn else 0) | (GF_OUT_F32 if out.dtype == torch.float32 else 0) | \
+        (GF_ACCUM if accumulate else 0)
+    rc = _lib.cuda().tb_gemm_grouped_pair(
+        a.data_ptr(), a.shape[0], a.shape[1], a.stride(0), b.data_ptr(), b.shape[0], b.shape[1], b.stride(0), out.data_ptr(),
+        out.numel() // out.shape[-1], out.stride(-2), n_limit, flags, tiles.desc.data_ptr(), tiles.count.data_ptr(), tiles.max_tiles, tiles.k,
+        _lib.ptr(a2), _lib.ptr(b2), tiles.k if a2 is not None else 0, kind, _lib.ptr(up), _lib.ptr(g), _lib.ptr(u),
+        _lib.status_buffer().data_ptr(), _lib.stream_ptr())
+    _lib.check(rc, "tb_gemm_grouped_pair")
+    _count()
+    return out
+
+
+def gemm_grouped_sum(a, b, a2, b2, out: torch.Tensor, n_limit: int, tiles: TileList) -> torch.Tensor:
+    """out = a x b[e] + a2 x b2[e] over `tiles` (on SM pairs, two products; b and b2 [E * k, n], contracted over an expert's rows)."""
+    assert all(t.dtype == torch.bfloat16 and t.is_contiguous() for t in (a, b, a2, b2)) and a.shape == a2.shape and b.shape == b2.shape
+    return _grouped_pair(a, b, out, n_limit, tiles, b_mn=True, a2=a2, b2=b2)
+
+
+def gemm_grouped_glu(x, gate, up, tiles: TileList, kind: int):
+    """(act(g) * u, g, u) with g = x gate[e]^T, u = x up[e]^T over `tiles` (on SM pairs, gated); gate, up [E * F, D]."""
+    assert all(t.dtype == torch.bfloat16 and t.is_contiguous() for t in (x, gate, up)) and gate.shape == up.shape
+    Fdim = tiles.n
+    h, g, u = (torch.empty((x.shape[0], Fdim), dtype=torch.bfloat16, device=x.device) for _ in range(3))
+    _grouped_pair(x, gate, h, Fdim, tiles, kind=kind, up=up, g=g, u=u)
+    return h, g, u
 
 
 def moe_zero_pad(buf: torch.Tensor, seg_off: torch.Tensor, counts: torch.Tensor) -> None:

@@ -49,18 +49,22 @@ class _ExpertsFn(torch.autograd.Function):
         xp = torch.empty((max_rows, D), dtype=torch.bfloat16, device=dev)
         K.moe_zero_pad(xp, seg_off, counts)
         K.moe_scatter_rows(x, pos, None, xp)
-        t_up = K.moe_tiles_rows(seg_off, max_rows, Fd, D, Fd)          # [R, F] <- xp [R, D] x W[e] [F, D]
-        t_down = K.moe_tiles_rows(seg_off, max_rows, D, Fd, D)         # [R, D] <- h  [R, F] x W[e] [D, F]
-        g = torch.empty((max_rows, Fd), dtype=torch.bfloat16, device=dev)
-        u = torch.empty_like(g)
-        K.gemm_grouped(xp, gate_w.view(E * Fd, D), g, Fd, t_up)
-        K.gemm_grouped(xp, up_w.view(E * Fd, D), u, Fd, t_up)
-        h = K.glu_fwd(g, u, kind)
+        pairs = K.moe_on_pairs(pos.numel(), E, Fd, D, gate_w, up_w, down_w)
+        t_up = K.moe_tiles_rows(seg_off, max_rows, Fd, D, Fd, pairs=pairs, glu=pairs)         # [R, F] <- xp [R, D] x W[e] [F, D]
+        t_down = K.moe_tiles_rows(seg_off, max_rows, D, Fd, D, pairs=pairs)                   # [R, D] <- h  [R, F] x W[e] [D, F]
+        if pairs:
+            h, g, u = K.gemm_grouped_glu(xp, gate_w.view(E * Fd, D), up_w.view(E * Fd, D), t_up, kind)
+        else:
+            g = torch.empty((max_rows, Fd), dtype=torch.bfloat16, device=dev)
+            u = torch.empty_like(g)
+            K.gemm_grouped(xp, gate_w.view(E * Fd, D), g, Fd, t_up)
+            K.gemm_grouped(xp, up_w.view(E * Fd, D), u, Fd, t_up)
+            h = K.glu_fwd(g, u, kind)
         y = torch.empty((max_rows, D), dtype=torch.bfloat16, device=dev)
         K.gemm_grouped(h, down_w.view(E * D, Fd), y, D, t_down)
         out = K.moe_gather_sum(y, pos, wts, residual)
         ctx.save_for_backward(xp, g, u, y, wts, pos, seg_off, counts, gate_w, up_w, down_w)
-        ctx.kind, ctx.max_rows, ctx.has_res = kind, max_rows, residual is not None
+        ctx.kind, ctx.max_rows, ctx.has_res, ctx.pairs = kind, max_rows, residual is not None, pairs
         ctx.w_refs = (gate_w, up_w, down_w)
         return out
 
@@ -78,8 +82,8 @@ class _ExpertsFn(torch.autograd.Function):
         h = K.glu_fwd(g, u, ctx.kind)
 
         def wgrad(a, b, w_ref, m_out, n_out):
-            tl = K.moe_tiles_expert(seg_off, m_out, n_out)
             mg = getattr(w_ref, "main_grad", None)
+            tl = K.moe_tiles_expert(seg_off, m_out, n_out, pairs=ctx.pairs and (mg is None or mg.data_ptr() % 16 == 0))
             if mg is not None:
                 K.gemm_grouped(a, b, mg.view(E, m_out, n_out), n_out, tl, a_mn=True, b_mn=True, accumulate=True)
                 w_ref.grad_added_to_main_grad = True
@@ -91,7 +95,7 @@ class _ExpertsFn(torch.autograd.Function):
         gw_ref, uw_ref, dw_ref = ctx.w_refs
         d_down = wgrad(dy, h, dw_ref, D, Fd) if ctx.needs_input_grad[8] else None
         # dh [R, F] = dy [R, D] x W_down[e] ([D, F], contracted over D: MN-major B)
-        t_dh = K.moe_tiles_rows(seg_off, R, Fd, D, D)
+        t_dh = K.moe_tiles_rows(seg_off, R, Fd, D, D, pairs=ctx.pairs)
         dh = h
         K.gemm_grouped(dy, down_w.view(E * D, Fd), dh, Fd, t_dh, b_mn=True)
         dg, du = K.glu_bwd(dh, g, u, ctx.kind, inplace=True)
@@ -100,10 +104,13 @@ class _ExpertsFn(torch.autograd.Function):
         dx = None
         if ctx.needs_input_grad[0]:
             # dxp [R, D] = dg x W_gate[e] + du x W_up[e] ([F, D], contracted over F)
-            t_dx = K.moe_tiles_rows(seg_off, R, D, Fd, Fd)
+            t_dx = K.moe_tiles_rows(seg_off, R, D, Fd, Fd, pairs=ctx.pairs, products=2 if ctx.pairs else 1)
             dxp = xp
-            K.gemm_grouped(dg, gate_w.view(E * Fd, D), dxp, D, t_dx, b_mn=True)
-            K.gemm_grouped(du, up_w.view(E * Fd, D), dxp, D, t_dx, b_mn=True, accumulate=True)
+            if ctx.pairs:
+                K.gemm_grouped_sum(dg, gate_w.view(E * Fd, D), du, up_w.view(E * Fd, D), dxp, D, t_dx)
+            else:
+                K.gemm_grouped(dg, gate_w.view(E * Fd, D), dxp, D, t_dx, b_mn=True)
+                K.gemm_grouped(du, up_w.view(E * Fd, D), dxp, D, t_dx, b_mn=True, accumulate=True)
             dx = K.moe_gather_sum(dxp, pos, None)
         dres = dout if ctx.has_res else None
         return dx, dwts, None, None, None, None, d_gate, d_up, d_down, dres, None
