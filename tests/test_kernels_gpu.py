@@ -761,3 +761,28 @@ def test_gated_product_of_few_rows(M, F_, K_):
         # one rounding, 2^-8 of a value at most, and few results to even it out
         assert _rel_err(out, torch.nn.functional.silu(g) * u) < 4e-3
     _check_status()
+
+
+@pytest.mark.parametrize("M,N,K_", [(5, 6144, 4096), (16, 1000, 520), (33, 136, 2056), (64, 4096, 12288), (4004, 16, 3584), (2056, 24, 1000),
+                                    (16, 3584, 4004), (776, 64, 512), (48, 9000, 640)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+def test_gemm_with_a_short_side(M, N, K_, a_mn, b_mn):
+    """One side of at most 64: the other in tiles of 128 with the contraction over a cluster; ragged tiles, columns and k-blocks, every layout
+    and way the result leaves, and more tiles than clusters (left to the other kernels)."""
+    k = _k()
+    up8 = lambda n: (n + 7) // 8 * 8  # noqa: E731
+    def operand(rows, mn, seed):          # strides are multiples of 8 whatever the sizes
+        t = _normal(*((K_, up8(rows)) if mn else (rows, up8(K_))), seed=seed).bfloat16()
+        return t[:, :rows] if mn else t[:, :K_]
+    a, b = operand(M, a_mn, 1), operand(N, b_mn, 2)
+    want = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    bias, res = _normal(N, seed=3).bfloat16(), _normal(M, N, seed=4).bfloat16()
+    kw = dict(a_mn=a_mn, b_mn=b_mn)
+    assert _rel_err(k.gemm(a, b, **kw), want) < 2e-3                         # one rounding
+    assert _rel_err(k.gemm(a, b, out_dtype=torch.float32, **kw), want) < 1e-5                 # sums of K_ products in 32 bits
+    assert _rel_err(k.gemm(a, b, bias=bias, residual=res, alpha=0.5, **kw), 0.5 * want + bias.double() + res.double()) < 2e-3
+    for dtype, tol in ((torch.bfloat16, 2e-3), (torch.float32, 1e-5)):
+        wide = torch.full((M, N + 3), 2.0, device="cuda", dtype=dtype)
+        k.gemm(a, b, out=wide[:, :N], accumulate=True, **kw)
+        assert _rel_err(wide[:, :N], want + 2.0) < tol and bool((wide[:, N:] == 2.0).all())
+    _check_status()

@@ -823,6 +823,8 @@ void clear_fused(GemmArgs& a) {
 
 }  // namespace
 
+int tb_gemm_stream_try(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int flags,
+                       const void* bias, const void* resid, long long ldr, float alpha, int* status, cudaStream_t stream);
 int tb_gemm_rows_try(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                      int flags, const void* bias, const void* resid, long long ldr, float alpha, cudaStream_t stream);
 int tb_gemm_splitk_try(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
@@ -936,6 +938,9 @@ TB_API int tb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int
     // up to four rows: a stream of the weight on the CUDA cores (gemm_rows.cu)
     const int gr = tb_gemm_rows_try(A, B, C, M, N, K, lda, ldb, ldc, flags, bias, resid, ldr, alpha, stream);
     if (gr != 0) return gr < 0 ? gr : 0;
+    // one side of at most 64: the other operand as the left one, K split over a cluster (gemm_stream.cu)
+    const int gs = tb_gemm_stream_try(A, B, C, M, N, K, lda, ldb, ldc, flags, bias, resid, ldr, alpha, status, stream);
+    if (gs != 0) return gs < 0 ? gs : 0;
   }
   if (max_ctas <= 0 && !no_splitk && !(flags & (GF_GLU_SILU | GF_GLU_GELU))) {
     // a few hundred rows: 256x256 tiles on CTA pairs with the K range split over a cluster (gemm_pair_splitk.cu)
