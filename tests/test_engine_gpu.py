@@ -639,3 +639,50 @@ def test_deleted_cache_gives_the_decode_graph_back():
         assert not pools() - before
         eng.reinitialize_cache()
     assert all(all(np.array_equal(a, b) for a, b in zip(o, outs[0])) for o in outs)
+
+
+def test_decode_graph_kept_from_call_to_call():
+    """A later call steps the last one's graph only where it would capture the same: its tokens are those of a new engine for other seeds,
+    weights changed in place, weights that have moved, other lengths, a hooked layer and forbidden tokens, and back again."""
+    from tunix_b200 import _lib
+    from tunix_b200.common.configs import CacheConfig
+    from tunix_b200.generate.engine import PagedEngine
+    model = _model()
+    make = lambda: PagedEngine(model, Tok(), CacheConfig(128, 2, 2, 64), page_size=16, max_running_requests=3, prefix_caching=False)  # noqa: E731
+    eng, captured = make(), []
+    capture = eng._capture_step
+    eng._capture_step = lambda st: captured.append(1) or capture(st)
+    rng = np.random.default_rng(4)
+    prompts = [[1] + rng.integers(3, 500, size=n).tolist() for n in (9, 30, 17, 5)]
+
+    def check(captures, steps=24, **kw):
+        kw = dict(prompt_token_ids=prompts, max_generation_steps=steps, eos_tokens=[2], return_logprobs=True, temperature=1.0, top_k=20,
+                  top_p=0.9, **kw)
+        captured.clear()
+        a, b = eng(**kw), make()(**kw)
+        assert all(np.array_equal(x, y) for x, y in zip(a.tokens, b.tokens)) and a.logprobs == b.logprobs
+        assert len(captured) == captures
+        return a
+    first = check(1, seed=5)
+    again = check(0, seed=6)
+    assert any(not np.array_equal(x, y) for x, y in zip(first.tokens, again.tokens))
+    check(0, seed=5)
+    check(0, seed=-1)
+    with torch.no_grad():
+        model.layers[1].mlp.down_proj.weight.mul_(-1.0)
+        model.layers[0].self_attn.q_proj.weight.mul_(0.5)
+    check(0, seed=5)
+    for p in model.parameters():
+        p.data = p.data.clone()
+    check(1, seed=5)
+    check(0, seed=7)
+    check(1, steps=9, seed=5)
+    check(1, seed=5, forbidden_tokens=[int(first.tokens[0][0])])
+    check(1, seed=5)
+    handle = model.layers[0].mlp.down_proj.register_forward_hook(lambda m, i, o: o * 2.0)
+    check(1, seed=5)
+    handle.remove()
+    check(1, seed=5)
+    model.layers[0].self_attn.window = 4
+    check(1, seed=5)
+    _lib.raise_if_kernel_error()

@@ -130,12 +130,13 @@ struct SampleShared {
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT)
 sample_kernel(float* __restrict__ logits, long long ld, int V, float inv_temp, int top_k, float top_p,
-              unsigned long long seed, int step_host, const int* __restrict__ step_dev, int greedy,
+              unsigned long long seed, const unsigned long long* __restrict__ seed_dev, int step_host, const int* __restrict__ step_dev, int greedy,
               long long* __restrict__ tokens, float* __restrict__ logprobs, float softcap,
               const int* __restrict__ forbidden, int n_forbidden) {
   pdl_trigger();
   pdl_wait();
-  const int step = step_dev ? *step_dev : step_host;  // device-resident step keeps the launch graph-capturable
+  const int step = step_dev ? *step_dev : step_host;  // device-resident step and seed keep the launch graph-capturable, and a graph usable
+  if (seed_dev) seed = *seed_dev;                     // for calls of other seeds
   __shared__ SampleShared sh;
   const cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
@@ -584,7 +585,7 @@ sample_kernel(float* __restrict__ logits, long long ld, int V, float inv_temp, i
 
 template <int NT>
 cudaError_t launch_clusters(int B, int C, float* logits, long long ld, int V, float inv_temp, int top_k, float top_p, unsigned long long seed,
-                            int step, const int* step_dev, int greedy, long long* tokens, float* logprobs, float softcap,
+                            const unsigned long long* seed_dev, int step, const int* step_dev, int greedy, long long* tokens, float* logprobs, float softcap,
                             const int* forbidden, int n_forbidden, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((long long)B * C));
@@ -598,22 +599,22 @@ cudaError_t launch_clusters(int B, int C, float* logits, long long ld, int V, fl
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = C > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, sample_kernel<NT>, logits, ld, V, inv_temp, top_k, top_p, seed, step, step_dev, greedy, tokens,
-                            logprobs, softcap, forbidden, n_forbidden);
+  return cudaLaunchKernelEx(&cfg, sample_kernel<NT>, logits, ld, V, inv_temp, top_k, top_p, seed, seed_dev, step, step_dev, greedy,
+                            tokens, logprobs, softcap, forbidden, n_forbidden);
 }
 
 // CTAs per row: up to 8, as long as the grid is one wave of two CTAs an SM. More CTAs shorten every pass over the row; past
 // one wave they only add exchanges. In the place of two, one CTA of twice the threads needs none: 128 rows of 151,936, no filter,
 // 51 us as two and 46 as one, 128 of 10,000 under top-p alone, flat, 66 and 36.
 int launch_sample(float* logits, long long ld, int B, int V, float temperature, int top_k, float top_p, unsigned long long seed,
-                  int step, const int* step_dev, long long* tokens, float* logprobs, float softcap, const int* forbidden,
+                  const unsigned long long* seed_dev, int step, const int* step_dev, long long* tokens, float* logprobs, float softcap, const int* forbidden,
                   int n_forbidden, cudaStream_t stream) {
   const int greedy = temperature <= 0.f;
   const float inv_temp = greedy ? 1.f : 1.f / temperature;
   int C = 8;
   while (C > 1 && ((long long)B * C > 296 || V < C * 4096)) C >>= 1;
   const auto run = C == 2 ? launch_clusters<1024> : launch_clusters<512>;
-  return run(B, C == 2 ? 1 : C, logits, ld, V, inv_temp, top_k, top_p, seed, step, step_dev, greedy, tokens, logprobs,
+  return run(B, C == 2 ? 1 : C, logits, ld, V, inv_temp, top_k, top_p, seed, seed_dev, step, step_dev, greedy, tokens, logprobs,
              softcap, forbidden, n_forbidden, stream) == cudaSuccess ? 0 : -5;
 }
 
@@ -625,7 +626,7 @@ TB_API int tb_sample(const float* logits, long long ld, int B, int V, float temp
                      unsigned long long seed, int step, const int* step_dev, long long* tokens, float* logprobs,
                      cudaStream_t stream) {
   if (B <= 0) return 0;
-  return launch_sample(const_cast<float*>(logits), ld, B, V, temperature, top_k, top_p, seed, step, step_dev, tokens, logprobs,
+  return launch_sample(const_cast<float*>(logits), ld, B, V, temperature, top_k, top_p, seed, nullptr, step, step_dev, tokens, logprobs,
                        0.f, nullptr, 0, stream);
 }
 
@@ -637,6 +638,16 @@ TB_API int tb_sample_ex(float* logits, long long ld, int B, int V, float tempera
                         float softcap, const int* forbidden, int n_forbidden, cudaStream_t stream) {
   if (B <= 0) return 0;
   if (n_forbidden < 0 || (n_forbidden > 0 && !forbidden)) return -2;
-  return launch_sample(logits, ld, B, V, temperature, top_k, top_p, seed, step, step_dev, tokens, logprobs, softcap, forbidden,
+  return launch_sample(logits, ld, B, V, temperature, top_k, top_p, seed, nullptr, step, step_dev, tokens, logprobs, softcap, forbidden,
+                       n_forbidden, stream);
+}
+
+// The same with the seed read on the device.
+TB_API int tb_sample_seed(float* logits, long long ld, int B, int V, float temperature, int top_k, float top_p,
+                          const unsigned long long* seed_dev, int step, const int* step_dev, long long* tokens, float* logprobs,
+                          float softcap, const int* forbidden, int n_forbidden, cudaStream_t stream) {
+  if (B <= 0) return 0;
+  if (!seed_dev || n_forbidden < 0 || (n_forbidden > 0 && !forbidden)) return -2;
+  return launch_sample(logits, ld, B, V, temperature, top_k, top_p, 0, seed_dev, step, step_dev, tokens, logprobs, softcap, forbidden,
                        n_forbidden, stream);
 }
