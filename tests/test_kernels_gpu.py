@@ -579,8 +579,9 @@ def test_qk_rope(tokens, N, KH, H, gap, norm):
         a, b = y[..., :H // 2], y[..., H // 2:]
         want.append(torch.cat([a * c - b * s, b * c + a * s], -1).flatten(1))
     yq, yk, rq, rk = k.qk_rope(*xs, H, pos, cos, sin, wq=ws[0], wk=ws[1], eps=1e-6, add_one=True, want_rstd=norm)
-    # one rounding to bf16: at most 2^-8 of a value, about 1.7e-3 in the norm of many
-    assert _rel_err(yq, want[0]) < 2e-3 and _rel_err(yk, want[1]) < 2e-3
+    # a rounding to bf16 is at most 2^-8 of a value, about 1.7e-3 in the norm of many; behind a norm there are two (2.4e-3)
+    tol = 3e-3 if norm else 2e-3
+    assert _rel_err(yq, want[0]) < tol and _rel_err(yk, want[1]) < tol
     torch.autograd.backward(want, [d.double() for d in ds])
     if norm:
         dxq, dxk, dwq, dwk = k.qk_rope_bwd(*ds, *xs, H, pos, cos, sin, *ws, rq, rk, True)
@@ -622,7 +623,8 @@ def test_model_joint_rotation_matches_separate(qk_norm):
         sep = run()
     finally:
         F.qk_rope = real
-    for a, b in zip(joint, sep):
+    assert torch.equal(joint[0], sep[0])                               # the same roundings forward
+    for a, b in zip(joint[1:], sep[1:]):
         assert _rel_err(a, b) < 2e-2, (a.shape, _rel_err(a, b))        # a few roundings to bf16 apart
     _check_status()
 
