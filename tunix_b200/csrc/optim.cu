@@ -192,11 +192,15 @@ TB_API int tb_adamw(float* p32, float* m, float* v, const void* g, int g_is_bf16
                           reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(g) |
                           (reinterpret_cast<uintptr_t>(p16) << 1);
   if (align & 15) return -2;  // flat buffers are always 16-byte aligned
+  // A block for every 1024 elements, not a loop of few blocks over all: the seven streams of a block then lie close together in time. bf16
+  // gradients, 654 M elements 2.94 ms (6.2 TB/s) in 2368 blocks, 2.66 (6.9) here; 60 M 0.274, 0.253. Eight elements a thread, two and four
+  // loads of each stream in flight or streaming loads and stores: 2.65 to 3.1.
+  const unsigned grid = (unsigned)std::min<long long>((n + 1023) / 1024, 0x7fffffffLL);
   if (g_is_bf16)
-    adamw_kernel<__nv_bfloat16><<<grid_for((n + 3) / 4, 256), 256, 0, stream>>>(
+    adamw_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
         p32, m, v, (const __nv_bfloat16*)g, (__nv_bfloat16*)p16, n, a);
   else
-    adamw_kernel<float><<<grid_for((n + 3) / 4, 256), 256, 0, stream>>>(p32, m, v, (const float*)g,
+    adamw_kernel<float><<<grid, 256, 0, stream>>>(p32, m, v, (const float*)g,
                                                               (__nv_bfloat16*)p16, n, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
