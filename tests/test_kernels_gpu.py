@@ -793,3 +793,42 @@ def test_gemm_with_a_short_side(M, N, K_, a_mn, b_mn):
         k.gemm(a, b, out=wide[:, :N], accumulate=True, **kw)
         assert _rel_err(wide[:, :N], want + 2.0) < tol and bool((wide[:, N:] == 2.0).all())
     _check_status()
+
+
+@pytest.mark.parametrize("rows,V,D,share,chunk", [(4094, 2048, 512, 0.6, 2048), (2250, 5000, 264, 0.5, 1000), (3000, 4096, 256, 0.0, 2048),
+                                                  (2048, 2304, 256, 1.0, 2048), (5000, 3080, 384, 0.02, 2048)])
+@pytest.mark.parametrize("softcap,want_ent", [(0.0, True), (30.0, False)])
+def test_head_over_the_rows_that_count(rows, V, D, share, chunk, softcap, want_ent, monkeypatch):
+    """Log-probs, entropies and gradients of the rows with a target; none, all, few rows, chunks that are no whole blocks of 64, a last
+    chunk with the one before, gradients added to what is there. The other rows hold values that would spoil any sum they took part in."""
+    from tunix_b200.ops import functional as F
+    monkeypatch.setattr(F, "_SCORED_MIN", 0)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    h, w = torch.randn(rows, D, device="cuda", generator=g).bfloat16(), (0.2 * torch.randn(V, D, device="cuda", generator=g)).bfloat16()
+    tg = torch.randint(0, V, (rows,), device="cuda", generator=g)
+    tg[torch.rand(rows, device="cuda", generator=g) >= share] = -1
+    on = tg >= 0
+    bad = h.clone()
+    bad[~on] = float("nan")
+    leaf, wl = bad.clone().requires_grad_(), w.clone().requires_grad_()
+    wl.main_grad = torch.ones(V, D, device="cuda")
+    logp, ent = F.lm_head_logprobs(leaf, wl, tg, softcap=softcap, temperature=0.8, want_entropy=want_ent, chunk=chunk, skip_ignored=True)
+    assert type(logp.grad_fn).__name__ == "_LmHeadScoredFnBackward"
+    z = h.double() @ w.double().t()
+    hd, wd = h.double().requires_grad_(), w.double().requires_grad_()
+    z = hd @ wd.t()
+    z = (softcap * torch.tanh(z / softcap) if softcap else z) / 0.8
+    lsm = torch.log_softmax(z, -1)
+    ref = torch.where(on, lsm.gather(1, tg.clamp(min=0)[:, None])[:, 0], 0.0)
+    ref_e = torch.where(on, -(lsm.exp() * lsm).sum(-1), 0.0)
+    wa, we = torch.randn(rows, device="cuda", generator=g), torch.randn(rows, device="cuda", generator=g)
+    (logp * wa + (ent * we if want_ent else 0.0)).sum().backward()
+    (ref * wa.double() + (ref_e * we.double() if want_ent else 0.0)).sum().backward()
+    assert bool((logp[~on] == 0).all()) and (not want_ent or bool((ent[~on] == 0).all()))
+    if share:
+        # 32-bit softmax of sums over bf16 rows; the capped score's tanh is off by 5e-4 of the cap
+        tol = 1e-4 if not softcap else 4e-3
+        assert _rel_err(logp, ref) < tol and (not want_ent or _rel_err(ent, ref_e) < tol)
+        assert _rel_err(leaf.grad[on], hd.grad[on]) < 1e-2              # dz rounded to bf16 on the way
+    assert bool((leaf.grad[~on] == 0).all()) and _rel_err(wl.main_grad, wd.grad + 1) < 1e-2 and wl.grad is None
+    _check_status()

@@ -49,6 +49,10 @@ struct Args2 {
   const TileDesc* tiles;   // null: a dense problem
   const int* num_tiles_dev;
   int M, N, K, flags;
+  // Rows that exist, known on the device: *limit - limit_off (null: all). Tiles of A rows past it are passed over, or with limit_k the
+  // contraction ends there (its last block is whole: zeros in one operand).
+  const int* limit;
+  int limit_off, limit_k;
   int group;             // tiles are walked in groups of this many rows of tiles (negative: columns), see tile_group
   // further products accumulated into the same TMEM tile, C += A_i[M, K_i] * B_i[N, K_i]^T with the layouts of A and B (a low-rank adapter
   // update carried by the base projection's GEMM, the input gradients of projections that share their input); 0 when absent
@@ -161,6 +165,8 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
   const int num_tiles = grouped ? *args.num_tiles_dev : num_m * num_n;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const bool a_mn = args.flags & GF_A_MN, b_mn = args.flags & GF_B_MN;
+  const int lim = args.limit ? *args.limit - args.limit_off : 0x7fffffff;
+  const int row_lim = args.limit_k ? 0x7fffffff : lim, kb_lim = args.limit_k ? max(0, min(num_kb, (lim + BK - 1) / BK)) : num_kb;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -201,7 +207,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
     const int size = by_n ? -args.group : args.group, along = by_n ? num_n : num_m, across = by_n ? num_m : num_n;
     const int g = t / (size * across), first = g * size, r = t - first * across, here = min(size, along - first);
     const int a = first + r % here, b = r / here;
-    return {(by_n ? b : a) * BM, (by_n ? a : b) * tile_n, M, 0, num_kb, 0, 0};
+    return {(by_n ? b : a) * BM, (by_n ? a : b) * tile_n, M, 0, kb_lim, 0, 0};
   };
 
   if (warp == 0) {
@@ -212,6 +218,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
         const Tile tile = tile_at(t);
+        if (tile.m0 >= row_lim) continue;
         const int m0 = tile.m0 + (int)rank * HM, n0 = tile.n0 + (glu ? 0 : (int)rank * HN);
         for (int kb = tile.kb0; kb < tile.kb1; ++kb) {
           if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1, abort_flag, args.status, ST_TIMEOUT_PRODUCER)) {
@@ -254,7 +261,8 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-        int kb0 = 0, kb1 = num_kb;
+        int kb0 = 0, kb1 = kb_lim;
+        if (args.limit && tile_at(t).m0 >= row_lim) continue;
         if (grouped) {
           kb0 = args.tiles[t].kb0;
           kb1 = args.tiles[t].kb1;
@@ -304,6 +312,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
     const bool dz_mode = args.dz_lse != nullptr;
     for (int t = pair; t < num_tiles; t += num_pairs) {
       const Tile tile = tile_at(t);
+      if (tile.m0 >= row_lim) continue;
       const int row = tile.m0 + (int)rank * HM + q * 32 + lane, row_end = tile.m_end, c_row = tile.c_row0 + row;
       const int n0 = tile.n0;
       const bool none = tile.kb1 <= tile.kb0;              // an expert without rows: its part of a sum over rows is zero
@@ -440,7 +449,7 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
               const float p = __expf(z - dz_l);
               float d = dz_gl * ((col0 + i == dz_t ? 1.f : 0.f) - p);
               if (dz_ge != 0.f) d -= dz_ge * p * (z - dz_l + dz_en);
-              v[i] = d * chain;
+              v[i] = row < row_lim ? d * chain : 0.f;
             }
           }
           if (has_bias) {
@@ -609,6 +618,10 @@ struct GluArgs {           // gated form where `up` is given: B is the gate proj
   void *g = nullptr, *u = nullptr;
   long long ldg = 0, ldu = 0;
 };
+struct Limit {             // see Args2::limit
+  const int* at = nullptr;
+  int off = 0, k = 0;
+};
 struct Product {           // a further product of the sum; K == 0 when absent
   const void *A = nullptr, *B = nullptr;
   int K = 0;
@@ -617,9 +630,10 @@ struct Product {           // a further product of the sum; K == 0 when absent
 
 // partial [M, num_n, 4] -> logp[row] = z[target] - lse (0 for targets outside [0, V)), lse, entropy = lse - E[z]
 __global__ void lse_combine_kernel(const float* __restrict__ partial, const int* __restrict__ targets, int M, int num_n,
-                                   int V, float* __restrict__ logp, float* __restrict__ lse_out, float* __restrict__ ent_out) {
+                                   int V, float* __restrict__ logp, float* __restrict__ lse_out, float* __restrict__ ent_out,
+                                   const int* __restrict__ limit) {
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= M) return;
+  if (row >= M || (limit && row >= *limit)) return;
   const int lane = threadIdx.x & 31;
   float mx = -INFINITY, sm = 0.f, sz = 0.f, zt = -INFINITY;
   for (int j = lane; j < num_n; j += 32) {
@@ -685,7 +699,7 @@ int start_2cta(const Maps2& maps, const Args2& a, int tiles, cudaStream_t stream
 int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                 int flags, const void* bias, const void* resid, long long ldr, float alpha, int* status,
                 cudaStream_t stream, const LseArgs& lse, const Product& p2 = Product{}, const Product& p3 = Product{},
-                const GluArgs& glu = GluArgs{}) {
+                const GluArgs& glu = GluArgs{}, const Limit& limit = Limit{}) {
   static const bool off = getenv("TUNIX_B200_NO_2CTA") != nullptr;
   if (off) return 0;
   if (!setup_2cta()) return -5;
@@ -743,6 +757,7 @@ int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long
   a.K2 = p2.K;
   a.K3 = p3.K;
   a.group = tile_group(num_m, num_n);
+  a.limit = limit.at; a.limit_off = limit.off; a.limit_k = limit.k;
   a.M = M; a.N = N; a.K = K; a.flags = flags; a.C = C; a.ldc = ldc;
   a.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   a.resid = reinterpret_cast<const __nv_bfloat16*>(resid);
@@ -840,30 +855,43 @@ TB_API int tb_gemm_glu(const void* x, const void* wg, const void* wu, void* h, i
 // the two-SM GEMM's epilogue leaves per-tile softmax statistics, a small kernel merges them.
 // h [M, K] bf16 (row stride ldh), w [V, K] bf16 (row stride ldw), targets int32 [M] (negative = ignored),
 // partial: fp32 scratch of M * ceil(V / 256) * 4 elements. Returns 1 when run here, 0 when the problem does not
-// qualify for the two-SM kernel (the caller uses its chunked path), negative on error.
+// qualify for the two-SM kernel (the caller uses its chunked path), negative on error. limit (device, null: M): rows from *limit on are left out.
 TB_API int tb_lm_head_lse(const void* h, long long ldh, const void* w, long long ldw, int M, int V, int K,
                           const int* targets, float inv_temp, float softcap, float* partial, float* logp, float* lse,
-                          float* entropy, int* status, cudaStream_t stream) {
+                          float* entropy, int* status, const int* limit, cudaStream_t stream) {
   LseArgs lse_args;
   lse_args.targets = targets; lse_args.partial = partial; lse_args.inv_temp = inv_temp; lse_args.softcap = softcap;
-  const int rc = launch_2cta(h, w, nullptr, M, V, K, ldh, ldw, 0, 0, nullptr, nullptr, 0, 1.0f, status, stream, lse_args);
+  const int rc = launch_2cta(h, w, nullptr, M, V, K, ldh, ldw, 0, 0, nullptr, nullptr, 0, 1.0f, status, stream, lse_args, Product{},
+                             Product{}, GluArgs{}, Limit{limit, 0, 0});
   if (rc != 1) return rc;
   const int num_n = (V + BN - 1) / BN;
-  lse_combine_kernel<<<(M + 7) / 8, 256, 0, stream>>>(partial, targets, M, num_n, V, logp, lse, entropy);
+  lse_combine_kernel<<<(M + 7) / 8, 256, 0, stream>>>(partial, targets, M, num_n, V, logp, lse, entropy, limit);
   return cudaGetLastError() == cudaSuccess ? 1 : -5;
 }
 
-// dz [M, V] (bf16, row stride ldo) = gradient of sum_rows(dlogp * logp + dent * entropy) with respect to the raw
+// dz [M, V] (bf16, row stride ldo) = gradient of sum_rows(dlogp * logp + dent * entropy) (rows from *limit - limit_off on, if given, are left
+// out, or zero in a tile with others) with respect to the raw
 // logits h W^T, computed in the epilogue of the two-SM GEMM that recomputes those logits: lse (and entropy, when dent
 // is given) are the row statistics saved by the forward pass. dlogp / dent / entropy may be null. Returns 1 when run
 // here, 0 when the problem does not qualify for the two-SM kernel, negative on error.
 TB_API int tb_lm_head_dlogits(const void* h, long long ldh, const void* w, long long ldw, int M, int V, int K,
                               const int* targets, const float* lse, const float* entropy, const float* dlogp,
                               const float* dent, float inv_temp, float softcap, void* out, long long ldo, int* status,
-                              cudaStream_t stream) {
+                              const int* limit, int limit_off, cudaStream_t stream) {
   if (!lse || !out) return -2;
   LseArgs e;
   e.targets = targets; e.inv_temp = inv_temp; e.softcap = softcap;
   e.dz_lse = lse; e.dz_dlogp = dlogp; e.dz_dent = dent; e.dz_ent = entropy;
-  return launch_2cta(h, w, out, M, V, K, ldh, ldw, ldo, 0, nullptr, nullptr, 0, 1.0f, status, stream, e);
+  return launch_2cta(h, w, out, M, V, K, ldh, ldw, ldo, 0, nullptr, nullptr, 0, 1.0f, status, stream, e, Product{}, Product{}, GluArgs{},
+                     Limit{limit, limit_off, 0});
+}
+
+// tb_gemm_bf16 for the first *limit - limit_off rows of A alone (the other rows of C are left as they are), or with limit_k for that much of the
+// contraction (zeros up to the next multiple of 64 in one operand). Returns 1 when launched, 0 when the two-SM kernel does not take the
+// sizes (nothing is launched), negative on error.
+TB_API int tb_gemm_limited(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int flags,
+                           const int* limit, int limit_off, int limit_k, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  return launch_2cta(A, B, C, M, N, K, lda, ldb, ldc, flags, nullptr, nullptr, 0, 1.f, status, stream, LseArgs{}, Product{}, Product{}, GluArgs{},
+                     Limit{limit, limit_off, limit_k});
 }

@@ -908,17 +908,18 @@ def gae_scan(rewards, values, mask, gamma: float, lam: float):
 # ------------------------------------------------------------------ fused lm_head -> log-softmax statistics
 _lib.register_cuda_sigs({
     "tb_lm_head_lse": [_lib.P, _lib.LL, _lib.P, _lib.LL, _lib.I, _lib.I, _lib.I, _lib.P, _lib.F, _lib.F, _lib.P, _lib.P, _lib.P,
-                       _lib.P, _lib.P, _lib.P],
+                       _lib.P, _lib.P, _lib.P, _lib.P],
     "tb_lm_head_dlogits": [_lib.P, _lib.LL, _lib.P, _lib.LL, _lib.I, _lib.I, _lib.I, _lib.P, _lib.P, _lib.P, _lib.P, _lib.P,
-                           _lib.F, _lib.F, _lib.P, _lib.LL, _lib.P, _lib.P],
+                           _lib.F, _lib.F, _lib.P, _lib.LL, _lib.P, _lib.P, _lib.P, _lib.I],
 })
 
 
 def lm_head_dlogits(h2: torch.Tensor, w: torch.Tensor, targets, lse, entropy, dlogp, dent, *, softcap: float,
-                    temperature: float, out: torch.Tensor) -> bool:
+                    temperature: float, out: torch.Tensor, limit: torch.Tensor | None = None, limit_off: int = 0) -> bool:
     """out [rows, V] bf16 = gradient with respect to the raw logits h W^T of sum(dlogp * logp + dent * entropy), from
     the epilogue of the GEMM that recomputes the logits (no fp32 logits in memory). Returns False when the problem is
-    too small for the two-SM kernel; the caller then recomputes logits into a buffer and runs `dlogits`."""
+    too small for the two-SM kernel; the caller then recomputes logits into a buffer and runs `dlogits`. `limit` (int32 [1] on the
+    device): rows from limit - limit_off on are left out, or zero where their tile has others."""
     import os
     if os.environ.get("TUNIX_B200_NO_FUSED_LSE"):
         return False
@@ -930,7 +931,7 @@ def lm_head_dlogits(h2: torch.Tensor, w: torch.Tensor, targets, lse, entropy, dl
     rc = _lib.cuda().tb_lm_head_dlogits(h2.data_ptr(), h2.stride(0), w.data_ptr(), w.stride(0), rows, V, Kd,
                                         _lib.ptr(targets), lse.data_ptr(), _lib.ptr(entropy), _lib.ptr(dlogp),
                                         _lib.ptr(dent), 1.0 / float(temperature), float(softcap or 0.0), out.data_ptr(),
-                                        out.stride(0), _lib.status_buffer().data_ptr(), _lib.stream_ptr())
+                                        out.stride(0), _lib.status_buffer().data_ptr(), _lib.ptr(limit), limit_off, _lib.stream_ptr())
     if rc < 0:
         _lib.check(rc, "tb_lm_head_dlogits")
     if rc == 1:
@@ -939,10 +940,10 @@ def lm_head_dlogits(h2: torch.Tensor, w: torch.Tensor, targets, lse, entropy, dl
 
 
 def lm_head_lse(h2: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, *, softcap: float, temperature: float,
-                logp: torch.Tensor, lse: torch.Tensor, entropy) -> bool:
+                logp: torch.Tensor, lse: torch.Tensor, entropy, limit: torch.Tensor | None = None) -> bool:
     """log p(target), log-sum-exp and (optionally) entropy of softcap(h W^T) / temperature, written into the given
     fp32 [rows] tensors, without materialising logits (csrc/gemm_2cta.cu). Returns False when the problem is too
-    small for the two-SM kernel; the caller then runs its chunked path."""
+    small for the two-SM kernel; the caller then runs its chunked path. Rows from `limit` (int32 [1] on the device) on are left out."""
     import os
     if os.environ.get("TUNIX_B200_NO_FUSED_LSE"):
         return False
@@ -954,11 +955,72 @@ def lm_head_lse(h2: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, *, sof
     partial = torch.empty(rows * num_n * 4, dtype=torch.float32, device=h2.device)
     rc = _lib.cuda().tb_lm_head_lse(h2.data_ptr(), h2.stride(0), w.data_ptr(), w.stride(0), rows, V, Kd, targets.data_ptr(),
                                     1.0 / float(temperature), float(softcap or 0.0), partial.data_ptr(), logp.data_ptr(),
-                                    lse.data_ptr(), _lib.ptr(entropy), _lib.status_buffer().data_ptr(), _lib.stream_ptr())
+                                    lse.data_ptr(), _lib.ptr(entropy), _lib.status_buffer().data_ptr(), _lib.ptr(limit), _lib.stream_ptr())
     if rc < 0:
         _lib.check(rc, "tb_lm_head_lse")
     if rc == 1:
         _count(2)
+    return rc == 1
+
+
+# ------------------------------------------------------------------ rows of the head that count (csrc/scored_rows.cu)
+def two_sm_takes(M: int, N: int, K_: int) -> bool:
+    """Whether the two-SM kernel takes a product of these sizes in rows of whole 16-byte pieces (a limit on M changes nothing)."""
+    import os
+    if os.environ.get("TUNIX_B200_NO_FUSED_LSE") or os.environ.get("TUNIX_B200_NO_2CTA"):
+        return False
+    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    return min(M, N, K_) >= 256 and (M + 255) // 256 * ((N + 255) // 256) >= sms // 2 * 3 // 5
+
+
+def scored_gather(h2: torch.Tensor, targets: torch.Tensor):
+    """Rows of h2 whose target is not negative, moved together: (rows, their targets, place of every row among them or -1, their number
+    int32 [1]), the first two with 63 rows of zeros (targets -1) behind them and anything behind those."""
+    rows, D = h2.shape
+    assert h2.dtype == torch.bfloat16 and _is2d_rowmajor(h2) and targets.dtype == torch.int32 and targets.is_contiguous()
+    hc = torch.empty((rows, D), dtype=torch.bfloat16, device=h2.device)
+    tc, pos = torch.empty((2, rows), dtype=torch.int32, device=h2.device).unbind(0)
+    count = torch.empty(1, dtype=torch.int32, device=h2.device)
+    rc = _lib.cuda().tb_scored_gather(h2.data_ptr(), h2.stride(0), targets.data_ptr(), rows, D, pos.data_ptr(), count.data_ptr(),
+                                      hc.data_ptr(), tc.data_ptr(), _lib.stream_ptr())
+    _lib.check(rc, "tb_scored_gather")
+    _count(2)
+    return hc, tc, pos, count
+
+
+def scored_scatter(src: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
+    """Row pos[r] of src for every r, zeros where that is -1."""
+    out = torch.empty_like(src)
+    rc = _lib.cuda().tb_scored_scatter(src.data_ptr(), pos.data_ptr(), pos.numel(), src.shape[1], out.data_ptr(), _lib.stream_ptr())
+    _lib.check(rc, "tb_scored_scatter")
+    _count()
+    return out
+
+
+def scored_numbers(a, b, pos: torch.Tensor, gather: bool):
+    """The same moves for fp32 numbers a row (a or b may be None)."""
+    outs = [None if t is None else torch.empty_like(t) for t in (a, b)]
+    rc = _lib.cuda().tb_scored_numbers(_lib.ptr(a), _lib.ptr(outs[0]), _lib.ptr(b), _lib.ptr(outs[1]), pos.data_ptr(), pos.numel(),
+                                       1 if gather else 0, _lib.stream_ptr())
+    _lib.check(rc, "tb_scored_numbers")
+    _count()
+    return outs
+
+
+def gemm_limited(a, b, out, limit: torch.Tensor, limit_off: int, *, a_mn: bool = False, b_mn: bool = False, accumulate: bool = False,
+                 contraction: bool = False) -> bool:
+    """`gemm` for the first limit - limit_off rows of a alone, or for that much of the contraction. False where the two-SM kernel does not
+    take the sizes: nothing has run then."""
+    K_, M = a.shape if a_mn else a.shape[::-1]
+    N = b.shape[1] if b_mn else b.shape[0]
+    assert a.dtype == b.dtype == torch.bfloat16 and all(_is2d_rowmajor(t) for t in (a, b, out)) and out.shape == (M, N)
+    flags = (GF_A_MN if a_mn else 0) | (GF_B_MN if b_mn else 0) | (GF_OUT_F32 if out.dtype == torch.float32 else 0) | (GF_ACCUM if accumulate else 0)
+    rc = _lib.cuda().tb_gemm_limited(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K_, a.stride(0), b.stride(0), out.stride(0), flags,
+                                     limit.data_ptr(), limit_off, 1 if contraction else 0, _lib.status_buffer().data_ptr(), _lib.stream_ptr())
+    if rc < 0:
+        _lib.check(rc, "tb_gemm_limited")
+    if rc == 1:
+        _count()
     return rc == 1
 
 

@@ -165,18 +165,18 @@ def grpo_loss_fn(model, train_example, algo_config, pad_id, eos_id, **kwargs) ->
     if segment_ids is not None:
         comp_seg = segment_ids[:, train_example.prompt_ids.shape[1]:] if segment_ids.shape[1] != completion_mask.shape[1] \
             else segment_ids
+    is_w = train_example.sampler_is_weights
+    fuse = (algo_config.use_rollout_logps and train_example.old_per_token_logps is not None and is_w is None
+            and not train_example.sampler_agreement_applied)
     logp, ent = common.compute_per_token_logps(
         model, train_example.prompt_ids, train_example.completion_ids, pad_id, eos_id,
         completion_mask=completion_mask, stop_gradient=False, return_entropy=True, segment_ids=segment_ids,
         segment_positions=getattr(train_example, "segment_positions", None),
         temperature=getattr(algo_config, "temperature", None), chunk_size=kwargs.get("compute_logps_chunk_size", 0),
-        routed_experts=getattr(train_example, "routed_experts", None))
+        routed_experts=getattr(train_example, "routed_experts", None), skip_masked=not fuse)
     logp = logp.float()
     adv = train_example.advantages.float()
-    is_w = train_example.sampler_is_weights
     sa_metrics: dict = {}
-    fuse = (algo_config.use_rollout_logps and train_example.old_per_token_logps is not None and is_w is None
-            and not train_example.sampler_agreement_applied)
     if fuse:
         sa_metrics, computed_w, filtered = common.sampler_trainer_agreement(
             train_example.old_per_token_logps.float(), logp.detach(), completion_mask,

@@ -101,11 +101,12 @@ def process_ids(prompt_tokens, completion_tokens, pad_id, eos_id, completion_mas
 def compute_per_token_logps(model, prompt_tokens, completion_tokens, pad_id, eos_id, *, completion_mask=None,
                             stop_gradient: bool = True, return_entropy: bool = False, segment_ids=None,
                             segment_positions=None, temperature: Optional[float] = None, chunk_size: int = 0,
-                            token_mask=None, routed_experts=None):
+                            token_mask=None, routed_experts=None, skip_masked: bool = False):
     """log pi(completion_t | prompt, completion_<t) for every completion position -> [B, C] fp32 (and entropy).
 
     Packed inputs pass `segment_ids` / `segment_positions` over the concatenated row; otherwise validity comes
-    from pad ids. The lm_head never materialises [B, T, V] logits."""
+    from pad ids. The lm_head never materialises [B, T, V] logits. `skip_masked`: the caller reads nothing where `completion_mask`
+    is 0, so those positions may hold 0."""
     P = prompt_tokens.shape[1]
     if segment_ids is not None:
         ids = torch.cat([prompt_tokens, completion_tokens], dim=1)
@@ -130,6 +131,10 @@ def compute_per_token_logps(model, prompt_tokens, completion_tokens, pad_id, eos
             # packed rows have no prompt side: token t is predicted from position t - 1, and nothing predicts the
             # first token of a row (it is a prompt token, masked out of every loss)
             h = torch.cat([torch.zeros_like(hidden[:, :1]), hidden[:, :-1]], dim=1)
+        if skip_masked and completion_mask is not None and getattr(model, "skips_ignored", False) and h.is_cuda and \
+                completion_mask.shape == completion_tokens.shape:
+            return model.token_logprobs(h, completion_tokens.masked_fill(completion_mask == 0, -1), temperature=temperature or 1.0,
+                                        want_entropy=return_entropy, chunk=chunk_size or None, skip_ignored=True)
         return model.token_logprobs(h, completion_tokens, temperature=temperature or 1.0,
                                     want_entropy=return_entropy, chunk=chunk_size or None)
 
