@@ -910,7 +910,7 @@ _lib.register_cuda_sigs({
     "tb_lm_head_lse": [_lib.P, _lib.LL, _lib.P, _lib.LL, _lib.I, _lib.I, _lib.I, _lib.P, _lib.F, _lib.F, _lib.P, _lib.P, _lib.P,
                        _lib.P, _lib.P, _lib.P, _lib.P],
     "tb_lm_head_dlogits": [_lib.P, _lib.LL, _lib.P, _lib.LL, _lib.I, _lib.I, _lib.I, _lib.P, _lib.P, _lib.P, _lib.P, _lib.P,
-                           _lib.F, _lib.F, _lib.P, _lib.LL, _lib.P, _lib.P, _lib.P, _lib.I],
+                           _lib.F, _lib.F, _lib.P, _lib.LL, _lib.P, _lib.P, _lib.I, _lib.P],
 })
 
 
