@@ -424,8 +424,9 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
               if (o == 0) {
                 float u[32];
                 get(BN / 2 + c + half * 32, u);
+                // of gate and up as they are kept: the activation of the rows that a backward reads, and of the separate kernels
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = act_fwd(v[i], args.glu_kind) * u[i];
+                for (int i = 0; i < 32; ++i) v[i] = act_fwd(round_bf16(v[i]), args.glu_kind) * round_bf16(u[i]);
               }
               put(to, half, v);
             }
