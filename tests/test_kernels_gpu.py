@@ -597,6 +597,24 @@ def test_qk_rope(tokens, N, KH, H, gap, norm):
     _check_status()
 
 
+@pytest.mark.parametrize("tokens,N,KH,H", [(3, 4, 2, 64), (1037, 16, 16, 64), (130, 8, 4, 128), (2100, 32, 4, 128), (700, 12, 8, 256)])
+def test_qk_rope_norms_like_the_norms_own_kernel(tokens, N, KH, H):
+    """1 / rms of every head bit for bit, in each of the norm's kernels for these widths; where the rotation runs by vectors (16384 units of
+    4 heads and 16 columns) the rotated rows too."""
+    k = _k()
+    pos = torch.arange(tokens, device="cuda", dtype=torch.int32) % 50
+    ang = _normal(50, H // 2, seed=3)
+    xs = [3 * _normal(tokens, n * H, seed=n) for n in (N, KH)]
+    xs, ws = [x.bfloat16() for x in xs], [(1 + 0.2 * _normal(H, seed=7 + i)).bfloat16() for i in (0, 1)]
+    got = k.qk_rope(*xs, H, pos, ang.cos(), ang.sin(), wq=ws[0], wk=ws[1], eps=1e-6, want_rstd=True)
+    for n, x, w, y, rstd in zip((N, KH), xs, ws, got[:2], got[2:]):
+        rows, want = k.rmsnorm_fwd(x.view(-1, H), w, 1e-6)
+        assert torch.equal(rstd, want)
+        if tokens * (H // 16) * ((n + 3) // 4) >= 16384:
+            assert torch.equal(y, k.rope_(rows.view(tokens, n, H), pos, ang.cos(), ang.sin()).view(tokens, -1))
+    _check_status()
+
+
 @pytest.mark.parametrize("qk_norm", [False, True])
 def test_model_joint_rotation_matches_separate(qk_norm):
     """The attention layer with the joint kernel and, made to by a hook or by a refusing kernel, with norm and rotation one by one."""

@@ -103,10 +103,14 @@ qk_rope_kernel(const QkArgs a) {
       unpack8(lo[h], p);
       unpack8(hi[h], q);
       if (NORM) {
-        float ss = 0.f;
+        // in the order of the norm's own kernels, where the two halves of a row belong to lanes that meet first
+        float sl = 0.f, sh = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ss += p[i] * p[i] + q[i] * q[i];
-        const float rstd = rsqrtf(row_sum<T>(ss) / (float)(2 * HALF) + a.eps);
+        for (int i = 0; i < 8; ++i) {
+          sl += p[i] * p[i];
+          sh += q[i] * q[i];
+        }
+        const float rstd = rsqrtf(row_sum<T>(sl + sh) / (float)(2 * HALF) + a.eps);
         if (h < n && j == 0 && r.rstd) r.rstd[(long long)tok * r.heads + h0 + h] = rstd;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {      // rounded as by the norm's own kernel and by the decode step's (decode.cu), so that all agree
