@@ -615,6 +615,21 @@ def test_qk_rope_norms_like_the_norms_own_kernel(tokens, N, KH, H):
     _check_status()
 
 
+@pytest.mark.parametrize("tokens,N,KH,H", [(5, 3, 1, 64), (2000, 14, 2, 64), (4100, 14, 2, 64), (1023, 8, 4, 128), (513, 32, 8, 128),
+                                           (255, 17, 4, 256)])
+@pytest.mark.parametrize("backward", [False, True])
+def test_qk_rope_rotates_like_the_rotations_own_kernels(tokens, N, KH, H, backward):
+    """Bit for bit, on both sides of the 16384 units of 4 heads and 16 columns that divide the rotation's kernels, for either tensor."""
+    k = _k()
+    pos = torch.arange(tokens, device="cuda", dtype=torch.int32) % 500
+    ang = _normal(500, H // 2, seed=3)
+    xs = [_normal(tokens, n * H, seed=n).bfloat16() for n in (N, KH)]
+    got = k.qk_rope(*xs, H, pos, ang.cos(), ang.sin(), backward=backward)
+    for n, x, y in zip((N, KH), xs, got):
+        assert torch.equal(y, k.rope_(x.view(tokens, n, H).clone(), pos, ang.cos(), ang.sin(), backward=backward).view(tokens, -1))
+    _check_status()
+
+
 @pytest.mark.parametrize("qk_norm", [False, True])
 def test_model_joint_rotation_matches_separate(qk_norm):
     """The attention layer with the joint kernel and, made to by a hook or by a refusing kernel, with norm and rotation one by one."""

@@ -383,3 +383,13 @@ int tb_make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint
 int tb_make_tmap_2d_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols);
 // Whole rows per box, as [cols / 64] slabs of [box_rows x 64] with the 128-byte swizzle: tma_load_3d at (0, row, 0). cols % 64 == 0.
 int tb_make_tmap_slabs_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
+
+// Rotary embedding by 16-byte vectors from 16384 units of 8 pairs by 4 heads on (up to what 32 bits count), by pairs below. The two round one
+// product each, in the second half of a row not the same one (rope_hi), and a joint kernel rounds what the tensor's own would have.
+constexpr int ROPE_HEADS = 4;
+inline long long rope_units(long long tokens, int heads, int H) { return tokens * (H / 16) * ((heads + ROPE_HEADS - 1) / ROPE_HEADS); }
+inline bool rope_by_vectors(long long units) { return units >= 16384 && units < (1LL << 31); }
+__device__ __forceinline__ float rope_lo(float lo, float hi, float c, float s) { return fmaf(lo, c, -(hi * s)); }
+__device__ __forceinline__ float rope_hi(float lo, float hi, float c, float s, bool vectors) {
+  return vectors ? fmaf(hi, c, lo * s) : fmaf(lo, s, hi * c);
+}

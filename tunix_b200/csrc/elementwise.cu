@@ -461,15 +461,13 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, const i
     uint32_t lo = *reinterpret_cast<uint32_t*>(base + j);
     uint32_t hi = *reinterpret_cast<uint32_t*>(base + half + j);
     const float a0 = bf16_lo(lo), a1 = bf16_hi(lo), b0 = bf16_lo(hi), b1 = bf16_hi(hi);
-    *reinterpret_cast<uint32_t*>(base + j) = pack_bf16(a0 * c.x - b0 * s.x, a1 * c.y - b1 * s.y);
-    *reinterpret_cast<uint32_t*>(base + half + j) =
-        pack_bf16(b0 * c.x + a0 * s.x, b1 * c.y + a1 * s.y);
+    *reinterpret_cast<uint32_t*>(base + j) = pack_bf16(rope_lo(a0, b0, c.x, s.x), rope_lo(a1, b1, c.y, s.y));
+    *reinterpret_cast<uint32_t*>(base + half + j) = pack_bf16(rope_hi(a0, b0, c.x, s.x, false), rope_hi(a1, b1, c.y, s.y, false));
   }
 }
 
 // The same with 16-byte accesses: a thread rotates 8 pairs of ROPE_HEADS heads of a token by the same angles. Bound by HBM: x read
 // and written once. B200, before -> after: 16384 x 32 x 128 79 -> 46 us, 4096 x 32 x 128 22 -> 14, 4004 x 16 x 256 21 -> 14.
-constexpr int ROPE_HEADS = 4;
 __global__ void __launch_bounds__(256)
 rope_vec_kernel(__nv_bfloat16* __restrict__ x, long long ld, const int* __restrict__ pos, const float* __restrict__ cos_t,
                 const float* __restrict__ sin_t, unsigned total, int heads, int H, float sign) {
@@ -501,8 +499,8 @@ rope_vec_kernel(__nv_bfloat16* __restrict__ x, long long ld, const int* __restri
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float a0 = bf16_lo(a[k]), a1 = bf16_hi(a[k]), b0 = bf16_lo(b[k]), b1 = bf16_hi(b[k]);
-        a[k] = pack_bf16(a0 * c[2 * k] - b0 * s[2 * k], a1 * c[2 * k + 1] - b1 * s[2 * k + 1]);
-        b[k] = pack_bf16(b0 * c[2 * k] + a0 * s[2 * k], b1 * c[2 * k + 1] + a1 * s[2 * k + 1]);
+        a[k] = pack_bf16(rope_lo(a0, b0, c[2 * k], s[2 * k]), rope_lo(a1, b1, c[2 * k + 1], s[2 * k + 1]));
+        b[k] = pack_bf16(rope_hi(a0, b0, c[2 * k], s[2 * k], true), rope_hi(a1, b1, c[2 * k + 1], s[2 * k + 1], true));
       }
       *reinterpret_cast<uint4*>(base + h * H) = make_uint4(a[0], a[1], a[2], a[3]);
       *reinterpret_cast<uint4*>(base + h * H + half) = make_uint4(b[0], b[1], b[2], b[3]);
@@ -750,11 +748,11 @@ TB_API int tb_rope(void* x, long long ld, const int* pos, const float* cos_t, co
                    long long tokens, int heads, int H, int backward, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (H % 4) return -2;
-  const long long units = tokens * (H / 16) * ((heads + ROPE_HEADS - 1) / ROPE_HEADS);
+  const long long units = rope_units(tokens, heads, H);
   // whole 16-byte pieces of both halves; a unit's number, and a turn's step beyond the last, fit 32 bits. Fewer units than these are
   // one short round of either kernel, of which the one by pairs has more threads (64 x 32 heads of 128, 4096 units: 2.2 us, 2.5 by
   // vectors; 256 x 32, 16384 units: 3.4, 2.7).
-  if (units >= 16384 && H % 16 == 0 && ld % 8 == 0 && units < (1LL << 31) &&
+  if (rope_by_vectors(units) && H % 16 == 0 && ld % 8 == 0 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15) == 0) {
     rope_vec_kernel<<<grid_for(units, 256), 256, 0, stream>>>((__nv_bfloat16*)x, ld, pos, cos_t, sin_t, (unsigned)units, heads, H,
                                                               backward ? -1.f : 1.f);

@@ -25,6 +25,7 @@ struct QkRows {                   // queries or keys: [tokens, heads * H], the h
   const __nv_bfloat16* w;         // [H]; null: no norm
   float* rstd;                    // [tokens * heads]
   int heads;
+  int vectors;                    // rotate as the tensor's own kernel by vectors does, else as the one by pairs
   // backward
   const __nv_bfloat16* dy;
   long long lddy;
@@ -122,8 +123,8 @@ qk_rope_kernel(const QkArgs a) {
         float o[8], t[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          o[i] = p[i] * c[i] - q[i] * s[i];
-          t[i] = q[i] * c[i] + p[i] * s[i];
+          o[i] = rope_lo(p[i], q[i], c[i], s[i]);
+          t[i] = rope_hi(p[i], q[i], c[i], s[i], r.vectors);
         }
         *reinterpret_cast<uint4*>(y + h * 2 * HALF) = pack8(o);
         *reinterpret_cast<uint4*>(y + h * 2 * HALF + HALF) = pack8(t);
@@ -251,8 +252,10 @@ TB_API int tb_qk_rope(const void* q, long long ldq, void* yq, long long ldyq, co
   if (tokens <= 0) return 0;
   if (tokens >= (1LL << 30) || (wq == nullptr) != (wk == nullptr) || (wq && backward)) return -2;
   QkArgs a = {};
-  a.q = {(const __nv_bfloat16*)q, (__nv_bfloat16*)yq, ldq, ldyq, (const __nv_bfloat16*)wq, rstd_q, heads_q, nullptr, 0, nullptr};
-  a.k = {(const __nv_bfloat16*)k, (__nv_bfloat16*)yk, ldk, ldyk, (const __nv_bfloat16*)wk, rstd_k, heads_k, nullptr, 0, nullptr};
+  a.q = {(const __nv_bfloat16*)q, (__nv_bfloat16*)yq, ldq, ldyq, (const __nv_bfloat16*)wq, rstd_q, heads_q,
+         rope_by_vectors(rope_units(tokens, heads_q, H)), nullptr, 0, nullptr};
+  a.k = {(const __nv_bfloat16*)k, (__nv_bfloat16*)yk, ldk, ldyk, (const __nv_bfloat16*)wk, rstd_k, heads_k,
+         rope_by_vectors(rope_units(tokens, heads_k, H)), nullptr, 0, nullptr};
   a.pos = pos; a.cos_t = cos_t; a.sin_t = sin_t; a.tokens = (unsigned)tokens; a.eps = eps; a.add_one = add_one;
   a.sign = backward ? -1.f : 1.f;
   if (!rows_ok(a.q) || !rows_ok(a.k) || !fits(a, H)) return -2;
@@ -277,9 +280,9 @@ TB_API int tb_qk_rope_bwd(const void* dyq, long long lddyq, const void* xq, long
   if (tokens <= 0) return 0;
   if (tokens >= (1LL << 30) || !wq || !wk || !rstd_q || !rstd_k) return -2;
   QkArgs a = {};
-  a.q = {(const __nv_bfloat16*)xq, (__nv_bfloat16*)dxq, ldxq, lddxq, (const __nv_bfloat16*)wq, const_cast<float*>(rstd_q), heads_q,
+  a.q = {(const __nv_bfloat16*)xq, (__nv_bfloat16*)dxq, ldxq, lddxq, (const __nv_bfloat16*)wq, const_cast<float*>(rstd_q), heads_q, 0,
          (const __nv_bfloat16*)dyq, lddyq, dwq};
-  a.k = {(const __nv_bfloat16*)xk, (__nv_bfloat16*)dxk, ldxk, lddxk, (const __nv_bfloat16*)wk, const_cast<float*>(rstd_k), heads_k,
+  a.k = {(const __nv_bfloat16*)xk, (__nv_bfloat16*)dxk, ldxk, lddxk, (const __nv_bfloat16*)wk, const_cast<float*>(rstd_k), heads_k, 0,
          (const __nv_bfloat16*)dyk, lddyk, dwk};
   a.pos = pos; a.cos_t = cos_t; a.sin_t = sin_t; a.tokens = (unsigned)tokens; a.add_one = add_one; a.sign = 1.f;
   if (!rows_ok(a.q) || !rows_ok(a.k) || !fits(a, H) || off16(dyq) || off16(dyk) || lddyq % 8 || lddyk % 8) return -2;
