@@ -252,6 +252,32 @@ def test_engine_packed_weights_match_unpacked():
         assert abs(la[0] - lb[0]) < 5e-2
 
 
+@pytest.mark.parametrize("family", [dict(qk_norm=True), dict(qk_norm=False, qkv_bias=True), dict(family="gemma2", post_norms=True, qk_norm=False)])
+def test_engine_few_sequences_round_behind_every_norm(family):
+    """Decode steps of one to four sequences of wide layers: log-probs bit for bit those of a model whose norms have to run by themselves."""
+    from tunix_b200 import _lib
+    from tunix_b200.common.configs import CacheConfig
+    from tunix_b200.generate.engine import PagedEngine
+    model = _model(hidden_dim=8192, **family)
+    with torch.no_grad():
+        for name, p in model.named_parameters():
+            if p.dim() == 1:
+                p.add_(0.3 * torch.randn(p.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(len(name))).to(p.dtype))
+    prompts = [[1, 5, 9, 77, 30], [1, 200, 3], [1] + list(range(10, 30)), [7, 8]]
+    cc = CacheConfig(cache_size=128, num_layers=2, num_kv_heads=2, head_dim=64)
+    for n in (1, 2, 4):
+        run = lambda: PagedEngine(model, Tok(), cc, page_size=16, max_running_requests=4)(  # noqa: E731
+            prompt_token_ids=prompts[:n], max_generation_steps=20, return_logprobs=True, eos_tokens=[511])
+        got = run()
+        hooks = [m.register_forward_hook(lambda *a: None) for layer in model.layers for m in layer.modules() if type(m).__name__ == "RMSNorm"]
+        want = run()
+        for h in hooks:
+            h.remove()
+        _lib.raise_if_kernel_error()
+        for t, u, x, y in zip(got.tokens, want.tokens, got.logprobs, want.logprobs):
+            assert list(t) == list(u) and list(x) == list(y)
+
+
 def test_engine_continuous_batching_matches_single_batch():
     """More requests than slots: finished sequences hand their slot to waiting ones; greedy results equal those of
     an engine that runs all requests side by side, and every page returns to the pool."""

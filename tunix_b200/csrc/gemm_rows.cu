@@ -25,8 +25,6 @@ struct RowsArgs {
   long long lda, ldb, ldc, ldr;
   int N, K, flags, kw;              // kw: warps that share a group of rows (1, 2, 4 or 8)
   int glu;                          // gated form: B is [2 N, K], gate rows above up rows; the activation (act_fwd)
-  const __nv_bfloat16* nw;          // NORM: weight [K] of the RMS norm that A passes first, and the numbers of that
-  float eps, add_one;
   void* C;
   const __nv_bfloat16 *bias, *resid;
   float alpha;
@@ -41,33 +39,29 @@ __device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
 }
 
 // GLU: a warp's R weight rows are R / 2 gate rows and their up rows, and one thread applies the activation to a pair of sums. One row of
-// 17920 x 1536 on packed weights and the tensor cores (tb_gemm_packed) 13.9 us, here: see tb_gemm_rows_ex.
-// NORM: A is multiplied by the norm's weight on the way and the sum by 1 / rms, whose square sum the same loads give. A norm of its own was a
-// launch of 2.7 us in front of the two products of a layer that begin with one (1536 columns), and a rounding.
-template <int M, int R, int U, bool GLU = false, bool NORM = false>
+// 17920 x 1536 on packed weights and the tensor cores (tb_gemm_packed) 13.9 us, here: see tb_gemm_rows_glu.
+template <int M, int R, int U, bool GLU = false>
 __global__ void __launch_bounds__(WARPS * 32)
 gemm_rows_kernel(const RowsArgs a) {
   constexpr int OUT = GLU ? R / 2 : R;                               // results of a group of rows
-  __shared__ float part[WARPS][R * M], part_ss[WARPS][M];
+  __shared__ float part[WARPS][R * M];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = WARPS / a.kw;                                      // groups of rows in this block
   const int n0 = (blockIdx.x * per + warp / a.kw) * OUT;
   const int k0 = (warp % a.kw) * STEP + lane * 8, stride = a.kw * STEP;
   pdl_trigger();
   pdl_wait();
-  float acc[R][M], ss[M];
+  float acc[R][M];
 #pragma unroll
-  for (int m = 0; m < M; ++m) {
-    ss[m] = 0.f;
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r][m] = 0.f;
-  }
+    for (int m = 0; m < M; ++m) acc[r][m] = 0.f;
   if (n0 < a.N) {
     const __nv_bfloat16* b[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) b[r] = a.B + ((long long)min(n0 + r % OUT, a.N - 1) + (r >= OUT ? a.N : 0)) * a.ldb;
     for (int k = k0; k < a.K; k += U * stride) {
-      uint4 w[U][R], x[U][M], nw[U];
+      uint4 w[U][R], x[U][M];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int at = k + u * stride;
@@ -80,34 +74,19 @@ gemm_rows_kernel(const RowsArgs a) {
 #pragma unroll
         for (int m = 0; m < M; ++m)
           x[u][m] = at < a.K ? *reinterpret_cast<const uint4*>(a.A + m * a.lda + at) : make_uint4(0u, 0u, 0u, 0u);
-        if (NORM) nw[u] = at < a.K ? *reinterpret_cast<const uint4*>(a.nw + at) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
         for (int m = 0; m < M; ++m) {
           const uint32_t xs[4] = {x[u][m].x, x[u][m].y, x[u][m].z, x[u][m].w};
-          float xf[8];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            xf[2 * i] = bf16_lo(xs[i]);
-            xf[2 * i + 1] = bf16_hi(xs[i]);
-          }
-          if (NORM) {
-            const uint32_t gs[4] = {nw[u].x, nw[u].y, nw[u].z, nw[u].w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              ss[m] = fmaf(xf[i], xf[i], ss[m]);
-              xf[i] *= (i & 1 ? bf16_hi(gs[i >> 1]) : bf16_lo(gs[i >> 1])) + a.add_one;
-            }
-          }
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const uint32_t ws[4] = {w[u][r].x, w[u][r].y, w[u][r].z, w[u][r].w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              acc[r][m] = fmaf(bf16_lo(ws[i]), xf[2 * i], acc[r][m]);
-              acc[r][m] = fmaf(bf16_hi(ws[i]), xf[2 * i + 1], acc[r][m]);
+              acc[r][m] = fmaf(bf16_lo(ws[i]), bf16_lo(xs[i]), acc[r][m]);
+              acc[r][m] = fmaf(bf16_hi(ws[i]), bf16_hi(xs[i]), acc[r][m]);
             }
           }
         }
@@ -120,30 +99,17 @@ gemm_rows_kernel(const RowsArgs a) {
       acc[r][m] = warp_sum(acc[r][m]);
       if (lane == 0) part[warp][r * M + m] = acc[r][m];
     }
-  if (NORM)
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      ss[m] = warp_sum(ss[m]);
-      if (lane == 0) part_ss[warp][m] = ss[m];
-    }
   __syncthreads();
   // one output a thread: group g of the block, row r of the group, row m of A
   if (threadIdx.x >= per * OUT * M) return;
   const int g = threadIdx.x / (OUT * M), rm = threadIdx.x % (OUT * M);
   const int n = (blockIdx.x * per + g) * OUT + rm / M, m = rm % M;
   if (n >= a.N) return;
-  float o = 0.f, rstd = 1.f;
+  float o = 0.f;
   for (int w = 0; w < a.kw; ++w) o += part[g * a.kw + w][rm];
-  if (NORM) {
-    float q = 0.f;
-    for (int w = 0; w < a.kw; ++w) q += part_ss[g * a.kw + w][m];
-    rstd = rsqrtf(q / (float)a.K + a.eps);
-    o *= rstd;
-  }
   if (GLU) {
     float up = 0.f;
     for (int w = 0; w < a.kw; ++w) up += part[g * a.kw + w][OUT * M + rm];
-    up *= rstd;
     reinterpret_cast<__nv_bfloat16*>(a.C)[m * a.ldc + n] = __float2bfloat16(act_fwd(o, a.glu) * up);
     return;
   }
@@ -199,34 +165,28 @@ int tb_gemm_rows_try(const void* A, const void* B, void* C, int M, int N, int K,
   return e == cudaSuccess ? 1 : -5;
 }
 
-// C [M, F] = act(A Wg^T) * (A Wu^T) for one to four rows, W = [Wg; Wu] [2 F, K] (glu >= 0: the activation), or C [M, F] = A W^T (+ bias), W
-// [F, K] (glu < 0). nw [K] (not null): A passes an RMS norm of that weight (+ add_one) and eps first. Returns 1 when launched, 0 when the call
-// is left to other kernels (more rows or weights than above, rows that are not whole 16-byte pieces), a negative code on error.
-TB_API int tb_gemm_rows_ex(const void* A, const void* W, void* C, int M, int F, int K, long long lda, long long ldw, long long ldc, int glu,
-                           const void* bias, const void* nw, float eps, float add_one, cudaStream_t stream) {
-  const int rows = glu >= 0 ? 2 * F : F;
-  if (M <= 0 || M > 4 || F <= 0 || K <= 0 || K % 8 || lda % 8 || ldw % 8 || (long long)rows * K > most_weights(M, rows) ||
-      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(nw)) & 15) || (glu >= 0 && bias))
+// C [M, F] = act(A Wg^T) * (A Wu^T) for one to four rows, W = [Wg; Wu] [2 F, K]. Returns 1 when launched, 0 when the call is left to the tensor
+// cores (more rows or weights than above, rows that are not whole 16-byte pieces), a negative code on error.
+TB_API int tb_gemm_rows_glu(const void* A, const void* W, void* C, int M, int F, int K, long long lda, long long ldw, long long ldc, int kind,
+                            cudaStream_t stream) {
+  if (M <= 0 || M > 4 || F <= 0 || K <= 0 || K % 8 || lda % 8 || ldw % 8 || 2LL * F * K > most_weights(M, 2 * F) ||
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15))
     return 0;
   RowsArgs a = {};
   a.A = reinterpret_cast<const __nv_bfloat16*>(A); a.B = reinterpret_cast<const __nv_bfloat16*>(W);
-  a.lda = lda; a.ldb = ldw; a.ldc = ldc; a.N = F; a.K = K; a.C = C; a.alpha = 1.f; a.glu = glu;
-  a.bias = reinterpret_cast<const __nv_bfloat16*>(bias); a.flags = bias ? GF_BIAS : 0;
-  a.nw = reinterpret_cast<const __nv_bfloat16*>(nw); a.eps = eps; a.add_one = add_one;
+  a.lda = lda; a.ldb = ldw; a.ldc = ldc; a.N = F; a.K = K; a.C = C; a.alpha = 1.f; a.glu = kind;
   constexpr int R = 4;
-  const int out = glu >= 0 ? R / 2 : R, groups = (F + out - 1) / out;
+  const int groups = (F + R / 2 - 1) / (R / 2);
   a.kw = 1;
   while (a.kw < WARPS && (long long)groups * a.kw / WARPS < 8 * 148 && a.kw * 2 * STEP <= K) a.kw *= 2;
   const int per = WARPS / a.kw;
   const dim3 grid((groups + per - 1) / per), block(WARPS * 32);
-  using Kernel = void (*)(RowsArgs);
-  const auto run = [&](Kernel plain, Kernel plain_norm, Kernel gated, Kernel gated_norm) {
-    return launch_pdl(glu >= 0 ? (nw ? gated_norm : gated) : nw ? plain_norm : plain, grid, block, 0, stream, a);
-  };
-#define ROWS_EX(m) run(gemm_rows_kernel<m, R, 1>, gemm_rows_kernel<m, R, 1, false, true>, gemm_rows_kernel<m, R, 1, true>, \
-                       gemm_rows_kernel<m, R, 1, true, true>)
-  const cudaError_t e = M == 1 && glu < 0 && F <= 2048 ? run(gemm_rows_kernel<1, R, 2>, gemm_rows_kernel<1, R, 2, false, true>, nullptr, nullptr) :
-                        M == 1 ? ROWS_EX(1) : M == 2 ? ROWS_EX(2) : M == 3 ? ROWS_EX(3) : ROWS_EX(4);
-#undef ROWS_EX
+  cudaError_t e;
+  switch (M) {
+    case 1: e = launch_pdl(gemm_rows_kernel<1, R, 1, true>, grid, block, 0, stream, a); break;
+    case 2: e = launch_pdl(gemm_rows_kernel<2, R, 1, true>, grid, block, 0, stream, a); break;
+    case 3: e = launch_pdl(gemm_rows_kernel<3, R, 1, true>, grid, block, 0, stream, a); break;
+    default: e = launch_pdl(gemm_rows_kernel<4, R, 1, true>, grid, block, 0, stream, a); break;
+  }
   return e == cudaSuccess ? 1 : -5;
 }

@@ -330,7 +330,7 @@ class PagedEngine(BaseSampler):
 
         def few(name, w):
             return name == "gu" and w is not None and self.exec is None and w.shape[0] >= self.ROWS_GLU_MIN and \
-                K.rows_takes(self._decode_rows, w.shape[0], w.shape[1])
+                K.rows_glu_takes(self._decode_rows, w.shape[0] // 2, w.shape[1])
         fresh = self._packed is None or len(self._packed) != len(srcs)
         if not fresh:
             for have, src in zip(self._packed, srcs):
@@ -392,22 +392,10 @@ class PagedEngine(BaseSampler):
     def _lin(self, mod, x, residual=None):
         return mod(x, residual=residual)   # Linear.forward handles LoRA; no autograd under no_grad
 
-    @staticmethod
-    def _rows(x, w, norm, **kw):
-        """A product of few rows whose norm the kernel applies (K.gemm_rows); None where either has to be done on its own."""
-        return K.gemm_rows(x, w, norm=norm.weight, eps=norm.eps, add_one=norm.add_one, **kw) if _bare(norm, RMSNorm) else None
-
-    def _mlp(self, layer, i, h, residual=None, decode=False, norm=None):
-        """`norm`: the layer's norm, which h has not passed yet."""
+    def _mlp(self, layer, i, h, residual=None, decode=False):
         wgu = self._wgu[i]
         if wgu is None and self.tpw > 1:
             raise NotImplementedError("tensor-parallel decode needs plain MLP weights (no adapters, no quantised base, no MoE)")
-        # `_pack_all` has left these out
-        few = decode and wgu is not None and wgu.shape[0] >= self.ROWS_GLU_MIN and K.rows_takes(h.numel() // h.shape[-1], *wgu.shape)
-        kind = None if wgu is None else K.GLU_SILU if layer.mlp.kind == "silu" else K.GLU_GELU
-        a = self._rows(h.reshape(-1, h.shape[-1]), wgu, norm, glu=kind) if few and norm is not None else None
-        if a is None and norm is not None:
-            h = norm(h)
         if wgu is None:
             if self.cfg.is_moe and h.dim() == 2:      # decode rows: the expert block wants [batch, time, D]
                 r3 = residual[:, None] if residual is not None else None
@@ -415,9 +403,10 @@ class PagedEngine(BaseSampler):
             return layer.mlp(h, residual=residual)
         Fd = wgu.shape[0] // 2
         h2 = h.reshape(-1, h.shape[-1])
+        kind = K.GLU_SILU if layer.mlp.kind == "silu" else K.GLU_GELU
+        few = decode and wgu.shape[0] >= self.ROWS_GLU_MIN and K.rows_glu_takes(h2.shape[0], Fd, h2.shape[1])        # `_pack_all` has left these out
         pgu = self._pk(i, "gu") if decode and not few else None
-        if a is None and few:
-            a = K.gemm_rows(h2, wgu, glu=kind)
+        a = K.gemm_rows_glu(h2, wgu, kind) if few else None
         if a is None and pgu is not None and pgu.glu:
             a = K.gemm_packed(h2, pgu, glu=kind)
         if a is None and pgu is None:
@@ -445,10 +434,10 @@ class PagedEngine(BaseSampler):
         cfg = self.cfg
         if cfg.post_norms:
             x = x + layer.post_attn_norm(attn_out)
-            m = self._mlp(layer, i, x, decode=decode, norm=layer.post_attention_layernorm)
+            m = self._mlp(layer, i, layer.post_attention_layernorm(x), decode=decode)
             return x + layer.post_ffw_norm(m)
         x = attn_out          # o_proj already added the residual
-        return self._mlp(layer, i, x, residual=x, decode=decode, norm=layer.post_attention_layernorm)
+        return self._mlp(layer, i, layer.post_attention_layernorm(x), residual=x, decode=decode)
 
     def _prefill(self, toks, positions, seg, slots, prev_len=None, write_from=None):
         """toks [B,P] left padded: the prompt tokens this call computes. `prev_len` [B] (or None): tokens of each row
@@ -600,15 +589,12 @@ class PagedEngine(BaseSampler):
         pos = st["positions"]           # position of the token being fed = seq_len before it is appended
         lens = st["seq_lens"]           # length including that token
         for i, layer in enumerate(self._model.layers):
-            at, wqkv, bq = layer.self_attn, self._wqkv[i], self._bqkv[i]
-            pq = self._pk(i, "qkv") if wqkv is not None else None
-            # (narrow layers round in front of every product, in a step of few rows as in one of many)
-            wide = wqkv is not None and pq is None and self._wgu[i] is not None and self._wgu[i].shape[0] >= self.ROWS_GLU_MIN
-            qkv = self._rows(x, wqkv, layer.input_layernorm, bias=bq) if wide else None
-            h = layer.input_layernorm(x) if qkv is None else None
-            if wqkv is not None:
-                if qkv is None:
-                    qkv = K.gemm_packed(h, pq, bias=bq) if pq is not None else F.linear(h, wqkv, bq)
+            h = layer.input_layernorm(x)
+            at = layer.self_attn
+            if self._wqkv[i] is not None:
+                pq = self._pk(i, "qkv")
+                bq = self._bqkv[i]
+                qkv = K.gemm_packed(h, pq, bias=bq) if pq is not None else F.linear(h, self._wqkv[i], bq)
                 cos, sin = self._rope(i)
                 qn, kn = (at.q_norm, at.k_norm) if cfg.qk_norm else (None, None)
                 K.qkv_post(qkv, st["slots"], pos, qn.weight if qn is not None else None,

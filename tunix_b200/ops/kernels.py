@@ -267,30 +267,26 @@ def gemm_glu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, kind: int, kee
     return h, g, u
 
 
-def rows_takes(M: int, rows: int, D: int) -> bool:
-    """Whether `gemm_rows` takes M rows by a weight of this many (aligned) rows."""
-    return 0 < M <= 4 and D % 8 == 0 and rows * D <= (128, 64, 16 if rows <= 4096 else 12, 16 if rows <= 4096 else 12)[M - 1] << 20
+def rows_glu_takes(M: int, Fdim: int, D: int) -> bool:
+    """Whether `gemm_rows_glu` takes M rows by these (aligned) weights."""
+    return M <= 4 and D % 8 == 0 and 2 * Fdim * D <= (128, 64, 16 if 2 * Fdim <= 4096 else 12, 16 if 2 * Fdim <= 4096 else 12)[M - 1] << 20
 
 
-def gemm_rows(x: torch.Tensor, w: torch.Tensor, *, glu: int | None = None, bias: torch.Tensor | None = None, norm: torch.Tensor | None = None,
-              eps: float = 0.0, add_one: bool = False):
-    """x @ w^T (+ bias), or with `glu` (an activation) act(x @ gate^T) * (x @ up^T) for w = [gate; up], of one to four rows; x passes an RMS norm
-    of weight `norm` first where that is given. None for calls that are left to other kernels."""
+def gemm_rows_glu(x: torch.Tensor, w: torch.Tensor, kind: int):
+    """act(x @ gate^T) * (x @ up^T) for one to four rows, w = [gate; up] [2 F, D]; None for calls that are left to the tensor cores."""
     assert x.dtype == w.dtype == torch.bfloat16 and _is2d_rowmajor(x) and _is2d_rowmajor(w) and x.shape[1] == w.shape[1]
-    (M, D), rows = x.shape, w.shape[0]
-    if not rows_takes(M, rows, D) or (norm is not None and (norm.dtype != torch.bfloat16 or not norm.is_contiguous() or norm.numel() != D)):
+    (M, D), Fdim = x.shape, w.shape[0] // 2
+    if not rows_glu_takes(M, Fdim, D):
         return None
-    assert bias is None or (glu is None and bias.dtype == torch.bfloat16 and bias.numel() == rows and bias.is_contiguous())
-    out = torch.empty((M, rows if glu is None else rows // 2), dtype=torch.bfloat16, device=x.device)
-    rc = _lib.cuda().tb_gemm_rows_ex(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, out.shape[1], D, x.stride(0), w.stride(0), out.stride(0),
-                                     -1 if glu is None else glu, _lib.ptr(bias), _lib.ptr(norm), float(eps), 1.0 if add_one else 0.0,
-                                     _lib.stream_ptr())
+    h = torch.empty((M, Fdim), dtype=torch.bfloat16, device=x.device)
+    rc = _lib.cuda().tb_gemm_rows_glu(x.data_ptr(), w.data_ptr(), h.data_ptr(), M, Fdim, D, x.stride(0), w.stride(0), Fdim, kind,
+                                      _lib.stream_ptr())
     if rc == 0:
         return None
     if rc < 0:
-        _lib.check(rc, "tb_gemm_rows_ex")
+        _lib.check(rc, "tb_gemm_rows_glu")
     _count()
-    return out
+    return h
 
 
 def embedding_fwd(ids: torch.Tensor, table: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
