@@ -278,6 +278,38 @@ def test_engine_few_sequences_round_behind_every_norm(family):
             assert list(t) == list(u) and list(x) == list(y)
 
 
+@pytest.mark.parametrize("n", [1, 3, 6])
+def test_engine_short_calls_and_few_sequences_read_packed_weights(n, monkeypatch):
+    """Calls of few steps and of few sequences multiply by packed weights as longer ones do, and so round alike; first tokens alone pack the
+    head, and a call after that packs the layers."""
+    from tunix_b200 import _lib
+    from tunix_b200.common.configs import CacheConfig
+    from tunix_b200.generate.engine import PagedEngine
+    from tunix_b200.ops import kernels as K
+    model = _model(hidden_dim=8192, vocab_size=1024)
+    prompts = [[1, 5, 9, 77, 30], [1, 200, 3], [1] + list(range(10, 30)), [7, 8], [9, 9, 4], [100]][:n]
+    seen, real = [], K.gemm_packed
+    monkeypatch.setattr(K, "gemm_packed", lambda x, pw, **kw: (seen.append(pw.N), real(x, pw, **kw))[1])
+    eng = PagedEngine(model, Tok(), CacheConfig(cache_size=128, num_layers=2, num_kv_heads=2, head_dim=64), page_size=16, max_running_requests=8)
+    eng.pack_min_rows = 1024
+    outs = []
+    for steps, widths in ((1, {1024}), (4, {1024, 16384}), (20, {1024, 16384}), (1, {1024})):
+        seen.clear()
+        outs.append(eng(prompt_token_ids=prompts, max_generation_steps=steps, return_logprobs=True, eos_tokens=[1023]))
+        assert set(seen) == widths
+    _lib.raise_if_kernel_error()
+    for out, steps in zip(outs, (1, 4, 20, 1)):
+        for t, u, x, y in zip(out.tokens, outs[2].tokens, out.logprobs, outs[2].logprobs):
+            assert list(t) == list(u)[:steps] and list(x) == list(y)[:steps]
+    with torch.no_grad():                # weights changed in place reach the buffers of a call for first tokens too
+        model.head_weight().mul_(0.5)
+    fresh = PagedEngine(model, Tok(), CacheConfig(cache_size=128, num_layers=2, num_kv_heads=2, head_dim=64), page_size=16, max_running_requests=8)
+    fresh.pack_min_rows = 1024
+    for steps in (1, 4):
+        got, want = (e(prompt_token_ids=prompts, max_generation_steps=steps, return_logprobs=True, eos_tokens=[1023]) for e in (eng, fresh))
+        assert [list(x) for x in got.logprobs] == [list(x) for x in want.logprobs]
+
+
 def test_engine_continuous_batching_matches_single_batch():
     """More requests than slots: finished sequences hand their slot to waiting ones; greedy results equal those of
     an engine that runs all requests side by side, and every page returns to the pool."""

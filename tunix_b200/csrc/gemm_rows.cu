@@ -11,7 +11,6 @@
 // Bound by latency (one wave: launch, one round of loads, one reduction) up to about 10 MB of weights and by HBM above. B200, one
 // row, in a graph with cold weights, tensor cores -> here: 256 x 1536 8.7 -> 2.4 us, 1536 x 1536 9.7 -> 3.7, 1536 x 8960 13.4 -> 7.6,
 // 4096 x 4096 12.2 -> 7.5, 4096 x 12288 24.2 -> 17.7; four rows 8.9 -> 3.4, 9.6 -> 4.7, 13.5 -> 9.2.
-#include "activation.cuh"
 #include "common.cuh"
 
 using namespace tb;
@@ -24,7 +23,6 @@ struct RowsArgs {
   const __nv_bfloat16 *A, *B;
   long long lda, ldb, ldc, ldr;
   int N, K, flags, kw;              // kw: warps that share a group of rows (1, 2, 4 or 8)
-  int glu;                          // gated form: B is [2 N, K], gate rows above up rows; the activation (act_fwd)
   void* C;
   const __nv_bfloat16 *bias, *resid;
   float alpha;
@@ -38,16 +36,13 @@ __device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
   return v;
 }
 
-// GLU: a warp's R weight rows are R / 2 gate rows and their up rows, and one thread applies the activation to a pair of sums. One row of
-// 17920 x 1536 on packed weights and the tensor cores (tb_gemm_packed) 13.9 us, here: see tb_gemm_rows_glu.
-template <int M, int R, int U, bool GLU = false>
+template <int M, int R, int U>
 __global__ void __launch_bounds__(WARPS * 32)
 gemm_rows_kernel(const RowsArgs a) {
-  constexpr int OUT = GLU ? R / 2 : R;                               // results of a group of rows
   __shared__ float part[WARPS][R * M];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = WARPS / a.kw;                                      // groups of rows in this block
-  const int n0 = (blockIdx.x * per + warp / a.kw) * OUT;
+  const int n0 = (blockIdx.x * per + warp / a.kw) * R;
   const int k0 = (warp % a.kw) * STEP + lane * 8, stride = a.kw * STEP;
   pdl_trigger();
   pdl_wait();
@@ -59,7 +54,7 @@ gemm_rows_kernel(const RowsArgs a) {
   if (n0 < a.N) {
     const __nv_bfloat16* b[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) b[r] = a.B + ((long long)min(n0 + r % OUT, a.N - 1) + (r >= OUT ? a.N : 0)) * a.ldb;
+    for (int r = 0; r < R; ++r) b[r] = a.B + (long long)min(n0 + r, a.N - 1) * a.ldb;
     for (int k = k0; k < a.K; k += U * stride) {
       uint4 w[U][R], x[U][M];
 #pragma unroll
@@ -101,18 +96,12 @@ gemm_rows_kernel(const RowsArgs a) {
     }
   __syncthreads();
   // one output a thread: group g of the block, row r of the group, row m of A
-  if (threadIdx.x >= per * OUT * M) return;
-  const int g = threadIdx.x / (OUT * M), rm = threadIdx.x % (OUT * M);
-  const int n = (blockIdx.x * per + g) * OUT + rm / M, m = rm % M;
+  if (threadIdx.x >= per * R * M) return;
+  const int g = threadIdx.x / (R * M), rm = threadIdx.x % (R * M);
+  const int n = (blockIdx.x * per + g) * R + rm / M, m = rm % M;
   if (n >= a.N) return;
   float o = 0.f;
   for (int w = 0; w < a.kw; ++w) o += part[g * a.kw + w][rm];
-  if (GLU) {
-    float up = 0.f;
-    for (int w = 0; w < a.kw; ++w) up += part[g * a.kw + w][OUT * M + rm];
-    reinterpret_cast<__nv_bfloat16*>(a.C)[m * a.ldc + n] = __float2bfloat16(act_fwd(o, a.glu) * up);
-    return;
-  }
   o *= a.alpha;
   if (a.flags & GF_BIAS) o += __bfloat162float(a.bias[n]);
   if (a.flags & GF_RESIDUAL) o += __bfloat162float(a.resid[m * a.ldr + n]);
@@ -124,8 +113,6 @@ gemm_rows_kernel(const RowsArgs a) {
     *c = __float2bfloat16((a.flags & GF_ACCUM) ? o + __bfloat162float(*c) : o);
   }
 }
-
-long long most_weights(int M, int N) { return (M == 1 ? 128LL : M == 2 ? 64LL : N <= 4096 ? 16LL : 12LL) << 20; }
 
 }  // namespace
 
@@ -139,8 +126,9 @@ int tb_gemm_rows_try(const void* A, const void* B, void* C, int M, int N, int K,
   // 9.9 / 12.3, 6144 x 4096 14.7 / 14.8; four, 12.6 / 12.3 and 14.7 / 14.7. Three and four rows of many short columns already meet
   // there below: four, 9728 x 896 8.4 / 8.8, 16384 x 1024 14.4 / 10.9, 65536 x 256 14.1 / 11.7 (1024 x 16384 12.3 / 18.6).
   if (M > 4 || K % 8 || (flags & ~(GF_OUT_F32 | GF_ACCUM | GF_BIAS | GF_RESIDUAL))) return 0;
-  if ((long long)N * K > most_weights(M, N)) return 0;
-  RowsArgs a = {};
+  const long long most = (M == 1 ? 128LL : M == 2 ? 64LL : N <= 4096 ? 16LL : 12LL) << 20;
+  if ((long long)N * K > most) return 0;
+  RowsArgs a;
   a.A = reinterpret_cast<const __nv_bfloat16*>(A); a.B = reinterpret_cast<const __nv_bfloat16*>(B);
   a.lda = lda; a.ldb = ldb; a.ldc = ldc; a.ldr = ldr; a.N = N; a.K = K; a.flags = flags; a.C = C;
   a.bias = reinterpret_cast<const __nv_bfloat16*>(bias); a.resid = reinterpret_cast<const __nv_bfloat16*>(resid); a.alpha = alpha;
@@ -161,32 +149,6 @@ int tb_gemm_rows_try(const void* A, const void* B, void* C, int M, int N, int K,
     case 2: e = launch_pdl(gemm_rows_kernel<2, R, 1>, grid, block, 0, stream, a); break;
     case 3: e = launch_pdl(gemm_rows_kernel<3, R, 1>, grid, block, 0, stream, a); break;
     default: e = launch_pdl(gemm_rows_kernel<4, R, 1>, grid, block, 0, stream, a); break;
-  }
-  return e == cudaSuccess ? 1 : -5;
-}
-
-// C [M, F] = act(A Wg^T) * (A Wu^T) for one to four rows, W = [Wg; Wu] [2 F, K]. Returns 1 when launched, 0 when the call is left to the tensor
-// cores (more rows or weights than above, rows that are not whole 16-byte pieces), a negative code on error.
-TB_API int tb_gemm_rows_glu(const void* A, const void* W, void* C, int M, int F, int K, long long lda, long long ldw, long long ldc, int kind,
-                            cudaStream_t stream) {
-  if (M <= 0 || M > 4 || F <= 0 || K <= 0 || K % 8 || lda % 8 || ldw % 8 || 2LL * F * K > most_weights(M, 2 * F) ||
-      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15))
-    return 0;
-  RowsArgs a = {};
-  a.A = reinterpret_cast<const __nv_bfloat16*>(A); a.B = reinterpret_cast<const __nv_bfloat16*>(W);
-  a.lda = lda; a.ldb = ldw; a.ldc = ldc; a.N = F; a.K = K; a.C = C; a.alpha = 1.f; a.glu = kind;
-  constexpr int R = 4;
-  const int groups = (F + R / 2 - 1) / (R / 2);
-  a.kw = 1;
-  while (a.kw < WARPS && (long long)groups * a.kw / WARPS < 8 * 148 && a.kw * 2 * STEP <= K) a.kw *= 2;
-  const int per = WARPS / a.kw;
-  const dim3 grid((groups + per - 1) / per), block(WARPS * 32);
-  cudaError_t e;
-  switch (M) {
-    case 1: e = launch_pdl(gemm_rows_kernel<1, R, 1, true>, grid, block, 0, stream, a); break;
-    case 2: e = launch_pdl(gemm_rows_kernel<2, R, 1, true>, grid, block, 0, stream, a); break;
-    case 3: e = launch_pdl(gemm_rows_kernel<3, R, 1, true>, grid, block, 0, stream, a); break;
-    default: e = launch_pdl(gemm_rows_kernel<4, R, 1, true>, grid, block, 0, stream, a); break;
   }
   return e == cudaSuccess ? 1 : -5;
 }

@@ -181,7 +181,6 @@ class PagedEngine(BaseSampler):
         self.pack_weights = pack_weights
         self.pack_min_rows = 16384
         self._packed_on = False     # per call: the packed form wins up to 128 running sequences (one row of tiles)
-        self._decode_rows = 0       # per call: rows of a decode step
         self._packed = None
         self.check_every = check_every
         self.max_pages_per_seq = (self.cache_size + page_size - 1) // page_size
@@ -301,17 +300,12 @@ class PagedEngine(BaseSampler):
     def _plain(mod) -> bool:
         return mod.quant is None and mod.bias is None and not (mod.lora_a is not None and mod.lora_enabled)
 
-    # Steps of a call that pay for packing: it reads and writes a weight once (24576 x 4096 154 us, 128256 x 4096 390 us) and a step of 64 rows
-    # gains 8 us with the one (activation in the epilogue included) and 18 us with the other.
-    PACK_STEPS = 16
-    # Rows of a gate / up weight from which one to four rows stream it as it is, activation included (K.gemm_rows), with nothing rounded in
-    # between; as they were packed from there. Narrower ones keep two launches.
-    ROWS_GLU_MIN = 16384
-
-    def _pack_all(self) -> None:
+    def _pack_all(self, steps: bool = True) -> None:
         """(Re)pack the weights the decode step multiplies by. The buffers are allocated once, so a captured
         decode graph keeps pointing at them; a projection with bias, LoRA or a quantised base is left to the
-        unpacked path (entry None), and so are gate / up weights that the step's few rows stream as they are."""
+        unpacked path (entry None). Without `steps` (a call for first tokens alone) the head alone: nothing reads the layers' packed
+        weights then, and the next call with steps packs them. (4 layers of 28672 x 4096 take 0.7 ms, and first tokens of 8 prompts of 4096
+        tokens 38.)"""
         if not self.pack_weights:
             self._packed = None
             return
@@ -327,29 +321,23 @@ class PagedEngine(BaseSampler):
             for name, w in src.items():
                 if w is not None and (w.shape[0] < self.pack_min_rows or w.dtype != torch.bfloat16 or w.shape[1] % 8):
                     src[name] = None
-
-        def few(name, w):
-            return name == "gu" and w is not None and self.exec is None and w.shape[0] >= self.ROWS_GLU_MIN and \
-                K.rows_glu_takes(self._decode_rows, w.shape[0] // 2, w.shape[1])
+        first = 0 if steps else len(srcs) - 1
         fresh = self._packed is None or len(self._packed) != len(srcs)
         if not fresh:
-            for have, src in zip(self._packed, srcs):
+            for have, src in zip(self._packed[first:], srcs[first:]):
                 for name, w in src.items():
                     pw = have.get(name)
-                    if few(name, w):          # not read in this call, whatever it holds
-                        continue
                     if (pw is None) != (w is None) or (pw is not None and (pw.N, pw.K) != tuple(w.shape)):
                         fresh = True
         if fresh:
             # the fused gate / up weight is packed with its rows interleaved, so that the GEMM's epilogue applies the
             # gated activation (no [rows, 2F] intermediate, no separate activation kernel)
-            self._packed = [{name: (K.PackedWeight(w, glu=(name == "gu" and w.shape[0] % 32 == 0))
-                                    if w is not None and not few(name, w) else None)
-                             for name, w in src.items()} for src in srcs]
+            self._packed = [{name: (K.PackedWeight(w, glu=(name == "gu" and w.shape[0] % 32 == 0)) if w is not None and i >= first else None)
+                             for name, w in src.items()} for i, src in enumerate(srcs)]
             return
-        for have, src in zip(self._packed, srcs):
+        for have, src in zip(self._packed[first:], srcs[first:]):
             for name, w in src.items():
-                if have[name] is not None and not few(name, w):
+                if have[name] is not None:
                     have[name].refresh(w)
 
     def _pk(self, i, name):
@@ -403,16 +391,14 @@ class PagedEngine(BaseSampler):
             return layer.mlp(h, residual=residual)
         Fd = wgu.shape[0] // 2
         h2 = h.reshape(-1, h.shape[-1])
+        pgu = self._pk(i, "gu") if decode else None
         kind = K.GLU_SILU if layer.mlp.kind == "silu" else K.GLU_GELU
-        few = decode and wgu.shape[0] >= self.ROWS_GLU_MIN and K.rows_glu_takes(h2.shape[0], Fd, h2.shape[1])        # `_pack_all` has left these out
-        pgu = self._pk(i, "gu") if decode and not few else None
-        a = K.gemm_rows_glu(h2, wgu, kind) if few else None
-        if a is None and pgu is not None and pgu.glu:
+        joint = K.gemm_glu(h2, wgu[:Fd], wgu[Fd:], kind) if pgu is None else None
+        if joint is not None:
+            a = joint[0]
+        elif pgu is not None and pgu.glu:
             a = K.gemm_packed(h2, pgu, glu=kind)
-        if a is None and pgu is None:
-            joint = K.gemm_glu(h2, wgu[:Fd], wgu[Fd:], kind)
-            a = None if joint is None else joint[0]
-        if a is None:
+        else:
             gu = K.gemm_packed(h2, pgu) if pgu is not None else F.linear(h2, wgu)
             a = K.glu_fwd(gu[:, :Fd], gu[:, Fd:], kind)
         pdown = self._pk(i, "down") if decode else None
@@ -671,10 +657,9 @@ class PagedEngine(BaseSampler):
         self._model.eval()
         prompts_all, plens_all = pad_prompts_left(rows, plen, pad_id)
         self._fuse_all()
-        self._decode_rows = min(self.max_running, len(rows))
-        self._packed_on = self.pack_weights and self._decode_rows <= 128 and max_generation_steps >= self.PACK_STEPS
+        self._packed_on = self.pack_weights and min(self.max_running, len(rows)) <= 128
         if self._packed_on:
-            self._pack_all()
+            self._pack_all(steps=max_generation_steps > 1)
         from .. import _lib
         _lib.register_cuda_sigs({"tb_set_pdl": [_lib.I]})
         _lib.cuda().tb_set_pdl(1 if self.use_pdl else 0)
@@ -1281,7 +1266,6 @@ class EngineServer:
                 torch.cuda.set_device(eng.device)
             with torch.no_grad():
                 eng._fuse_all()
-                eng._decode_rows = eng.max_running
                 eng._packed_on = eng.pack_weights and eng.max_running <= 128
                 if eng._packed_on:
                     eng._pack_all()

@@ -267,28 +267,6 @@ def gemm_glu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, kind: int, kee
     return h, g, u
 
 
-def rows_glu_takes(M: int, Fdim: int, D: int) -> bool:
-    """Whether `gemm_rows_glu` takes M rows by these (aligned) weights."""
-    return M <= 4 and D % 8 == 0 and 2 * Fdim * D <= (128, 64, 16 if 2 * Fdim <= 4096 else 12, 16 if 2 * Fdim <= 4096 else 12)[M - 1] << 20
-
-
-def gemm_rows_glu(x: torch.Tensor, w: torch.Tensor, kind: int):
-    """act(x @ gate^T) * (x @ up^T) for one to four rows, w = [gate; up] [2 F, D]; None for calls that are left to the tensor cores."""
-    assert x.dtype == w.dtype == torch.bfloat16 and _is2d_rowmajor(x) and _is2d_rowmajor(w) and x.shape[1] == w.shape[1]
-    (M, D), Fdim = x.shape, w.shape[0] // 2
-    if not rows_glu_takes(M, Fdim, D):
-        return None
-    h = torch.empty((M, Fdim), dtype=torch.bfloat16, device=x.device)
-    rc = _lib.cuda().tb_gemm_rows_glu(x.data_ptr(), w.data_ptr(), h.data_ptr(), M, Fdim, D, x.stride(0), w.stride(0), Fdim, kind,
-                                      _lib.stream_ptr())
-    if rc == 0:
-        return None
-    if rc < 0:
-        _lib.check(rc, "tb_gemm_rows_glu")
-    _count()
-    return h
-
-
 def embedding_fwd(ids: torch.Tensor, table: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     assert ids.dtype == torch.int32 and ids.is_contiguous() and table.dtype == torch.bfloat16
     tokens = ids.numel()
