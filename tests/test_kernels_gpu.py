@@ -826,6 +826,25 @@ def test_gemm_with_a_short_side(M, N, K_, a_mn, b_mn):
     _check_status()
 
 
+@pytest.mark.parametrize("M,N,K_", [(64, 4096, 12288), (5, 4096, 8192), (16, 1536, 8960), (33, 3590, 14336), (48, 800, 9000), (17, 4096, 4096),
+                                    (64, 2304, 4104), (64, 9472, 4096)])
+def test_gemm_of_a_few_rows_sums_the_same_partial_products(M, N, K_):
+    """Bit for bit what the kernel for higher problems gives (the same rows among 65, which it takes from K = 8192 on, or the product scaled by
+    two, which it takes always), whatever the rows, ragged columns and k-blocks and way out."""
+    k = _k()
+    a, b = _normal(65, K_, seed=1).bfloat16(), _normal(N, K_, seed=2).bfloat16()
+    bias, res, base = _normal(N, seed=3).bfloat16(), _normal(65, N, seed=4).bfloat16(), _normal(65, N, seed=5).bfloat16()
+    for kw in (dict(), dict(bias=bias), dict(bias=bias, residual=res), dict(out_dtype=torch.float32)):
+        cut = {key: v[:M] if key == "residual" else v for key, v in kw.items()}
+        got = k.gemm(a[:M], b, **cut)
+        assert torch.equal(2 * got, k.gemm(a[:M], b, alpha=2.0, **{key: v if key == "out_dtype" else 2 * v for key, v in cut.items()}))
+        if K_ >= 8192:
+            assert torch.equal(got, k.gemm(a, b, **kw)[:M])
+    got, two = base[:M].clone(), 2 * base[:M]
+    assert torch.equal(2 * k.gemm(a[:M], b, out=got, accumulate=True), k.gemm(a[:M], b, out=two, accumulate=True, alpha=2.0))
+    _check_status()
+
+
 @pytest.mark.parametrize("rows,V,D,share,chunk", [(4094, 2048, 512, 0.6, 2048), (2250, 5000, 264, 0.5, 1000), (3000, 4096, 256, 0.0, 2048),
                                                   (2048, 2304, 256, 1.0, 2048), (5000, 3080, 384, 0.02, 2048)])
 @pytest.mark.parametrize("softcap,want_ent", [(0.0, True), (30.0, False)])

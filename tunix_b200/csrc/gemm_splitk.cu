@@ -236,11 +236,9 @@ int g_sk_sms = 0;
 
 }  // namespace
 
-// Returns 1 when the problem was launched here, 0 when it is not a split-K case (the caller runs the persistent
-// kernel), a negative code on error. A and B K-major, same conventions as tb_gemm_bf16.
-int tb_gemm_splitk_try(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                       long long ldc, int flags, const void* bias, const void* resid, long long ldr, float alpha,
-                       int* status, cudaStream_t stream, const void* b_packed) {
+// The split of the K range for a problem that this kernel takes, 0 for others, a negative code on error. (Also asked by gemm_stream.cu, which sums
+// the same partial products.)
+int tb_gemm_splitk_split(int M, int N, int K, int flags) {
   if (flags & 3) return 0;                              // MN-major operands stay on the persistent kernel
   // Measured on B200 against the persistent kernel's narrow tiles: the split pays once the K loop is long
   // (down projections, K >= 8192: 40 -> 28 us at 64 x 4096 x 12288); at K = 4096 it wins up to 64 rows
@@ -293,6 +291,17 @@ int tb_gemm_splitk_try(const void* A, const void* B, void* C, int M, int N, int 
   for (int s = 1; s <= 8; ++s)
     if (eff[s] >= 0.92 * best) { S = s; break; }
   if (S == 1 && tiles >= g_sk_sms) return 0;            // enough tiles for the persistent kernel
+  return S;
+}
+
+// Returns 1 when the problem was launched here, 0 when it is not a split-K case (the caller runs the persistent
+// kernel), a negative code on error. A and B K-major, same conventions as tb_gemm_bf16.
+int tb_gemm_splitk_try(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                       long long ldc, int flags, const void* bias, const void* resid, long long ldr, float alpha,
+                       int* status, cudaStream_t stream, const void* b_packed) {
+  const int S = tb_gemm_splitk_split(M, N, K, flags);
+  if (S <= 0) return S;
+  const int num_m = (M + BM - 1) / BM, num_n = (N + BN - 1) / BN;
   CUtensorMap tmA, tmB;
   if (tb_make_tmap_2d_bf16(&tmA, A, M, K, lda, BM, BK, 1)) return -3;
   if (b_packed != nullptr) tmB = tmA;                  // unused by the kernel

@@ -3,15 +3,18 @@
 //   C[M,N] = epilogue( A[M,K] * B[N,K]^T ),  min(M, N) <= 64, each operand K-major or MN-major
 //
 // The long operand is the left one of the product: 128 of its rows are a tile's lanes in TMEM and the short side is its columns, so a tile
-// costs what the short side costs and the accumulator is as small as the result. The K range of a tile is split over the S CTAs of a
-// cluster:
+// costs what the short side costs and the accumulator is as small as the result. The K range of a tile is V partial products (partial p
+// sums k blocks [p KB / V, (p + 1) KB / V), and the partials are added in their order), spread over the S CTAs of a cluster:
 //
-//   * grid (S, tiles), cluster (S, 1, 1); CTA z owns k blocks [z KB / S, (z + 1) KB / S)
-//   * warp 0: TMA into a ring of 8 to 10 stages of 16 KB of the long operand and the k block of the short one; warp 1: one-thread
-//     tcgen05.mma
-//   * warps 2..5: the partial tile from TMEM straight into the shared memory of the CTAs that sum its columns (CTA o has the o-th
+//   * grid (S, tiles), cluster (S, 1, 1); CTA z owns partials [z V / S, (z + 1) V / S), each with an accumulator in TMEM
+//   * warp 0: TMA into a ring of 6 to 10 stages of 16 KB of the long operand and the k block of the short one; warp 1: one-thread tcgen05.mma
+//   * warps 2..5: the partial tiles from TMEM straight into the shared memory of the CTAs that sum their columns (CTA o has the o-th
 //     share of the padded columns): stores cross the cluster once and nobody waits for a remote load
 //   * one cluster barrier; each CTA sums its columns of all partial tiles and writes them
+//
+// V. Few rows by a K-major weight, the products of decode steps, have the partial products of gemm_splitk.cu, which took them before and takes
+// what is left out here: both give the same bits, whoever runs a step. For the others V is S; they were one sum over all of K, which the
+// tensor cores cut off at every step, so that V of them are nearer to 64 bits (64 x 4096 x 12288, fp32 out: 1.4e-5 -> below 1e-5).
 //
 // Bound by fixed costs (launch, first loads, the exchange) up to some 20 MB of the long operand and by HBM above.
 // Every wait is bounded; a timeout sets *status and falls through to the cluster barriers, which every thread reaches on every path.
@@ -24,13 +27,14 @@ namespace {
 constexpr int TILE = 128, BK = 64, UMMA_K = 16, MAX_STAGES = 10;
 constexpr int W_BYTES = TILE * BK * 2;
 constexpr int COLS = 16;                 // columns that a CTA sums at most
-constexpr int RING_BYTES = 8 * (W_BYTES + 64 * BK * 2);                // 192 KB: 8 stages of 64 rows, 9 of 32, 10 of 16
-constexpr int SMEM_BYTES = RING_BYTES + 64 * TILE * 4 + 256 + 1024;    // ring, partial sums, barriers
+constexpr int MAX_PARTS = 8, TMEM_COLS = 128;                          // accumulators of a CTA: V / S (rounded up) of P columns, see the choice of S
+constexpr int DATA_BYTES = 224 * 1024;   // ring (6 to 10 stages of 18 to 24 KB) and partial sums (up to 64 KB)
+constexpr int SMEM_BYTES = DATA_BYTES + 256 + 1024;
 
 enum { GF_A_MN = 1, GF_B_MN = 2, GF_OUT_F32 = 4, GF_ACCUM = 8, GF_BIAS = 16, GF_RESIDUAL = 32 };
 
 struct StreamArgs {
-  int rows, cols, K, flags, S, P, log_share, stages;    // rows: of the long operand; P: cols padded to 16, 32 or 64; log_share: of P / S / 4
+  int rows, cols, K, flags, S, V, P, log_share, stages;    // rows: of the long operand; P: cols padded to 16, 32 or 64; log_share: of P / S / 4
   int w_mn, x_mn;          // the long and the short operand are MN-major
   int tall;                // C is [rows, cols], else [cols, rows]
   int x_bytes;             // of a k block of the short operand
@@ -64,20 +68,22 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t part_base = smem_base + RING_BYTES, bar_base = part_base + 64 * TILE * 4;
-  const float4* const part = reinterpret_cast<const float4*>(smem_al + RING_BYTES);   // [S][128 rows][columns of a CTA]
+  const int stages = args.stages, stage_bytes = W_BYTES + args.x_bytes;
+  const uint32_t part_base = smem_base + stages * stage_bytes, bar_base = smem_base + DATA_BYTES;
+  const float4* const part = reinterpret_cast<const float4*>(smem_al + stages * stage_bytes);   // [V][128 rows][columns of a CTA]
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (MAX_STAGES + s); };
   const uint32_t tfull_bar = bar_base + 8u * (2 * MAX_STAGES);
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_al + RING_BYTES + 64 * TILE * 4 + 8 * (2 * MAX_STAGES + 1));
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_al + DATA_BYTES + 8 * (2 * MAX_STAGES + 1));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rows = args.rows, cols = args.cols, S = args.S, P = args.P, stages = args.stages;
+  const int rows = args.rows, cols = args.cols, S = args.S, V = args.V, P = args.P;
   const int z = blockIdx.x, n0 = blockIdx.y * TILE;                              // z: rank in the cluster
   const int num_kb = (args.K + BK - 1) / BK;
-  const int kb_begin = (int)((long long)z * num_kb / S), kb_end = (int)((long long)(z + 1) * num_kb / S);
-  const int stage_bytes = W_BYTES + args.x_bytes;
+  const int p_begin = z * V / S, here = (z + 1) * V / S - p_begin;                // this CTA's partial products: from k block kb_of(p) on
+  auto kb_of = [&](int p) { return (int)((long long)p * num_kb / V); };
+  const int kb_begin = kb_of(p_begin), kb_end = kb_of(p_begin + here);
   const int pieces = P / S / 4;                        // of four columns that a CTA sums (powers of two)
 
   pdl_trigger();
@@ -93,7 +99,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     prefetch_tensormap(&tmW);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32((const void*)tmem_slot), 64);
+    tmem_alloc(smem_u32((const void*)tmem_slot), TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -131,7 +137,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      int p = p_begin, kb_next = kb_of(p + 1);
+      uint32_t d = tmem, more = 0;                     // accumulator of partial p, and whether it holds something
       for (int kb = kb_begin; kb < kb_end; ++kb) {
+        if (kb == kb_next) {                           // (no partial product is empty)
+          kb_next = kb_of(++p + 1);
+          d += P;
+          more = 0;
+        }
         if (!mbar_wait_bounded(full_bar(stage), phase, abort_flag, args.status, ST_TIMEOUT_MMA)) {
           ok = false;
           break;
@@ -140,8 +153,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         const uint32_t sw = smem_base + stage * stage_bytes, sx = sw + W_BYTES;
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k)
-          umma_f16_ss(tmem, make_smem_desc(sw + k * w_step, w_lbo, 1024), make_smem_desc(sx + k * x_step, x_lbo, 1024), idesc,
-                      (kb > kb_begin || k > 0) ? 1u : 0u);
+          umma_f16_ss(d, make_smem_desc(sw + k * w_step, w_lbo, 1024), make_smem_desc(sx + k * x_step, x_lbo, 1024), idesc, more | (k > 0));
+        more = 1;
         umma_commit(empty_bar(stage));
         if (++stage == stages) { stage = 0; phase ^= 1; }
       }
@@ -166,20 +179,23 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     tc_fence_after();
     cluster_wait();                                    // the peers run
 #pragma unroll 1
-    for (int c = 0; c < cols; c += 16) {
-      uint32_t v[16];
-      if (ok) {
-        tmem_ld_32x16(tmem + ((uint32_t)(q * 32) << 16) + c, v);
-        tmem_ld_wait();
-      } else {
+    for (int p = 0; p < here; ++p) {
+#pragma unroll 1
+      for (int c = 0; c < cols; c += 16) {
+        uint32_t v[16];
+        if (ok) {
+          tmem_ld_32x16(tmem + ((uint32_t)(q * 32) << 16) + p * P + c, v);
+          tmem_ld_wait();
+        } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0u;
-      }
+          for (int i = 0; i < 16; ++i) v[i] = 0u;
+        }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int piece = c / 4 + i, o = piece >> args.log_share;                 // the CTA that sums these columns
-        const uint32_t to = part_base + (uint32_t)((z * TILE * pieces + piece_at(r, piece & (pieces - 1), pieces)) << 4);
-        if (piece * 4 < cols) st_cluster(map_to_cta(to, (uint32_t)o), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        for (int i = 0; i < 4; ++i) {
+          const int piece = c / 4 + i, o = piece >> args.log_share;                 // the CTA that sums these columns
+          const uint32_t to = part_base + (uint32_t)(((p_begin + p) * TILE * pieces + piece_at(r, piece & (pieces - 1), pieces)) << 4);
+          if (piece * 4 < cols) st_cluster(map_to_cta(to, (uint32_t)o), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
       }
     }
     tc_fence_before();
@@ -188,7 +204,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     auto sum = [&](int piece) {
       float o[4] = {0.f, 0.f, 0.f, 0.f};
       const float4* p = part + piece_at(r, piece, pieces);
-      for (int s = 0; s < S; ++s) {
+      for (int s = 0; s < V; ++s) {
         const float4 v = p[s * TILE * pieces];
         o[0] += v.x;
         o[1] += v.y;
@@ -229,7 +245,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 64);
+    tmem_dealloc(tmem, TMEM_COLS);
   }
 }
 
@@ -252,15 +268,23 @@ cudaLaunchConfig_t stream_config(int S, int tiles, cudaStream_t stream, cudaLaun
 
 }  // namespace
 
+int tb_gemm_splitk_split(int M, int N, int K, int flags);
+
 // Returns 1 when the problem was launched here, 0 when it is not one of this kernel's (the caller goes on), a negative code on error.
 // Same conventions as tb_gemm_bf16, whose caller has checked alignment and strides.
 int tb_gemm_stream_try(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int flags,
                        const void* bias, const void* resid, long long ldr, float alpha, int* status, cudaStream_t stream) {
-  if ((flags & ~(GF_A_MN | GF_B_MN | GF_OUT_F32 | GF_ACCUM | GF_BIAS | GF_RESIDUAL)) || K < 512) return 0;
+  if (flags & ~(GF_A_MN | GF_B_MN | GF_OUT_F32 | GF_ACCUM | GF_BIAS | GF_RESIDUAL)) return 0;
   const bool tall = M > N;
-  const int rows = tall ? M : N, cols = tall ? N : M;
-  if (cols > 64 || rows < TILE) return 0;
-  const int tiles = (rows + TILE - 1) / TILE, num_kb = (K + BK - 1) / BK;
+  const int rows = tall ? M : N, cols = tall ? N : M, num_kb = (K + BK - 1) / BK;
+  if (cols > 64 || rows < TILE || K < 512) return 0;
+  int parts = 0;                                       // 0: as many as CTAs
+  if (!tall && !(flags & (GF_A_MN | GF_B_MN))) {
+    parts = tb_gemm_splitk_split(M, N, K, flags);
+    if (parts < 0) return parts;
+    if (parts < 2 || parts > MAX_PARTS || alpha != 1.f) return 0;      // (a product by alpha may join the sum behind it in one rounding, or not)
+  }
+  const int tiles = (rows + TILE - 1) / TILE;
   static DeviceOnce once;
   static int clusters[9] = {0};                        // co-resident clusters per size, asked of the runtime once
   if (once.first()) {
@@ -277,18 +301,21 @@ int tb_gemm_stream_try(const void* A, const void* B, void* C, int M, int N, int 
       clusters[s] = n;
     }
   }
-  // One wave of clusters, each CTA with four k blocks or more and at most 16 columns to sum (a thread's results leave one by one; beyond
-  // that, and at short contractions, narrow tiles are faster). Of those splits the one with the shortest stream: a CTA draws up to about 60
-  // bytes a nanosecond, all together what HBM gives; every further CTA of a cluster adds to the exchange. us, other kernels -> here: 64 rows by
-  // 4096 x 4096 16.7 -> 13.5, 4096 x 12288 30.9 -> 24.8, 1536 x 8960 16.5 -> 12.2, 16 rows 13.2 -> 10.3, 25.9 -> 21.2, 14.4 -> 9.4; factors of
-  // rank 16 of 4004 tokens, [4004, 3584] by [16, 3584] 17.3 -> 7.3, [4004, 14336]^T by [4004, 16] 29.6 -> 26.0, by [14336, 16] 54.4 -> 23.5. Left out: 64
-  // rows by 6144 x 4096 (32 columns a CTA) 18.9 / 19.1, 8192 x 2048 13.4 / 16.2, 32 by 1024 x 512 6.0 / 6.5.
+  // One wave of clusters; of few rows each CTA with whole partial products, of the others with four k blocks or more; and at most 16
+  // columns to sum (a thread's results leave one by one; beyond that, and at short contractions, narrow tiles are faster). Of those sizes the
+  // one with the shortest stream: a CTA draws up to about 60 bytes a nanosecond, all together what HBM gives; every further CTA of a cluster
+  // adds to the exchange. us in a graph with cold weights, other kernels -> here: 64 rows by 4096 x 4096 16.1 -> 14.5, 4096 x 12288 30.1 -> 27.0,
+  // 1536 x 8960 16.5 -> 12.1, 3072 x 8192 18.5 -> 18.3; 16 rows 13.0 -> 11.2, 25.6 -> 22.4, 14.3 -> 9.4, 16.3 -> 13.3 (with V = S, and so other bits, 10.4,
+  // 21.1, 9.1, 12.9); factors of rank 16 of 4004 tokens, [4004, 3584] by [16, 3584] 17.3 -> 7.3, [4004, 14336]^T by [4004, 16] 29.6 -> 26.0, by [14336, 16]
+  // 54.4 -> 23.5. Left out: 64 rows by 6144 x 4096 and 8192 x 4096 (32 columns a CTA; 18.4 and 22.5 in the other kernels).
   int best = 0, pad = 0;
   double cost = 0.0;
   for (int s = 1; s <= 8; s *= 2) {
     const int p = cols <= 16 && s <= 4 ? 16 : cols <= 32 ? 32 : 64;       // four columns a CTA or more
-    if (clusters[s] < tiles || num_kb / s < 4 || p / s > 16 || (K < 768 && p > 16)) continue;
-    const double rate = 6400.0 / (tiles * s), t = ((num_kb + s - 1) / s) * (W_BYTES * 1e-3) / (rate < 60.0 ? rate : 60.0) + 0.25 * s;
+    if (clusters[s] < tiles || num_kb / s < 4 || p / s > COLS || (K < 768 && p > 16)) continue;
+    if (parts && (parts < s || (parts + s - 1) / s * p > TMEM_COLS)) continue;
+    const int most = parts ? (parts + s - 1) / s * ((num_kb + parts - 1) / parts) : (num_kb + s - 1) / s;       // k blocks of a CTA
+    const double rate = 6400.0 / (tiles * s), t = most * (W_BYTES * 1e-3) / (rate < 60.0 ? rate : 60.0) + 0.25 * s;
     if (best == 0 || t < cost) {
       best = s;
       pad = p;
@@ -297,14 +324,15 @@ int tb_gemm_stream_try(const void* A, const void* B, void* C, int M, int N, int 
   }
   if (best == 0) return 0;
   StreamArgs a;
-  a.rows = rows; a.cols = cols; a.K = K; a.flags = flags; a.S = best; a.C = C; a.ldc = ldc; a.tall = tall;
+  a.rows = rows; a.cols = cols; a.K = K; a.flags = flags; a.S = best; a.V = parts ? parts : best; a.C = C; a.ldc = ldc; a.tall = tall;
   a.w_mn = (flags & (tall ? GF_A_MN : GF_B_MN)) != 0;
   a.x_mn = (flags & (tall ? GF_B_MN : GF_A_MN)) != 0;
   a.P = pad;
   a.x_bytes = (a.x_mn ? 64 : a.P) * BK * 2;             // an MN-major block is 64 wide, zeros past its columns
   a.log_share = 0;
   while ((a.P / best / 4) >> (a.log_share + 1)) ++a.log_share;
-  a.stages = RING_BYTES / (W_BYTES + a.x_bytes);
+  a.stages = (DATA_BYTES - a.V * TILE * (pad / best) * 4) / (W_BYTES + a.x_bytes);
+  if (a.stages > MAX_STAGES) a.stages = MAX_STAGES;
   a.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   a.resid = reinterpret_cast<const __nv_bfloat16*>(resid);
   a.ldr = ldr; a.alpha = alpha; a.status = status;
