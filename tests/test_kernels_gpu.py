@@ -882,3 +882,76 @@ def test_head_over_the_rows_that_count(rows, V, D, share, chunk, softcap, want_e
         assert _rel_err(leaf.grad[on], hd.grad[on]) < 1e-2              # dz rounded to bf16 on the way
     assert bool((leaf.grad[~on] == 0).all()) and _rel_err(wl.main_grad, wd.grad + 1) < 1e-2 and wl.grad is None
     _check_status()
+
+
+@pytest.mark.parametrize("count", [0, 1, 64, 700, 2048, 2049, 2500, 4094])
+@pytest.mark.parametrize("off", [0, 2048])
+def test_products_that_end_at_a_number_on_the_device(count, off):
+    """`gemm_limited` at sizes that the kernel takes: rows (tiles past the limit stay as they are) and contractions that end inside a block
+    of 64, on its edge, before the chunk and past it, over operands that are NaN behind the zeros up to the block's end; a contraction of
+    nothing leaves what it would add to alone, the sign of its zeros too."""
+    k = _k()
+    M, N, K_ = 2046, 2560, 1536
+    n = max(0, min(M, count - off))
+    limit = torch.tensor([count], dtype=torch.int32, device="cuda")
+    a, b = _normal(M, K_, seed=1).bfloat16(), (0.1 * _normal(K_, N, seed=2)).bfloat16()
+    out = torch.full((M, N), -7.0, device="cuda", dtype=torch.bfloat16)
+    assert k.gemm_limited(a, b, out, limit, off, b_mn=True)
+    assert n == 0 or _rel_err(out[:n], a[:n].double() @ b.double()) < 2e-3
+    assert bool((out[-(-n // 256) * 256:] == -7.0).all())
+    x, y = _normal(M, N, seed=3).bfloat16(), (0.1 * _normal(M, K_, seed=4)).bfloat16()
+    x[n:] = y[n:] = 0
+    x[n + 63:] = y[n + 63:] = float("nan")
+    for dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 3e-3)):
+        for start in (-0.0, 1.0):
+            out = torch.full((N, K_), start, device="cuda", dtype=dtype)
+            assert k.gemm_limited(x, y, out, limit, off, a_mn=True, b_mn=True, accumulate=True, contraction=True)
+            if n:
+                assert _rel_err(out, x[:n].double().t() @ y[:n].double() + start) < tol
+            else:
+                assert bool((out == start).all()) and bool((out.signbit() == (start == 0)).all())
+    out = torch.full((N, K_), 5.0, device="cuda")
+    assert k.gemm_limited(x, y, out, limit, off, a_mn=True, b_mn=True, contraction=True)
+    assert _rel_err(out, x[:n].double().t() @ y[:n].double()) < 1e-5 if n else bool((out == 0).all())
+    _check_status()
+
+
+@pytest.mark.parametrize("count", [0, 1, 700, 2111, 4094])
+@pytest.mark.parametrize("held", [False, True])
+def test_head_over_the_rows_that_count_on_sm_pairs(count, held, monkeypatch):
+    """The head at sizes where every product runs on SM pairs, with a gradient kept in 32 bits or not: the second chunk empty, ending inside a
+    block, or full."""
+    from tunix_b200.ops import functional as F
+    rows, V, D = 4094, 8192, 3072
+    monkeypatch.setattr(F, "_SCORED_MIN", 0)
+    ran, real = [], F.K.gemm_limited
+    monkeypatch.setattr(F.K, "gemm_limited", lambda *a, **kw: (ran.append(real(*a, **kw)), ran[-1])[1])
+    g = torch.Generator(device="cuda").manual_seed(count)
+    h, w = torch.randn(rows, D, device="cuda", generator=g).bfloat16(), (0.05 * torch.randn(V, D, device="cuda", generator=g)).bfloat16()
+    tg = torch.randint(0, V, (rows,), device="cuda", generator=g)
+    on = torch.zeros(rows, dtype=torch.bool, device="cuda")
+    on[torch.randperm(rows, device="cuda", generator=g)[:count]] = True
+    tg[~on] = -1
+    bad = h.clone()
+    bad[~on] = float("nan")
+    leaf, wl = bad.requires_grad_(), w.clone().requires_grad_()
+    if held:
+        wl.main_grad = torch.ones(V, D, device="cuda")
+    logp, _ = F.lm_head_logprobs(leaf, wl, tg, chunk=2048, skip_ignored=True)
+    wa = torch.randn(rows, device="cuda", generator=g)
+    (logp * wa).sum().backward()
+    assert ran == [True] * 4
+    z = h[on].double() @ w.double().t()
+    lsm = torch.log_softmax(z, -1)
+    assert bool((logp[~on] == 0).all()) and bool((leaf.grad[~on] == 0).all())
+    dz = -lsm.exp()
+    dz[torch.arange(count, device="cuda"), tg[on]] += 1
+    dz *= wa[on].double()[:, None]
+    dw = dz.t() @ h[on].double()
+    got = wl.main_grad - 1 if held else wl.grad
+    if count:
+        assert _rel_err(logp[on], lsm.gather(1, tg[on][:, None])[:, 0]) < 1e-4
+        assert _rel_err(leaf.grad[on], dz @ w.double()) < 1e-2 and _rel_err(got, dw) < 1e-2          # dz rounded to bf16 on the way
+    else:
+        assert bool((got == 0).all())
+    _check_status()
