@@ -744,3 +744,52 @@ def test_decode_graph_kept_from_call_to_call():
     model.layers[0].self_attn.window = 4
     check(1, seed=5)
     _lib.raise_if_kernel_error()
+
+
+def test_kept_decode_graph_reads_refreshed_packed_weights():
+    """The graph of the last call steps packed buffers that a call refreshes in place: weights changed between two calls that share it, a call for
+    first tokens alone in between (which refreshes the head and nothing else), and one whose buffers are new."""
+    from tunix_b200 import _lib
+    from tunix_b200.common.configs import CacheConfig
+    from tunix_b200.generate.engine import PagedEngine
+    model = _model()
+
+    def make(packs=True):
+        eng = PagedEngine(model, Tok(), CacheConfig(128, 2, 2, 64), page_size=16, max_running_requests=3, prefix_caching=False, pack_weights=packs)
+        eng.pack_min_rows = 0
+        return eng
+    eng, captured = make(), []
+    capture = eng._capture_step
+    eng._capture_step = lambda st: captured.append(1) or capture(st)
+    rng = np.random.default_rng(4)
+    prompts = [[1] + rng.integers(3, 500, size=n).tolist() for n in (9, 30, 17)]
+
+    def run(e, steps):
+        return e(prompt_token_ids=prompts, max_generation_steps=steps, eos_tokens=[2], return_logprobs=True)
+
+    def check(captures, steps=24):
+        captured.clear()
+        a, b, plain = run(eng, steps), run(make(), steps), run(make(False), steps)
+        assert eng._packed_on and all(pw is not None for src in eng._packed for pw in src.values()) or steps == 1
+        assert all(np.array_equal(x, y) for x, y in zip(a.tokens, b.tokens)) and a.logprobs == b.logprobs
+        assert len(captured) == captures
+        for t, u, x, y in zip(a.tokens, plain.tokens, a.logprobs, plain.logprobs):
+            n = next((i for i, (p, q) in enumerate(zip(t, u)) if p != q), len(t))         # a near tie may part the two
+            assert n > 0 and np.allclose(x[:n], y[:n], atol=5e-2)
+        return a
+    first = check(1)
+    assert any(len(t) > 4 for t in first.tokens)
+    check(0)
+    for names in (("gate_proj", "up_proj"), ("q_proj", "o_proj"), ("down_proj",), ("lm_head", "embed_tokens")):
+        with torch.no_grad():
+            for name, p in model.named_parameters():
+                if any(n in name for n in names):
+                    p.mul_(-0.7)
+        if names == ("down_proj",):
+            check(0, steps=1)             # (a call of other numbers ends the kept graph)
+        changed = check(int(names == ("down_proj",)))
+        assert changed.logprobs != first.logprobs
+        first = changed
+    eng._packed = None
+    check(1)
+    _lib.raise_if_kernel_error()
