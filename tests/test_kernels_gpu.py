@@ -955,3 +955,17 @@ def test_head_over_the_rows_that_count_on_sm_pairs(count, held, monkeypatch):
     else:
         assert bool((got == 0).all())
     _check_status()
+
+
+@pytest.mark.parametrize("M,N,K_", [(256, 11264, 256), (256, 11008, 256), (255, 32768, 512), (2816, 1024, 248), (2816, 1024, 256), (1100, 2304, 4096)])
+def test_the_head_asks_the_kernels_own_rule(M, N, K_, monkeypatch):
+    """`two_sm_takes` says what a limited product of these sizes does, also where a switch has changed since the kernels read it."""
+    k = _k()
+    a, b, limit = _normal(M, K_, seed=1).bfloat16(), _normal(N, K_, seed=2).bfloat16(), torch.tensor([M], dtype=torch.int32, device="cuda")
+    out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    k.gemm(a, b)
+    for switch in (None, "TUNIX_B200_NO_2CTA"):
+        if switch:
+            monkeypatch.setenv(switch, "1")
+        assert k.two_sm_takes(M, N, K_) == k.gemm_limited(a, b, out, limit, 0)
+    _check_status()

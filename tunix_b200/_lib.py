@@ -30,6 +30,7 @@ _CUDA_SIGS = {
     "tb_gemm_bf16_ext": [P, P, P, I, I, I, LL, LL, LL, I, P, P, LL, F, P, P, I, LL, LL, P, P, I, LL, LL, P, P],
     "tb_gemm_glu": [P, P, P, P, I, I, I, LL, LL, LL, LL, P, P, LL, LL, I, P, P],
     "tb_gemm_limited": [P, P, P, I, I, I, LL, LL, LL, I, P, I, I, P, P],
+    "tb_two_sm_takes": [I, I, I],
     "tb_scored_gather": [P, LL, P, I, I, P, P, P, P, P],
     "tb_scored_scatter": [P, P, I, I, P, P],
     "tb_scored_numbers": [P, P, P, P, P, I, I, P],

@@ -700,18 +700,21 @@ int start_2cta(const Maps2& maps, const Args2& a, int tiles, cudaStream_t stream
   return cudaLaunchKernelEx(&cfg, gemm2_kernel, maps, a) == cudaSuccess ? 1 : -5;
 }
 
+// Worth it when the pairs have most of a wave of 256 x 256 tiles (tile_n columns) and the K loop amortises the prologue.
+bool takes_2cta(int M, int N, int K, int tile_n) {
+  static const bool off = getenv("TUNIX_B200_NO_2CTA") != nullptr;
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + tile_n - 1) / tile_n);
+  return !off && N >= tile_n && M >= 256 && K >= 256 && tiles >= (g_sms2 / 2 * 3) / 5;
+}
+
 int launch_2cta(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                 int flags, const void* bias, const void* resid, long long ldr, float alpha, int* status,
                 cudaStream_t stream, const LseArgs& lse, const Product& p2 = Product{}, const Product& p3 = Product{},
                 const GluArgs& glu = GluArgs{}, const Limit& limit = Limit{}) {
-  static const bool off = getenv("TUNIX_B200_NO_2CTA") != nullptr;
-  if (off) return 0;
   if (!setup_2cta()) return -5;
   const int tile_n = glu.up ? BN / 2 : BN;
   const int num_m = (M + BM - 1) / BM, num_n = (N + tile_n - 1) / tile_n;
-  const int pairs = g_sms2 / 2;
-  // worth it when the pairs have at least a wave of 256 x 256 tiles and the K loop amortises the prologue
-  if (N < tile_n || M < 256 || K < 256 || (long long)num_m * num_n < (pairs * 3) / 5) return 0;
+  if (!takes_2cta(M, N, K, tile_n)) return 0;
   const bool a_mn = flags & GF_A_MN, b_mn = flags & GF_B_MN;
   // (the up projection takes the place of a second product: both read all of A)
   const Product sum[SEGS] = {{A, B, K, lda, ldb}, glu.up ? Product{A, glu.up, K, lda, glu.ldup} : p2, p3};
@@ -890,6 +893,9 @@ TB_API int tb_lm_head_dlogits(const void* h, long long ldh, const void* w, long 
   return launch_2cta(h, w, out, M, V, K, ldh, ldw, ldo, 0, nullptr, nullptr, 0, 1.0f, status, stream, e, Product{}, Product{}, GluArgs{},
                      Limit{limit, limit_off, 0});
 }
+
+// Whether the kernel takes a product of these sizes in rows of whole 16-byte pieces: 1 or 0, or a negative code.
+TB_API int tb_two_sm_takes(int M, int N, int K) { return setup_2cta() ? takes_2cta(M, N, K, BN) : -5; }
 
 // tb_gemm_bf16 for the first *limit - limit_off rows of A alone (the other rows of C are left as they are), or with limit_k for that much of the
 // contraction (zeros up to the next multiple of 64 in one operand). Returns 1 when launched, 0 when the two-SM kernel does not take the

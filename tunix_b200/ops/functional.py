@@ -14,6 +14,7 @@ accumulates into it in its epilogue and autograd sees no gradient for that param
 from __future__ import annotations
 
 import contextlib
+import os
 
 import torch
 
@@ -705,8 +706,9 @@ def lm_head_logprobs(h, w, targets, *, softcap: float = 0.0, temperature: float 
         chunk = int(chunk) if chunk and chunk > 0 else 2048
         fn = _LmHeadLogprobFn
         # sizes that the two-SM kernel takes in every chunk of the backward
-        if skip_ignored and torch.is_grad_enabled() and h.requires_grad and targets.numel() * w.numel() >= max(_SCORED_MIN, 1) and \
-                w.shape[0] % 8 == 0 and w.is_contiguous() and _aligned16(w) and \
+        if skip_ignored and torch.is_grad_enabled() and h.requires_grad and targets.numel() and \
+                targets.numel() * w.numel() >= _SCORED_MIN and w.shape[0] % 8 == 0 and w.is_contiguous() and _aligned16(w) and \
+                not os.environ.get("TUNIX_B200_NO_FUSED_LSE") and \
                 K.two_sm_takes(min(e - s0 for s0, e in _head_chunks(targets.numel(), chunk)), w.shape[0], h.shape[-1]):
             fn = _LmHeadScoredFn
         return fn.apply(h, w, targets, float(softcap or 0.0), float(temperature), bool(want_entropy), chunk)

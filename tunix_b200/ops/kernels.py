@@ -940,11 +940,10 @@ def lm_head_lse(h2: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, *, sof
 # ------------------------------------------------------------------ rows of the head that count (csrc/scored_rows.cu)
 def two_sm_takes(M: int, N: int, K_: int) -> bool:
     """Whether the two-SM kernel takes a product of these sizes in rows of whole 16-byte pieces (a limit on M changes nothing)."""
-    import os
-    if os.environ.get("TUNIX_B200_NO_FUSED_LSE") or os.environ.get("TUNIX_B200_NO_2CTA"):
-        return False
-    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-    return min(M, N, K_) >= 256 and (M + 255) // 256 * ((N + 255) // 256) >= sms // 2 * 3 // 5
+    rc = _lib.cuda().tb_two_sm_takes(M, N, K_)
+    if rc < 0:
+        _lib.check(rc, "tb_two_sm_takes")
+    return rc == 1
 
 
 def scored_gather(h2: torch.Tensor, targets: torch.Tensor):
