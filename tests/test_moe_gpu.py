@@ -109,6 +109,32 @@ def test_experts_on_sm_pairs(T, E, k, D, Fd, acc):
         assert rel(w.grad, r.grad) < 1e-2 if acc is None else rel(w.main_grad, r.grad + 0.5) < 1e-2
 
 
+@pytest.mark.parametrize("T,E,k,D,Fd", [(1024, 8, 2, 256, 320), (1500, 4, 2, 1536, 256)])
+def test_experts_on_sm_pairs_without_gradients(T, E, k, D, Fd, monkeypatch):
+    """Nothing is kept for a backward that nobody asks for, and the result is the same bit for bit: no gradients, or none wanted of any input."""
+    from tunix_b200.ops import moe
+    kept, real = [], moe.K.gemm_grouped_glu
+
+    def spy(*a, **kw):
+        out = real(*a, **kw)
+        kept.append(out[1] is not None and out[2] is not None)
+        return out
+    monkeypatch.setattr(moe.K, "gemm_grouped_glu", spy)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *n: (0.1 * torch.randn(*n, device="cuda", generator=g)).bfloat16()  # noqa: E731
+    x, ws = 5 * rnd(T, D), [rnd(E, Fd, D), rnd(E, Fd, D), rnd(E, D, Fd)]
+    wts, idx = torch.topk(torch.softmax(torch.randn(T, E, device="cuda", generator=g), -1), k, -1)
+    plain = moe.experts(x, wts, idx, *ws)
+    grads = [w.clone().requires_grad_() for w in ws]
+    want = moe.experts(x, wts, idx, *grads)
+    with torch.no_grad():
+        again = moe.experts(x, wts, idx, *grads)
+    assert kept == [False, True, False] and torch.equal(plain, want) and torch.equal(again, want)
+    want.sum().backward()
+    assert all(w.grad is not None and bool(w.grad.isfinite().all()) for w in grads)
+
+
+
 def test_row_tiles_cover_every_segment_once():
     """The planned tiles of 128 and 256 rows against the segments, empty ones and an odd number of 128 rows among them."""
     import numpy as np

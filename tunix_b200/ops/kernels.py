@@ -611,7 +611,10 @@ def _grouped_bn(n: int) -> int:
     return 256 if n >= 256 else (128 if n >= 128 else 64)
 
 
-# Rows an expert from which grouped products run on SM pairs: a tile of 256 rows that is half empty costs what two of 128 do.
+# Rows an expert from which grouped products run on SM pairs: a tile of 256 rows that is half empty costs what two of 128 do. us of a layer,
+# tiles of 128 on one SM -> pairs, forward alone / with its backward, experts x rows, D x F: 64 x 256, 512 x 512 266 -> 245 / 718 -> 480, 2048 x 768 446 ->
+# 373 / 2286 -> 1204; 128 x 512, 512 x 512 417 -> 406 / 1367 -> 966, 2048 x 768 1006 -> 870 / 5158 -> 2989. Forward alone, narrow rows and segments that
+# end just past a tile lose a little (64 x 512, 256 x 256 212 -> 234, 512 x 512 271 -> 282), with the backward nothing does (439 -> 377, 799 -> 577).
 PAIR_ROWS = 256
 
 
@@ -689,11 +692,11 @@ def gemm_grouped_sum(a, b, a2, b2, out: torch.Tensor, n_limit: int, tiles: TileL
     return _grouped_pair(a, b, out, n_limit, tiles, b_mn=True, a2=a2, b2=b2)
 
 
-def gemm_grouped_glu(x, gate, up, tiles: TileList, kind: int):
-    """(act(g) * u, g, u) with g = x gate[e]^T, u = x up[e]^T over `tiles` (on SM pairs, gated); gate, up [E * F, D]."""
+def gemm_grouped_glu(x, gate, up, tiles: TileList, kind: int, keep: bool = True):
+    """(act(g) * u, g, u) with g = x gate[e]^T, u = x up[e]^T over `tiles` (on SM pairs, gated); gate, up [E * F, D]. g and u only with `keep`."""
     assert all(t.dtype == torch.bfloat16 and t.is_contiguous() for t in (x, gate, up)) and gate.shape == up.shape
     Fdim = tiles.n
-    h, g, u = (torch.empty((x.shape[0], Fdim), dtype=torch.bfloat16, device=x.device) for _ in range(3))
+    h, g, u = (torch.empty((x.shape[0], Fdim), dtype=torch.bfloat16, device=x.device) if want else None for want in (True, keep, keep))
     _grouped_pair(x, gate, h, Fdim, tiles, kind=kind, up=up, g=g, u=u)
     return h, g, u
 
