@@ -116,3 +116,34 @@ def test_gemma4_forward_backward_matches_reference(case):
 def test_smoke_entry():
     import __graft_entry__ as ge
     ge.smoke()
+
+
+@pytest.mark.parametrize("how", ["subclass", "instance"])
+def test_losses_call_a_replaced_token_logprobs_as_it_is_declared(how):
+    """A model whose `token_logprobs` has been replaced, by a method or function that knows nothing of rows to pass over, trains as it did: the
+    losses hand it every target and no further argument."""
+    from tunix_b200.models.config import ModelConfig
+    from tunix_b200.models.transformer import Transformer, create_model
+    from tunix_b200.rl.common import compute_per_token_logps
+    from tunix_b200.sft.peft_trainer import _default_loss_fn
+    cfg = ModelConfig(num_layers=2, vocab_size=2048, embed_dim=256, hidden_dim=768, num_heads=4, head_dim=64, num_kv_heads=2, max_position=512,
+                      dtype=torch.bfloat16)
+    model = create_model(cfg, device=torch.device("cuda"), seed=0)
+    seen = []
+
+    class Own(type(model)):
+        def token_logprobs(self, hidden, targets, *, temperature=1.0, want_entropy=False, chunk=None):
+            seen.append(int(targets.min()))
+            return Transformer.token_logprobs(self, hidden, targets, temperature=temperature, want_entropy=want_entropy, chunk=chunk)
+    toks = torch.randint(3, 200, (2, 40), device="cuda")
+    mask = torch.ones_like(toks)
+    mask[:, :11] = 0
+    want = _default_loss_fn(model, toks, mask)
+    if how == "subclass":
+        model.__class__ = Own
+    else:
+        model.token_logprobs = Own.token_logprobs.__get__(model)
+    got = _default_loss_fn(model, toks, mask)
+    assert float((got.loss.value() - want.loss.value()).detach().abs()) < 1e-4
+    lp = compute_per_token_logps(model, toks[:, :20], toks[:, 20:], 0, -1, completion_mask=mask[:, :20], stop_gradient=False, skip_masked=True)
+    assert lp.shape == (2, 20) and len(seen) == 2 and min(seen) >= 3

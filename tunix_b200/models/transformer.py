@@ -504,8 +504,6 @@ class Transformer(nn.Module):
     def compute_final_logits(self, hidden):
         return F.lm_head_logits(hidden, self.head_weight(), softcap=self.config.final_logit_softcap)
 
-    skips_ignored = True       # `token_logprobs` takes skip_ignored
-
     def token_logprobs(self, hidden, targets, *, temperature: float = 1.0, want_entropy: bool = False,
                        chunk: Optional[int] = None, skip_ignored: bool = False):
         """log p(targets) from final hidden states without materialising [tokens, vocab] logits. `skip_ignored`: see
@@ -513,6 +511,8 @@ class Transformer(nn.Module):
         return F.lm_head_logprobs(hidden, self.head_weight(), targets, softcap=self.config.final_logit_softcap,
                                   temperature=temperature, want_entropy=want_entropy,
                                   chunk=chunk or self.config.logprob_chunk, skip_ignored=skip_ignored)
+
+    token_logprobs.skips_ignored = True       # of the method: one that takes its place need not take skip_ignored
 
     def routed_experts_of_last_forward(self):
         """[B, T, num_layers, top_k] expert ids the MoE layers chose in the last forward (None for dense models)."""

@@ -131,7 +131,7 @@ def compute_per_token_logps(model, prompt_tokens, completion_tokens, pad_id, eos
             # packed rows have no prompt side: token t is predicted from position t - 1, and nothing predicts the
             # first token of a row (it is a prompt token, masked out of every loss)
             h = torch.cat([torch.zeros_like(hidden[:, :1]), hidden[:, :-1]], dim=1)
-        if skip_masked and completion_mask is not None and getattr(model, "skips_ignored", False) and h.is_cuda and \
+        if skip_masked and completion_mask is not None and getattr(model.token_logprobs, "skips_ignored", False) and h.is_cuda and \
                 completion_mask.shape == completion_tokens.shape:
             return model.token_logprobs(h, completion_tokens.masked_fill(completion_mask == 0, -1), temperature=temperature or 1.0,
                                         want_entropy=return_entropy, chunk=chunk_size or None, skip_ignored=True)

@@ -87,7 +87,7 @@ def _default_loss_fn(model, input_tokens, input_mask, positions=None, attention_
     else:
         targets = local_batch(model, input_tokens)[:, 1:]
         mask = local_batch(model, input_mask)[:, 1:].to(torch.float32)
-        if getattr(model, "skips_ignored", False) and hidden.is_cuda:       # tokens that weigh nothing need no log-prob
+        if getattr(model.token_logprobs, "skips_ignored", False) and hidden.is_cuda:       # tokens that weigh nothing need no log-prob
             logp, _ = model.token_logprobs(hidden[:, :-1], targets.masked_fill(mask == 0, -1), skip_ignored=True)
         else:
             logp, _ = model.token_logprobs(hidden[:, :-1], targets)
