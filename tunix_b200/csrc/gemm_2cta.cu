@@ -417,24 +417,32 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
 #pragma unroll 1
         for (int c = 0; c < BN / 2; c += 64) {
           if (n0 + c >= N) break;
-#pragma unroll 1
-          for (int o = args.glu_keep ? 2 : 0; o >= 0; --o) {
-            uint8_t* const to = acquire();
+          // gate and up as they are kept, rounded in pairs: the activation is that of the rows that a backward reads, and of the separate kernels
+          uint32_t g[32], u[32];
+          auto columns = [&](int col, uint32_t (&to)[32]) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
               float v[32];
-              get(c + half * 32 + (o == 2 ? BN / 2 : 0), v);
-              if (o == 0) {
-                float u[32];
-                get(BN / 2 + c + half * 32, u);
-                // of gate and up as they are kept: the activation of the rows that a backward reads, and of the separate kernels
+              get(col + half * 32, v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = act_fwd(round_bf16(v[i]), args.glu_kind) * round_bf16(u[i]);
-              }
-              put(to, half, v);
+              for (int i = 0; i < 16; ++i) to[half * 16 + i] = pack_bf16(v[2 * i], v[2 * i + 1]);
             }
+          };
+          auto leave = [&](int o, const uint32_t (&v)[32]) {
+            uint8_t* const to = acquire();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              *reinterpret_cast<uint4*>(to + ((i ^ (lane & 7)) << 4)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
             release(&maps.c[o], n0 + c, false);
-          }
+          };
+          columns(BN / 2 + c, u);
+          if (args.glu_keep) leave(2, u);
+          columns(c, g);
+          if (args.glu_keep) leave(1, g);
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            g[i] = pack_bf16(act_fwd(bf16_lo(g[i]), args.glu_kind) * bf16_lo(u[i]), act_fwd(bf16_hi(g[i]), args.glu_kind) * bf16_hi(u[i]));
+          leave(0, g);
         }
       } else {
         // 32 columns of the row, up to what is stored
@@ -495,7 +503,8 @@ gemm2_kernel(const __grid_constant__ Maps2 maps, const Args2 args) {
         };
         if (args.tma_c) {
           // Blocks of 32 rows and 128 bytes leave through shared memory and TMA, two in flight a warp: whole lines, and no thread waits for C
-          // or its address. bf16 results by a lane a row and fp32 sums by rows of lanes before (us): see launch_2cta.
+          // or its address. us in a loop, bf16 results by a lane a row -> here: 4096^3 110 -> 107, 8192 x 1024 x 4096 with B MN-major 65 -> 58, added to
+          // bf16 4096^3 118 -> 113, 4096 x 14336 x 4096 385 -> 364; added to fp32, by rows of lanes before, 404 -> 389.
 #pragma unroll 1
           for (int c = 0; c < BN; c += out_f32 ? 32 : 64) {
             const int col0 = n0 + c;
@@ -846,9 +855,10 @@ TB_API int tb_gemm_grouped_pair(const void* A, long long a_rows, long long a_col
 // h [M, F] = act(x Wg^T) * (x Wu^T), both products and the activation in one launch; gate and up projections [M, F] are written too where
 // g and u are given. x [M, K], Wg and Wu [F, K], bf16; F % 8 == 0. Returns 1 when launched, 0 when the call is left to separate kernels
 // (too small, or rows that are not whole 16-byte pieces), negative on error.
-// A loop under the power cap, us, two products and the activation by itself -> here, gate and up kept / not kept: 4096 x 14336 x 4096 742 -> 691 / 668,
-// 16384 x 12288 x 4096 2503 -> 2326 / 2230, 2048 x 8960 x 1536 115 -> 106 / 94, 512 x 8192 x 3072 61 -> 52 / 50. Below K = 1536 three results of a
-// tile take longer than its products: 2331 x 4864 x 896 59 -> 63 / 53. The activation's gradient in the epilogue of dy Wd was slower
+// us, two products and the activation by itself -> here, gate and up kept / not kept: 4096 x 14336 x 4096 677 -> 635 / 608, 16384 x 12288 x 4096 2260 ->
+// 2180 / 2050, 2048 x 8960 x 1536 103 -> 93 / 88, 512 x 8192 x 3072 60 -> 48 / 47. Gate and up are read from the accumulator once, as pairs of bf16
+// (a rounding at a time, each read twice: 2048 x 8960 x 1536 in a loop 156, against 138 by themselves). Below K = 1536 three results of a tile took
+// longer than its products: 2331 x 4864 x 896 59 -> 63 / 53. The activation's gradient in the epilogue of dy Wd was slower
 // everywhere (4096 x 14336 x 4096 442 -> 519): its rows of gate and up arrive by a lane a row.
 TB_API int tb_gemm_glu(const void* x, const void* wg, const void* wu, void* h, int M, int F, int K, long long ldx, long long ldwg,
                        long long ldwu, long long ldh, void* g, void* u, long long ldg, long long ldu, int kind, int* status,
