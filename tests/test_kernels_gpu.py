@@ -969,3 +969,15 @@ def test_the_head_asks_the_kernels_own_rule(M, N, K_, monkeypatch):
             monkeypatch.setenv(switch, "1")
         assert k.two_sm_takes(M, N, K_) == k.gemm_limited(a, b, out, limit, 0)
     _check_status()
+
+
+@pytest.mark.parametrize("M,F_,D", [(300, 2816, 8192), (512, 3072, 9000), (300, 2816, 4096), (513, 2816, 8192)])
+def test_gated_products_sum_like_separate_products(M, F_, D):
+    """Gate and up bit for bit those of the two products, also where these are sums of several parts (which the joint launch leaves to them)."""
+    k = _k()
+    x, wg, wu = _normal(M, D, seed=1).bfloat16(), (0.05 * _normal(F_, D, seed=2)).bfloat16(), (0.05 * _normal(F_, D, seed=3)).bfloat16()
+    out = k.gemm_glu(x, wg, wu, k.GLU_SILU, keep=True)
+    assert (out is None) == (M <= 512 and D >= 8192)
+    if out is not None:
+        assert torch.equal(out[1], k.gemm(x, wg)) and torch.equal(out[2], k.gemm(x, wu))
+    _check_status()

@@ -852,6 +852,8 @@ TB_API int tb_gemm_grouped_pair(const void* A, long long a_rows, long long a_col
   return rc == 1 ? 0 : rc;
 }
 
+int tb_gemm_splitk_split(int M, int N, int K, int flags);   // gemm_splitk.cu
+
 // h [M, F] = act(x Wg^T) * (x Wu^T), both products and the activation in one launch; gate and up projections [M, F] are written too where
 // g and u are given. x [M, K], Wg and Wu [F, K], bf16; F % 8 == 0. Returns 1 when launched, 0 when the call is left to separate kernels
 // (too small, or rows that are not whole 16-byte pieces), negative on error.
@@ -864,6 +866,8 @@ TB_API int tb_gemm_glu(const void* x, const void* wg, const void* wu, void* h, i
                        long long ldwu, long long ldh, void* g, void* u, long long ldg, long long ldu, int kind, int* status,
                        cudaStream_t stream) {
   if (M <= 0 || F <= 0 || K < 1536 || F % 8) return 0;
+  const int split = tb_gemm_splitk_split(M, F, K, 0);   // a few hundred rows by narrow layers of 8192 and more: sums in parts, which are nearer to
+  if (split != 0) return split < 0 ? split : 0;         // 64 bits than one, stay with the kernel that makes them
   GluArgs a;
   a.kind = kind; a.up = wu; a.ldup = ldwu; a.g = g; a.u = u; a.ldg = ldg; a.ldu = ldu;
   return launch_2cta(x, wg, h, M, F, K, ldx, ldwg, ldh, 0, nullptr, nullptr, 0, 1.f, status, stream, LseArgs{}, Product{}, Product{}, a);
