@@ -6,8 +6,8 @@
 // place through a view cost autograd four more copies of its gradient.
 // (reference: per-head norms tunix/models/qwen3/model.py, rotation tunix/models/llama3/model.py:249-270)
 //
-// B200, us, four launches -> one: 16384 tokens of 32 / 8 heads of 128 146 -> 79, backward 222 -> 95; 4096 tokens 45 -> 23 and 73 -> 32; 2331 of 14 / 2
-// heads of 64 42 -> 22 and 52 -> 26; without norms (two launches) 61 -> 56, 18 -> 13, 13 -> 10.
+// B200, us in a graph, four launches -> one: 16384 tokens of 32 / 8 heads of 128 126 -> 83, backward 207 -> 88; 4096 tokens 36 -> 19 and 61 -> 27; 2331 of
+// 14 / 2 heads of 64 10.4 -> 4.7 and 13.6 -> 6.4; without norms (two launches) 55 -> 53, 11.1 -> 9.5, 4.4 -> 3.3.
 // Bound by HBM: every row read and written once (the backward reads two). A thread holds 8 pairs (x[j], x[j + H / 2]) of QK_HEADS
 // heads of one token, which share the angles; H / 16 lanes make a row.
 #include "common.cuh"
